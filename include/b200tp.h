@@ -181,6 +181,30 @@ int b200tp_linear_ce_bwd_train(const b200tp_ce_args* a, const float* lse, const 
                                int32_t d_hidden_dtype, int32_t accumulate, void* d_weight, void* workspace,
                                size_t workspace_bytes, void* stream, int* status);
 
+/* Forward of a FROZEN head that also forms the gradient of the hidden states, for callers that will ask for
+ * it: two contractions over N x V x D where b200tp_linear_ce_fwd + b200tp_linear_ce_bwd take three (the
+ * logits are not computed again).  Per row the gradient of the loss is
+ *   exp(ref - lse) * sum_{v != t} exp(z_v - ref) W_v  +  (p_t - 1) W_t
+ * for any reference `ref`; with ref = the target's logit the sum is formed chunk by chunk beside the row sums,
+ * its exponentials rounded to bf16 before the second contraction like g in b200tp_linear_ce_bwd, the target's
+ * term in fp32.  Rows whose logits exceed the target's by 69 would overflow: the call then sets a flag in
+ * `state` and b200tp_linear_ce_bwd_grad recomputes as b200tp_linear_ce_bwd does (lse / nll / tgt_logit are
+ * right in any case, and every decision is taken on the device).
+ *   state : b200tp_linear_ce_grad_state_bytes, 256-byte aligned, kept by the caller until the backward
+ *           (fp32 sums of d_hidden, the references and the flag)
+ * bf16 hidden, D % 8 == 0, the whole vocabulary (v_offset = 0); the *_bytes functions return 0 where the call
+ * would be refused.  b200tp_linear_ce_bwd_grad may be called more than once on one state. */
+size_t b200tp_linear_ce_grad_state_bytes(const b200tp_ce_args* a);
+size_t b200tp_linear_ce_fwd_grad_workspace_bytes(const b200tp_ce_args* a);
+int b200tp_linear_ce_fwd_grad(const b200tp_ce_args* a, float* tgt_logit, float* lse, float* nll, void* state,
+                              size_t state_bytes, void* workspace, size_t workspace_bytes, void* stream,
+                              int* status);
+/* d_hidden (N, D) bf16 = cotangent * that gradient (0 on ignored rows). */
+size_t b200tp_linear_ce_bwd_grad_workspace_bytes(const b200tp_ce_args* a);
+int b200tp_linear_ce_bwd_grad(const b200tp_ce_args* a, const float* lse, const float* tgt_logit, const float* cotangent,
+                              void* state, size_t state_bytes, void* d_hidden, void* workspace, size_t workspace_bytes,
+                              void* stream, int* status);
+
 /* Dequantise rows [row0, row0 + rows) of a 4-bit affine head into `out` (rows, D) bf16/f32:
  * w = scale * code + bias in fp32, rounded once; `out` 16-byte aligned.  core/kernel/source.py:193-208. */
 int b200tp_dequant_int4(const uint32_t* w_q, const void* scales, const void* biases, int32_t qparam_dtype,

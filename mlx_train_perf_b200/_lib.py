@@ -82,6 +82,14 @@ SIGNATURES = {
     "b200tp_linear_ce_bwd_train": (C.c_int, [C.POINTER(CeArgs), C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32,
                                              C.c_int32, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p,
                                              C.c_void_p]),
+    "b200tp_linear_ce_grad_state_bytes": (C.c_size_t, [C.POINTER(CeArgs)]),
+    "b200tp_linear_ce_fwd_grad_workspace_bytes": (C.c_size_t, [C.POINTER(CeArgs)]),
+    "b200tp_linear_ce_fwd_grad": (C.c_int, [C.POINTER(CeArgs), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                            C.c_size_t, C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]),
+    "b200tp_linear_ce_bwd_grad_workspace_bytes": (C.c_size_t, [C.POINTER(CeArgs)]),
+    "b200tp_linear_ce_bwd_grad": (C.c_int, [C.POINTER(CeArgs), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                            C.c_size_t, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p,
+                                            C.c_void_p]),
     "b200tp_selftest_bounded_wait": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
     "b200tp_qk_norm_rope_fwd": (C.c_int, [C.POINTER(PrestepArgs), C.c_void_p, C.c_void_p, C.c_void_p]),
     "b200tp_qk_norm_rope_bwd_workspace_bytes": (C.c_size_t, [C.POINTER(PrestepArgs)]),

@@ -24,6 +24,7 @@ SOURCES = [
     "common.cu",
     "linear_ce_tc.cu",
     "linear_ce_simt.cu",
+    "linear_ce_grad.cu",
     "capi_ce.cu",
     "linear_ce_static.cu",
     "flash_simt.cu",

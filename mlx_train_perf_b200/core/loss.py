@@ -338,13 +338,69 @@ def ce_backward_raw(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, 
     return out
 
 
+def _forms_grad(impl: str, hidden_wants_grad: bool) -> bool:
+    """Whether the forward of a frozen head also forms the gradient of the hidden states (two contractions over
+    N x V x D in all, where a backward that computes the logits again makes it three): on the tensor-core path,
+    when autograd may ask for that gradient.  A forward whose gradient is never wanted is best run under
+    `torch.no_grad()`, where it stays at one contraction."""
+    return hidden_wants_grad and impl in ("tc", "tc_chunked")
+
+
+def ce_forward_grad(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, *,
+                    ignore_index: int = IGNORE_INDEX, impl: str = "tc"):
+    """((3, N) fp32 rows tgt_logit, lse, nll; state): the forward that also forms the gradient.  `state` is what
+    `ce_backward_grad` needs: fp32 sums of d_hidden and a few words per row."""
+    lib = _lib.load()
+    dev = hidden.device
+    n = hidden.shape[0]
+    a, keep = _ce_args(hidden, head, targets, v_offset=0, ignore_index=ignore_index, impl=impl)
+    out = torch.empty((3, n), dtype=torch.float32, device=dev)
+    sbytes = lib.b200tp_linear_ce_grad_state_bytes(C.byref(a))
+    nbytes = lib.b200tp_linear_ce_fwd_grad_workspace_bytes(C.byref(a))
+    state, ws = _workspace(sbytes, dev), _workspace(nbytes, dev)
+    base = out.data_ptr()
+    with torch.cuda.device(dev):
+        rc = lib.b200tp_linear_ce_fwd_grad(C.byref(a), base, base + 4 * n, base + 8 * n, _ptr(state), sbytes,
+                                           _ptr(ws), nbytes, _stream(dev), device_status(dev).data_ptr())
+    _lib.check(rc)
+    del keep
+    return out, state
+
+
+def ce_backward_grad(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, out: torch.Tensor,
+                     state: torch.Tensor, cotangent: torch.Tensor, *, ignore_index: int = IGNORE_INDEX,
+                     impl: str = "tc") -> torch.Tensor:
+    """d_hidden (N, D) from what `ce_forward_grad` returned and the upstream gradient of the per-row losses."""
+    lib = _lib.load()
+    dev = hidden.device
+    n = hidden.shape[0]
+    a, keep = _ce_args(hidden, head, targets, v_offset=0, ignore_index=ignore_index, impl=impl)
+    d_hidden = torch.empty_like(hidden)
+    ct = cotangent.to(torch.float32).contiguous()
+    nbytes = lib.b200tp_linear_ce_bwd_grad_workspace_bytes(C.byref(a))
+    ws = _workspace(nbytes, dev)
+    base = out.data_ptr()
+    with torch.cuda.device(dev):
+        rc = lib.b200tp_linear_ce_bwd_grad(C.byref(a), base + 4 * n, base, ct.data_ptr(), state.data_ptr(),
+                                           state.numel(), d_hidden.data_ptr(), _ptr(ws), nbytes, _stream(dev),
+                                           device_status(dev).data_ptr())
+    _lib.check(rc)
+    del keep
+    return d_hidden
+
+
 class _FusedLinearCE(torch.autograd.Function):
     """(hidden, targets) -> (nll, lse, tgt); the head is a constant (frozen)."""
 
     @staticmethod
     def forward(ctx, hidden, targets, head, ignore_index, impl):
-        _, _, tgt, lse, nll = ce_forward_raw(hidden, head, targets, ignore_index=ignore_index, impl=impl)
-        ctx.save_for_backward(hidden, targets, lse)
+        if _forms_grad(impl, ctx.needs_input_grad[0]):
+            out, state = ce_forward_grad(hidden, head, targets, ignore_index=ignore_index, impl=impl)
+            tgt, lse, nll = out[0], out[1], out[2]
+            ctx.save_for_backward(hidden, targets, out, state)
+        else:
+            _, _, tgt, lse, nll = ce_forward_raw(hidden, head, targets, ignore_index=ignore_index, impl=impl)
+            ctx.save_for_backward(hidden, targets, lse)
         ctx.head = head
         ctx.ignore_index = ignore_index
         ctx.impl = impl
@@ -355,9 +411,15 @@ class _FusedLinearCE(torch.autograd.Function):
     def backward(ctx, g_nll, _g_lse, _g_tgt):
         key = "quantized" if isinstance(ctx.head, QuantizedHead) else "dense"
         VJP_CALLS[key] = VJP_CALLS.get(key, 0) + 1
-        hidden, targets, lse = ctx.saved_tensors
-        d_hidden = ce_backward_raw(hidden, ctx.head, targets, lse, g_nll, ignore_index=ctx.ignore_index,
-                                   impl=ctx.impl)
+        saved = ctx.saved_tensors
+        if len(saved) == 4:
+            hidden, targets, out, state = saved
+            d_hidden = ce_backward_grad(hidden, ctx.head, targets, out, state, g_nll, ignore_index=ctx.ignore_index,
+                                        impl=ctx.impl)
+        else:
+            hidden, targets, lse = saved
+            d_hidden = ce_backward_raw(hidden, ctx.head, targets, lse, g_nll, ignore_index=ctx.ignore_index,
+                                       impl=ctx.impl)
         return d_hidden, None, None, None, None
 
 
@@ -406,7 +468,13 @@ class _FusedLinearCEReduced(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, weight, targets, head, ignore_index, impl, mean):
         use = DenseHead(weight=weight) if weight is not None else head
-        _, _, _, lse, nll = ce_forward_raw(hidden, use, targets, ignore_index=ignore_index, impl=impl)
+        if weight is None and _forms_grad(impl, ctx.needs_input_grad[0]):
+            rows, state = ce_forward_grad(hidden, use, targets, ignore_index=ignore_index, impl=impl)
+            nll, saved = rows[2], [rows, state]
+        else:
+            _, _, _, lse, nll = ce_forward_raw(hidden, use, targets, ignore_index=ignore_index, impl=impl)
+            saved = [lse] + ([weight] if weight is not None else [])
+        ctx.trains_weight, ctx.has_grad = weight is not None, weight is None and len(saved) == 2
         lib = _lib.load()
         dev = hidden.device
         out3 = torch.empty(3, dtype=torch.float32, device=dev)
@@ -414,8 +482,7 @@ class _FusedLinearCEReduced(torch.autograd.Function):
             rc = lib.b200tp_linear_ce_reduce(nll.data_ptr(), targets.data_ptr(), hidden.shape[0], ignore_index,
                                              out3.data_ptr(), _stream(dev))
         _lib.check(rc)
-        saved = [hidden, targets, lse, out3] + ([weight] if weight is not None else [])
-        ctx.save_for_backward(*saved)
+        ctx.save_for_backward(hidden, targets, out3, *saved)
         ctx.head, ctx.ignore_index, ctx.impl, ctx.mean = head, ignore_index, impl, mean
         loss, count = out3[1 if mean else 0], out3[2]
         ctx.mark_non_differentiable(count)
@@ -424,8 +491,8 @@ class _FusedLinearCEReduced(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_loss, _g_count):
         saved = ctx.saved_tensors
-        hidden, targets, lse, out3 = saved[:4]
-        weight = saved[4] if len(saved) == 5 else None
+        hidden, targets, out3, rows = saved[:4]      # rows: lse, or the three rows of `ce_forward_grad`
+        weight = saved[4] if ctx.trains_weight else None
         head = DenseHead(weight=weight) if weight is not None else ctx.head
         key = "dense_trainable" if weight is not None else ("quantized" if isinstance(head, QuantizedHead) else "dense")
         VJP_CALLS[key] = VJP_CALLS.get(key, 0) + 1
@@ -438,10 +505,14 @@ class _FusedLinearCEReduced(torch.autograd.Function):
             rc = lib.b200tp_linear_ce_cotangent(targets.data_ptr(), n, ctx.ignore_index, g.data_ptr(),
                                                 out3[2:].data_ptr() if ctx.mean else None, ct.data_ptr(), _stream(dev))
         _lib.check(rc)
+        if ctx.has_grad:
+            d_hidden = ce_backward_grad(hidden, head, targets, rows, saved[4], ct, ignore_index=ctx.ignore_index,
+                                        impl=ctx.impl)
+            return d_hidden, None, None, None, None, None, None
         d_w = None
         if weight is not None and ctx.needs_input_grad[1]:
             d_w = torch.empty_like(weight, memory_format=torch.contiguous_format)
-        d_hidden = ce_backward_raw(hidden, head, targets, lse, ct, ignore_index=ctx.ignore_index, impl=ctx.impl,
+        d_hidden = ce_backward_raw(hidden, head, targets, rows, ct, ignore_index=ctx.ignore_index, impl=ctx.impl,
                                    d_weight=d_w)
         return d_hidden, d_w, None, None, None, None, None
 

@@ -3,6 +3,7 @@
 #include <string>
 
 #include "common.h"
+#include "linear_ce_grad.h"
 #include "linear_ce_simt.h"
 #include "linear_ce_tc.h"
 
@@ -108,15 +109,17 @@ bool quant_inline(const b200tp_ce_args* a, bool backward) {
   return !backward && a->n <= kInlineMaxRows;
 }
 
-QuantHead quant_head(const b200tp_ce_args* a, bool backward) {
+QuantHead packed_head(const b200tp_ce_args* a) {
   QuantHead q{};
-  if (quant_inline(a, backward)) {
-    q.wq = a->w_q;
-    q.scales = a->scales;
-    q.biases = a->biases;
-    q.qp_f32 = a->qparam_dtype == B200TP_F32 ? 1 : 0;
-  }
+  q.wq = a->w_q;
+  q.scales = a->scales;
+  q.biases = a->biases;
+  q.qp_f32 = a->qparam_dtype == B200TP_F32 ? 1 : 0;
   return q;
+}
+
+QuantHead quant_head(const b200tp_ce_args* a, bool backward) {
+  return quant_inline(a, backward) ? packed_head(a) : QuantHead{};
 }
 
 // 1 = tcgen05, 2 = SIMT, negative = refusal already recorded
@@ -217,6 +220,59 @@ BwdPlan plan_bwd(const b200tp_ce_args* a, int out_dtype, void* ws) {
   }
   p.bytes = align_up(b.off, 256);
   return p;
+}
+
+// Forward that also forms the gradient: what it leaves for the backward (`state`) and its scratch.  The chunks
+// are the recomputing backward's, so the scratch is that backward's: one (N, chunk) bf16 tile, one dequantised
+// chunk of a 4-bit head, plus the forward's partial triples.
+struct GradPlan {
+  bool ok;
+  int64_t chunk, num_chunks;
+  int shares;            // partial sums of d_hidden (see ce_tc_dh_ksplit)
+  int64_t total_splits;
+  // state
+  int* overflow;
+  float* ref2;           // (n)
+  float* acc;            // (shares, n, d)
+  size_t state_bytes;
+  // scratch
+  void* g;
+  void* deq;
+  float* pm; float* ps; float* pt;
+  size_t bytes;          // forward
+  size_t bwd_bytes;      // backward: g and deq alone, for calls whose overflow flag is set
+};
+
+GradPlan plan_grad(const b200tp_ce_args* a, void* state, void* ws) {
+  GradPlan p{};
+  p.ok = pick_impl(a) == 1 && a->impl != B200TP_IMPL_SIMT && (a->reserved & kReservedInline) == 0;
+  if (!p.ok) return p;
+  p.chunk = tc_chunk_rows(a, &p.num_chunks);
+  p.shares = ce_tc_dh_ksplit(a->n, a->d, static_cast<int>(p.chunk));
+  Bump st(state);
+  p.overflow = st.take<int>(1);
+  p.ref2 = st.take<float>(a->n);
+  p.acc = st.take<float>(static_cast<size_t>(p.shares) * a->n * a->d);
+  p.state_bytes = align_up(st.off, 256);
+  Bump b(ws);
+  p.g = b.take<char>(static_cast<size_t>(a->n) * p.chunk * 2);
+  if (a->quant_bits != 0) p.deq = b.take<char>(static_cast<size_t>(p.chunk) * a->d * 2);
+  p.bwd_bytes = align_up(b.off, 256);
+  for (int64_t c = 0; c < p.num_chunks; ++c)
+    p.total_splits += ce_tc_fwd_splits(a->n, std::min<int64_t>(p.chunk, a->v_local - c * p.chunk));
+  p.pm = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
+  p.ps = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
+  p.pt = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
+  p.bytes = align_up(b.off, 256);
+  return p;
+}
+
+int check_grad_args(const b200tp_ce_args* a) {
+  int rc = check_args(a);
+  if (rc) return rc;
+  if (a->v_offset != 0)
+    return fail(B200TP_ERR_LOSS_INPUT, "the forward with gradient needs the whole vocabulary (v_offset = 0)");
+  return B200TP_OK;
 }
 
 int check_workspace(void* ws, size_t have, size_t need) {
@@ -395,7 +451,7 @@ static int bwd_impl(const b200tp_ce_args* a, const float* lse, const float* cota
       }
       if (stage == 0) {
         rc = ce_tc_launch_bwd_g(a->hidden, wmat, wrows, a->n, a->d, row0, row0 + w, vocab_id0, a->targets,
-                                a->ignore_index, lse, cotangent, p.g, p.ldg, qp, stream, status);
+                                a->ignore_index, lse, cotangent, p.g, p.ldg, qp, LaunchGuard{}, stream, status);
         if (rc) return rc;
       }
       const int k_total = static_cast<int>(align_up(w, kCeTileCols));
@@ -412,7 +468,7 @@ static int bwd_impl(const b200tp_ce_args* a, const float* lse, const float* cota
         out_bf16 = last ? d_hidden : nullptr;
       }
       rc = ce_tc_launch_dh(p.g, p.ldg, k_total, a->n, wmat, wrows, a->d, row0, acc_in, acc_out, out_bf16,
-                           last ? tile0 : -1, last ? tile1 : -1, qp, stream, status);
+                           last ? tile0 : -1, last ? tile1 : -1, 1, qp, LaunchGuard{}, stream, status);
       if (rc) return rc;
       if (d_weight != nullptr) {
         void* block = static_cast<char*>(d_weight) + static_cast<size_t>(r0) * a->d * elem_size(a->dtype);
@@ -474,6 +530,120 @@ int b200tp_linear_ce_bwd_train(const b200tp_ce_args* a, const float* lse, const 
   if (d_weight == nullptr) return fail(B200TP_ERR_LOSS_INPUT, "d_weight is null");
   return bwd_impl(a, lse, cotangent, d_hidden, d_hidden_dtype, accumulate, d_weight, 1, 0, nullptr, workspace,
                   workspace_bytes, stream_v, status);
+}
+
+size_t b200tp_linear_ce_grad_state_bytes(const b200tp_ce_args* a) {
+  return check_grad_args(a) == B200TP_OK ? plan_grad(a, nullptr, nullptr).state_bytes : 0;
+}
+
+size_t b200tp_linear_ce_fwd_grad_workspace_bytes(const b200tp_ce_args* a) {
+  return check_grad_args(a) == B200TP_OK ? plan_grad(a, nullptr, nullptr).bytes : 0;
+}
+
+size_t b200tp_linear_ce_bwd_grad_workspace_bytes(const b200tp_ce_args* a) {
+  return check_grad_args(a) == B200TP_OK ? plan_grad(a, nullptr, nullptr).bwd_bytes : 0;
+}
+
+int b200tp_linear_ce_fwd_grad(const b200tp_ce_args* a, float* tgt_logit, float* lse, float* nll, void* state,
+                              size_t state_bytes, void* workspace, size_t workspace_bytes, void* stream_v,
+                              int* status) {
+  int rc = check_grad_args(a);
+  if (rc) return rc;
+  if (tgt_logit == nullptr || lse == nullptr || nll == nullptr)
+    return fail(B200TP_ERR_LOSS_INPUT, "tgt_logit / lse / nll outputs are required");
+  rc = require_sm100();
+  if (rc) return rc;
+  const GradPlan p = plan_grad(a, state, workspace);
+  if (!p.ok)
+    return fail(B200TP_ERR_UNSUPPORTED_HEAD, "the forward with gradient runs on the tensor-core path, 4-bit heads chunk-wise");
+  rc = check_workspace(state, state_bytes, p.state_bytes);
+  if (rc) return rc;
+  rc = check_workspace(workspace, workspace_bytes, p.bytes);
+  if (rc) return rc;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  const QuantHead q = packed_head(a);
+  rc = launch_ce_reference(a->hidden, a->weight, a->quant_bits != 0 ? &q : nullptr, a->n, a->d, a->v_local, a->targets,
+                           a->ignore_index, p.ref2, p.overflow, stream);
+  if (rc) return rc;
+  int64_t slot = 0;
+  for (int64_t c = 0; c < p.num_chunks; ++c) {
+    const int64_t r0 = c * p.chunk;
+    const int64_t w = std::min<int64_t>(p.chunk, a->v_local - r0);
+    const void* wmat = a->weight;
+    int64_t wrows = a->v_local, row0 = r0, vocab_id0 = 0;
+    if (p.deq != nullptr) {
+      rc = launch_dequant_int4(a->w_q, a->scales, a->biases, a->qparam_dtype, r0, w, a->d, a->group_size, p.deq,
+                               B200TP_BF16, stream);
+      if (rc) return rc;
+      wmat = p.deq;
+      wrows = w;
+      row0 = 0;
+      vocab_id0 = r0;
+    }
+    const int splits = ce_tc_fwd_splits(a->n, w);
+    rc = ce_tc_launch_fwd_grad(a->hidden, wmat, wrows, a->n, a->d, row0, row0 + w, vocab_id0, a->targets,
+                               a->ignore_index, p.ref2, p.overflow, splits, p.pm + slot * a->n, p.ps + slot * a->n,
+                               p.pt + slot * a->n, p.g, static_cast<int>(p.chunk), stream, status);
+    if (rc) return rc;
+    slot += splits;
+    // once the flag is set the sums are void: no need to go on with them
+    rc = ce_tc_launch_dh(p.g, static_cast<int>(p.chunk), static_cast<int>(align_up(w, kCeTileCols)), a->n, wmat, wrows,
+                         a->d, row0, c == 0 ? nullptr : p.acc, p.acc, nullptr, -1, -1, p.shares, nullptr,
+                         LaunchGuard{p.overflow, 0}, stream, status);
+    if (rc) return rc;
+  }
+  return launch_combine(p.pm, p.ps, p.pt, a->n, static_cast<int>(p.total_splits), a->n, a->targets, a->ignore_index,
+                        nullptr, nullptr, tgt_logit, lse, nll, stream);
+}
+
+int b200tp_linear_ce_bwd_grad(const b200tp_ce_args* a, const float* lse, const float* tgt_logit, const float* cotangent,
+                              void* state, size_t state_bytes, void* d_hidden, void* workspace, size_t workspace_bytes,
+                              void* stream_v, int* status) {
+  int rc = check_grad_args(a);
+  if (rc) return rc;
+  if (lse == nullptr || tgt_logit == nullptr || cotangent == nullptr || d_hidden == nullptr)
+    return fail(B200TP_ERR_LOSS_INPUT, "lse / tgt_logit / cotangent / d_hidden is null");
+  rc = require_sm100();
+  if (rc) return rc;
+  const GradPlan p = plan_grad(a, state, workspace);
+  if (!p.ok)
+    return fail(B200TP_ERR_UNSUPPORTED_HEAD, "the forward with gradient runs on the tensor-core path, 4-bit heads chunk-wise");
+  rc = check_workspace(state, state_bytes, p.state_bytes);
+  if (rc) return rc;
+  rc = check_workspace(workspace, workspace_bytes, p.bwd_bytes);
+  if (rc) return rc;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  const QuantHead q = packed_head(a);
+  rc = launch_ce_grad_finish(p.acc, p.shares, p.ref2, p.overflow, a->weight, a->quant_bits != 0 ? &q : nullptr, a->n,
+                             a->d, a->v_local, a->targets, a->ignore_index, lse, tgt_logit, cotangent, d_hidden, stream);
+  if (rc) return rc;
+  // Overflowed references: recompute the logits chunk by chunk.  The sums in `state` are void then, so their
+  // first share serves as the fp32 accumulator.
+  const LaunchGuard guard{p.overflow, 1};
+  for (int64_t c = 0; c < p.num_chunks; ++c) {
+    const int64_t r0 = c * p.chunk;
+    const int64_t w = std::min<int64_t>(p.chunk, a->v_local - r0);
+    const void* wmat = a->weight;
+    int64_t wrows = a->v_local, row0 = r0, vocab_id0 = 0;
+    if (p.deq != nullptr) {
+      rc = launch_dequant_int4(a->w_q, a->scales, a->biases, a->qparam_dtype, r0, w, a->d, a->group_size, p.deq,
+                               B200TP_BF16, stream, p.overflow);
+      if (rc) return rc;
+      wmat = p.deq;
+      wrows = w;
+      row0 = 0;
+      vocab_id0 = r0;
+    }
+    rc = ce_tc_launch_bwd_g(a->hidden, wmat, wrows, a->n, a->d, row0, row0 + w, vocab_id0, a->targets, a->ignore_index,
+                            lse, cotangent, p.g, static_cast<int>(p.chunk), nullptr, guard, stream, status);
+    if (rc) return rc;
+    const bool last = c == p.num_chunks - 1;
+    rc = ce_tc_launch_dh(p.g, static_cast<int>(p.chunk), static_cast<int>(align_up(w, kCeTileCols)), a->n, wmat, wrows,
+                         a->d, row0, c == 0 ? nullptr : p.acc, last ? nullptr : p.acc, last ? d_hidden : nullptr, -1, -1,
+                         1, nullptr, guard, stream, status);
+    if (rc) return rc;
+  }
+  return B200TP_OK;
 }
 
 int b200tp_dequant_int4(const uint32_t* w_q, const void* scales, const void* biases, int32_t qparam_dtype, int64_t row0,

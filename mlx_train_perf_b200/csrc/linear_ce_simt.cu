@@ -327,7 +327,8 @@ loss_cotangent_kernel(const long long* __restrict__ targets, long long n, long l
 template <typename TP, typename TO>
 __global__ void dequant_int4_kernel(const uint32_t* __restrict__ wq, const TP* __restrict__ scales,
                                     const TP* __restrict__ biases, long long row0, long long rows, int d, int group,
-                                    TO* __restrict__ out) {
+                                    TO* __restrict__ out, const int* run_if_set) {
+  if (run_if_set != nullptr && *run_if_set == 0) return;
   const int words = d / 8;
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= rows * words) return;
@@ -367,7 +368,9 @@ __device__ __forceinline__ void st_global_32b(void* p, const uint32_t (&v)[8]) {
 template <typename TP, typename TO>
 __global__ void __launch_bounds__(256)
 dequant_int4_x4_kernel(const uint32_t* __restrict__ wq, const TP* __restrict__ scales, const TP* __restrict__ biases,
-                       long long row0, long long rows, int d, int group, TO* __restrict__ out) {
+                       long long row0, long long rows, int d, int group, TO* __restrict__ out,
+                       const int* run_if_set) {
+  if (run_if_set != nullptr && *run_if_set == 0) return;
   const int quads = d / 32;
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= rows * quads) return;
@@ -406,7 +409,7 @@ dequant_int4_x4_kernel(const uint32_t* __restrict__ wq, const TP* __restrict__ s
 
 template <typename TP, typename TO>
 void launch_dequant_typed(const uint32_t* w_q, const void* scales, const void* biases, int64_t row0, int64_t rows, int d,
-                          int group, void* out, cudaStream_t stream) {
+                          int group, void* out, cudaStream_t stream, const int* run_if_set) {
   const bool wide = d % 32 == 0 && group % 32 == 0 && (reinterpret_cast<uintptr_t>(w_q) & 15) == 0 &&
                     (reinterpret_cast<uintptr_t>(out) & 31) == 0;
   const int threads = 256;
@@ -414,12 +417,12 @@ void launch_dequant_typed(const uint32_t* w_q, const void* scales, const void* b
     const unsigned blocks = static_cast<unsigned>(ceil_div(rows * (d / 32), threads));
     dequant_int4_x4_kernel<TP, TO><<<blocks, threads, 0, stream>>>(w_q, static_cast<const TP*>(scales),
                                                                    static_cast<const TP*>(biases), row0, rows, d, group,
-                                                                   static_cast<TO*>(out));
+                                                                   static_cast<TO*>(out), run_if_set);
   } else {
     const unsigned blocks = static_cast<unsigned>(ceil_div(rows * (d / 8), threads));
     dequant_int4_kernel<TP, TO><<<blocks, threads, 0, stream>>>(w_q, static_cast<const TP*>(scales),
                                                                 static_cast<const TP*>(biases), row0, rows, d, group,
-                                                                static_cast<TO*>(out));
+                                                                static_cast<TO*>(out), run_if_set);
   }
 }
 
@@ -455,16 +458,21 @@ int launch_loss_cotangent(const int64_t* targets, int64_t n, int64_t ignore_inde
 }
 
 int launch_dequant_int4(const uint32_t* w_q, const void* scales, const void* biases, int qparam_dtype, int64_t row0,
-                        int64_t rows, int d, int group, void* out, int out_dtype, cudaStream_t stream) {
+                        int64_t rows, int d, int group, void* out, int out_dtype, cudaStream_t stream,
+                        const int* run_if_set) {
   if (rows <= 0) return B200TP_OK;
   if (qparam_dtype == B200TP_BF16 && out_dtype == B200TP_BF16)
-    launch_dequant_typed<__nv_bfloat16, __nv_bfloat16>(w_q, scales, biases, row0, rows, d, group, out, stream);
+    launch_dequant_typed<__nv_bfloat16, __nv_bfloat16>(w_q, scales, biases, row0, rows, d, group, out, stream,
+                                                       run_if_set);
   else if (qparam_dtype == B200TP_BF16 && out_dtype == B200TP_F32)
-    launch_dequant_typed<__nv_bfloat16, float>(w_q, scales, biases, row0, rows, d, group, out, stream);
+    launch_dequant_typed<__nv_bfloat16, float>(w_q, scales, biases, row0, rows, d, group, out, stream,
+                                                       run_if_set);
   else if (qparam_dtype == B200TP_F32 && out_dtype == B200TP_BF16)
-    launch_dequant_typed<float, __nv_bfloat16>(w_q, scales, biases, row0, rows, d, group, out, stream);
+    launch_dequant_typed<float, __nv_bfloat16>(w_q, scales, biases, row0, rows, d, group, out, stream,
+                                                       run_if_set);
   else
-    launch_dequant_typed<float, float>(w_q, scales, biases, row0, rows, d, group, out, stream);
+    launch_dequant_typed<float, float>(w_q, scales, biases, row0, rows, d, group, out, stream,
+                                                       run_if_set);
   B200TP_CUDA_OK(cudaGetLastError());
   return B200TP_OK;
 }

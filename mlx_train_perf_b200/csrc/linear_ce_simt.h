@@ -18,8 +18,10 @@ int launch_loss_reduce(const float* nll, const int64_t* targets, int64_t n, int6
 int launch_loss_cotangent(const int64_t* targets, int64_t n, int64_t ignore_index, const float* upstream,
                           const float* count, float* ct, cudaStream_t stream);
 
+// `run_if_set` (device flag) non-null: the launch does nothing unless it is set.
 int launch_dequant_int4(const uint32_t* w_q, const void* scales, const void* biases, int qparam_dtype, int64_t row0,
-                        int64_t rows, int d, int group, void* out, int out_dtype, cudaStream_t stream);
+                        int64_t rows, int d, int group, void* out, int out_dtype, cudaStream_t stream,
+                        const int* run_if_set = nullptr);
 
 // logits_ws (n, width) f32 = hidden @ w_chunk^T, folded into run_m / run_s / run_t.
 int ce_simt_fwd_chunk(const void* hidden, const void* w_chunk, int dtype, int64_t n, int d, int64_t width,

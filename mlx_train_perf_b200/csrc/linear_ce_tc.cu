@@ -67,8 +67,15 @@ constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + 1024;  // + alignm
 constexpr int SMEM_BYTES_Q = SMEM_BYTES + CODE_BYTES;
 constexpr uint32_t TMEM_COLS = 512;                                  // two 256-column accumulators
 
-enum { MODE_FWD = 0, MODE_BWD_G = 1 };
+enum { MODE_FWD = 0, MODE_BWD_G = 1, MODE_FWD_GRAD = 2 };
 
+// MODE_FWD_GRAD: exponents (log2 units, relative to the row's reference) above this raise the overflow flag.
+// Sums of 2^27 terms of 2^100 stay below the largest fp32, and 2^100 = e^69.
+constexpr float kRefHeadroom = 100.f;
+
+__device__ __forceinline__ bool guard_skips(const LaunchGuard& g) {
+  return g.flag != nullptr && (*g.flag != 0) != (g.run_if_set != 0);
+}
 
 struct LogitsParams {
   int n_rows;            // N
@@ -85,8 +92,12 @@ struct LogitsParams {
   // BWD_G
   const float* lse;
   const float* ct;
-  __nv_bfloat16* g;
+  __nv_bfloat16* g;         // BWD_G, FWD_GRAD
   int ldg;
+  // FWD_GRAD
+  const float* ref2;        // per row: reference of the exponentials, log2 units
+  int* overflow;            // set to 1 when some logit exceeds its row's reference by kRefHeadroom
+  LaunchGuard guard;
   int* status;
   // QUANT: the packed head (rows indexed like the tensor map of a dense weight would be)
   const uint32_t* wq;
@@ -105,8 +116,11 @@ struct DhParams {
   const float* acc_in;   // fp32 (N, D) partial sums to add, or nullptr
   float* acc_out;        // fp32 (N, D) destination, or nullptr
   __nv_bfloat16* out_bf16;  // bf16 (N, D) destination, or nullptr
+  LaunchGuard guard;
   int* status;
-  int tile0, tile1;         // tiles [tile0, tile1) of the row-block-major order are computed by this launch
+  int tile0, tile1;         // units [tile0, tile1) are computed by this launch; unit = split * tiles + tile
+  int ksplit;               // shares of the contraction: share s adds into acc + s * split_stride (ksplit 1: no shares)
+  long long split_stride;
   // QUANT: the packed head
   const uint32_t* wq;
   const void* scales;
@@ -246,6 +260,7 @@ template <int MODE, bool QUANT>
 __global__ void __launch_bounds__(QUANT ? THREADS_Q : THREADS, 1)
 ce_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_constant__ CUtensorMap tmap_w,
                  const LogitsParams p) {
+  if (guard_skips(p.guard)) return;
   extern __shared__ uint8_t smem_raw[];
   const SmemView sm = carve_smem(smem_raw, QUANT);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // provably warp-uniform
@@ -444,12 +459,14 @@ ce_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_consta
       if (row_ok) target = p.targets[row];
       const bool tvalid = row_ok && target != p.ignore_index;
 
-      float run_m = -INFINITY, run_s = 0.f, run_t = 0.f;  // FWD state (log2 domain for m)
+      float run_m = -INFINITY, run_s = 0.f, run_t = 0.f;  // FWD, FWD_GRAD state (log2 domain for m)
+      bool over = false;                                  // FWD_GRAD: some exponent left the reference's range
       float lse2 = 0.f, ctv = 0.f;                        // BWD_G state
       if (MODE == MODE_BWD_G && row_ok) {
         lse2 = p.lse[row] * kLog2e;
         ctv = tvalid ? p.ct[row] : 0.f;
       }
+      if (MODE == MODE_FWD_GRAD) run_m = row_ok ? p.ref2[row] : 0.f;
 
       for (int vt = vt0; vt < vt1 && ok; ++vt, ++tile) {
         const uint32_t as = tile & 1;
@@ -497,6 +514,50 @@ ce_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_consta
             for (int j = 0; j < 32; ++j) acc += fast_exp2(fmaf(x[j], kLog2e, -new_m));
             run_s = run_s * fast_exp2(run_m - new_m) + acc;
             run_m = new_m;
+          } else if (MODE == MODE_FWD_GRAD) {
+            // One exponential per logit serves both the row sum and the unnormalised gradient: relative to a
+            // reference fixed before the launch, e = exp(z - ref) needs neither the row maximum nor the final
+            // log-sum-exp, and the row's factor exp(ref - lse) is applied to d_hidden afterwards.
+            float x[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              x[j] = __uint_as_float(r[j]);
+              if (j >= cvalid) x[j] = -INFINITY;
+            }
+            const int tj = (tcol >= 0 && (tcol >> 5) == c) ? (tcol & 31) : -1;
+            float xm = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              if (j == tj) run_t = x[j];
+              x[j] = fmaf(x[j], kLog2e, -run_m);
+              xm = fmaxf(xm, x[j]);
+            }
+            if (xm > kRefHeadroom) {   // rare: move this thread's own sum to a larger reference; g is void then
+              over = true;
+              run_s *= fast_exp2(-xm);
+              run_m += xm;
+#pragma unroll
+              for (int j = 0; j < 32; ++j) x[j] -= xm;
+            }
+            float acc4[4] = {0.f, 0.f, 0.f, 0.f};
+            uint32_t packed[16];
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              float e0 = fast_exp2(x[j]), e1 = fast_exp2(x[j + 1]);
+              acc4[(j >> 1) & 3] += e0 + e1;
+              // the target's own term p - 1 is added to d_hidden in fp32 later: rounding p to bf16 here would
+              // lose it on rows whose target is nearly certain
+              if (j == tj) e0 = 0.f;
+              if (j + 1 == tj) e1 = 0.f;
+              packed[j >> 1] = tvalid ? pack_bf16x2(e0, e1) : 0u;
+            }
+            run_s += (acc4[0] + acc4[1]) + (acc4[2] + acc4[3]);
+            if (row_ok) {
+              uint4* dst = reinterpret_cast<uint4*>(p.g + static_cast<size_t>(row) * p.ldg + (vt * BN + c * 32));
+#pragma unroll
+              for (int q4 = 0; q4 < 4; ++q4)
+                dst[q4] = make_uint4(packed[4 * q4], packed[4 * q4 + 1], packed[4 * q4 + 2], packed[4 * q4 + 3]);
+            }
           } else {
             uint32_t packed[16];
 #pragma unroll
@@ -522,7 +583,8 @@ ce_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_consta
         if (lane == 0) mbar_arrive(&sm.tempty[as]);
       }
 
-      if (MODE == MODE_FWD && ok && row_ok) {
+      if (MODE == MODE_FWD_GRAD && over) *p.overflow = 1;
+      if ((MODE == MODE_FWD || MODE == MODE_FWD_GRAD) && ok && row_ok) {
         const size_t o = static_cast<size_t>(split) * p.n_rows + row;
         p.pm[o] = run_m * kLn2;  // back to natural-log units
         p.ps[o] = run_s;
@@ -544,6 +606,7 @@ template <bool QUANT>
 __global__ void __launch_bounds__(QUANT ? THREADS_Q : THREADS, 1)
 ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__ CUtensorMap tmap_w,
              const DhParams p) {
+  if (guard_skips(p.guard)) return;
   extern __shared__ uint8_t smem_raw[];
   const SmemView sm = carve_smem(smem_raw, QUANT);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // provably warp-uniform
@@ -553,6 +616,12 @@ ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
   const int total_tiles = p.tile1;
   const int first_tile = p.tile0 + blockIdx.x;
   const int kblocks = p.k_total / BK;
+  const int tiles = p.num_rb * p.num_nt;
+  // k blocks [kb0, kb1) of a unit; a share can be empty when a later chunk is narrower than the first
+  auto k_range = [&](int split, int& kb0, int& kb1) {
+    kb0 = static_cast<int>(static_cast<long long>(split) * kblocks / p.ksplit);
+    kb1 = static_cast<int>(static_cast<long long>(split + 1) * kblocks / p.ksplit);
+  };
 
   if (QUANT && warp >= THREADS / 32) {
     // ------------------------------ dequantising warps ------------------------------
@@ -639,10 +708,13 @@ ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
       tma_prefetch_desc(&tmap_w);
       uint32_t it = 0;
       bool ok = true;
-      for (int t = first_tile; t < total_tiles && ok; t += gridDim.x) {
+      for (int u = first_tile; u < total_tiles && ok; u += gridDim.x) {
+        const int split = u / tiles, t = u - split * tiles;
         const int rb = t / p.num_nt;
         const int nt = t - rb * p.num_nt;
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+        int kb0, kb1;
+        k_range(split, kb0, kb1);
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(&sm.empty[s], ((it / STAGES) & 1) ^ 1, sm.abort_flag)) {
             raise_abort(sm, p.status, kDevTimeoutProducer);
@@ -684,7 +756,10 @@ ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
     constexpr uint32_t dhi = desc_hi_sw128(1024);
     uint32_t it = 0, tile = 0;
     bool ok = true;
-    for (int t = first_tile; t < total_tiles && ok; t += gridDim.x, ++tile) {
+    for (int u = first_tile; u < total_tiles && ok; u += gridDim.x) {
+      int kb0, kb1;
+      k_range(u / tiles, kb0, kb1);
+      if (kb0 >= kb1) continue;
       const uint32_t as = tile & 1;
       if (!mbar_wait_warp(&sm.tempty[as], ((tile >> 1) & 1) ^ 1, sm.abort_flag)) {
         if (lane == 0) raise_abort(sm, p.status, kDevTimeoutMma);
@@ -692,7 +767,7 @@ ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
       }
       tc_fence_after_sync();
       const uint32_t d_tmem = tmem_base + as * BN;
-      for (int kb = 0; kb < kblocks; ++kb, ++it) {
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const int s = it % STAGES;
         if (!mbar_wait_warp(&sm.full[s], (it / STAGES) & 1, sm.abort_flag)) {
           if (lane == 0) raise_abort(sm, p.status, kDevTimeoutMma);
@@ -706,21 +781,26 @@ ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
         if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
-            umma_ss_w(d_tmem, a_lo + k * 2, dhi, b_lo + k * 128, dhi, idesc, (kb | k) != 0 ? 1u : 0u);
+            umma_ss_w(d_tmem, a_lo + k * 2, dhi, b_lo + k * 128, dhi, idesc, kb != kb0 || k != 0 ? 1u : 0u);
           umma_commit(&sm.empty[s]);
         }
         __syncwarp();
       }
       if (ok && elect_one()) umma_commit(&sm.tfull[as]);
       __syncwarp();
+      ++tile;
     }
   } else {
     const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;
     uint32_t tile = 0;
-    for (int t = first_tile; t < total_tiles; t += gridDim.x, ++tile) {
+    for (int u = first_tile; u < total_tiles; u += gridDim.x) {
+      const int split = u / tiles, t = u - split * tiles;
       const int rb = t / p.num_nt;
       const int nt = t - rb * p.num_nt;
+      int kb0, kb1;
+      k_range(split, kb0, kb1);
+      if (kb0 >= kb1) continue;   // nothing to add: the share keeps what earlier chunks left (see the host side)
       const uint32_t as = tile & 1;
       if (!mbar_wait_warp(&sm.tfull[as], (tile >> 1) & 1, sm.abort_flag)) {
         raise_abort(sm, p.status, kDevTimeoutEpilogue);
@@ -739,7 +819,7 @@ ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
         tmem_wait_ld();
         tmem_regs_ready(r);
         if (row_ok) {
-          const size_t off = static_cast<size_t>(row) * p.d_cols + col0;
+          const size_t off = static_cast<size_t>(split) * p.split_stride + static_cast<size_t>(row) * p.d_cols + col0;
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
             if (col0 + j < p.d_cols) {  // d_cols is a multiple of 8
@@ -761,6 +841,7 @@ ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.tempty[as]);
+      ++tile;
     }
   }
   cta_teardown(sm, warp, tmem_base);
@@ -948,6 +1029,8 @@ static int configure_kernels() {
                                       SMEM_BYTES));
   B200TP_CUDA_OK(cudaFuncSetAttribute(ce_logits_kernel<MODE_BWD_G, false>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  B200TP_CUDA_OK(cudaFuncSetAttribute(ce_logits_kernel<MODE_FWD_GRAD, false>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   B200TP_CUDA_OK(cudaFuncSetAttribute(ce_logits_kernel<MODE_FWD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       SMEM_BYTES_Q));
   B200TP_CUDA_OK(cudaFuncSetAttribute(ce_logits_kernel<MODE_BWD_G, true>,
@@ -1024,8 +1107,8 @@ int ce_tc_launch_fwd(const void* hidden, const void* w, int64_t w_rows_total, in
 
 int ce_tc_launch_bwd_g(const void* hidden, const void* w, int64_t w_rows_total, int64_t n, int d, int64_t vrow0,
                        int64_t vrow1, int64_t vocab_id0, const int64_t* targets, int64_t ignore_index,
-                       const float* lse, const float* ct, void* g, int ldg, const QuantHead* q, cudaStream_t stream,
-                       int* status) {
+                       const float* lse, const float* ct, void* g, int ldg, const QuantHead* q,
+                       const LaunchGuard& guard, cudaStream_t stream, int* status) {
   int rc = configure_kernels();
   if (rc) return rc;
   CUtensorMap tmap_h, tmap_w;
@@ -1050,6 +1133,7 @@ int ce_tc_launch_bwd_g(const void* hidden, const void* w, int64_t w_rows_total, 
   p.ct = ct;
   p.g = reinterpret_cast<__nv_bfloat16*>(g);
   p.ldg = ldg;
+  p.guard = guard;
   p.status = status;
   fill_quant(p, q);
   const int grid = std::min<long long>(sm_count(), static_cast<long long>(p.num_rb) * p.splits);
@@ -1061,8 +1145,65 @@ int ce_tc_launch_bwd_g(const void* hidden, const void* w, int64_t w_rows_total, 
   return B200TP_OK;
 }
 
+int ce_tc_launch_fwd_grad(const void* hidden, const void* w, int64_t w_rows_total, int64_t n, int d, int64_t vrow0,
+                          int64_t vrow1, int64_t vocab_id0, const int64_t* targets, int64_t ignore_index,
+                          const float* ref2, int* overflow, int splits, float* pm, float* ps, float* pt, void* g,
+                          int ldg, cudaStream_t stream, int* status) {
+  int rc = configure_kernels();
+  if (rc) return rc;
+  CUtensorMap tmap_h, tmap_w;
+  rc = make_tmap_2d_bf16(&tmap_h, hidden, n, d, d, BM, BK);
+  if (rc) return rc;
+  rc = make_tmap_2d_bf16(&tmap_w, w, w_rows_total, d, d, BN, BK);
+  if (rc) return rc;
+  LogitsParams p{};
+  p.n_rows = static_cast<int>(n);
+  p.k_dim = d;
+  p.vrow0 = static_cast<int>(vrow0);
+  p.vrow1 = static_cast<int>(vrow1);
+  p.vocab_id0 = vocab_id0;
+  p.num_rb = static_cast<int>(ceil_div(n, BM));
+  p.num_vt = static_cast<int>(ceil_div(vrow1 - vrow0, BN));
+  p.splits = splits;
+  p.targets = reinterpret_cast<const long long*>(targets);
+  p.ignore_index = ignore_index;
+  p.pm = pm;
+  p.ps = ps;
+  p.pt = pt;
+  p.g = reinterpret_cast<__nv_bfloat16*>(g);
+  p.ldg = ldg;
+  p.ref2 = ref2;
+  p.overflow = overflow;
+  p.status = status;
+  const int grid = std::min<long long>(sm_count(), static_cast<long long>(p.num_rb) * splits);
+  ce_logits_kernel<MODE_FWD_GRAD, false><<<grid, THREADS, SMEM_BYTES, stream>>>(tmap_h, tmap_w, p);
+  B200TP_CUDA_OK(cudaGetLastError());
+  return B200TP_OK;
+}
+
 int ce_tc_dh_tiles(int64_t n, int d) {
   return static_cast<int>(ceil_div(n, BM) * ceil_div(d, BN));
+}
+
+// Shares of the d_hidden contraction.  A call with few rows has few 128 x 256 tiles (four at 60 rows and
+// D = 1024), and one CTA each would leave most of the chip idle; the shares' fp32 sums are added in a fixed order
+// afterwards.  The cost of a choice is the busiest CTA's k blocks plus, per unit, what its prologue and
+// epilogue take (about kUnitCost k blocks of 0.27 us).
+int ce_tc_dh_ksplit(int64_t n, int d, int k_total) {
+  constexpr int kUnitCost = 8, kMostShares = 64;
+  const int64_t tiles = ce_tc_dh_tiles(n, d);
+  const int kblocks = k_total / BK, ctas = sm_count();
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int ks = 1; ks <= std::min(kMostShares, kblocks); ++ks) {
+    const int64_t cost = ceil_div(tiles * ks, ctas) * (ceil_div(kblocks, ks) + kUnitCost);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = ks;
+    }
+    if (tiles * ks >= 4 * ctas) break;   // more shares than this only add partial sums
+  }
+  return best;
 }
 
 int ce_tc_dh_rows_done(int64_t n, int d, int tiles_done) {
@@ -1073,7 +1214,10 @@ int ce_tc_dh_rows_done(int64_t n, int d, int tiles_done) {
 
 int ce_tc_launch_dh(const void* g, int ldg, int k_total, int64_t n, const void* w, int64_t w_rows_total, int d,
                     int64_t wrow0, const float* acc_in, float* acc_out, void* out_bf16, int tile0, int tile1,
-                    const QuantHead* q, cudaStream_t stream, int* status) {
+                    int ksplit, const QuantHead* q, const LaunchGuard& guard, cudaStream_t stream, int* status) {
+  if (ksplit > 1 && (out_bf16 != nullptr || (q != nullptr && q->wq != nullptr) ||
+                     (acc_in == nullptr && ksplit > k_total / BK) || (acc_in != nullptr && acc_in != acc_out)))
+    return fail(B200TP_ERR_CUDA, "d_hidden shares: fp32 sums of a dense weight, in place, no empty share at first");
   int rc = configure_kernels();
   if (rc) return rc;
   CUtensorMap tmap_g, tmap_w;
@@ -1092,7 +1236,10 @@ int ce_tc_launch_dh(const void* g, int ldg, int k_total, int64_t n, const void* 
   p.acc_out = acc_out;
   p.out_bf16 = reinterpret_cast<__nv_bfloat16*>(out_bf16);
   p.status = status;
-  const int total = p.num_rb * p.num_nt;
+  p.guard = guard;
+  p.ksplit = ksplit;
+  p.split_stride = static_cast<long long>(n) * d;
+  const int total = p.num_rb * p.num_nt * ksplit;
   p.tile0 = tile0 < 0 ? 0 : tile0;
   p.tile1 = tile1 < 0 ? total : std::min(tile1, total);
   p.w_rows = static_cast<int>(w_rows_total);

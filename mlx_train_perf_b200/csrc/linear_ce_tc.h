@@ -18,6 +18,13 @@ struct QuantHead {
   int qp_f32;
 };
 
+// A launch that is only needed when a flag in device memory is set (or is not): every CTA reads it first and
+// leaves at once otherwise.  A null `flag` means "always".
+struct LaunchGuard {
+  const int* flag = nullptr;
+  int run_if_set = 0;
+};
+
 // Vocab splits the forward uses for (n rows, v_rows vocab rows): one partial triple per
 // (row, split) lands in the workspace.
 int ce_tc_fwd_splits(int64_t n, int64_t v_rows);
@@ -32,19 +39,30 @@ int ce_tc_launch_fwd(const void* hidden, const void* w, int64_t w_rows_total, in
 // up to the next multiple of 256 are written (zeros past vrow1).
 int ce_tc_launch_bwd_g(const void* hidden, const void* w, int64_t w_rows_total, int64_t n, int d, int64_t vrow0,
                        int64_t vrow1, int64_t vocab_id0, const int64_t* targets, int64_t ignore_index,
-                       const float* lse, const float* ct, void* g, int ldg, const QuantHead* q, cudaStream_t stream,
-                       int* status);
+                       const float* lse, const float* ct, void* g, int ldg, const QuantHead* q,
+                       const LaunchGuard& guard, cudaStream_t stream, int* status);
+
+// Forward partials as ce_tc_launch_fwd and, from the same exponentials, g[n][ldg] (bf16) = exp(z - ref) with
+// `ref2` = ref log2(e) per row, zero at the target's column and on ignored rows.  A row whose logits reach
+// 69 above its reference sets *overflow (g is void then; the partials are right in any case).  Dense weights.
+int ce_tc_launch_fwd_grad(const void* hidden, const void* w, int64_t w_rows_total, int64_t n, int d, int64_t vrow0,
+                          int64_t vrow1, int64_t vocab_id0, const int64_t* targets, int64_t ignore_index,
+                          const float* ref2, int* overflow, int splits, float* pm, float* ps, float* pt, void* g,
+                          int ldg, cudaStream_t stream, int* status);
 
 // dH = [acc_in +] G[:, :k_total] @ W[wrow0 : wrow0 + k_total, :]; written to acc_out (f32)
 // and/or out_bf16.  k_total is a multiple of 64; rows of W past w_rows_total read as zero.
 // The 128 x 256 output tiles are numbered row-block-major; this launch computes tiles
 // [tile0, tile1) (negative: from the first / through the last).  `ce_tc_dh_rows_done(n, d, t)` is
 // the number of leading rows of d_hidden that are complete once tiles [0, t) have run.
+// `ksplit` > 1 shares each tile's contraction between that many units, share s summing into acc + s * n * d
+// (fp32, in place over chunks); `ce_tc_dh_ksplit` picks it for chunks of k_total columns.
 int ce_tc_dh_tiles(int64_t n, int d);
+int ce_tc_dh_ksplit(int64_t n, int d, int k_total);
 int ce_tc_dh_rows_done(int64_t n, int d, int tiles_done);
 int ce_tc_launch_dh(const void* g, int ldg, int k_total, int64_t n, const void* w, int64_t w_rows_total, int d,
                     int64_t wrow0, const float* acc_in, float* acc_out, void* out_bf16, int tile0, int tile1,
-                    const QuantHead* q, cudaStream_t stream, int* status);
+                    int ksplit, const QuantHead* q, const LaunchGuard& guard, cudaStream_t stream, int* status);
 
 // d_weight block (v_rows, d) bf16 = G[:, :v_rows]^T @ hidden: g (n, ldg) bf16 as written by
 // ce_tc_launch_bwd_g, hidden (n, d) bf16.  fp32 accumulation over the n rows, one rounding.

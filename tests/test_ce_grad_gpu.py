@@ -1,0 +1,119 @@
+"""The forward that also forms the gradient of a frozen head, against the fp64 evaluation of the oracle.
+
+Bound, per row of d_hidden in the 2-norm: the exponentials are rounded to bf16 before the second contraction
+(2^-9 of each term at most, errors independent) and the result is rounded once (2^-9 of each element), so a row is
+off by at most 2 x 2^-9 = 4e-3 of its norm unless its terms cancel; 1e-2 leaves room for that.  On top, the target's
+term (p - 1) W_t with p = exp(tgt - lse) <= 1 moves by the absolute error of tgt - lse: an error of the target's
+logit is in both and cancels, their roundings to fp32 (2^-24 each) and those of the logarithm and the scale (as much
+again) do not.  It is what limits rows whose target is certain.
+Forward: D / 16 accumulation steps per logit, each off by at most 2^-23 of the running sum, beside the 1e-5 that small
+logits are held to.
+"""
+import pytest
+import torch
+
+from mlx_train_perf_b200 import configs
+from mlx_train_perf_b200.core import loss as L
+from mlx_train_perf_b200.core.loss import DenseHead, QuantizedHead, fused_linear_ce
+from oracle import linear_ce as oc
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(dev, hidden, head, targets, ct):
+    h = hidden.to(dev).requires_grad_(True)
+    nll, lse, tgt = fused_linear_ce(h, head, targets.to(dev))
+    (nll * ct.to(dev)).sum().backward(retain_graph=True)
+    first = h.grad.clone()
+    h.grad = None
+    (nll * ct.to(dev)).sum().backward()
+    torch.cuda.synchronize()
+    L.check_device_status()
+    assert torch.equal(first, h.grad)            # the forward's sums serve a second backward unchanged
+    return nll.detach().cpu(), lse.detach().cpu(), tgt.detach().cpu(), h.grad.double().cpu()
+
+
+def _check(got, hidden, w, targets, ct):
+    nll, lse, tgt, dh = got
+    r_nll, r_lse, r_tgt = oc.naive_linear_ce(hidden, w, targets, dtype=torch.float64)
+    r_dh, _ = oc.chunked_backward(hidden, w, targets, r_lse, ct.double(), chunk_size=4096, dtype=torch.float64)
+    top = max(r_lse.abs().max().item(), r_tgt.abs().max().item())
+    fwd = 1e-5 + hidden.shape[1] / 16 * 2.0 ** -23 * top
+    for x, y in ((nll, r_nll), (lse, r_lse), (tgt, r_tgt)):
+        assert (x.double() - y).abs().max().item() < fwd
+    ign = targets == configs.IGNORE_INDEX
+    assert (dh[ign] == 0).all() and (nll[ign] == 0).all()
+    err, norm = (dh - r_dh)[~ign].norm(dim=1), r_dh[~ign].norm(dim=1)
+    floor = 2.0 ** -22 * top * ct.double().abs()[~ign] * w[targets[~ign]].double().norm(dim=1)
+    assert (err <= 1e-2 * norm + floor).all(), (err / (1e-2 * norm + floor)).max().item()
+
+
+# rows around a tile, hidden sizes around a k block and a column tile, vocabularies around a tile and over
+# several chunks; few rows share each tile's contraction over many CTAs, many rows do not
+SHAPES = [(1, 8, 1), (1, 64, 257), (127, 72, 255), (128, 256, 512), (129, 264, 4099), (60, 1024, 33000),
+          (300, 320, 16385), (1500, 136, 2049)]
+
+
+@pytest.mark.parametrize("certain", [False, True])
+@pytest.mark.parametrize(("n", "d", "v"), SHAPES)
+def test_dense(cuda_device, n, d, v, certain):
+    inp = configs.ce_dense(n, d, v, dtype=torch.bfloat16, ignore_frac=0.05 if n > 1 else 0.0, seed=n + v)
+    if certain:      # targets from unlikely to certain: pushed towards their weight rows by up to 30
+        t = inp.targets.clamp(min=0)
+        push = torch.linspace(0, 30, n)[:, None]
+        inp.hidden = (inp.hidden.float() + push * inp.weight[t].float()).to(torch.bfloat16)
+    ct = torch.linspace(0.5, 1.5, n) * torch.where(torch.arange(n) % 2 == 0, 1.0, -1.0)
+    got = _run(cuda_device, inp.hidden, DenseHead(inp.weight.to(cuda_device), trainable=False), inp.targets, ct)
+    if v == 1:       # the loss of the only class is zero and so is its gradient
+        assert got[3].abs().max() < 1e-5 and got[0].abs().max() < 1e-5
+        return
+    _check(got, inp.hidden, inp.weight, inp.targets, ct)
+
+
+@pytest.mark.parametrize("params", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize(("n", "d", "v"), [(1, 64, 300), (130, 320, 4099), (70, 128, 40000)])
+def test_int4(cuda_device, n, d, v, params):
+    inp = configs.ce_quant(n, d, v, ignore_frac=0.05 if n > 1 else 0.0, seed=v)
+    sc, bi = inp.scales.to(params), inp.biases.to(params)
+    w = oc.dequantize_int4(inp.w_q, sc, bi, out_dtype=torch.bfloat16)
+    head = QuantizedHead(*(x.to(cuda_device) for x in (inp.w_q, sc, bi)))
+    ct = torch.full((n,), 1.0 / n)
+    _check(_run(cuda_device, inp.hidden, head, inp.targets, ct), inp.hidden, w, inp.targets, ct)
+
+
+@pytest.mark.parametrize("quant", [False, True])
+@pytest.mark.parametrize("scale", [20.0, 200.0])
+def test_logits_far_above_the_target(cuda_device, quant, scale):
+    """Logits 70 and more above the target's leave the range of the fixed reference: the backward then computes
+    them again.  At 20 some rows do, at 200 all; ignored rows (reference: vocab row 0) do as well."""
+    n, d, v = 200, 128, 20000
+    if quant:
+        inp = configs.ce_quant(n, d, v, ignore_frac=0.1, seed=3)
+        w = oc.dequantize_int4(inp.w_q, inp.scales, inp.biases, out_dtype=torch.bfloat16)
+        head = QuantizedHead(*(x.to(cuda_device) for x in (inp.w_q, inp.scales, inp.biases)))
+    else:
+        inp = configs.ce_dense(n, d, v, dtype=torch.bfloat16, ignore_frac=0.1, seed=3)
+        w, head = inp.weight, DenseHead(inp.weight.to(cuda_device), trainable=False)
+    hidden = (inp.hidden.float() * scale).to(torch.bfloat16)
+    ct = torch.full((n,), 1.0 / n)
+    got = _run(cuda_device, hidden, head, inp.targets, ct)
+    nll, lse, _, dh = got
+    r_nll, r_lse, _ = oc.naive_linear_ce(hidden, w, inp.targets, dtype=torch.float64)
+    assert r_nll.max() > 80
+    r_dh, _ = oc.chunked_backward(hidden, w, inp.targets, r_lse, ct.double(), chunk_size=4096, dtype=torch.float64)
+    # fp32 sums of 128 products of size up to 4 scale: 2^-24 of the largest partial sum per addition
+    assert ((lse.double() - r_lse).abs() <= 2e-6 * scale * 4).all()
+    assert torch.isfinite(nll).all()
+    # a probability moves by the absolute error of its logit, and g is rounded to bf16
+    assert ((dh - r_dh).norm() / r_dh.norm()).item() < 1e-2
+
+
+def test_no_gradient_wanted_runs_the_plain_forward(cuda_device):
+    inp = configs.ce_dense(100, 128, 3000, dtype=torch.bfloat16, seed=1)
+    head = DenseHead(inp.weight.to(cuda_device), trainable=False)
+    h, t = inp.hidden.to(cuda_device), inp.targets.to(cuda_device)
+    a = fused_linear_ce(h, head, t)
+    b = fused_linear_ce(h.clone().requires_grad_(True), head, t)
+    assert a[0].grad_fn is None and b[0].grad_fn is not None
+    for x, y in zip(a, b):
+        assert (x - y.detach()).abs().max().item() < 1e-5
