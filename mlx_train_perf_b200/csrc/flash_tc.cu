@@ -201,6 +201,35 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* raw) {
   return raw + (((addr + 1023u) & ~1023u) - addr);
 }
 
+// Packed rows: segment ids never decrease along a row, so what row i may see is the interval
+// [first index of its segment, i], and who sees key k is [k, end of its segment).  Every masked element is then
+// one unsigned compare against two values found once per thread, and a warp masks only where its own rows and
+// columns need it.  Reading the ids element by element took 64 loads a row and block in each pass and four more per
+// block to decide.  Forward + backward, 32 / 8 heads: one row of 16384 tokens in documents of 128 to 4096, 2353 ->
+// 1870 us; forward of 2 x 2500 at head_dim 64 (diagonal blocks only), 136 -> 113 us.
+//
+// First index of row i's segment: `starts[i]` where it is one (the contract), else a search.
+__device__ __forceinline__ int segment_first(const int* __restrict__ segs, const int* __restrict__ starts, int i) {
+  const int sid = segs[i], st = max(0, min(starts[i], i));
+  if (segs[st] == sid && (st == 0 || segs[st - 1] != sid)) return st;
+  int lo = 0, hi = i;   // segs[hi] == sid throughout
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (segs[mid] < sid) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+// First index past k's segment, searched up to `limit` (> k).
+__device__ __forceinline__ int segment_end(const int* __restrict__ segs, int k, int limit) {
+  const int sid = segs[k];
+  int lo = k + 1, hi = limit;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (segs[mid] > sid) hi = mid; else lo = mid + 1;
+  }
+  return lo;
+}
+
 // One query row's entry of the statistics tile: -L / scale and -D, each split into three bf16 terms whose
 // sum is the fp32 value exactly (each remainder is formed exactly in fp32), then two zeros:
 //   [v_hi, v_mid, v_lo, d_hi, d_mid, d_lo, 0, 0].
@@ -372,8 +401,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const int ig = q0 + r;
     const int igc = min(ig, p.S - 1);  // rows past the end mask like the last row; never stored
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const int my_seg = packed ? segs[igc] : 0;
-    const int q_last = min(q0 + TILE - 1, p.S - 1);
+    const int row_lo = packed ? segment_first(segs, p.seg_start + static_cast<long long>(b) * p.S, igc) : 0;
+    const int lo_max = __reduce_max_sync(0xffffffffu, row_lo);   // of this warp's rows
     float m = -INFINITY, l = 0.f, alpha_prev = 1.f;
     float acc[FWD_COLS];
 #pragma unroll
@@ -384,24 +413,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       const int buf = n & 1;
       if (!mbar_wait_warp(&s_full[buf], (n >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
-      bool need_mask = (j == qi);
-      if (packed) {
-        const int k_first = j * TILE, k_last = min(j * TILE + TILE - 1, p.S - 1);
-        const int sid = segs[k_first];
-        need_mask = need_mask || sid != segs[k_last] || sid != segs[q0] || sid != segs[q_last];
-      }
+      const int c_first = j * TILE + part * FWD_COLS;   // this warp's keys of the block
+      const bool need_mask = c_first + FWD_COLS - 1 > q0 + quad * 32 || c_first < lo_max;
       // ---- this warp's 32 scores of the row, read from tensor memory once
       uint32_t sv[FWD_COLS];
       tmem_ld_cols<FWD_COLS>(tmem_base + buf * 128 + lane_off + part * FWD_COLS, sv);
       tmem_wait_ld();
       if (need_mask) {
 #pragma unroll
-        for (int e = 0; e < FWD_COLS; ++e) {
-          const int jg = j * TILE + part * FWD_COLS + e;
-          bool allowed = jg <= igc;
-          if (packed && allowed) allowed = segs[jg] == my_seg;
-          if (!allowed) sv[e] = 0xff800000u;  // -inf
-        }
+        for (int e = 0; e < FWD_COLS; ++e)
+          if (static_cast<uint32_t>(c_first - row_lo + e) > static_cast<uint32_t>(igc - row_lo))
+            sv[e] = 0xff800000u;  // -inf
       }
       // ---- partial row max (raw scores; scale > 0 so max commutes with the scaling)
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -771,9 +793,9 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       auto sum_slot = [&](int half) -> volatile float* {
         return reinterpret_cast<float*>(q_sm + t * TILE_BYTES) + half * TILE + r;
       };
-      const int my_seg = packed ? segs[igc] : 0;
-      const int q_last = min(me.q0 + TILE - 1, p.S - 1);
-      const int qi = me.q0 / TILE;
+      const int row_lo = packed ? segment_first(segs, p.seg_start + static_cast<long long>(b) * p.S, igc) : 0;
+      const int lo_max = __reduce_max_sync(0xffffffffu, row_lo);   // of this warp's rows
+      const int span = igc - row_lo;                               // keys row_lo .. row_lo + span are visible
       const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
       float m_used = -INFINITY, l = 0.f;   // l: this thread's half of the row sum
       bool ok = true;
@@ -782,12 +804,8 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         // S(j) complete; the commit also covers P V(j-1), so O may be rescaled below.
         if (!mbar_wait_warp(&s_full[t], n & 1, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
-        bool need_mask = (j == qi);
-        if (packed) {
-          const int k_first = j * TILE, k_last = min(j * TILE + TILE - 1, p.S - 1);
-          const int sid = segs[k_first];
-          need_mask = need_mask || sid != segs[k_last] || sid != segs[me.q0] || sid != segs[q_last];
-        }
+        const int c_first = j * TILE + ch * 64;   // this warp's keys of the block
+        const bool need_mask = c_first + 63 > me.q0 + quad * 32 || c_first < lo_max;
         // 32 of this thread's 64 scores, masked; called once per pass (the scores are read twice from
         // tensor memory rather than held in 64 registers across the exchange)
         auto load_scores = [&](int c, uint32_t (&sv)[32]) {
@@ -795,12 +813,9 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           tmem_wait_ld();
           if (need_mask) {
 #pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              const int jg = j * TILE + ch * 64 + c * 32 + e;
-              bool allowed = jg <= igc;
-              if (packed && allowed) allowed = segs[jg] == my_seg;
-              if (!allowed) sv[e] = 0xff800000u;  // -inf
-            }
+            for (int e = 0; e < 32; ++e)
+              if (static_cast<uint32_t>(c_first + c * 32 - row_lo + e) > static_cast<uint32_t>(span))
+                sv[e] = 0xff800000u;  // -inf
           }
         };
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -1227,8 +1242,8 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tmap_k64, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(a_ready);
     }
-    const int my_seg = packed ? segs[igc] : 0;
-    const int q_last = min(q0 + TILE - 1, p.S - 1);
+    const int row_lo = packed ? segment_first(segs, p.seg_start + static_cast<long long>(b) * p.S, igc) : 0;
+    const int lo_max = __reduce_max_sync(0xffffffffu, row_lo);   // of this warp's rows
     const long long ridx = (static_cast<long long>(b) * p.Hq + h) * p.S + igc;
     // -D and -L * log2(e) of this row.  All sixteen elementwise warps: the half-row sums are in shared memory
     asm volatile("bar.sync 1, %0;" ::"r"(32 * DQ_EW_WARPS) : "memory");
@@ -1245,13 +1260,10 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tmap_k64, const __grid_const
       const int buf = n & 1;
       if (!mbar_wait_warp(&sp_full[buf], (n >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
-      const int k_first = j * 64, k_last = min(j * 64 + 63, p.S - 1);
-      bool need_mask = k_first + 63 > q0;  // touches the diagonal (or runs past the sequence)
-      if (packed) {
-        const int sid = segs[k_first];
-        need_mask = need_mask || sid != segs[k_last] || sid != segs[q0] || sid != segs[q_last];
-      }
       const int c0 = part * DQ_CW;
+      const int c_first = j * 64 + c0;   // this warp's keys of the item
+      // some of them above the diagonal (or past the sequence), or in an earlier segment
+      const bool need_mask = c_first + DQ_CW - 1 > q0 + quad * 32 || c_first < lo_max;
       uint32_t sv[DQ_CW], dv[DQ_CW];
       tmem_ld_cols<DQ_CW>(tm_s + buf * 64 + lane_off + c0, sv);
       tmem_ld_cols<DQ_CW>(tm_dp + buf * 64 + lane_off + c0, dv);
@@ -1263,12 +1275,9 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tmap_k64, const __grid_const
         f2_unpack(f2_fma(f2_pack_bits(sv[e], sv[e + 1]), sc2, nl2_2), x0, x1);
         float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
         if (need_mask) {
-          const int jg = k_first + c0 + e;
-          bool a0 = jg <= igc, a1 = jg + 1 <= igc;
-          if (packed && a0) a0 = segs[jg] == my_seg;
-          if (packed && a1) a1 = segs[jg + 1] == my_seg;
-          if (!a0) p0 = 0.f;
-          if (!a1) p1 = 0.f;
+          const uint32_t rel = static_cast<uint32_t>(c_first - row_lo + e), span = static_cast<uint32_t>(igc - row_lo);
+          if (rel > span) p0 = 0.f;
+          if (rel + 1 > span) p1 = 0.f;
         }
         float y0, y1;
         f2_unpack(f2_mul(f2_pack(p0, p1), f2_add(f2_pack_bits(dv[e], dv[e + 1]), nd2)), y0, y1);
@@ -1342,10 +1351,9 @@ constexpr int DKV_CW = 64 / DKV_PARTS;
 constexpr int DKV_CTRL_WARPS = 3;                     // TMA producer and two MMA issuers
 constexpr int DKV_THREADS = 32 * DKV_CTRL_WARPS + 32 * DKV_EW_WARPS;
 constexpr int DKV_OCOLS = HD / DKV_PARTS;             // dK / dV columns each warp writes in the epilogue
-constexpr int DKV_SCAL_BYTES = DKV_EW_WARPS * 32 * 4;   // per warp: the segment ids of an item's queries (packed rows)
 constexpr int DKV_STAT_BYTES = 2048;                   // one 64-query block of the statistics tile
 constexpr int DKV_ONES_BYTES = 4096;                   // [2 chunks][128 rows][8 bf16]: a constant A operand
-constexpr int DKV_SMEM_BYTES = 2 * TILE_BYTES + DKV_RING * 2 * HALF_TILE_BYTES + 256 + DKV_SCAL_BYTES +
+constexpr int DKV_SMEM_BYTES = 2 * TILE_BYTES + DKV_RING * 2 * HALF_TILE_BYTES + 256 +
                                DKV_RING * DKV_STAT_BYTES + 2 * DKV_ONES_BYTES + 1024;
 
 template <int D>
@@ -1360,8 +1368,7 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q64, const __grid_cons
   uint8_t* v_sm = sm + TILE_BYTES;
   uint8_t* ring_sm = sm + 2 * TILE_BYTES;                        // stage s: Q at +0, dO at +16 KiB
   uint64_t* bars = reinterpret_cast<uint64_t*>(ring_sm + DKV_RING * 2 * HALF_TILE_BYTES);
-  uint8_t* scal_sm = ring_sm + DKV_RING * 2 * HALF_TILE_BYTES + 256;
-  uint8_t* stat_sm = scal_sm + DKV_SCAL_BYTES;                  // [DKV_RING][2048]
+  uint8_t* stat_sm = ring_sm + DKV_RING * 2 * HALF_TILE_BYTES + 256;   // [DKV_RING][2048]
   uint8_t* ones_sm = stat_sm + DKV_RING * DKV_STAT_BYTES;       // ones in columns 0-2, then ones in columns 3-5
   uint64_t* kv_full = bars;
   uint64_t* qdo_full = bars + 1;                 // [DKV_RING]
@@ -1399,16 +1406,25 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q64, const __grid_cons
     }
     mbar_init(acc_done, 2);
     *abort_flag = 0;
-    // last query block that can see any key of this block
-    int ihi = nqb - 1;
-    if (packed) {
-      const int k_last = min(k0 + TILE - 1, p.S - 1);
-      const int* starts = p.seg_start + static_cast<long long>(b) * p.S;
-      ihi = ilo;
-      while (ihi + 1 < nqb && starts[(ihi + 1) * 64] <= k_last) ++ihi;
-    }
-    *ihi_sm = ihi;
+    if (!packed) *ihi_sm = nqb - 1;
     fence_mbar_init();
+  }
+  if (packed && warp == 2) {
+    // last query block that can see any key of this block; 32 blocks per step (one thread walking them took as
+    // many dependent loads as the longest document has blocks)
+    const int k_last = min(k0 + TILE - 1, p.S - 1);
+    const int* starts = p.seg_start + static_cast<long long>(b) * p.S;
+    int ihi = ilo;
+    for (;;) {
+      const int i = ihi + 1 + lane;
+      const uint32_t past = __ballot_sync(0xffffffffu, i >= nqb || starts[i * 64] > k_last);
+      if (past != 0) {
+        ihi += __ffs(past) - 1;
+        break;
+      }
+      ihi += 32;
+    }
+    if (lane == 0) *ihi_sm = ihi;
   }
   if (warp == 1) {
     tmem_alloc(tmem_ptr, TMEM_COLS);
@@ -1525,10 +1541,11 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q64, const __grid_cons
     const int r = quad * 32 + lane;        // key row inside the block
     const int kg = k0 + r;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const int my_seg = (packed && kg < p.S) ? segs[kg] : 0;
-    // Warp-private staging of the segment ids of an item's queries (packed rows, masked items only), read
-    // back as broadcast vector loads.
-    int* my_sg = reinterpret_cast<int*>(scal_sm) + ew * 32;
+    // queries [kg, q_end) see this key; q_end does not decrease along the block
+    int q_end = p.S;
+    if (packed && kg < p.S) q_end = segment_end(segs, kg, min(p.S, (ihi + 1) * 64));
+    const uint32_t span = static_cast<uint32_t>(max(q_end - kg, 0));
+    const int end_min = __reduce_min_sync(0xffffffffu, q_end);
     const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
     bool ok = true;
     for (int t = 0; t < total; ++t) {
@@ -1537,16 +1554,8 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q64, const __grid_cons
       const int buf = t & 1;
       const uint32_t ph = (t >> 1) & 1;
       const int q_first = i * 64 + part * DKV_CW;
-      // Warp-uniform: can any (key, query) pair of this warp's 128 x DKV_CW sub-block be masked?
-      // Segment ids do not decrease along a row, so comparing the two ends covers the block.
-      bool need_mask = q_first < k0 + TILE - 1 || q_first + DKV_CW - 1 >= p.S;
-      if (packed && !need_mask) need_mask = segs[k0] != segs[q_first + DKV_CW - 1];
-      if (packed && need_mask) {
-        const int qmine = q_first + lane;
-        __syncwarp();   // the previous masked item's reads of the staging area are done
-        if (lane < DKV_CW) my_sg[lane] = qmine < p.S ? segs[qmine] : -1;
-        __syncwarp();
-      }
+      // Warp-uniform: can any (key, query) pair of this warp's 32 x DKV_CW sub-block be masked?
+      const bool need_mask = q_first < k0 + quad * 32 + 31 || q_first + DKV_CW > end_min;
       if (!mbar_wait_warp(&sp_full[buf], ph, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       uint32_t sv[DKV_CW], dv[DKV_CW];
@@ -1562,14 +1571,9 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q64, const __grid_cons
         float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
         if (need_mask) {
           // visible iff the query exists, is at or after this key, and shares its segment
-          bool a0 = kg <= q_first + e && q_first + e < p.S, a1 = kg <= q_first + e + 1 && q_first + e + 1 < p.S;
-          if (packed) {
-            const int2 sg = *reinterpret_cast<const int2*>(my_sg + e);
-            a0 = a0 && sg.x == my_seg;
-            a1 = a1 && sg.y == my_seg;
-          }
-          if (!a0) p0 = 0.f;
-          if (!a1) p1 = 0.f;
+          const uint32_t rel = static_cast<uint32_t>(q_first - kg + e);
+          if (rel >= span) p0 = 0.f;
+          if (rel + 1 >= span) p1 = 0.f;
         }
         float y0, y1;
         f2_unpack(f2_mul(f2_pack(p0, p1), f2_pack_bits(dv[e], dv[e + 1])), y0, y1);
