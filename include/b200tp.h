@@ -87,7 +87,9 @@ typedef struct b200tp_ce_args {
                        * 0x10000 expands the head inside the kernels whatever N is, 0x20000 always dequantises chunk
                        * by chunk into the workspace (default: the forward expands inside the kernel for N <= 512,
                        * where that is the cheaper form and needs no weight scratch, and is chunked beyond; the
-                       * backward is chunked at every N) */
+                       * backward is chunked at every N); 0x40000: fp32
+                       * operands of a dense head run on the tensor cores as three bf16 planes each at any size (by default
+                       * from 2^28 multiplications a contraction; impl = auto, D % 8 == 0) */
 } b200tp_ce_args;
 
 /* Forward: per-row log-sum-exp pieces and target logit over this call's vocab rows.  A 4-bit head is

@@ -65,7 +65,7 @@ def tied_head(embedding_weight: torch.Tensor, *, trainable: bool = False) -> Den
 # weight scratch), "tc_chunked" always dequantises chunk by chunk ahead of the dense kernels; plain "tc" /
 # "auto" lets the library choose (the forward inside the kernel up to 512 rows, everything else chunked).
 _TC_QUANT_IMPLS = ("tc_inline", "tc_chunked")
-_QUANT_RESERVED = {"tc_inline": 0x10000, "tc_chunked": 0x20000}
+_RESERVED = {"tc_inline": 0x10000, "tc_chunked": 0x20000, "split": 0x40000}   # "split": fp32 as bf16 planes at any size
 
 
 @dataclass(frozen=True)
@@ -98,8 +98,9 @@ def resolve_impl(*, head: HeadRef, dtype: torch.dtype, n: int, d: int | None = N
                  impl: str = "auto") -> Resolution:
     """Pick the kernel family; never falls back silently (core/loss.py:94-123).
 
-    "auto"/"kernel": tensor-core (tcgen05) kernels for bf16 with D % 8 == 0, CUDA-core
-    kernels for fp32 (exact fp32 accumulation) and odd D.  "tc"/"simt" force one family and
+    "auto"/"kernel": tensor-core (tcgen05) kernels for bf16 with D % 8 == 0; what resolves to "simt"
+    (fp32, odd D) the library serves at fp32 precision: fp32 with a dense head and D % 8 == 0 on the
+    tensor cores as three bf16 planes from some size on, the rest on the CUDA cores.  "tc"/"simt" force one family and
     raise `UnsupportedHeadError` when it cannot serve the input."""
     if n <= 0:
         raise LossInputError(f"n must be positive (hidden's row count); got n={n}")
@@ -118,7 +119,7 @@ def resolve_impl(*, head: HeadRef, dtype: torch.dtype, n: int, d: int | None = N
         return Resolution(impl, f"explicit impl={impl!r}")
     if tc_ok:
         return Resolution("tc", "bf16 operands: tcgen05 kernels")
-    return Resolution("simt", f"{dtype} operands: CUDA-core kernels with fp32 accumulation")
+    return Resolution("simt", f"{dtype} operands: fp32 sums, no bf16 rounding of an operand")
 
 
 def _validate_inputs(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, *,
@@ -222,8 +223,8 @@ def _ce_args(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, *, v_of
     a.dtype = _dtype_code(hidden.dtype)
     a.v_offset = v_offset
     a.ignore_index = ignore_index
-    a.impl = _lib.IMPL["tc" if impl in _TC_QUANT_IMPLS else impl]
-    a.reserved = _QUANT_RESERVED.get(impl, 0)
+    a.impl = _lib.IMPL["tc" if impl in _TC_QUANT_IMPLS else "auto" if impl == "split" else impl]
+    a.reserved = _RESERVED.get(impl, 0)
     if isinstance(head, DenseHead):
         w = head.weight.detach()
         if not w.is_contiguous():
@@ -564,7 +565,10 @@ def _prepare(hidden, head, targets, *, impl, validate_targets, ignore_index):
         hidden2 = hidden2.contiguous()
     targets2 = targets.reshape(-1).to(device=hidden.device, dtype=torch.int64).contiguous()
     res = resolve_impl(head=head, dtype=hidden2.dtype, n=hidden2.shape[0], d=d, impl=impl)
-    return hidden2, targets2, leading, res
+    # "auto" leaves what is not bf16 to the library: fp32 with a dense head runs on the tensor cores as bf16 planes,
+    # the rest on the CUDA cores; an explicit impl="simt" is always the CUDA cores.
+    native = "auto" if res.impl == "simt" and impl != "simt" else res.impl
+    return hidden2, targets2, leading, native
 
 
 def fused_linear_ce(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, *,
@@ -573,9 +577,9 @@ def fused_linear_ce(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, 
 
     hidden (N, D) or (B, S, D); targets integer, `ignore_index` rows masked.  Differentiable
     w.r.t. `hidden` through `nll` only."""
-    hidden2, targets2, leading, res = _prepare(hidden, head, targets, impl=impl,
+    hidden2, targets2, leading, native = _prepare(hidden, head, targets, impl=impl,
                                                validate_targets=validate_targets, ignore_index=ignore_index)
-    nll, lse, tgt = _apply(hidden2, targets2, head, ignore_index, res.impl)
+    nll, lse, tgt = _apply(hidden2, targets2, head, ignore_index, native)
     return nll.reshape(leading), lse.reshape(leading), tgt.reshape(leading)
 
 
@@ -588,9 +592,9 @@ def linear_cross_entropy(hidden: torch.Tensor, head: HeadRef, targets: torch.Ten
     if reduction not in ("none", "mean", "sum"):
         raise LossInputError(f"unknown reduction {reduction!r}; expected 'none', 'mean', or 'sum'")
     if reduction == "none":
-        hidden2, targets2, leading, res = _prepare(hidden, head, targets, impl=impl,
+        hidden2, targets2, leading, native = _prepare(hidden, head, targets, impl=impl,
                                                    validate_targets=validate_targets, ignore_index=ignore_index)
-        nll, _, _ = _apply(hidden2, targets2, head, ignore_index, res.impl)
+        nll, _, _ = _apply(hidden2, targets2, head, ignore_index, native)
         return nll.reshape(leading)
     return reduced_linear_cross_entropy(hidden, head, targets, impl=impl, reduction=reduction,
                                         ignore_index=ignore_index, validate_targets=validate_targets)[0]
@@ -604,6 +608,6 @@ def reduced_linear_cross_entropy(hidden: torch.Tensor, head: HeadRef, targets: t
     returns as `(loss, ntoks)` (adapters/mlx_lm.py:192-216).  Nothing on this path synchronises with the host."""
     if reduction not in ("mean", "sum"):
         raise LossInputError(f"unknown reduction {reduction!r}; expected 'mean' or 'sum'")
-    hidden2, targets2, _leading, res = _prepare(hidden, head, targets, impl=impl,
+    hidden2, targets2, _leading, native = _prepare(hidden, head, targets, impl=impl,
                                                 validate_targets=validate_targets, ignore_index=ignore_index)
-    return _apply_reduced(hidden2, targets2, head, ignore_index, res.impl, reduction == "mean")
+    return _apply_reduced(hidden2, targets2, head, ignore_index, native, reduction == "mean")

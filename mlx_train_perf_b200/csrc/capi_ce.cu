@@ -5,6 +5,7 @@
 #include "common.h"
 #include "linear_ce_grad.h"
 #include "linear_ce_simt.h"
+#include "linear_ce_split.h"
 #include "linear_ce_tc.h"
 
 namespace b200tp {
@@ -21,6 +22,11 @@ constexpr int64_t kTcChunkRowsMax = 16384;
 constexpr int64_t kTcChunkRowsMin = 2048;
 constexpr int64_t kTcScratchBytes = 512ll << 20;
 constexpr int64_t kSimtChunkRows = 4096;  // vocab rows per SIMT chunk
+// fp32 on the tensor cores: bound of what a chunk's planes take (weight rows, in the backward g too), as much as
+// the CUDA-core path's (N, 4096) fp32 tile at 8192 rows, and the chunk widths it may give
+constexpr int64_t kSplitScratchBytes = 128ll << 20;
+constexpr int64_t kSplitWorkMin = 1ll << 28;   // multiplications of a contraction (see pick_impl)
+constexpr int64_t kSplitChunkRowsMin = 2048, kSplitChunkRowsMax = 16384;
 
 // Vocab rows per tensor-core backward chunk for a shard of `v` rows.  The bound (the default above, or what
 // the caller asked for in `reserved`) trades scratch for launches: the (N, chunk) bf16 matrix of g is the
@@ -29,6 +35,7 @@ constexpr int64_t kSimtChunkRows = 4096;  // vocab rows per SIMT chunk
 // round trip).
 constexpr int kReservedInline = 0x10000;    // 4-bit head: expand inside the kernels whatever the row count
 constexpr int kReservedChunked = 0x20000;   // 4-bit head: dequantise chunk by chunk whatever the row count
+constexpr int kReservedSplit = 0x40000;     // fp32, dense head: the tensor cores whatever the size
 constexpr int64_t kInlineMaxRows = 512;     // default: the forward expands in the kernel up to this many rows of hidden
 
 int64_t tc_chunk_rows(const b200tp_ce_args* a, int64_t* num_chunks) {
@@ -81,11 +88,11 @@ int check_args(const b200tp_ce_args* a) {
   }
   if (a->impl != B200TP_IMPL_AUTO && a->impl != B200TP_IMPL_TC && a->impl != B200TP_IMPL_SIMT)
     return fail(B200TP_ERR_LOSS_INPUT, "unknown impl selector");
-  if (a->reserved < 0 || (a->reserved & ~(0xFFFF | kReservedInline | kReservedChunked)) != 0 ||
+  if (a->reserved < 0 || (a->reserved & ~(0xFFFF | kReservedInline | kReservedChunked | kReservedSplit)) != 0 ||
       (a->reserved & (kReservedInline | kReservedChunked)) == (kReservedInline | kReservedChunked))
     return fail(B200TP_ERR_LOSS_INPUT,
                 "reserved holds the backward chunk bound (low 16 bits, units of 256 vocab rows) and at most one of "
-                "the 4-bit dequantisation selectors 0x10000 / 0x20000");
+                "the 4-bit dequantisation selectors 0x10000 / 0x20000, and 0x40000");
   return B200TP_OK;
 }
 
@@ -122,7 +129,13 @@ QuantHead quant_head(const b200tp_ce_args* a, bool backward) {
   return quant_inline(a, backward) ? packed_head(a) : QuantHead{};
 }
 
-// 1 = tcgen05, 2 = SIMT, negative = refusal already recorded
+// 1 = tcgen05, 2 = SIMT, 3 = tcgen05 over the three bf16 planes of fp32 operands, negative = refusal already
+// recorded.  3 is the default for fp32 with a dense head: 2048 x 1024 x 32768 forward + backward 18.5 -> 2.57 ms, with
+// a third of the CUDA-core path's distance to float64 .  A trained fp32 head's backward stays on the CUDA
+// cores, and so do D % 8 != 0 (TMA strides), a 4-bit head under fp32 hidden states, and calls whose contraction is
+// under 2^28 multiplications: there the CUDA cores need no longer than the split's extra launches take (forward /
+// forward + backward, CUDA cores against split: 128 x 512 x 2000 65 / 259 against 90 / 282 us, 32 x 1024 x 32000
+// 1001 / 4151 against 173 / 430 us).
 int pick_impl(const b200tp_ce_args* a) {
   const bool tc_ok = a->dtype == B200TP_BF16 && a->d % 8 == 0;
   if (a->impl == B200TP_IMPL_SIMT) return 2;
@@ -138,7 +151,18 @@ int pick_impl(const b200tp_ce_args* a) {
     }
     return 1;
   }
-  return tc_ok ? 1 : 2;
+  if (tc_ok) return 1;
+  const bool large = (a->reserved & kReservedSplit) != 0 || a->n * a->v_local >= kSplitWorkMin / a->d;
+  return a->dtype == B200TP_F32 && a->quant_bits == 0 && a->d % 8 == 0 && large ? 3 : 2;
+}
+
+int64_t split_chunk_rows(const b200tp_ce_args* a, int64_t bytes_per_row, int64_t* num_chunks) {
+  int64_t bound = static_cast<int64_t>(a->reserved & 0xFFFF) * kCeTileCols;
+  if (bound <= 0)
+    bound = std::min(kSplitChunkRowsMax,
+                     std::max(kSplitChunkRowsMin, kSplitScratchBytes / bytes_per_row / kCeTileCols * kCeTileCols));
+  *num_chunks = ceil_div(a->v_local, bound);
+  return static_cast<int64_t>(align_up(static_cast<size_t>(ceil_div(a->v_local, *num_chunks)), kCeTileCols));
 }
 
 size_t elem_size(int dtype) { return dtype == B200TP_BF16 ? 2 : 4; }
@@ -152,6 +176,10 @@ struct FwdPlan {
   float* pm; float* ps; float* pt;
   void* deq;
   float* logits;
+  // fp32 on the tensor cores: the planes; `logits` overlays the weight's, `simt_chunk` columns of it fit
+  int* flag;
+  void* h3; void* w3;
+  int64_t simt_chunk;
   size_t bytes;
 };
 
@@ -179,10 +207,25 @@ FwdPlan plan_fwd(const b200tp_ce_args* a, void* ws) {
     p.pm = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
     p.ps = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
     p.pt = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
+  } else if (p.impl == 3) {
+    p.chunk = split_chunk_rows(a, 6ll * a->d, &p.num_chunks);
+    for (int64_t c = 0; c < p.num_chunks; ++c)
+      p.total_splits += 2 * ce_tc_fwd_splits(a->n, std::min<int64_t>(p.chunk, a->v_local - c * p.chunk));
+    p.flag = b.take<int>(1);
+    p.h3 = b.take<char>(static_cast<size_t>(a->n) * a->d * 6);
+    const size_t planes = static_cast<size_t>(p.chunk) * a->d * 6;
+    const size_t least = static_cast<size_t>(a->n) * std::min<int64_t>(kSimtChunkRows, a->v_local) * 4;
+    p.w3 = b.take<char>(std::max(planes, least));
+    p.logits = static_cast<float*>(p.w3);
+    p.simt_chunk = std::min<int64_t>(a->v_local, static_cast<int64_t>(std::max(planes, least) / 4) / a->n);
+    p.pm = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
+    p.ps = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
+    p.pt = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
   } else {
     p.chunk = std::min<int64_t>(kSimtChunkRows, a->v_local);
     p.num_chunks = ceil_div(a->v_local, p.chunk);
     p.logits = b.take<float>(static_cast<size_t>(a->n) * p.chunk);
+    p.simt_chunk = p.chunk;
     if (a->quant_bits != 0) p.deq = b.take<char>(static_cast<size_t>(p.chunk) * a->d * elem_size(a->dtype));
   }
   p.bytes = align_up(b.off, 256);
@@ -197,6 +240,12 @@ struct BwdPlan {
   float* logits;  // simt: f32 (n, chunk)
   float* acc;     // f32 (n, d) when the output is bf16 and must be accumulated in fp32
   void* deq;
+  // fp32 on the tensor cores: the planes, `shares` partial sums of d_hidden; `logits` overlays g's planes
+  int* flag;
+  void* h3; void* w3; void* g3;
+  float* shares_acc;
+  int shares;
+  int64_t simt_chunk;
   size_t bytes;
 };
 
@@ -211,10 +260,22 @@ BwdPlan plan_bwd(const b200tp_ce_args* a, int out_dtype, void* ws) {
     p.g = b.take<char>(static_cast<size_t>(a->n) * p.ldg * 2);
     if (out_dtype == B200TP_BF16 && p.num_chunks > 1) p.acc = b.take<float>(static_cast<size_t>(a->n) * a->d);
     if (a->quant_bits != 0 && !quant_inline(a, true)) p.deq = b.take<char>(static_cast<size_t>(p.chunk) * a->d * 2);
+  } else if (p.impl == 3) {
+    p.chunk = split_chunk_rows(a, 6ll * (a->n + a->d), &p.num_chunks);
+    p.ldg = static_cast<int>(p.chunk);
+    p.shares = ce_split_dh_shares(a->n, a->d, p.chunk);
+    p.flag = b.take<int>(1);
+    p.h3 = b.take<char>(static_cast<size_t>(a->n) * a->d * 6);
+    p.w3 = b.take<char>(static_cast<size_t>(p.chunk) * a->d * 6);
+    p.g3 = b.take<char>(static_cast<size_t>(a->n) * p.chunk * 6);
+    p.shares_acc = b.take<float>(static_cast<size_t>(p.shares) * a->n * a->d);
+    p.logits = static_cast<float*>(p.g3);
+    p.simt_chunk = std::min<int64_t>(a->v_local, p.chunk * 6 / 4);
   } else {
     p.chunk = std::min<int64_t>(kSimtChunkRows, a->v_local);
     p.num_chunks = ceil_div(a->v_local, p.chunk);
     p.logits = b.take<float>(static_cast<size_t>(a->n) * p.chunk);
+    p.simt_chunk = p.chunk;
     if (out_dtype == B200TP_BF16) p.acc = b.take<float>(static_cast<size_t>(a->n) * a->d);
     if (a->quant_bits != 0) p.deq = b.take<char>(static_cast<size_t>(p.chunk) * a->d * elem_size(a->dtype));
   }
@@ -339,10 +400,31 @@ int b200tp_linear_ce_fwd(const b200tp_ce_args* a, float* row_max, float* row_sum
                           a->ignore_index, row_max, row_sumexp, tgt_logit, lse, nll, stream);
   }
 
-  // SIMT: running triples live directly in the caller's output arrays.
-  for (int64_t c = 0; c < p.num_chunks; ++c) {
-    const int64_t r0 = c * p.chunk;
-    const int64_t w = std::min<int64_t>(p.chunk, a->v_local - r0);
+  if (p.impl == 3) {
+    B200TP_CUDA_OK(cudaMemsetAsync(p.flag, 0, sizeof(int), stream));
+    rc = ce_split_planes(static_cast<const float*>(a->hidden), a->n * a->d, p.h3, p.flag, stream);
+    if (rc) return rc;
+    int64_t slot = 0;
+    for (int64_t c = 0; c < p.num_chunks; ++c) {
+      const int64_t r0 = c * p.chunk;
+      const int64_t w = std::min<int64_t>(p.chunk, a->v_local - r0);
+      rc = ce_split_planes(static_cast<const float*>(a->weight) + r0 * a->d, w * a->d, p.w3, p.flag, stream);
+      if (rc) return rc;
+      const int splits = ce_tc_fwd_splits(a->n, w);
+      rc = ce_split_fwd(p.h3, p.w3, a->n, a->d, w, a->v_offset + r0, a->targets, a->ignore_index, splits,
+                        p.pm + slot * a->n, p.ps + slot * a->n, p.pt + slot * a->n, stream, status);
+      if (rc) return rc;
+      slot += 2 * splits;
+    }
+    rc = launch_combine(p.pm, p.ps, p.pt, a->n, static_cast<int>(p.total_splits), a->n, a->targets, a->ignore_index,
+                        row_max, row_sumexp, tgt_logit, lse, nll, stream);
+    if (rc) return rc;
+  }
+
+  // SIMT: running triples live directly in the caller's output arrays.  After the split path: only where it met
+  // values its planes cannot hold.
+  for (int64_t r0 = 0; r0 < a->v_local; r0 += p.simt_chunk) {
+    const int64_t w = std::min<int64_t>(p.simt_chunk, a->v_local - r0);
     const void* wc;
     if (a->quant_bits == 0) {
       wc = static_cast<const char*>(a->weight) + static_cast<size_t>(r0) * a->d * elem_size(a->dtype);
@@ -353,11 +435,11 @@ int b200tp_linear_ce_fwd(const b200tp_ce_args* a, float* row_max, float* row_sum
       wc = p.deq;
     }
     rc = ce_simt_fwd_chunk(a->hidden, wc, a->dtype, a->n, a->d, w, a->v_offset + r0, a->targets, a->ignore_index,
-                           p.logits, row_max, row_sumexp, tgt_logit, c == 0 ? 1 : 0, stream);
+                           p.logits, row_max, row_sumexp, tgt_logit, r0 == 0 ? 1 : 0, stream, p.flag);
     if (rc) return rc;
   }
   return launch_combine(row_max, row_sumexp, tgt_logit, a->n, 1, a->n, a->targets, a->ignore_index, nullptr, nullptr,
-                        tgt_logit, lse, nll, stream);
+                        tgt_logit, lse, nll, stream, p.flag);
 }
 
 int b200tp_linear_ce_combine(const float* parts, int32_t num_parts, int64_t n, const int64_t* targets,
@@ -479,13 +561,33 @@ static int bwd_impl(const b200tp_ce_args* a, const float* lse, const float* cota
     return B200TP_OK;
   }
 
-  // CUDA-core path: not staged (everything runs in stage 0)
+  // The other two paths are not staged (everything runs in stage 0).
   if (rows_done != nullptr) *rows_done = a->n;
   if (stage > 0) return B200TP_OK;
+  if (p.impl == 3 && d_weight == nullptr) {
+    B200TP_CUDA_OK(cudaMemsetAsync(p.flag, 0, sizeof(int), stream));
+    rc = ce_split_planes(static_cast<const float*>(a->hidden), a->n * a->d, p.h3, p.flag, stream);
+    if (rc) return rc;
+    for (int64_t c = 0; c < p.num_chunks; ++c) {
+      const int64_t r0 = c * p.chunk;
+      const int64_t w = std::min<int64_t>(p.chunk, a->v_local - r0);
+      rc = ce_split_planes(static_cast<const float*>(a->weight) + r0 * a->d, w * a->d, p.w3, p.flag, stream);
+      if (rc) return rc;
+      rc = ce_split_bwd_g(p.h3, p.w3, a->n, a->d, w, a->v_offset + r0, a->targets, a->ignore_index, lse, cotangent,
+                          ce_tc_fwd_splits(a->n, w), p.g3, p.ldg, p.flag, stream, status);
+      if (rc) return rc;
+      rc = ce_split_dh(p.g3, p.ldg, p.w3, a->n, a->d, w, p.shares, p.shares_acc, c > 0, stream, status);
+      if (rc) return rc;
+    }
+    // d_hidden is only touched once it is known that the planes held every value
+    rc = ce_split_sum(p.shares_acc, p.shares, a->n * a->d, static_cast<float*>(d_hidden), accumulate, p.flag, stream);
+    if (rc) return rc;
+  } else {
+    p.flag = nullptr;   // the CUDA-core path, unconditionally
+  }
   float* acc = out_f32 ? static_cast<float*>(d_hidden) : p.acc;
-  for (int64_t c = 0; c < p.num_chunks; ++c) {
-    const int64_t r0 = c * p.chunk;
-    const int64_t w = std::min<int64_t>(p.chunk, a->v_local - r0);
+  for (int64_t r0 = 0; r0 < a->v_local; r0 += p.simt_chunk) {
+    const int64_t w = std::min<int64_t>(p.simt_chunk, a->v_local - r0);
     const void* wc;
     if (a->quant_bits == 0) {
       wc = static_cast<const char*>(a->weight) + static_cast<size_t>(r0) * a->d * elem_size(a->dtype);
@@ -495,9 +597,9 @@ static int bwd_impl(const b200tp_ce_args* a, const float* lse, const float* cota
       if (rc) return rc;
       wc = p.deq;
     }
-    const int acc_flag = (c > 0 || (out_f32 && accumulate)) ? 1 : 0;
+    const int acc_flag = (r0 > 0 || (out_f32 && accumulate)) ? 1 : 0;
     rc = ce_simt_bwd_chunk(a->hidden, wc, a->dtype, a->n, a->d, w, a->v_offset + r0, a->targets, a->ignore_index, lse,
-                           cotangent, p.logits, acc, acc_flag, stream);
+                           cotangent, p.logits, acc, acc_flag, stream, p.flag);
     if (rc) return rc;
     if (d_weight != nullptr) {
       void* block = static_cast<char*>(d_weight) + static_cast<size_t>(r0) * a->d * elem_size(a->dtype);

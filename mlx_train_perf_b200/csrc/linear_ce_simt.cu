@@ -30,7 +30,8 @@ constexpr int TK = 16;
 template <typename TA, typename TB>
 __global__ void __launch_bounds__(256)
 gemm_nt_kernel(const TA* __restrict__ A, long long lda, const TB* __restrict__ B, long long ldb, float* __restrict__ C,
-               long long ldc, int M, int Nn, int K) {
+               long long ldc, int M, int Nn, int K, const int* run_if_set) {
+  if (run_if_set != nullptr && *run_if_set == 0) return;
   __shared__ float As[TK][TS + 1];
   __shared__ float Bs[TK][TS + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -79,7 +80,9 @@ gemm_nt_kernel(const TA* __restrict__ A, long long lda, const TB* __restrict__ B
 template <typename TB>
 __global__ void __launch_bounds__(256)
 gemm_nn_acc_kernel(const float* __restrict__ A, long long lda, const TB* __restrict__ B, long long ldb,
-                   float* __restrict__ C, long long ldc, int M, int Nn, int K, int accumulate) {
+                   float* __restrict__ C, long long ldc, int M, int Nn, int K, int accumulate,
+                   const int* run_if_set) {
+  if (run_if_set != nullptr && *run_if_set == 0) return;
   __shared__ float As[TK][TS + 1];
   __shared__ float Bs[TK][TS + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -193,7 +196,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 __global__ void __launch_bounds__(256)
 rows_fwd_kernel(const float* __restrict__ logits, long long ld, int n_rows, int width, long long vocab_id0,
                 const long long* __restrict__ targets, long long ignore_index, float* run_m, float* run_s,
-                float* run_t, int first) {
+                float* run_t, int first, const int* run_if_set) {
+  if (run_if_set != nullptr && *run_if_set == 0) return;
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= n_rows) return;
@@ -226,7 +230,8 @@ template <bool ROUND_BF16>
 __global__ void __launch_bounds__(256)
 rows_bwd_kernel(float* __restrict__ logits, long long ld, int n_rows, int width, long long vocab_id0,
                 const long long* __restrict__ targets, long long ignore_index, const float* __restrict__ lse,
-                const float* __restrict__ ct) {
+                const float* __restrict__ ct, const int* run_if_set) {
+  if (run_if_set != nullptr && *run_if_set == 0) return;
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= n_rows) return;
@@ -260,7 +265,8 @@ __global__ void __launch_bounds__(32 * kCombineGroups)
 combine_kernel(const float* __restrict__ pm, const float* __restrict__ ps, const float* __restrict__ pt,
                long long stride, int parts, long long n, const long long* __restrict__ targets,
                long long ignore_index, float* row_max, float* row_sumexp, float* tgt_out, float* lse_out,
-               float* nll_out) {
+               float* nll_out, const int* run_if_set) {
+  if (run_if_set != nullptr && *run_if_set == 0) return;
   __shared__ float s_m[kCombineGroups][32], s_s[kCombineGroups][32], s_t[kCombineGroups][32];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const long long row = static_cast<long long>(blockIdx.x) * 32 + lane;
@@ -452,12 +458,12 @@ void launch_dequant_typed(const uint32_t* w_q, const void* scales, const void* b
 
 int launch_combine(const float* pm, const float* ps, const float* pt, int64_t stride, int parts, int64_t n,
                    const int64_t* targets, int64_t ignore_index, float* row_max, float* row_sumexp, float* tgt_out,
-                   float* lse_out, float* nll_out, cudaStream_t stream) {
+                   float* lse_out, float* nll_out, cudaStream_t stream, const int* run_if_set) {
   if (n <= 0) return B200TP_OK;
   const unsigned blocks = static_cast<unsigned>(ceil_div(n, 32));
   combine_kernel<<<blocks, 32 * kCombineGroups, 0, stream>>>(pm, ps, pt, stride, parts, n,
                                                  reinterpret_cast<const long long*>(targets), ignore_index, row_max,
-                                                 row_sumexp, tgt_out, lse_out, nll_out);
+                                                 row_sumexp, tgt_out, lse_out, nll_out, run_if_set);
   B200TP_CUDA_OK(cudaGetLastError());
   return B200TP_OK;
 }
@@ -500,56 +506,57 @@ int launch_dequant_int4(const uint32_t* w_q, const void* scales, const void* bia
 
 int ce_simt_fwd_chunk(const void* hidden, const void* w_chunk, int dtype, int64_t n, int d, int64_t width,
                       int64_t vocab_id0, const int64_t* targets, int64_t ignore_index, float* logits_ws, float* run_m,
-                      float* run_s, float* run_t, int first, cudaStream_t stream) {
+                      float* run_s, float* run_t, int first, cudaStream_t stream, const int* run_if_set) {
   dim3 grid(static_cast<unsigned>(ceil_div(width, TS)), static_cast<unsigned>(ceil_div(n, TS)));
   if (dtype == B200TP_F32)
     gemm_nt_kernel<float, float><<<grid, 256, 0, stream>>>(static_cast<const float*>(hidden), d,
                                                            static_cast<const float*>(w_chunk), d, logits_ws, width,
-                                                           static_cast<int>(n), static_cast<int>(width), d);
+                                                           static_cast<int>(n), static_cast<int>(width), d, run_if_set);
   else
     gemm_nt_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(hidden), d, static_cast<const __nv_bfloat16*>(w_chunk), d, logits_ws, width,
-        static_cast<int>(n), static_cast<int>(width), d);
+        static_cast<int>(n), static_cast<int>(width), d, run_if_set);
   B200TP_CUDA_OK(cudaGetLastError());
   rows_fwd_kernel<<<static_cast<unsigned>(ceil_div(n, 8)), 256, 0, stream>>>(
       logits_ws, width, static_cast<int>(n), static_cast<int>(width), vocab_id0,
-      reinterpret_cast<const long long*>(targets), ignore_index, run_m, run_s, run_t, first);
+      reinterpret_cast<const long long*>(targets), ignore_index, run_m, run_s, run_t, first, run_if_set);
   B200TP_CUDA_OK(cudaGetLastError());
   return B200TP_OK;
 }
 
 int ce_simt_bwd_chunk(const void* hidden, const void* w_chunk, int dtype, int64_t n, int d, int64_t width,
                       int64_t vocab_id0, const int64_t* targets, int64_t ignore_index, const float* lse,
-                      const float* ct, float* logits_ws, float* dh_acc, int accumulate, cudaStream_t stream) {
+                      const float* ct, float* logits_ws, float* dh_acc, int accumulate, cudaStream_t stream,
+                      const int* run_if_set) {
   dim3 grid(static_cast<unsigned>(ceil_div(width, TS)), static_cast<unsigned>(ceil_div(n, TS)));
   dim3 grid2(static_cast<unsigned>(ceil_div(d, TS)), static_cast<unsigned>(ceil_div(n, TS)));
   const unsigned row_blocks = static_cast<unsigned>(ceil_div(n, 8));
   if (dtype == B200TP_F32) {
     gemm_nt_kernel<float, float><<<grid, 256, 0, stream>>>(static_cast<const float*>(hidden), d,
                                                            static_cast<const float*>(w_chunk), d, logits_ws, width,
-                                                           static_cast<int>(n), static_cast<int>(width), d);
+                                                           static_cast<int>(n), static_cast<int>(width), d, run_if_set);
     B200TP_CUDA_OK(cudaGetLastError());
     rows_bwd_kernel<false><<<row_blocks, 256, 0, stream>>>(logits_ws, width, static_cast<int>(n),
                                                            static_cast<int>(width), vocab_id0,
                                                            reinterpret_cast<const long long*>(targets), ignore_index,
-                                                           lse, ct);
+                                                           lse, ct, run_if_set);
     B200TP_CUDA_OK(cudaGetLastError());
     gemm_nn_acc_kernel<float><<<grid2, 256, 0, stream>>>(logits_ws, width, static_cast<const float*>(w_chunk), d,
                                                          dh_acc, d, static_cast<int>(n), d, static_cast<int>(width),
-                                                         accumulate);
+                                                         accumulate, run_if_set);
   } else {
     gemm_nt_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(hidden), d, static_cast<const __nv_bfloat16*>(w_chunk), d, logits_ws, width,
-        static_cast<int>(n), static_cast<int>(width), d);
+        static_cast<int>(n), static_cast<int>(width), d, run_if_set);
     B200TP_CUDA_OK(cudaGetLastError());
     rows_bwd_kernel<true><<<row_blocks, 256, 0, stream>>>(logits_ws, width, static_cast<int>(n),
                                                           static_cast<int>(width), vocab_id0,
                                                           reinterpret_cast<const long long*>(targets), ignore_index,
-                                                          lse, ct);
+                                                          lse, ct, run_if_set);
     B200TP_CUDA_OK(cudaGetLastError());
     gemm_nn_acc_kernel<__nv_bfloat16><<<grid2, 256, 0, stream>>>(
         logits_ws, width, static_cast<const __nv_bfloat16*>(w_chunk), d, dh_acc, d, static_cast<int>(n), d,
-        static_cast<int>(width), accumulate);
+        static_cast<int>(width), accumulate, run_if_set);
   }
   B200TP_CUDA_OK(cudaGetLastError());
   return B200TP_OK;

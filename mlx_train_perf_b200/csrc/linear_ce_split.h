@@ -1,0 +1,34 @@
+// Launchers of the fp32 linear cross-entropy on the tensor cores (linear_ce_split.cu).
+//
+// Operands are planes: an fp32 matrix (rows, cols) as (3, rows, cols) bf16 whose sum it is.
+#pragma once
+
+#include "common.h"
+
+namespace b200tp {
+
+// x (count values, a multiple of 8) -> planes; sets *flag when a value has no such form (inf, NaN, or so near the
+// largest fp32 that bf16 rounds it to infinity).
+int ce_split_planes(const float* x, int64_t count, void* planes, int* flag, cudaStream_t stream);
+
+// Forward partials of one vocab chunk (`width` rows from `vocab_id0`): 2 * splits triples per row.
+int ce_split_fwd(const void* h3, const void* w3, int64_t n, int d, int64_t width, int64_t vocab_id0,
+                 const int64_t* targets, int64_t ignore_index, int splits, float* pm, float* ps, float* pt,
+                 cudaStream_t stream, int* status);
+
+// g3 (3, n, ldg) = (exp(z - lse) - onehot) * ct of one chunk, zero past its width up to the next multiple of 256;
+// sets *flag when a value is not finite.
+int ce_split_bwd_g(const void* h3, const void* w3, int64_t n, int d, int64_t width, int64_t vocab_id0,
+                   const int64_t* targets, int64_t ignore_index, const float* lse, const float* ct, int splits,
+                   void* g3, int ldg, int* flag, cudaStream_t stream, int* status);
+
+// out (ksplit shares of (n, d) fp32, `keep`: added to) = g @ w over the chunk.
+int ce_split_dh_shares(int64_t n, int d, int64_t width);
+int ce_split_dh(const void* g3, int ldg, const void* w3, int64_t n, int d, int64_t width, int ksplit, float* out,
+                int keep, cudaStream_t stream, int* status);
+
+// out = (keep ? out : 0) + sum of the shares in index order; nothing while *skip_if_set is set.
+int ce_split_sum(const float* acc, int shares, int64_t count, float* out, int keep, const int* skip_if_set,
+                 cudaStream_t stream);
+
+}  // namespace b200tp

@@ -1,6 +1,8 @@
 """Packed rows whose document boundaries fall on and around the kernels' blocks, tensor-core kernels against the
 CUDA-core ones.  Both round O and the gradients to bf16 once; the tensor-core kernels also round P and dS to bf16
-(2^-9 of each term, independent): 2^-8 of the largest value covers the two, 2e-2 is the class the parity tests use."""
+(2^-9 of each term, independent): 2^-8 of the largest value covers the two, 2e-2 is the class the parity tests use.
+A one-token document's dS = P (dP - D) is zero; formed from two fp32 sums of 64 products of up to 4 x 4 it is off by
+64 x 16 x 2^-24 = 6e-5 at most, times |k| <= 4 and the scale 1/8: 3e-5 absolute."""
 import pytest
 import torch
 
@@ -32,8 +34,8 @@ def test_boundaries(cuda_device, lengths, impl):
     want = _run(q, k, v, d_o, seg, "simt")
     got = _run(q, k, v, d_o, seg, impl)
     for a, b in zip(got, want):
-        assert (a - b).abs().max() <= 2e-2 * b.abs().max()
+        assert (a - b).abs().max() <= 2e-2 * b.abs().max() + 3e-5
     # starts that are only a lower bound (nothing skipped): the ids alone decide
     loose = PackedMask(seg_id=seg.seg_id, seg_start=torch.zeros_like(seg.seg_start))
     for a, b in zip(_run(q, k, v, d_o, loose, impl), got):
-        assert (a - b).abs().max() <= 2e-2 * b.abs().max()
+        assert (a - b).abs().max() <= 2e-2 * b.abs().max() + 3e-5

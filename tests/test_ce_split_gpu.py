@@ -1,0 +1,97 @@
+"""fp32 losses on the tensor cores (three bf16 planes an operand) against fp64 and against the CUDA-core kernels.
+
+Bounds: a logit is a sum of D exact products, dropped terms below 2^-25 of each; its segments of 128 round towards
+zero at most nine times at 2^-23 of the running sum, and there are D / 128 additions of them: (9 + D / 128) 2^-23 of the
+largest partial sum, |h| |w| at most.  Probabilities move by that, d_hidden rows by it times sum_v |g_v| |W_v|, plus
+the same for the second contraction over V."""
+import math
+
+import pytest
+import torch
+
+from mlx_train_perf_b200.core import loss as L
+from mlx_train_perf_b200.core.loss import DenseHead
+from oracle import linear_ce as oc
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(n, d, v):
+    g = torch.Generator().manual_seed(n + d + v)
+    w = torch.randn(v, d, generator=g) * d ** -0.5
+    h = torch.randn(n, d, generator=g)
+    t = torch.randint(0, v, (n,), generator=g)
+    h += torch.linspace(0, 20, n)[:, None] * w[t]
+    t[2::7] = -100
+    return h, w, t
+
+
+def _run(dev, h, w, t, ct, impl="split"):
+    h, t, head = h.to(dev), t.to(dev), DenseHead(w.to(dev), trainable=False)
+    _, _, tgt, lse, nll = L.ce_forward_raw(h, head, t, impl=impl)
+    dh = L.ce_backward_raw(h, head, t, lse, ct.to(dev), impl=impl)
+    L.check_device_status()
+    return nll.cpu(), lse.cpu(), tgt.cpu(), dh.cpu()
+
+
+# rows, hidden sizes and vocabularies around tiles, k blocks and accumulator segments; several chunks; shares
+@pytest.mark.parametrize(("n", "d", "v"), [(1, 8, 1), (1, 64, 257), (127, 72, 255), (128, 128, 512), (129, 136, 4099),
+                                           (60, 1024, 17000), (300, 264, 2500), (33, 2056, 600)])
+def test_against_fp64(cuda_device, n, d, v):
+    h, w, t = _inputs(n, d, v)
+    ct = torch.linspace(-1, 1.5, n)
+    nll, lse, tgt, dh = _run(cuda_device, h, w, t, ct)
+    r_nll, r_lse, r_tgt = oc.naive_linear_ce(h, w, t, dtype=torch.float64)
+    r_dh, _ = oc.chunked_backward(h, w, t, r_lse, ct.double(), chunk_size=4096, dtype=torch.float64)
+    rows = h.double().norm(dim=1) * w.double().norm(dim=1).max()
+    z = (9 + d / 128) * 2.0 ** -23 * rows + 2.0 ** -22 * (1 + r_lse.abs())
+    ok = t != -100
+    assert ((lse.double() - r_lse).abs() <= z).all()
+    assert ((tgt.double() - r_tgt).abs() <= z)[ok].all() and ((nll.double() - r_nll).abs() <= 2 * z)[ok].all()
+    assert (nll[~ok] == 0).all() and (dh[~ok] == 0).all()
+    wn = w.double().norm(dim=1).max()
+    bound = ct.double().abs() * wn * 2 * (z + (9 + v / 128) * 2.0 ** -23)
+    assert ((dh.double() - r_dh).norm(dim=1) <= bound + 1e-12).all()
+    # no less precise than the CUDA cores, up to the last rounding of the results
+    s_nll, s_lse, _, s_dh = _run(cuda_device, h, w, t, ct, impl="simt")
+    assert (lse.double() - r_lse).norm() <= (s_lse.double() - r_lse).norm() + 2.0 ** -24 * r_lse.norm()
+    assert (dh.double() - r_dh).norm() <= (s_dh.double() - r_dh).norm() + 2.0 ** -24 * r_dh.norm()
+
+
+def test_accumulates_into_fp32(cuda_device):
+    h, w, t = _inputs(70, 264, 5000)
+    dev, ct = cuda_device, torch.ones(70)
+    head = DenseHead(w.to(dev), trainable=False)
+    out = L.ce_forward_buffer(h.to(dev), head, t.to(dev), impl="split")
+    base = torch.randn(70 * 264 + 1, device=dev)[1:].reshape(70, 264)      # not 16-byte aligned
+    buf = torch.empty(70 * 264 + 1, device=dev)[1:].reshape(70, 264).copy_(base)
+    one = L.ce_backward_raw(h.to(dev), head, t.to(dev), out[3], ct.to(dev), impl="split")
+    L.ce_backward_raw(h.to(dev), head, t.to(dev), out[3], ct.to(dev), out=buf, accumulate=True,
+                      out_dtype=torch.float32, impl="split")
+    assert torch.equal(buf, base + one)        # added once, after the shares' own sum
+
+
+@pytest.mark.parametrize("what", ["inf", "nan", "largest", "cotangent"])
+def test_values_without_planes(cuda_device, what):
+    """bf16 cannot hold them: the CUDA-core kernels give the result, bit for bit theirs."""
+    h, w, t = _inputs(40, 64, 700)
+    ct = torch.ones(40)
+    if what == "inf":
+        w[5] = 0
+        w[5, 3] = -math.inf
+        h[:, 3] = h[:, 3].abs() + 0.1
+    elif what == "nan":
+        h[7, 2] = math.nan
+    elif what == "largest":
+        w[9] = 0
+        w[9, 1] = -3.4e38
+        h[:, 1] = h[:, 1].abs().clamp(max=0.9)
+    else:
+        ct[3] = math.inf
+    for a, b in zip(_run(cuda_device, h, w, t, ct), _run(cuda_device, h, w, t, ct, impl="simt")):
+        if what == "cotangent" and a.ndim == 1:
+            continue                      # the forward saw no such value
+        if what == "cotangent":           # nor did the saved lse come from the same kernels
+            assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+            continue
+        assert torch.equal(a.nan_to_num(7e7), b.nan_to_num(7e7))
