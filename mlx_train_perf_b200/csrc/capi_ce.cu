@@ -38,11 +38,19 @@ constexpr int kReservedChunked = 0x20000;   // 4-bit head: dequantise chunk by c
 constexpr int kReservedSplit = 0x40000;     // fp32, dense head: the tensor cores whatever the size
 constexpr int64_t kInlineMaxRows = 512;     // default: the forward expands in the kernel up to this many rows of hidden
 
-int64_t tc_chunk_rows(const b200tp_ce_args* a, int64_t* num_chunks) {
+// `grow` (the forward that also forms the gradient, dense heads): few rows take wider chunks, up to the scratch that
+// 8192 rows use anyway.  A chunk ends in a partly filled wave of tiles and an fp32 round trip of d_hidden in each of
+// its two GEMMs: at 1000 x 4096 x 151936 ten chunks make 40 tile times of logits out of 32.1 full waves, two make
+// 34 (training step 2.63 -> 2.30 ms; 60 x 1024 x 32768 in one chunk instead of two: GPU time 94 -> 58 us).
+constexpr int64_t kGrowScratchBytes = 256ll << 20;
+
+int64_t tc_chunk_rows(const b200tp_ce_args* a, int64_t* num_chunks, bool grow = false) {
   int64_t bound = static_cast<int64_t>(a->reserved & 0xFFFF) * kCeTileCols;
   if (bound <= 0) {
     const int64_t fit = kTcScratchBytes / (2 * std::max<int64_t>(a->n, 1)) / kCeTileCols * kCeTileCols;
     bound = std::min(kTcChunkRowsMax, std::max(kTcChunkRowsMin, fit));
+    if (grow && a->quant_bits == 0)
+      bound = std::max(bound, kGrowScratchBytes / (2 * a->n) / kCeTileCols * kCeTileCols);
   }
   const int64_t nc = ceil_div(a->v_local, bound);
   *num_chunks = nc;
@@ -283,9 +291,9 @@ BwdPlan plan_bwd(const b200tp_ce_args* a, int out_dtype, void* ws) {
   return p;
 }
 
-// Forward that also forms the gradient: what it leaves for the backward (`state`) and its scratch.  The chunks
-// are the recomputing backward's, so the scratch is that backward's: one (N, chunk) bf16 tile, one dequantised
-// chunk of a 4-bit head, plus the forward's partial triples.
+// Forward that also forms the gradient: what it leaves for the backward (`state`) and its scratch.  The scratch
+// is like the recomputing backward's: one (N, chunk) bf16 tile, one dequantised chunk of a 4-bit head, plus the
+// forward's partial triples.
 struct GradPlan {
   bool ok;
   int64_t chunk, num_chunks;
@@ -308,7 +316,7 @@ GradPlan plan_grad(const b200tp_ce_args* a, void* state, void* ws) {
   GradPlan p{};
   p.ok = pick_impl(a) == 1 && a->impl != B200TP_IMPL_SIMT && (a->reserved & kReservedInline) == 0;
   if (!p.ok) return p;
-  p.chunk = tc_chunk_rows(a, &p.num_chunks);
+  p.chunk = tc_chunk_rows(a, &p.num_chunks, true);
   p.shares = ce_tc_dh_ksplit(a->n, a->d, static_cast<int>(p.chunk));
   Bump st(state);
   p.overflow = st.take<int>(1);
