@@ -272,6 +272,11 @@ size_t b200tp_flash_bwd_workspace_bytes(const b200tp_attn_args* a);
 int b200tp_flash_bwd(const b200tp_attn_args* a, const void* q, const void* k, const void* v, const void* o,
                      const float* lse, const void* d_o, void* dq, void* dk, void* dv, void* workspace,
                      size_t workspace_bytes, void* stream, int* status);
+/* The same with d_o's own element strides over (B, H, S), unit over d (null: o's).  Tensor-core path only: multiples
+ * of 8, d_o 16-byte aligned, no two elements at one address. */
+int b200tp_flash_bwd_strided(const b200tp_attn_args* a, const void* q, const void* k, const void* v, const void* o,
+                             const float* lse, const void* d_o, const int64_t* d_o_stride, void* dq, void* dk, void* dv,
+                             void* workspace, size_t workspace_bytes, void* stream, int* status);
 
 /* ---------------------------------------------------------------------------------------
  * Attention pre-step: per-head RMSNorm (optional) + rotary position embedding

@@ -119,6 +119,13 @@ size_t b200tp_flash_bwd_workspace_bytes(const b200tp_attn_args* a) {
 int b200tp_flash_bwd(const b200tp_attn_args* a, const void* q, const void* k, const void* v, const void* o,
                      const float* lse, const void* d_o, void* dq, void* dk, void* dv, void* workspace,
                      size_t workspace_bytes, void* stream, int* status) {
+  return b200tp_flash_bwd_strided(a, q, k, v, o, lse, d_o, nullptr, dq, dk, dv, workspace, workspace_bytes, stream,
+                                  status);
+}
+
+int b200tp_flash_bwd_strided(const b200tp_attn_args* a, const void* q, const void* k, const void* v, const void* o,
+                             const float* lse, const void* d_o, const int64_t* d_o_stride, void* dq, void* dk, void* dv,
+                             void* workspace, size_t workspace_bytes, void* stream, int* status) {
   int rc = check_attn(a);
   if (rc) return rc;
   if (q == nullptr || k == nullptr || v == nullptr || o == nullptr || lse == nullptr || d_o == nullptr ||
@@ -132,8 +139,14 @@ int b200tp_flash_bwd(const b200tp_attn_args* a, const void* q, const void* k, co
   if (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0 || workspace_bytes < need)
     return fail(B200TP_ERR_WORKSPACE, "attention backward workspace missing, misaligned or smaller than " +
                                           std::to_string(need) + " bytes");
-  if (impl == 1)
-    return flash_tc_bwd(a, q, k, v, o, lse, d_o, dq, dk, dv, workspace, static_cast<cudaStream_t>(stream), status);
+  const int64_t* ds = d_o_stride != nullptr ? d_o_stride : a->o_stride;
+  if (impl == 1) {
+    if (ds[0] % 8 != 0 || ds[1] % 8 != 0 || ds[2] % 8 != 0)
+      return fail(B200TP_ERR_ATTN_INPUT, "d_o strides must be multiples of 16 bytes on the tensor-core path");
+    return flash_tc_bwd(a, q, k, v, o, lse, d_o, ds, dq, dk, dv, workspace, static_cast<cudaStream_t>(stream), status);
+  }
+  if (ds[0] != a->o_stride[0] || ds[1] != a->o_stride[1] || ds[2] != a->o_stride[2])
+    return fail(B200TP_ERR_ATTN_INPUT, "the CUDA-core path takes d_o with o's strides");
   return flash_simt_bwd(a, q, k, v, o, lse, d_o, dq, dk, dv, static_cast<float*>(workspace),
                         static_cast<cudaStream_t>(stream));
 }

@@ -20,7 +20,7 @@ int flash_tc_fwd(const b200tp_attn_args* a, const void* q, const void* k, const 
                  void* workspace, size_t workspace_bytes, cudaStream_t stream, int* status);
 size_t flash_tc_bwd_workspace_bytes(const b200tp_attn_args* a);
 int flash_tc_bwd(const b200tp_attn_args* a, const void* q, const void* k, const void* v, const void* o,
-                 const float* lse, const void* d_o, void* dq, void* dk, void* dv, void* workspace,
-                 cudaStream_t stream, int* status);
+                 const float* lse, const void* d_o, const int64_t* do_stride, void* dq, void* dk, void* dv,
+                 void* workspace, cudaStream_t stream, int* status);
 
 }  // namespace b200tp

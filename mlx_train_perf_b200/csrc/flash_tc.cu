@@ -171,7 +171,8 @@ struct AttnParams {
   long long out_sb, out_sh, out_ss;
   float* lse_out;           // forward only
   const float* lse;         // backward
-  const __nv_bfloat16* o_saved;   // dQ kernel: the forward's O (same strides as dO), for D = rowsum(dO * O)
+  const __nv_bfloat16* o_saved;   // dQ kernel: the forward's O, for D = rowsum(dO * O)
+  long long o_sb, o_sh, o_ss;
   // The row statistics of the backward (-D, -L / scale) as a bf16 operand tile for the dK / dV kernel, which
   // adds them to its products with one extra K = 16 MMA step each (see `stat_row`): per (b, q head)
   // `stat_blocks` blocks of 64 rows, each block 2048 bytes = [2 chunks][64 rows][8 bf16], the shared-memory
@@ -1217,7 +1218,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tmap_k64, const __grid_const
         }
         if (!is_q && ig < p.S) {
           const __nv_bfloat16* osrc =
-              p.o_saved + b * do_sb + h * do_sh + static_cast<long long>(igc) * do_ss + (col0 & 63) * 2 + c * 64;
+              p.o_saved + b * p.o_sb + h * p.o_sh + static_cast<long long>(igc) * p.o_ss + (col0 & 63) * 2 + c * 64;
           float acc4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int g = 0; g < 8; ++g) {
@@ -1661,8 +1662,8 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q64, const __grid_cons
 // (attention/kernel/source.py:614-649) and -L / scale, written as the statistics tile of the dK / dV
 // kernel.  Only launched when the dQ kernel, which forms the same tile in its prologue, is left out.
 __global__ void __launch_bounds__(128)
-bwd_d_kernel(int S, int Hq, int d, const __nv_bfloat16* __restrict__ d_o, const __nv_bfloat16* __restrict__ o, long long sb,
-             long long sh, long long ss, const float* __restrict__ lse, __nv_bfloat16* __restrict__ stat,
+bwd_d_kernel(int S, int Hq, int d, const __nv_bfloat16* __restrict__ d_o, const __nv_bfloat16* __restrict__ o, long long do_sb,
+             long long do_sh, long long do_ss, long long sb, long long sh, long long ss, const float* __restrict__ lse, __nv_bfloat16* __restrict__ stat,
              int stat_blocks, float scale_log2) {
   griddep_launch_dependents();
   griddep_wait();
@@ -1675,8 +1676,9 @@ bwd_d_kernel(int S, int Hq, int d, const __nv_bfloat16* __restrict__ d_o, const 
     return;
   }
   const long long off = b * sb + h * sh + static_cast<long long>(i) * ss + lane * 4;
+  const long long do_off = b * do_sb + h * do_sh + static_cast<long long>(i) * do_ss + lane * 4;
   const bool has_cols = lane * 4 < d;   // four head_dim columns per lane
-  const uint2 a = has_cols ? *reinterpret_cast<const uint2*>(d_o + off) : make_uint2(0u, 0u);
+  const uint2 a = has_cols ? *reinterpret_cast<const uint2*>(d_o + do_off) : make_uint2(0u, 0u);
   const uint2 c = has_cols ? *reinterpret_cast<const uint2*>(o + off) : make_uint2(0u, 0u);
   const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
   const __nv_bfloat162* c2 = reinterpret_cast<const __nv_bfloat162*>(&c);
@@ -1891,8 +1893,8 @@ size_t flash_tc_bwd_workspace_bytes(const b200tp_attn_args* a) {
 
 template <int D>
 static int bwd_impl(const b200tp_attn_args* a, const void* q, const void* k, const void* v, const void* o,
-                    const float* lse, const void* d_o, void* dq, void* dk, void* dv, void* workspace,
-                    cudaStream_t stream, int* status) {
+                    const float* lse, const void* d_o, const int64_t* do_stride, void* dq, void* dk, void* dv,
+                    void* workspace, cudaStream_t stream, int* status) {
   int rc = configure();
   if (rc) return rc;
   if (!(a->scale > 0.f)) return fail(B200TP_ERR_ATTN_INPUT, "scale must be positive");
@@ -1907,14 +1909,10 @@ static int bwd_impl(const b200tp_attn_args* a, const void* q, const void* k, con
     dk_part = reinterpret_cast<float*>(static_cast<char*>(workspace) + after_stat);
     dv_part = reinterpret_cast<float*>(static_cast<char*>(workspace) + after_stat + part_bytes);
   }
-  CUtensorMap tq, tk, tv, tdo;
-  rc = make_tmap_bhsd_bf16(&tq, q, a->b, a->hq, a->s, D, a->q_stride[0], a->q_stride[1], a->q_stride[2], TILE, 64);
-  if (rc) return rc;
+  CUtensorMap tk, tv;
   rc = make_tmap_bhsd_bf16(&tk, k, a->b, a->hkv, a->s, D, a->k_stride[0], a->k_stride[1], a->k_stride[2], TILE, 64);
   if (rc) return rc;
   rc = make_tmap_bhsd_bf16(&tv, v, a->b, a->hkv, a->s, D, a->v_stride[0], a->v_stride[1], a->v_stride[2], TILE, 64);
-  if (rc) return rc;
-  rc = make_tmap_bhsd_bf16(&tdo, d_o, a->b, a->hq, a->s, D, a->o_stride[0], a->o_stride[1], a->o_stride[2], TILE, 64);
   if (rc) return rc;
   CUtensorMap tq64, tk64, tv64, tdo64;  // 64-row boxes for the operand that is streamed in half tiles
   rc = make_tmap_bhsd_bf16(&tq64, q, a->b, a->hq, a->s, D, a->q_stride[0], a->q_stride[1], a->q_stride[2], 64, 64);
@@ -1923,7 +1921,7 @@ static int bwd_impl(const b200tp_attn_args* a, const void* q, const void* k, con
   if (rc) return rc;
   rc = make_tmap_bhsd_bf16(&tv64, v, a->b, a->hkv, a->s, D, a->v_stride[0], a->v_stride[1], a->v_stride[2], 64, 64);
   if (rc) return rc;
-  rc = make_tmap_bhsd_bf16(&tdo64, d_o, a->b, a->hq, a->s, D, a->o_stride[0], a->o_stride[1], a->o_stride[2], 64, 64);
+  rc = make_tmap_bhsd_bf16(&tdo64, d_o, a->b, a->hq, a->s, D, do_stride[0], do_stride[1], do_stride[2], 64, 64);
   if (rc) return rc;
 
   // Row statistics (-D, -L log2 e): formed by the dQ kernel for its own rows and published for the dK / dV
@@ -1932,14 +1930,17 @@ static int bwd_impl(const b200tp_attn_args* a, const void* q, const void* k, con
     dim3 gd(stat_blocks * 16, a->hq, a->b);   // four rows per block, whole 64-row blocks of the statistics tile
     B200TP_CUDA_OK(launch_pdl(bwd_d_kernel, gd, dim3(128), 0, stream, a->s, a->hq, D,
                               static_cast<const __nv_bfloat16*>(d_o), static_cast<const __nv_bfloat16*>(o),
-                              static_cast<long long>(a->o_stride[0]), static_cast<long long>(a->o_stride[1]),
-                              static_cast<long long>(a->o_stride[2]), lse, stat, stat_blocks,
+                              static_cast<long long>(do_stride[0]), static_cast<long long>(do_stride[1]),
+                              static_cast<long long>(do_stride[2]), static_cast<long long>(a->o_stride[0]),
+                              static_cast<long long>(a->o_stride[1]), static_cast<long long>(a->o_stride[2]), lse, stat,
+                              stat_blocks,
                               a->scale * kLog2e));
   }
 
   AttnParams p = base_params(a, status);
   p.lse = lse;
   p.o_saved = static_cast<const __nv_bfloat16*>(o);
+  p.o_sb = a->o_stride[0]; p.o_sh = a->o_stride[1]; p.o_ss = a->o_stride[2];
   p.stat_w = stat;
   p.stat = stat;
   p.stat_blocks = stat_blocks;
@@ -1956,8 +1957,8 @@ static int bwd_impl(const b200tp_attn_args* a, const void* q, const void* k, con
     B200TP_CUDA_OK(launch_pdl(flash_dq_kernel<D>, gq, dim3(DQ_THREADS), DQ_SMEM_BYTES, stream, tk64, tv64,
                               static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(d_o),
                               static_cast<long long>(a->q_stride[0]), static_cast<long long>(a->q_stride[1]),
-                              static_cast<long long>(a->q_stride[2]), static_cast<long long>(a->o_stride[0]),
-                              static_cast<long long>(a->o_stride[1]), static_cast<long long>(a->o_stride[2]), p));
+                              static_cast<long long>(a->q_stride[2]), static_cast<long long>(do_stride[0]),
+                              static_cast<long long>(do_stride[1]), static_cast<long long>(do_stride[2]), p));
   }
   if (a->reserved & 256) return B200TP_OK;
   p.dk_part = dk_part;
@@ -1979,12 +1980,12 @@ static int bwd_impl(const b200tp_attn_args* a, const void* q, const void* k, con
 }
 
 int flash_tc_bwd(const b200tp_attn_args* a, const void* q, const void* k, const void* v, const void* o,
-                 const float* lse, const void* d_o, void* dq, void* dk, void* dv, void* workspace, cudaStream_t stream,
-                 int* status) {
+                 const float* lse, const void* d_o, const int64_t* do_stride, void* dq, void* dk, void* dv,
+                 void* workspace, cudaStream_t stream, int* status) {
   switch (a->d) {
-    case 64: return bwd_impl<64>(a, q, k, v, o, lse, d_o, dq, dk, dv, workspace, stream, status);
-    case 96: return bwd_impl<96>(a, q, k, v, o, lse, d_o, dq, dk, dv, workspace, stream, status);
-    case 128: return bwd_impl<128>(a, q, k, v, o, lse, d_o, dq, dk, dv, workspace, stream, status);
+    case 64: return bwd_impl<64>(a, q, k, v, o, lse, d_o, do_stride, dq, dk, dv, workspace, stream, status);
+    case 96: return bwd_impl<96>(a, q, k, v, o, lse, d_o, do_stride, dq, dk, dv, workspace, stream, status);
+    case 128: return bwd_impl<128>(a, q, k, v, o, lse, d_o, do_stride, dq, dk, dv, workspace, stream, status);
     default: return fail(B200TP_ERR_UNSUPPORTED_ATTN, "head_dim must be 64, 96 or 128");
   }
 }

@@ -39,3 +39,19 @@ def test_boundaries(cuda_device, lengths, impl):
     loose = PackedMask(seg_id=seg.seg_id, seg_start=torch.zeros_like(seg.seg_start))
     for a, b in zip(_run(q, k, v, d_o, loose, impl), got):
         assert (a - b).abs().max() <= 2e-2 * b.abs().max() + 3e-5
+
+
+@pytest.mark.parametrize("d", [64, 96, 128])
+def test_gradient_in_another_layout(cuda_device, d):
+    """d_o as it comes back through `o.transpose(1, 2)` is read where it lies: the same bits as its copy in o's
+    layout; layouts the kernels cannot read are copied."""
+    g, s = torch.Generator().manual_seed(d), 333
+    q, k, v = (torch.randn(2, h, s, d, generator=g).bfloat16().to(cuda_device) for h in (4, 2, 2))
+    base = torch.randn(2, s, 4, d + 8, generator=g).bfloat16().to(cuda_device)
+    views = [base[..., :d].transpose(1, 2), base[..., 8:].contiguous().transpose(1, 2),
+             base[..., 4:d + 4].transpose(1, 2),                      # not 16-byte aligned
+             base[:1, :, :, :d].transpose(1, 2).expand(2, 4, s, d)]   # batches share memory
+    for d_o in views:
+        want = _run(q, k, v, d_o.contiguous(), None, "auto")
+        for a, b in zip(_run(q, k, v, d_o, None, "auto"), want):
+            assert torch.equal(a, b)
