@@ -85,7 +85,7 @@ typedef struct b200tp_ce_args {
                        * 512 MiB): the backward's scratch is that matrix, so
                        * a smaller bound trades launches for memory.  4-bit heads on the tensor-core path:
                        * 0x10000 expands the head inside the kernels whatever N is, 0x20000 always dequantises chunk
-                       * by chunk into the workspace (default: the forward expands inside the kernel for N <= 512,
+                       * by chunk into the workspace (default: the forward expands inside the kernel for N <= 2048,
                        * where that is the cheaper form and needs no weight scratch, and is chunked beyond; the
                        * backward is chunked at every N); 0x40000: fp32
                        * operands of a dense head run on the tensor cores as three bf16 planes each at any size (by default

@@ -25,6 +25,7 @@ SOURCES = [
     "linear_ce_tc.cu",
     "linear_ce_simt.cu",
     "linear_ce_grad.cu",
+    "linear_ce_int4.cu",
     "linear_ce_split.cu",
     "capi_ce.cu",
     "linear_ce_static.cu",

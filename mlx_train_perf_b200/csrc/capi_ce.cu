@@ -36,7 +36,7 @@ constexpr int64_t kSplitChunkRowsMin = 2048, kSplitChunkRowsMax = 16384;
 constexpr int kReservedInline = 0x10000;    // 4-bit head: expand inside the kernels whatever the row count
 constexpr int kReservedChunked = 0x20000;   // 4-bit head: dequantise chunk by chunk whatever the row count
 constexpr int kReservedSplit = 0x40000;     // fp32, dense head: the tensor cores whatever the size
-constexpr int64_t kInlineMaxRows = 512;     // default: the forward expands in the kernel up to this many rows of hidden
+constexpr int64_t kInlineMaxRows = 2048;    // default: the forward expands in the kernel up to this many rows of hidden
 
 // `grow` (the forward that also forms the gradient, dense heads): few rows take wider chunks, up to the scratch that
 // 8192 rows use anyway.  A chunk ends in a partly filled wave of tiles and an fp32 round trip of d_hidden in each of
@@ -105,16 +105,16 @@ int check_args(const b200tp_ce_args* a) {
 }
 
 // Where a 4-bit head is expanded on the tensor-core path.
-//   in the kernels: the weight operand never exists in global memory, but every CTA that meets a weight
-//     tile expands it again, i.e. once per 128 rows of hidden: ALU work that grows with N and, past a few
-//     row blocks, exceeds what the tensor pipe leaves idle (measured at N=8192: 2.2x the dense forward);
-//   chunk by chunk into a bf16 scratch (one pass over the codes per GEMM pass, 0.06 ms per 16384 x 4096
-//     chunk) followed by the dense kernels: the cheaper form for training-sized batches.
-// Default, from timings at D=4096, V=151936 (in-kernel / chunked, ms): forward 0.36 / 1.25 at N=128,
-// 1.02 / 1.25 at 512, 1.93 / 1.56 at 1024 -- in the kernel up to kInlineMaxRows rows, with no weight
-// scratch at all; backward 3.2 / 1.9 at N=128, 3.8 / 2.1 at 512 -- always chunked: with few row blocks
-// the d_hidden GEMM has only D / 256 tiles, so a handful of CTAs would each expand their 256 columns of
-// the whole head, while the dequantisation kernel spreads the same work over every SM.  `reserved`
+//   in the kernels: the weight operand never exists in global memory.  The forward's default kernel expands a code
+//     once per 320 rows of hidden (linear_ce_int4.cu); the kernels that `reserved` selects (bit for bit the dense ones
+//     on dequantised weights, and the only ones of the backward) once per 128;
+//   chunk by chunk into a bf16 scratch (one pass over the codes per GEMM pass, 0.03 ms per 16384 x 4096
+//     chunk) followed by the dense kernels.
+// Default, from timings at D=4096, V=151936 (in-kernel / chunked, us): forward 260 / 691 at N=60, 304 / 884 at 257,
+// 563 / 927 at 512, 1176 / 1481 at 1024, 2050 / 2427 at 2048, 4373 / 4228 at 4096 -- in the kernel up to
+// kInlineMaxRows rows, with no weight scratch at all; backward 3.2 / 1.9 ms at N=128, 3.8 / 2.1 at 512 -- always
+// chunked: with few row blocks the d_hidden GEMM has only D / 256 tiles, so a handful of CTAs would each expand their
+// 256 columns of the whole head, while the dequantisation kernel spreads the same work over every SM.  `reserved`
 // can force either form in both directions (in-kernel needs no weight scratch).  The in-kernel path
 // needs a 16-byte aligned w_q (TMA).
 bool quant_inline(const b200tp_ce_args* a, bool backward) {
@@ -180,6 +180,7 @@ struct FwdPlan {
   int64_t chunk;        // vocab rows per launch (tc dense: all)
   int64_t num_chunks;
   int64_t total_splits; // tc only
+  bool int4;            // tc: the head is expanded into tensor memory (linear_ce_int4.cu)
   // workspace pointers
   float* pm; float* ps; float* pt;
   void* deq;
@@ -201,7 +202,8 @@ FwdPlan plan_fwd(const b200tp_ce_args* a, void* ws) {
       // one launch over the whole shard (a 4-bit head is expanded inside the kernel, tile by tile)
       p.chunk = a->v_local;
       p.num_chunks = 1;
-      p.total_splits = ce_tc_fwd_splits(a->n, a->v_local);
+      p.int4 = a->quant_bits != 0 && (a->reserved & kReservedInline) == 0;
+      p.total_splits = p.int4 ? ce_int4_fwd_splits(a->n, a->v_local) : ce_tc_fwd_splits(a->n, a->v_local);
     } else {
       // 4-bit head, chunked: dequantise a chunk of vocab rows, run the dense kernel over it
       p.chunk = tc_chunk_rows(a, &p.num_chunks);
@@ -385,8 +387,12 @@ int b200tp_linear_ce_fwd(const b200tp_ce_args* a, float* row_max, float* row_sum
     if (p.deq == nullptr) {
       const int splits = static_cast<int>(p.total_splits);
       const QuantHead q = quant_head(a, false);
-      rc = ce_tc_launch_fwd(a->hidden, a->weight, a->v_local, a->n, a->d, 0, a->v_local, a->v_offset, a->targets,
-                            a->ignore_index, splits, p.pm, p.ps, p.pt, &q, stream, status);
+      if (p.int4)
+        rc = ce_int4_launch_fwd(a->hidden, q, a->v_local, a->n, a->d, a->v_offset, a->targets,
+                                a->ignore_index, splits, p.pm, p.ps, p.pt, stream, status);
+      else
+        rc = ce_tc_launch_fwd(a->hidden, a->weight, a->v_local, a->n, a->d, 0, a->v_local, a->v_offset, a->targets,
+                              a->ignore_index, splits, p.pm, p.ps, p.pt, &q, stream, status);
       if (rc) return rc;
     } else {
       int64_t slot = 0;

@@ -4,7 +4,7 @@
 // stores the 32 bf16 pairs into that row's lane.  The tokens are the N side: a CTA keeps up to kMostTokens of them
 // against one 128-row weight tile, so a code is expanded once per kMostTokens tokens.  (With the tokens on the M side
 // a weight tile was expanded again for every 128 of them, and padding went to multiples of 128: 257 rows x 4096 x
-// 151936 took 773 us where this takes T4_US, 60 rows T4_60.)  An MMA reads only the tokens from shared memory, which
+// 151936 took 773 us where this takes 304.)  An MMA reads only the tokens from shared memory, which
 // leaves room for the TMA writes beside it; both operands there would need more than its bandwidth.
 //
 // The accumulator is transposed: a lane holds a vocab row, a column a token.  The epilogue warps turn 32 x 32 blocks
@@ -14,7 +14,7 @@
 // Tensor-bound from about 200 tokens on, expansion-bound below (about 170 instructions per 64 weights; eight warps in
 // two groups, each taking every other k block, keep it under the MMAs of 272 tokens).
 //
-// Roles (18 warps): TMA producer, MMA issuer, eight epilogue warps, eight expanding warps.  Waits are bounded and end
+// Roles (19 warps): two TMA producers, MMA issuer, eight epilogue warps, eight expanding warps.  Waits are bounded and end
 // like those of linear_ce_tc.cu.  Replaces core/kernel/source.py:199-340 (K2) of the reference.
 #include "linear_ce_tc.h"
 
@@ -35,7 +35,8 @@ constexpr int STAGE_BYTES = kMostTokens * KB * 2;     // 40 KiB
 constexpr int CODE_SLOTS = 4;
 constexpr int CODE_BYTES = VROWS * 64;                // one row's codes of two k blocks: 64 bytes
 constexpr int EPI_WARPS = 8, DQ_WARPS = 8;
-constexpr int THREADS = 32 * (2 + EPI_WARPS + DQ_WARPS);
+constexpr int CTRL_WARPS = 3;                         // token producer, MMA issuer, code producer
+constexpr int THREADS = 32 * (CTRL_WARPS + EPI_WARPS + DQ_WARPS);
 constexpr int TURN_FLOATS = 32 * 33;                  // per epilogue warp: a 32 x 32 block, padded against conflicts
 constexpr int BAR_BYTES = 256;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + CODE_SLOTS * CODE_BYTES + EPI_WARPS * TURN_FLOATS * 4 + BAR_BYTES + 1024;
@@ -161,24 +162,12 @@ int4_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_cons
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&tmap_h);
-      tma_prefetch_desc(&tmap_c);
       const uint32_t box_bytes = static_cast<uint32_t>(p.n0) * KB * 2;
-      uint32_t it = 0, ci = 0;
+      uint32_t it = 0;
       bool ok = true;
       for (TileWalk w(p); !w.done(p) && ok; w.next(p)) {
         const int row0 = (w.u % p.groups) * p.gsz;
         for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
-          if ((kb & 1) == 0) {
-            const uint32_t cs = ci % CODE_SLOTS;
-            if (!mbar_wait(&sm.cempty[cs], ((ci / CODE_SLOTS) & 1) ^ 1, sm.abort_flag)) {
-              raise(sm, p.status, kDevTimeoutProducer);
-              ok = false;
-              break;
-            }
-            mbar_arrive_expect_tx(&sm.cfull[cs], CODE_BYTES);
-            tma_load_2d(sm.codes + cs * CODE_BYTES, &tmap_c, &sm.cfull[cs], kb * 8, w.vt * VROWS);
-            ++ci;
-          }
           const int s = it % STAGES;
           if (!mbar_wait(&sm.empty[s], ((it / STAGES) & 1) ^ 1, sm.abort_flag)) {
             raise(sm, p.status, kDevTimeoutProducer);
@@ -190,11 +179,31 @@ int4_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_cons
             tma_load_2d(sm.base + s * STAGE_BYTES + b * box_bytes, &tmap_h, &sm.full[s], kb * KB, row0 + b * p.n0);
         }
       }
-      if (!ok) {
+      if (!ok)
         for (uint32_t j = it > STAGES ? it - STAGES : 0; j < it; ++j) mbar_wait_drain(&sm.full[j % STAGES], (j / STAGES) & 1);
+    }
+  } else if (warp == 2) {
+    // The codes come from HBM and the tokens from L2, and codes must be asked for further ahead than the stages reach:
+    // issued in step with the tokens, four k blocks ahead, stages waited for them (257 rows: 322 us, now 304).
+    if (lane == 0) {
+      tma_prefetch_desc(&tmap_c);
+      uint32_t ci = 0;
+      bool ok = true;
+      for (TileWalk w(p); !w.done(p) && ok; w.next(p)) {
+        for (int cb = 0; cb < cblocks; ++cb, ++ci) {
+          const uint32_t cs = ci % CODE_SLOTS;
+          if (!mbar_wait(&sm.cempty[cs], ((ci / CODE_SLOTS) & 1) ^ 1, sm.abort_flag)) {
+            raise(sm, p.status, kDevTimeoutProducer);
+            ok = false;
+            break;
+          }
+          mbar_arrive_expect_tx(&sm.cfull[cs], CODE_BYTES);
+          tma_load_2d(sm.codes + cs * CODE_BYTES, &tmap_c, &sm.cfull[cs], cb * 16, w.vt * VROWS);
+        }
+      }
+      if (!ok)
         for (uint32_t c = ci > CODE_SLOTS ? ci - CODE_SLOTS : 0; c < ci; ++c)
           mbar_wait_drain(&sm.cfull[c % CODE_SLOTS], (c / CODE_SLOTS) & 1);
-      }
     }
   } else if (warp == 1) {
     // whole-warp issue loop, one elected lane issues (see ce_logits_kernel)
@@ -226,10 +235,10 @@ int4_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_cons
       __syncwarp();
     }
     if (!ok && lane == 0) raise(sm, p.status, kDevTimeoutMma);
-  } else if (warp < 2 + EPI_WARPS) {
-    const int quad = warp & 3, half = (warp - 2) >> 2;   // lanes (vocab rows); every other 32-token chunk
+  } else if (warp < CTRL_WARPS + EPI_WARPS) {
+    const int quad = warp & 3, half = (warp - CTRL_WARPS) >> 2;   // lanes (vocab rows); every other 32-token chunk
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
-    float* turn = sm.turn + (warp - 2) * TURN_FLOATS;
+    float* turn = sm.turn + (warp - CTRL_WARPS) * TURN_FLOATS;
     uint32_t tile = 0;
     bool ok = true;
     TileWalk w(p);
@@ -329,7 +338,7 @@ int4_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_cons
     }
   } else {
     // expanding warps: group g takes the k blocks with kb % 2 == g
-    const int grp = (warp - 2 - EPI_WARPS) >> 2, quad = warp & 3;
+    const int grp = (warp - CTRL_WARPS - EPI_WARPS) >> 2, quad = warp & 3;
     const int trow = quad * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t swz = static_cast<uint32_t>((trow >> 1) & 3);

@@ -943,6 +943,8 @@ static int configure_kernels() {
   return B200TP_OK;
 }
 
+int ce_tc_choose_splits(int num_rb, int num_vt) { return choose_splits(num_rb, num_vt, sm_count()); }
+
 int ce_tc_fwd_splits(int64_t n, int64_t v_rows) {
   const int num_rb = static_cast<int>(ceil_div(n, BM));
   const int num_vt = static_cast<int>(ceil_div(v_rows, BN));

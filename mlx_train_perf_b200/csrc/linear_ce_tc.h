@@ -28,12 +28,20 @@ struct LaunchGuard {
 // Vocab splits the forward uses for (n rows, v_rows vocab rows): one partial triple per
 // (row, split) lands in the workspace.
 int ce_tc_fwd_splits(int64_t n, int64_t v_rows);
+// The split count behind it, for `num_rb` row groups and `num_vt` vocab tiles.
+int ce_tc_choose_splits(int num_rb, int num_vt);
 
 // Forward partials over weight rows [vrow0, vrow1) of a (w_rows_total, d) bf16 matrix whose
 // row 0 has global vocab id `vocab_id0`.  pm/ps/pt: [splits][n] f32.
 int ce_tc_launch_fwd(const void* hidden, const void* w, int64_t w_rows_total, int64_t n, int d, int64_t vrow0,
                      int64_t vrow1, int64_t vocab_id0, const int64_t* targets, int64_t ignore_index, int splits,
                      float* pm, float* ps, float* pt, const QuantHead* q, cudaStream_t stream, int* status);
+
+// The same partials for a 4-bit head expanded inside the kernel into tensor memory (linear_ce_int4.cu).
+int ce_int4_fwd_splits(int64_t n, int64_t v_rows);
+int ce_int4_launch_fwd(const void* hidden, const QuantHead& q, int64_t v_rows, int64_t n, int d, int64_t vocab_id0,
+                       const int64_t* targets, int64_t ignore_index, int splits, float* pm, float* ps, float* pt,
+                       cudaStream_t stream, int* status);
 
 // g[n][ldg] (bf16) = (exp(z - lse) - onehot) * ct over weight rows [vrow0, vrow1); columns
 // up to the next multiple of 256 are written (zeros past vrow1).
