@@ -5,9 +5,12 @@ The library is loaded lazily and exactly once; a missing or unloadable library r
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import threading
 from pathlib import Path
+
+import torch
 
 from mlx_train_perf_b200.errors import (
     AttentionInputError, DeviceTimeoutError, LossInputError, NativeLibraryError,
@@ -140,6 +143,20 @@ def load() -> C.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def on(device: torch.device):
+    """Context in which launches go to `device`.  On the current device already (the usual case) nothing is switched:
+    the four launch sites of a 60-row training step spent 20 us of its host time entering and leaving contexts."""
+    return _SAME_DEVICE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+def stream(device: torch.device) -> int:
+    """The raw handle of torch's current stream on `device` (no `torch.cuda.Stream` object around it)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 
 _ERRORS = {

@@ -92,6 +92,8 @@ def _non_overlapping(t: torch.Tensor) -> bool:
     up the other axes from the smallest stride, each stride at least the extent below it.  Expanded
     (stride 0) heads or batches fail this; the backward writes gradients through these strides, so an
     aliasing view would make different heads race on the same memory."""
+    if t.is_contiguous():
+        return t.stride(-1) == 1
     if t.stride(-1) != 1:
         return False
     extent = t.shape[-1]
@@ -118,9 +120,7 @@ def _attn_args(q, k, v, o, *, scale, segments, impl):
     a.hkv = k.shape[1]
     a.dtype = _lib.BF16 if q.dtype == torch.bfloat16 else _lib.F32
     for name, t in (("q_stride", q), ("k_stride", k), ("v_stride", v), ("o_stride", o)):
-        arr = getattr(a, name)
-        for i in range(3):
-            arr[i] = t.stride(i)
+        setattr(a, name, t.stride()[:3])
     a.scale = float(scale)
     a.causal = 1
     if segments is not None:
@@ -180,10 +180,10 @@ def flash_fwd_raw(q, k, v, *, scale: float, segments: PackedMask | None = None, 
     # scratch for the split over keys a small grid gets (0 bytes for most shapes)
     nbytes = lib.b200tp_flash_fwd_workspace_bytes(C.byref(a))
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
-    with torch.cuda.device(dev):
+    with _lib.on(dev):
         rc = lib.b200tp_flash_fwd_ws(C.byref(a), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
                                      lse.data_ptr(), ws.data_ptr() if nbytes else None, nbytes,
-                                     torch.cuda.current_stream(dev).cuda_stream, device_status(dev).data_ptr())
+                                     _lib.stream(dev), device_status(dev).data_ptr())
     _lib.check(rc)
     return o, lse
 
@@ -228,11 +228,11 @@ def flash_bwd_raw(q, k, v, o, lse, d_o, *, scale: float, segments: PackedMask | 
     nbytes = lib.b200tp_flash_bwd_workspace_bytes(C.byref(a))
     a.reserved |= _BWD_PARTS[parts]
     ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on(dev):
         rc = lib.b200tp_flash_bwd_strided(C.byref(a), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
                                           lse.data_ptr(), d_o.data_ptr(), do_stride, dq.data_ptr(), dk.data_ptr(),
                                           dv.data_ptr(), ws.data_ptr(), ws.numel(),
-                                          torch.cuda.current_stream(dev).cuda_stream, device_status(dev).data_ptr())
+                                          _lib.stream(dev), device_status(dev).data_ptr())
     _lib.check(rc)
     return dq, dk, dv
 
@@ -249,10 +249,13 @@ class _FlashAttention(torch.autograd.Function):
         ctx.scale = scale
         ctx.impl = impl
         ctx.mark_non_differentiable(lse)
+        ctx.set_materialize_grads(False)      # no (B, H, N) zeros for L's gradient
         return o, lse
 
     @staticmethod
     def backward(ctx, d_o, _d_l):
+        if d_o is None:
+            return (None,) * 7
         VJP_CALLS["flash_attention"] = VJP_CALLS.get("flash_attention", 0) + 1
         saved = ctx.saved_tensors
         q, k, v, o, lse = saved[:5]

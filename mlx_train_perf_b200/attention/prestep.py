@@ -23,9 +23,7 @@ def _args(x: torch.Tensor, y: torch.Tensor, weight, eps: float, cos: torch.Tenso
     a = _lib.PrestepArgs()
     a.b, a.l, a.h, a.d = x.shape
     a.dtype = _lib.BF16 if x.dtype == torch.bfloat16 else _lib.F32
-    for i in range(3):
-        a.x_stride[i] = x.stride(i)
-        a.y_stride[i] = y.stride(i)
+    a.x_stride, a.y_stride = x.stride()[:3], y.stride()[:3]
     a.weight = None if weight is None else weight.data_ptr()
     a.eps = float(eps)
     a.cos, a.sin = cos.data_ptr(), sin.data_ptr()
@@ -71,9 +69,9 @@ class _NormRope(torch.autograd.Function):
         lib = _lib.load()
         y = torch.empty_like(x, memory_format=torch.preserve_format)
         a = _args(x, y, weight, eps, cos, sin)
-        with torch.cuda.device(x.device):
+        with _lib.on(x.device):
             rc = lib.b200tp_qk_norm_rope_fwd(C.byref(a), x.data_ptr(), y.data_ptr(),
-                                             torch.cuda.current_stream(x.device).cuda_stream)
+                                             _lib.stream(x.device))
         _lib.check(rc)
         ctx.save_for_backward(x, weight, cos, sin)
         ctx.eps = eps
@@ -91,11 +89,11 @@ class _NormRope(torch.autograd.Function):
         dw = torch.empty(x.shape[-1], dtype=torch.float32, device=x.device) if want_dw else None
         nbytes = lib.b200tp_qk_norm_rope_bwd_workspace_bytes(C.byref(a)) if want_dw else 0
         ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=x.device) if want_dw else None
-        with torch.cuda.device(x.device):
+        with _lib.on(x.device):
             rc = lib.b200tp_qk_norm_rope_bwd(C.byref(a), x.data_ptr(), dy.data_ptr(), dx.data_ptr(),
                                              None if dw is None else dw.data_ptr(),
                                              None if ws is None else ws.data_ptr(), nbytes,
-                                             torch.cuda.current_stream(x.device).cuda_stream)
+                                             _lib.stream(x.device))
         _lib.check(rc)
         return dx, (None if dw is None else dw.to(weight.dtype)), None, None, None
 

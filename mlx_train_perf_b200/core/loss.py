@@ -63,7 +63,7 @@ def tied_head(embedding_weight: torch.Tensor, *, trainable: bool = False) -> Den
 
 # 4-bit heads on the tensor-core path: "tc_inline" expands the head inside the kernels whatever N is (no
 # weight scratch), "tc_chunked" always dequantises chunk by chunk ahead of the dense kernels; plain "tc" /
-# "auto" lets the library choose (the forward inside the kernel up to 512 rows, everything else chunked).
+# "auto" lets the library choose (the forward inside the kernel up to 2048 rows, everything else chunked).
 _TC_QUANT_IMPLS = ("tc_inline", "tc_chunked")
 _RESERVED = {"tc_inline": 0x10000, "tc_chunked": 0x20000, "split": 0x40000}   # "split": fp32 as bf16 planes at any size
 
@@ -226,9 +226,9 @@ def _ce_args(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, *, v_of
     a.impl = _lib.IMPL["tc" if impl in _TC_QUANT_IMPLS else "auto" if impl == "split" else impl]
     a.reserved = _RESERVED.get(impl, 0)
     if isinstance(head, DenseHead):
-        w = head.weight.detach()
+        w = head.weight
         if not w.is_contiguous():
-            w = w.contiguous()
+            w = w.detach().contiguous()
         keep.append(w)
         a.weight = w.data_ptr()
         a.v_local = w.shape[0]
@@ -247,10 +247,6 @@ def _ce_args(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, *, v_of
         a.group_size = head.group_size
         a.qparam_dtype = _dtype_code(sc.dtype)
     return a, keep
-
-
-def _stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
 
 
 def _workspace(nbytes: int, device: torch.device) -> torch.Tensor | None:
@@ -278,11 +274,12 @@ def ce_forward_buffer(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor
     out = torch.empty((5, n), dtype=torch.float32, device=dev)
     nbytes = lib.b200tp_linear_ce_fwd_workspace_bytes(C.byref(a))
     ws = _workspace(nbytes, dev)
-    with torch.cuda.device(dev):
+    base = out.data_ptr()
+    with _lib.on(dev):
         rc = lib.b200tp_linear_ce_fwd(
-            C.byref(a), out[0].data_ptr(), out[1].data_ptr(), out[2].data_ptr(),
-            out[3].data_ptr() if want_lse else None, out[4].data_ptr() if want_lse else None,
-            _ptr(ws), nbytes, _stream(dev), device_status(dev).data_ptr())
+            C.byref(a), base, base + 4 * n, base + 8 * n,
+            base + 12 * n if want_lse else None, base + 16 * n if want_lse else None,
+            _ptr(ws), nbytes, _lib.stream(dev), device_status(dev).data_ptr())
     _lib.check(rc)
     del keep
     return out
@@ -325,15 +322,15 @@ def ce_backward_raw(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, 
         if (d_weight.dtype != head.weight.dtype or tuple(d_weight.shape) != tuple(head.weight.shape)
                 or not d_weight.is_contiguous() or d_weight.device != dev):
             raise LossInputError("d_weight must be a contiguous tensor shaped and typed like the head weight")
-    with torch.cuda.device(dev):
+    with _lib.on(dev):
         if d_weight is None:
             rc = lib.b200tp_linear_ce_bwd(C.byref(a), lse.data_ptr(), ct.data_ptr(), out.data_ptr(),
-                                          _dtype_code(odt), 1 if accumulate else 0, _ptr(ws), nbytes, _stream(dev),
+                                          _dtype_code(odt), 1 if accumulate else 0, _ptr(ws), nbytes, _lib.stream(dev),
                                           device_status(dev).data_ptr())
         else:
             rc = lib.b200tp_linear_ce_bwd_train(C.byref(a), lse.data_ptr(), ct.data_ptr(), out.data_ptr(),
                                                 _dtype_code(odt), 1 if accumulate else 0, d_weight.data_ptr(),
-                                                _ptr(ws), nbytes, _stream(dev), device_status(dev).data_ptr())
+                                                _ptr(ws), nbytes, _lib.stream(dev), device_status(dev).data_ptr())
     _lib.check(rc)
     del keep
     return out
@@ -360,9 +357,9 @@ def ce_forward_grad(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, 
     nbytes = lib.b200tp_linear_ce_fwd_grad_workspace_bytes(C.byref(a))
     state, ws = _workspace(sbytes, dev), _workspace(nbytes, dev)
     base = out.data_ptr()
-    with torch.cuda.device(dev):
+    with _lib.on(dev):
         rc = lib.b200tp_linear_ce_fwd_grad(C.byref(a), base, base + 4 * n, base + 8 * n, _ptr(state), sbytes,
-                                           _ptr(ws), nbytes, _stream(dev), device_status(dev).data_ptr())
+                                           _ptr(ws), nbytes, _lib.stream(dev), device_status(dev).data_ptr())
     _lib.check(rc)
     del keep
     return out, state
@@ -381,9 +378,9 @@ def ce_backward_grad(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor,
     nbytes = lib.b200tp_linear_ce_bwd_grad_workspace_bytes(C.byref(a))
     ws = _workspace(nbytes, dev)
     base = out.data_ptr()
-    with torch.cuda.device(dev):
+    with _lib.on(dev):
         rc = lib.b200tp_linear_ce_bwd_grad(C.byref(a), base + 4 * n, base, ct.data_ptr(), state.data_ptr(),
-                                           state.numel(), d_hidden.data_ptr(), _ptr(ws), nbytes, _stream(dev),
+                                           state.numel(), d_hidden.data_ptr(), _ptr(ws), nbytes, _lib.stream(dev),
                                            device_status(dev).data_ptr())
     _lib.check(rc)
     del keep
@@ -402,6 +399,7 @@ class _FusedLinearCE(torch.autograd.Function):
         else:
             _, _, tgt, lse, nll = ce_forward_raw(hidden, head, targets, ignore_index=ignore_index, impl=impl)
             ctx.save_for_backward(hidden, targets, lse)
+        ctx.set_materialize_grads(False)      # no zeros for the gradients of lse and target_logit
         ctx.head = head
         ctx.ignore_index = ignore_index
         ctx.impl = impl
@@ -410,6 +408,8 @@ class _FusedLinearCE(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g_nll, _g_lse, _g_tgt):
+        if g_nll is None:
+            return (None,) * 5
         key = "quantized" if isinstance(ctx.head, QuantizedHead) else "dense"
         VJP_CALLS[key] = VJP_CALLS.get(key, 0) + 1
         saved = ctx.saved_tensors
@@ -437,10 +437,13 @@ class _FusedLinearCETrainable(torch.autograd.Function):
         ctx.ignore_index = ignore_index
         ctx.impl = impl
         ctx.mark_non_differentiable(lse, tgt)
+        ctx.set_materialize_grads(False)
         return nll, lse, tgt
 
     @staticmethod
     def backward(ctx, g_nll, _g_lse, _g_tgt):
+        if g_nll is None:
+            return (None,) * 5
         VJP_CALLS["dense_trainable"] = VJP_CALLS.get("dense_trainable", 0) + 1
         hidden, weight, targets, lse = ctx.saved_tensors
         d_w = torch.empty_like(weight, memory_format=torch.contiguous_format) if ctx.needs_input_grad[1] else None
@@ -479,18 +482,21 @@ class _FusedLinearCEReduced(torch.autograd.Function):
         lib = _lib.load()
         dev = hidden.device
         out3 = torch.empty(3, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on(dev):
             rc = lib.b200tp_linear_ce_reduce(nll.data_ptr(), targets.data_ptr(), hidden.shape[0], ignore_index,
-                                             out3.data_ptr(), _stream(dev))
+                                             out3.data_ptr(), _lib.stream(dev))
         _lib.check(rc)
         ctx.save_for_backward(hidden, targets, out3, *saved)
         ctx.head, ctx.ignore_index, ctx.impl, ctx.mean = head, ignore_index, impl, mean
+        ctx.set_materialize_grads(False)      # no zeros for the count's gradient
         loss, count = out3[1 if mean else 0], out3[2]
         ctx.mark_non_differentiable(count)
         return loss, count
 
     @staticmethod
     def backward(ctx, g_loss, _g_count):
+        if g_loss is None:
+            return (None,) * 7
         saved = ctx.saved_tensors
         hidden, targets, out3, rows = saved[:4]      # rows: lse, or the three rows of `ce_forward_grad`
         weight = saved[4] if ctx.trains_weight else None
@@ -502,9 +508,9 @@ class _FusedLinearCEReduced(torch.autograd.Function):
         n = hidden.shape[0]
         g = g_loss.to(torch.float32).reshape(1).contiguous()
         ct = torch.empty(n, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on(dev):
             rc = lib.b200tp_linear_ce_cotangent(targets.data_ptr(), n, ctx.ignore_index, g.data_ptr(),
-                                                out3[2:].data_ptr() if ctx.mean else None, ct.data_ptr(), _stream(dev))
+                                                out3.data_ptr() + 8 if ctx.mean else None, ct.data_ptr(), _lib.stream(dev))
         _lib.check(rc)
         if ctx.has_grad:
             d_hidden = ce_backward_grad(hidden, head, targets, rows, saved[4], ct, ignore_index=ctx.ignore_index,
@@ -536,12 +542,12 @@ def masked_loss(nll: torch.Tensor, targets: torch.Tensor, *, mean: bool = True,
     out3 = torch.empty(3, dtype=torch.float32, device=dev)
     ct = torch.empty(n, dtype=torch.float32, device=dev)
     g = torch.ones(1, dtype=torch.float32, device=dev) if upstream is None else upstream.to(torch.float32).reshape(1)
-    with torch.cuda.device(dev):
+    with _lib.on(dev):
         rc = lib.b200tp_linear_ce_reduce(nll.data_ptr(), targets.data_ptr(), n, ignore_index, out3.data_ptr(),
-                                         _stream(dev))
+                                         _lib.stream(dev))
         _lib.check(rc)
         rc = lib.b200tp_linear_ce_cotangent(targets.data_ptr(), n, ignore_index, g.data_ptr(),
-                                            out3[2:].data_ptr() if mean else None, ct.data_ptr(), _stream(dev))
+                                            out3[2:].data_ptr() if mean else None, ct.data_ptr(), _lib.stream(dev))
         _lib.check(rc)
     return out3[1 if mean else 0], out3[2], ct
 
