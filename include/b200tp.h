@@ -194,14 +194,15 @@ int b200tp_linear_ce_bwd_train(const b200tp_ce_args* a, const float* lse, const 
  * right in any case, and every decision is taken on the device).
  *   state : b200tp_linear_ce_grad_state_bytes, 256-byte aligned, kept by the caller until the backward
  *           (fp32 sums of d_hidden, the references and the flag)
- * bf16 hidden, D % 8 == 0, the whole vocabulary (v_offset = 0); the *_bytes functions return 0 where the call
- * would be refused.  b200tp_linear_ce_bwd_grad may be called more than once on one state. */
+ * bf16 hidden, or fp32 where the tensor cores serve it (see `reserved`: its exponentials keep fp32 precision, and
+ * inputs without bf16 planes set the flag too); D % 8 == 0, the whole vocabulary (v_offset = 0); the *_bytes functions
+ * return 0 where the call would be refused.  b200tp_linear_ce_bwd_grad may be called more than once on one state. */
 size_t b200tp_linear_ce_grad_state_bytes(const b200tp_ce_args* a);
 size_t b200tp_linear_ce_fwd_grad_workspace_bytes(const b200tp_ce_args* a);
 int b200tp_linear_ce_fwd_grad(const b200tp_ce_args* a, float* tgt_logit, float* lse, float* nll, void* state,
                               size_t state_bytes, void* workspace, size_t workspace_bytes, void* stream,
                               int* status);
-/* d_hidden (N, D) bf16 = cotangent * that gradient (0 on ignored rows). */
+/* d_hidden (N, D) in the hidden dtype = cotangent * that gradient (0 on ignored rows). */
 size_t b200tp_linear_ce_bwd_grad_workspace_bytes(const b200tp_ce_args* a);
 int b200tp_linear_ce_bwd_grad(const b200tp_ce_args* a, const float* lse, const float* tgt_logit, const float* cotangent,
                               void* state, size_t state_bytes, void* d_hidden, void* workspace, size_t workspace_bytes,

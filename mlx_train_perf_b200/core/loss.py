@@ -336,12 +336,17 @@ def ce_backward_raw(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, 
     return out
 
 
-def _forms_grad(impl: str, hidden_wants_grad: bool) -> bool:
+def _forms_grad(impl: str, hidden_wants_grad: bool, hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor) -> bool:
     """Whether the forward of a frozen head also forms the gradient of the hidden states (two contractions over
     N x V x D in all, where a backward that computes the logits again makes it three): on the tensor-core path,
     when autograd may ask for that gradient.  A forward whose gradient is never wanted is best run under
     `torch.no_grad()`, where it stays at one contraction."""
-    return hidden_wants_grad and impl in ("tc", "tc_chunked")
+    if not hidden_wants_grad or impl in ("tc", "tc_chunked"):
+        return hidden_wants_grad
+    if impl not in ("auto", "split") or hidden.dtype != torch.float32:
+        return False
+    a, keep = _ce_args(hidden, head, targets, v_offset=0, ignore_index=IGNORE_INDEX, impl=impl)
+    return _lib.load().b200tp_linear_ce_grad_state_bytes(C.byref(a)) > 0      # fp32: where the library's rule says so
 
 
 def ce_forward_grad(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, *,
@@ -392,7 +397,7 @@ class _FusedLinearCE(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, hidden, targets, head, ignore_index, impl):
-        if _forms_grad(impl, ctx.needs_input_grad[0]):
+        if _forms_grad(impl, ctx.needs_input_grad[0], hidden, head, targets):
             out, state = ce_forward_grad(hidden, head, targets, ignore_index=ignore_index, impl=impl)
             tgt, lse, nll = out[0], out[1], out[2]
             ctx.save_for_backward(hidden, targets, out, state)
@@ -472,7 +477,7 @@ class _FusedLinearCEReduced(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, weight, targets, head, ignore_index, impl, mean):
         use = DenseHead(weight=weight) if weight is not None else head
-        if weight is None and _forms_grad(impl, ctx.needs_input_grad[0]):
+        if weight is None and _forms_grad(impl, ctx.needs_input_grad[0], hidden, use, targets):
             rows, state = ce_forward_grad(hidden, use, targets, ignore_index=ignore_index, impl=impl)
             nll, saved = rows[2], [rows, state]
         else:

@@ -220,7 +220,7 @@ FwdPlan plan_fwd(const b200tp_ce_args* a, void* ws) {
   } else if (p.impl == 3) {
     p.chunk = split_chunk_rows(a, 6ll * a->d, &p.num_chunks);
     for (int64_t c = 0; c < p.num_chunks; ++c)
-      p.total_splits += 2 * ce_tc_fwd_splits(a->n, std::min<int64_t>(p.chunk, a->v_local - c * p.chunk));
+      p.total_splits += 2 * ce_split_splits(a->n, std::min<int64_t>(p.chunk, a->v_local - c * p.chunk));
     p.flag = b.take<int>(1);
     p.h3 = b.take<char>(static_cast<size_t>(a->n) * a->d * 6);
     const size_t planes = static_cast<size_t>(p.chunk) * a->d * 6;
@@ -298,12 +298,13 @@ BwdPlan plan_bwd(const b200tp_ce_args* a, int out_dtype, void* ws) {
 // forward's partial triples.
 struct GradPlan {
   bool ok;
+  int impl;              // 1 or 3, as pick_impl's
   int64_t chunk, num_chunks;
   int shares;            // partial sums of d_hidden (see ce_tc_dh_ksplit)
   int64_t total_splits;
   // state
-  int* overflow;
-  float* ref2;           // (n)
+  int* overflow;         // [0]: the sums are void; [1]: (fp32) an operand had no planes
+  float* ref2;           // (n), log2 units; fp32: natural units
   float* acc;            // (shares, n, d)
   size_t state_bytes;
   // scratch
@@ -312,12 +313,40 @@ struct GradPlan {
   float* pm; float* ps; float* pt;
   size_t bytes;          // forward
   size_t bwd_bytes;      // backward: g and deq alone, for calls whose overflow flag is set
+  // fp32: planes; `logits` overlays g's
+  void* h3; void* w3;
+  float* logits;
+  int64_t simt_chunk;
 };
 
 GradPlan plan_grad(const b200tp_ce_args* a, void* state, void* ws) {
   GradPlan p{};
-  p.ok = pick_impl(a) == 1 && a->impl != B200TP_IMPL_SIMT && (a->reserved & kReservedInline) == 0;
+  p.impl = pick_impl(a);
+  p.ok = p.impl == 3 || (p.impl == 1 && (a->reserved & kReservedInline) == 0);
   if (!p.ok) return p;
+  if (p.impl == 3) {
+    p.chunk = split_chunk_rows(a, 6ll * (a->n + a->d), &p.num_chunks);
+    p.shares = ce_split_dh_shares(a->n, a->d, p.chunk);
+    Bump st(state);
+    p.overflow = st.take<int>(2);
+    p.ref2 = st.take<float>(a->n);
+    p.acc = st.take<float>(static_cast<size_t>(p.shares) * a->n * a->d);
+    p.state_bytes = align_up(st.off, 256);
+    Bump b(ws);
+    p.g = b.take<char>(static_cast<size_t>(a->n) * p.chunk * 6);
+    p.logits = static_cast<float*>(p.g);
+    p.simt_chunk = std::min<int64_t>(a->v_local, p.chunk * 6 / 4);
+    p.bwd_bytes = align_up(b.off, 256);
+    p.h3 = b.take<char>(static_cast<size_t>(a->n) * a->d * 6);
+    p.w3 = b.take<char>(static_cast<size_t>(p.chunk) * a->d * 6);
+    for (int64_t c = 0; c < p.num_chunks; ++c)
+      p.total_splits += 2 * ce_split_splits(a->n, std::min<int64_t>(p.chunk, a->v_local - c * p.chunk));
+    p.pm = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
+    p.ps = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
+    p.pt = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
+    p.bytes = align_up(b.off, 256);
+    return p;
+  }
   p.chunk = tc_chunk_rows(a, &p.num_chunks, true);
   p.shares = ce_tc_dh_ksplit(a->n, a->d, static_cast<int>(p.chunk));
   Bump st(state);
@@ -424,7 +453,7 @@ int b200tp_linear_ce_fwd(const b200tp_ce_args* a, float* row_max, float* row_sum
       const int64_t w = std::min<int64_t>(p.chunk, a->v_local - r0);
       rc = ce_split_planes(static_cast<const float*>(a->weight) + r0 * a->d, w * a->d, p.w3, p.flag, stream);
       if (rc) return rc;
-      const int splits = ce_tc_fwd_splits(a->n, w);
+      const int splits = ce_split_splits(a->n, w);
       rc = ce_split_fwd(p.h3, p.w3, a->n, a->d, w, a->v_offset + r0, a->targets, a->ignore_index, splits,
                         p.pm + slot * a->n, p.ps + slot * a->n, p.pt + slot * a->n, stream, status);
       if (rc) return rc;
@@ -588,7 +617,7 @@ static int bwd_impl(const b200tp_ce_args* a, const float* lse, const float* cota
       rc = ce_split_planes(static_cast<const float*>(a->weight) + r0 * a->d, w * a->d, p.w3, p.flag, stream);
       if (rc) return rc;
       rc = ce_split_bwd_g(p.h3, p.w3, a->n, a->d, w, a->v_offset + r0, a->targets, a->ignore_index, lse, cotangent,
-                          ce_tc_fwd_splits(a->n, w), p.g3, p.ldg, p.flag, stream, status);
+                          ce_split_splits(a->n, w), p.g3, p.ldg, p.flag, stream, status);
       if (rc) return rc;
       rc = ce_split_dh(p.g3, p.ldg, p.w3, a->n, a->d, w, p.shares, p.shares_acc, c > 0, stream, status);
       if (rc) return rc;
@@ -677,6 +706,44 @@ int b200tp_linear_ce_fwd_grad(const b200tp_ce_args* a, float* tgt_logit, float* 
   rc = check_workspace(workspace, workspace_bytes, p.bytes);
   if (rc) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  if (p.impl == 3) {
+    const float* hidden = static_cast<const float*>(a->hidden);
+    const float* weight = static_cast<const float*>(a->weight);
+    int *void_sums = p.overflow, *bad = p.overflow + 1;
+    B200TP_CUDA_OK(cudaMemsetAsync(p.overflow, 0, 2 * sizeof(int), stream));
+    rc = ce_split_reference(hidden, weight, a->n, a->d, a->v_local, a->targets, a->ignore_index, p.ref2, stream);
+    if (rc) return rc;
+    rc = ce_split_planes(hidden, a->n * a->d, p.h3, bad, stream);
+    if (rc) return rc;
+    int64_t slot = 0;
+    for (int64_t c = 0; c < p.num_chunks; ++c) {
+      const int64_t r0 = c * p.chunk;
+      const int64_t w = std::min<int64_t>(p.chunk, a->v_local - r0);
+      rc = ce_split_planes(weight + r0 * a->d, w * a->d, p.w3, bad, stream);
+      if (rc) return rc;
+      const int splits = ce_split_splits(a->n, w);
+      rc = ce_split_fwd_grad(p.h3, p.w3, a->n, a->d, w, r0, a->targets, a->ignore_index, p.ref2, splits,
+                             p.pm + slot * a->n, p.ps + slot * a->n, p.pt + slot * a->n, p.g,
+                             static_cast<int>(p.chunk), bad, void_sums, stream, status);
+      if (rc) return rc;
+      slot += 2 * splits;
+      rc = ce_split_dh(p.g, static_cast<int>(p.chunk), p.w3, a->n, a->d, w, p.shares, p.acc, c > 0, stream, status);
+      if (rc) return rc;
+    }
+    rc = launch_combine(p.pm, p.ps, p.pt, a->n, static_cast<int>(p.total_splits), a->n, a->targets, a->ignore_index,
+                        nullptr, nullptr, tgt_logit, lse, nll, stream);
+    if (rc) return rc;
+    // void sums: the CUDA cores, here and in the backward (which wants lse from the same logits as its own); the
+    // partials' space holds their running triples
+    for (int64_t r0 = 0; r0 < a->v_local; r0 += p.simt_chunk) {
+      const int64_t w = std::min<int64_t>(p.simt_chunk, a->v_local - r0);
+      rc = ce_simt_fwd_chunk(hidden, weight + r0 * a->d, a->dtype, a->n, a->d, w, r0, a->targets, a->ignore_index,
+                             p.logits, p.pm, p.ps, tgt_logit, r0 == 0 ? 1 : 0, stream, void_sums);
+      if (rc) return rc;
+    }
+    return launch_combine(p.pm, p.ps, tgt_logit, a->n, 1, a->n, a->targets, a->ignore_index, nullptr, nullptr,
+                          tgt_logit, lse, nll, stream, void_sums);
+  }
   const QuantHead q = packed_head(a);
   rc = launch_ce_reference(a->hidden, a->weight, a->quant_bits != 0 ? &q : nullptr, a->n, a->d, a->v_local, a->targets,
                            a->ignore_index, p.ref2, p.overflow, stream);
@@ -729,6 +796,20 @@ int b200tp_linear_ce_bwd_grad(const b200tp_ce_args* a, const float* lse, const f
   rc = check_workspace(workspace, workspace_bytes, p.bwd_bytes);
   if (rc) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  if (p.impl == 3) {
+    const float* weight = static_cast<const float*>(a->weight);
+    float* out = static_cast<float*>(d_hidden);
+    rc = ce_split_finish(p.acc, p.shares, p.ref2, p.overflow, weight, a->n, a->d, a->v_local, a->targets,
+                         a->ignore_index, lse, tgt_logit, cotangent, out, stream);
+    if (rc) return rc;
+    for (int64_t r0 = 0; r0 < a->v_local; r0 += p.simt_chunk) {
+      const int64_t w = std::min<int64_t>(p.simt_chunk, a->v_local - r0);
+      rc = ce_simt_bwd_chunk(a->hidden, weight + r0 * a->d, a->dtype, a->n, a->d, w, r0, a->targets, a->ignore_index,
+                             lse, cotangent, p.logits, out, r0 > 0, stream, p.overflow);
+      if (rc) return rc;
+    }
+    return B200TP_OK;
+  }
   const QuantHead q = packed_head(a);
   rc = launch_ce_grad_finish(p.acc, p.shares, p.ref2, p.overflow, a->weight, a->quant_bits != 0 ? &q : nullptr, a->n,
                              a->d, a->v_local, a->targets, a->ignore_index, lse, tgt_logit, cotangent, d_hidden, stream);

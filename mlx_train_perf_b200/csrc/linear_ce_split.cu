@@ -15,11 +15,12 @@
 //
 //   split_planes_kernel    fp32 rows -> three bf16 planes; raises a flag on values bf16 cannot hold (inf, NaN,
 //                          within 2^-9 of the largest fp32), for which the CUDA-core kernels take over
-//   split_logits_kernel    Z = H W^T per 128 x 256 tile, K = D; row sums (FWD) or g as three planes (BWD_G)
+//   split_logits_kernel    Z = H W^T per 128 x 256 tile, K = D; row sums (FWD), g as three planes (BWD_G), or row sums
+//                          and exp(z - ref) as three planes (FWD_GRAD, as linear_ce_grad.cu does for bf16)
 //   split_dh_kernel        dH (128 x 256) (+)= G W over the chunk's vocab rows
 //   share_sum_kernel       adds the shares of a contraction that was spread over several CTAs
 //
-// Roles as in linear_ce_tc.cu, with eight accumulating warps (two per lane quadrant, 128 columns each).
+// Roles as in linear_ce_tc.cu (single CTAs), with eight accumulating warps (two per lane quadrant, 128 columns each).
 // Replaces core/chunked.py:35-90 of the reference for fp32 heads, beside linear_ce_simt.cu.
 #include "linear_ce_split.h"
 
@@ -42,7 +43,8 @@ constexpr uint32_t PLANE_B = 0u | 2u << 2 | 1u << 4 | 0u << 6 | 1u << 8 | 0u << 
 __device__ __forceinline__ int plane_a(int pr) { return (PLANE_A >> (2 * pr)) & 3; }
 __device__ __forceinline__ int plane_b(int pr) { return (PLANE_B >> (2 * pr)) & 3; }
 
-enum { SPLIT_FWD = 0, SPLIT_BWD_G = 1 };
+enum { SPLIT_FWD = 0, SPLIT_BWD_G = 1, SPLIT_FWD_GRAD = 2 };
+constexpr float kHeadroom = 69.f;   // FWD_GRAD: exponents above this raise the flag; 2^27 terms of e^69 fit fp32
 
 __device__ __forceinline__ void split3(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   hi = __bfloat16_as_ushort(__float2bfloat16_rn(x));
@@ -118,7 +120,9 @@ struct SplitLogitsParams {
   const float* ct;
   __nv_bfloat16* g;      // (3, N, ldg)
   int ldg;
-  int* flag;             // BWD_G: set when a value of g is not finite
+  const float* ref;      // FWD_GRAD: reference of the row's exponentials
+  const int* bad;        // FWD_GRAD: an operand had no planes; raises the flag
+  int* flag;             // BWD_G: set when a value of g is not finite; FWD_GRAD: when g is void
   int* status;
 };
 
@@ -274,6 +278,7 @@ split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
       const bool tvalid = row_ok && target != p.ignore_index;
       float run_m = -INFINITY, run_s = 0.f, run_t = 0.f;   // FWD
       float lse = 0.f, ct = 0.f;                           // BWD_G
+      if (MODE == SPLIT_FWD_GRAD) run_m = row_ok ? p.ref[row] : 0.f;
       if (MODE == SPLIT_BWD_G && row_ok) {
         lse = p.lse[row];
         ct = tvalid ? p.ct[row] : 0.f;
@@ -308,27 +313,54 @@ split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
         } else if (row_ok) {
           __nv_bfloat16* dst = p.g + static_cast<long long>(row) * p.ldg + col0;
           const long long plane = static_cast<long long>(p.n_rows) * p.ldg;
+          if (MODE == SPLIT_FWD_GRAD) {
+            float xm = -INFINITY;
+#pragma unroll
+            for (int e = 0; e < HALF; ++e) {
+              if (e >= ncols) acc[e] = -INFINITY;
+              if (e == tcol) run_t = acc[e];
+              acc[e] -= run_m;
+              xm = fmaxf(xm, acc[e]);
+            }
+            if (xm > kHeadroom) {   // rare: this thread's own sum moves to a larger reference; g is void then
+              bad = true;
+              run_s *= expf(-xm);
+              run_m += xm;
+#pragma unroll
+              for (int e = 0; e < HALF; ++e) acc[e] -= xm;
+            }
+          }
+          float s4[4] = {run_s, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int e = 0; e < HALF; e += 8) {
             float g[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
+              if (MODE == SPLIT_FWD_GRAD) {
+                // the target's own term p - 1 is added to d_hidden at the end
+                const float v = expf(acc[e + k]);
+                s4[k & 3] += v;
+                g[k] = tvalid && e + k != tcol ? v : 0.f;
+                continue;
+              }
               float v = expf(acc[e + k] - lse);
               if (e + k == tcol) v -= 1.f;
               g[k] = e + k < ncols ? v * ct : 0.f;
             }
             bad = split_store8(g, dst + e, plane) || bad;
           }
+          if (MODE == SPLIT_FWD_GRAD) run_s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
         }
       }
-      if (MODE == SPLIT_FWD && ok && row_ok) {
+      if (MODE != SPLIT_BWD_G && ok && row_ok) {
         const size_t o = static_cast<size_t>(split * 2 + half) * p.n_rows + row;
         p.pm[o] = run_m;
         p.ps[o] = run_s;
         p.pt[o] = run_t;
       }
     }
-    if (MODE == SPLIT_BWD_G && bad) *p.flag = 1;
+    if (MODE != SPLIT_FWD && bad) *p.flag = 1;
+    if (MODE == SPLIT_FWD_GRAD && blockIdx.x == 0 && warp == 2 && lane == 0 && *p.bad != 0) *p.flag = 1;
   }
   cta_teardown(sm, warp, tmem_base);
 }
@@ -407,6 +439,44 @@ split_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constan
   cta_teardown(sm, warp, tmem_base);
 }
 
+// ref[row] = the target's logit (any vocab row's, where there is no target).  One warp per row; no alignment wanted.
+__global__ void __launch_bounds__(128)
+split_reference_kernel(const float* __restrict__ hidden, const float* __restrict__ w, int n, int d, long long v,
+                       const long long* __restrict__ targets, long long ignore_index, float* __restrict__ ref) {
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= n) return;
+  const long long tg = targets[row], t = tg != ignore_index && tg >= 0 && tg < v ? tg : 0;
+  const float *h = hidden + static_cast<long long>(row) * d, *wt = w + t * d;
+  float acc = 0.f;
+#pragma unroll 8
+  for (int i = lane; i < d; i += 32) acc = fmaf(__ldg(h + i), __ldg(wt + i), acc);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) ref[row] = acc;
+}
+
+// d_hidden = ct (exp(ref - lse) sum of shares + (p_t - 1) W_t); HBM-bound, one column per thread.
+__global__ void __launch_bounds__(256)
+split_finish_kernel(const float* __restrict__ acc, int shares, const float* __restrict__ ref,
+                    const int* __restrict__ skip_if_set, const float* __restrict__ w, int n, int d, long long v,
+                    const long long* __restrict__ targets, long long ignore_index, const float* __restrict__ lse,
+                    const float* __restrict__ tgt, const float* __restrict__ ct, float* __restrict__ out) {
+  const int row = blockIdx.x, i = blockIdx.y * 256 + threadIdx.x;
+  if (*skip_if_set != 0 || i >= d) return;
+  const long long off = static_cast<long long>(row) * d + i, t = targets[row];
+  if (t == ignore_index) {
+    out[off] = 0.f;
+    return;
+  }
+  float s = 0.f;
+#pragma unroll 4
+  for (int k = 0; k < shares; ++k) s += __ldcs(acc + static_cast<long long>(k) * n * d + off);
+  const float c = ct[row], l = lse[row];
+  float g = expf(ref[row] - l) * s;
+  if (t >= 0 && t < v) g = fmaf(expm1f(tgt[row] - l), __ldg(w + t * d + i), g);
+  out[off] = c * g;
+}
+
 std::atomic<int> g_configured[64];
 
 int configure() {
@@ -417,6 +487,8 @@ int configure() {
                                       SMEM_BYTES));
   B200TP_CUDA_OK(cudaFuncSetAttribute(split_logits_kernel<SPLIT_BWD_G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       SMEM_BYTES));
+  B200TP_CUDA_OK(cudaFuncSetAttribute(split_logits_kernel<SPLIT_FWD_GRAD>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   B200TP_CUDA_OK(cudaFuncSetAttribute(split_dh_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   if (dev >= 0 && dev < 64) g_configured[dev].store(1, std::memory_order_release);
   return B200TP_OK;
@@ -449,6 +521,10 @@ int launch_logits(const void* h3, const void* w3, int64_t n, int d, int64_t widt
 }
 
 }  // namespace
+
+int ce_split_splits(int64_t n, int64_t width) {
+  return ce_tc_choose_splits(static_cast<int>(ceil_div(n, BM)), static_cast<int>(ceil_div(width, BN)));
+}
 
 int ce_split_planes(const float* x, int64_t count, void* planes, int* flag, cudaStream_t stream) {
   const unsigned blocks = static_cast<unsigned>(ceil_div(count, 256 * 8));
@@ -491,6 +567,45 @@ int ce_split_bwd_g(const void* h3, const void* w3, int64_t n, int d, int64_t wid
   p.ldg = ldg;
   p.status = status;
   return launch_logits<SPLIT_BWD_G>(h3, w3, n, d, width, p, stream);
+}
+
+int ce_split_reference(const float* hidden, const float* w, int64_t n, int d, int64_t v, const int64_t* targets,
+                       int64_t ignore_index, float* ref, cudaStream_t stream) {
+  split_reference_kernel<<<static_cast<unsigned>(ceil_div(n, 4)), 128, 0, stream>>>(
+      hidden, w, static_cast<int>(n), d, v, reinterpret_cast<const long long*>(targets), ignore_index, ref);
+  B200TP_CUDA_OK(cudaGetLastError());
+  return B200TP_OK;
+}
+
+int ce_split_fwd_grad(const void* h3, const void* w3, int64_t n, int d, int64_t width, int64_t vocab_id0,
+                      const int64_t* targets, int64_t ignore_index, const float* ref, int splits, float* pm, float* ps,
+                      float* pt, void* g3, int ldg, const int* bad, int* flag, cudaStream_t stream, int* status) {
+  SplitLogitsParams p{};
+  p.vocab_id0 = vocab_id0;
+  p.splits = splits;
+  p.targets = reinterpret_cast<const long long*>(targets);
+  p.ignore_index = ignore_index;
+  p.pm = pm;
+  p.ps = ps;
+  p.pt = pt;
+  p.g = static_cast<__nv_bfloat16*>(g3);
+  p.ldg = ldg;
+  p.ref = ref;
+  p.bad = bad;
+  p.flag = flag;
+  p.status = status;
+  return launch_logits<SPLIT_FWD_GRAD>(h3, w3, n, d, width, p, stream);
+}
+
+int ce_split_finish(const float* acc, int shares, const float* ref, const int* skip_if_set, const float* w, int64_t n,
+                    int d, int64_t v, const int64_t* targets, int64_t ignore_index, const float* lse, const float* tgt,
+                    const float* ct, float* out, cudaStream_t stream) {
+  const dim3 grid(static_cast<unsigned>(n), static_cast<unsigned>(ceil_div(d, 256)));
+  split_finish_kernel<<<grid, 256, 0, stream>>>(acc, shares, ref, skip_if_set, w, static_cast<int>(n), d, v,
+                                                reinterpret_cast<const long long*>(targets), ignore_index, lse, tgt,
+                                                ct, out);
+  B200TP_CUDA_OK(cudaGetLastError());
+  return B200TP_OK;
 }
 
 // Shares of the d_hidden contraction: the fewest that keep the busiest CTA's work (k blocks, plus about two per unit

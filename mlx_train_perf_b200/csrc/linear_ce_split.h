@@ -11,6 +11,9 @@ namespace b200tp {
 // largest fp32 that bf16 rounds it to infinity).
 int ce_split_planes(const float* x, int64_t count, void* planes, int* flag, cudaStream_t stream);
 
+// Vocab shares of a logits launch.
+int ce_split_splits(int64_t n, int64_t width);
+
 // Forward partials of one vocab chunk (`width` rows from `vocab_id0`): 2 * splits triples per row.
 int ce_split_fwd(const void* h3, const void* w3, int64_t n, int d, int64_t width, int64_t vocab_id0,
                  const int64_t* targets, int64_t ignore_index, int splits, float* pm, float* ps, float* pt,
@@ -21,6 +24,19 @@ int ce_split_fwd(const void* h3, const void* w3, int64_t n, int d, int64_t width
 int ce_split_bwd_g(const void* h3, const void* w3, int64_t n, int d, int64_t width, int64_t vocab_id0,
                    const int64_t* targets, int64_t ignore_index, const float* lse, const float* ct, int splits,
                    void* g3, int ldg, int* flag, cudaStream_t stream, int* status);
+
+// The forward that also forms the gradient's sum (see linear_ce_grad.h): ref, then per chunk the partials and
+// g3 = exp(z - ref), zero at the target and on ignored rows; *flag is set when g3 is void (a logit more than 69 above
+// its reference, or *bad), the partials are right unless *bad.
+int ce_split_reference(const float* hidden, const float* w, int64_t n, int d, int64_t v, const int64_t* targets,
+                       int64_t ignore_index, float* ref, cudaStream_t stream);
+int ce_split_fwd_grad(const void* h3, const void* w3, int64_t n, int d, int64_t width, int64_t vocab_id0,
+                      const int64_t* targets, int64_t ignore_index, const float* ref, int splits, float* pm, float* ps,
+                      float* pt, void* g3, int ldg, const int* bad, int* flag, cudaStream_t stream, int* status);
+// d_hidden from the shares' sums; nothing while *skip_if_set is set.
+int ce_split_finish(const float* acc, int shares, const float* ref, const int* skip_if_set, const float* w, int64_t n,
+                    int d, int64_t v, const int64_t* targets, int64_t ignore_index, const float* lse, const float* tgt,
+                    const float* ct, float* out, cudaStream_t stream);
 
 // out (ksplit shares of (n, d) fp32, `keep`: added to) = g @ w over the chunk.
 int ce_split_dh_shares(int64_t n, int d, int64_t width);

@@ -95,3 +95,47 @@ def test_values_without_planes(cuda_device, what):
             assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
             continue
         assert torch.equal(a.nan_to_num(7e7), b.nan_to_num(7e7))
+
+
+@pytest.mark.parametrize(("n", "d", "v", "push"), [(1, 64, 257, 3.0), (129, 136, 4099, 20.0), (60, 1024, 17000, 20.0),
+                                                   (40, 264, 2500, -90.0)])
+def test_forward_that_forms_the_gradient(cuda_device, n, d, v, push):
+    """Same bounds as above; at push -90 logits lie 69 and more above the target's and the CUDA cores take over."""
+    dev, (h, w, t) = cuda_device, _inputs(n, d, v)
+    h = h + torch.linspace(0, push - 20, n)[:, None] * w[t]
+    ct = torch.linspace(-1, 1.5, n)
+    r_nll, r_lse, _ = oc.naive_linear_ce(h, w, t, dtype=torch.float64)
+    r_dh, _ = oc.chunked_backward(h, w, t, r_lse, ct.double(), chunk_size=4096, dtype=torch.float64)
+    assert push > 0 or r_nll.max() > 75
+    hd, td, head = h.to(dev), t.to(dev), DenseHead(w.to(dev), trainable=False)
+    rows, state = L.ce_forward_grad(hd, head, td, impl="split")
+    got = [L.ce_backward_grad(hd, head, td, rows, state, ct.to(dev), impl="split") for _ in range(2)]
+    L.check_device_status()
+    assert torch.equal(got[0], got[1])
+    s_nll, s_lse, _, s_dh = _run(dev, h, w, t, ct, impl="simt")
+    if push < 0:
+        for a, b in ((rows[1], s_lse), (rows[2], s_nll), (got[0], s_dh)):
+            assert torch.equal(a.cpu(), b)
+        return
+    _, lse, nll = rows.double().cpu()
+    dh, ok = got[0].double().cpu(), t != -100
+    z = (9 + d / 128) * 2.0 ** -23 * h.double().norm(dim=1) * w.double().norm(dim=1).max() + 2.0 ** -22 * (1 + r_lse.abs())
+    assert ((lse - r_lse).abs() <= z).all() and ((nll - r_nll).abs() <= 2 * z)[ok].all()
+    wn = w.double().norm(dim=1).max()
+    assert ((dh - r_dh).norm(dim=1) <= ct.double().abs() * wn * 2 * (2 * z + (9 + v / 128) * 2.0 ** -23) + 1e-12).all()
+    # no less precise than the recomputing form, up to the last rounding of the results
+    assert (dh - r_dh).norm() <= (s_dh.double() - r_dh).norm() + 2.0 ** -24 * r_dh.norm()
+
+
+def test_forward_that_forms_the_gradient_without_planes(cuda_device):
+    h, w, t = _inputs(40, 64, 700)
+    w[5] = 0
+    w[5, 3] = -math.inf
+    h[:, 3] = h[:, 3].abs() + 0.1
+    dev, ct = cuda_device, torch.ones(40)
+    hd, td, head = h.to(dev), t.to(dev), DenseHead(w.to(dev), trainable=False)
+    rows, state = L.ce_forward_grad(hd, head, td, impl="split")
+    dh = L.ce_backward_grad(hd, head, td, rows, state, ct.to(dev), impl="split")
+    nll, lse, tgt, s_dh = _run(dev, h, w, t, ct, impl="simt")
+    for a, b in ((rows[0], tgt), (rows[1], lse), (rows[2], nll), (dh, s_dh)):
+        assert torch.equal(a.cpu().nan_to_num(7e7), b.nan_to_num(7e7))
