@@ -203,14 +203,14 @@ FwdPlan plan_fwd(const b200tp_ce_args* a, void* ws) {
       p.chunk = a->v_local;
       p.num_chunks = 1;
       p.int4 = a->quant_bits != 0 && (a->reserved & kReservedInline) == 0;
-      p.total_splits = p.int4 ? ce_int4_fwd_splits(a->n, a->v_local) : ce_tc_fwd_splits(a->n, a->v_local);
+      p.total_splits = p.int4 ? ce_int4_fwd_splits(a->n, a->v_local) : ce_tc_fwd_splits(a->n, a->d, a->v_local);
     } else {
       // 4-bit head, chunked: dequantise a chunk of vocab rows, run the dense kernel over it
       p.chunk = tc_chunk_rows(a, &p.num_chunks);
       p.total_splits = 0;
       for (int64_t c = 0; c < p.num_chunks; ++c) {
         const int64_t w = std::min<int64_t>(p.chunk, a->v_local - c * p.chunk);
-        p.total_splits += ce_tc_fwd_splits(a->n, w);
+        p.total_splits += ce_tc_fwd_splits(a->n, a->d, w);
       }
       p.deq = b.take<char>(static_cast<size_t>(p.chunk) * a->d * 2);
     }
@@ -359,7 +359,7 @@ GradPlan plan_grad(const b200tp_ce_args* a, void* state, void* ws) {
   if (a->quant_bits != 0) p.deq = b.take<char>(static_cast<size_t>(p.chunk) * a->d * 2);
   p.bwd_bytes = align_up(b.off, 256);
   for (int64_t c = 0; c < p.num_chunks; ++c)
-    p.total_splits += ce_tc_fwd_splits(a->n, std::min<int64_t>(p.chunk, a->v_local - c * p.chunk));
+    p.total_splits += ce_tc_fwd_splits(a->n, a->d, std::min<int64_t>(p.chunk, a->v_local - c * p.chunk));
   p.pm = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
   p.ps = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
   p.pt = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
@@ -431,7 +431,7 @@ int b200tp_linear_ce_fwd(const b200tp_ce_args* a, float* row_max, float* row_sum
         rc = launch_dequant_int4(a->w_q, a->scales, a->biases, a->qparam_dtype, r0, w, a->d, a->group_size, p.deq,
                                  B200TP_BF16, stream);
         if (rc) return rc;
-        const int splits = ce_tc_fwd_splits(a->n, w);
+        const int splits = ce_tc_fwd_splits(a->n, a->d, w);
         rc = ce_tc_launch_fwd(a->hidden, p.deq, w, a->n, a->d, 0, w, a->v_offset + r0, a->targets, a->ignore_index,
                               splits, p.pm + slot * a->n, p.ps + slot * a->n, p.pt + slot * a->n, nullptr, stream,
                               status);
@@ -763,7 +763,7 @@ int b200tp_linear_ce_fwd_grad(const b200tp_ce_args* a, float* tgt_logit, float* 
       row0 = 0;
       vocab_id0 = r0;
     }
-    const int splits = ce_tc_fwd_splits(a->n, w);
+    const int splits = ce_tc_fwd_splits(a->n, a->d, w);
     rc = ce_tc_launch_fwd_grad(a->hidden, wmat, wrows, a->n, a->d, row0, row0 + w, vocab_id0, a->targets,
                                a->ignore_index, p.ref2, p.overflow, splits, p.pm + slot * a->n, p.ps + slot * a->n,
                                p.pt + slot * a->n, p.g, static_cast<int>(p.chunk), stream, status);

@@ -15,6 +15,10 @@ constexpr int STAGES = 4;
 constexpr int A_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int B_BYTES = BN * BK * 2;  // 32 KiB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+// CTA pairs: a CTA holds half of B's tile, so its ring has six stages in the same space
+constexpr int PAIR_STAGES = 6;
+constexpr int PAIR_STAGE_BYTES = A_BYTES + B_BYTES / 2;
+static_assert(PAIR_STAGES * PAIR_STAGE_BYTES == STAGES * STAGE_BYTES, "one ring size");
 constexpr int DQ_WARPS = 8;                       // dequantising warps of the QUANT kernels
 constexpr int CODE_BYTES = 32 * 1024;             // QUANT: ring of packed-code tiles filled by TMA
 constexpr int CODE_SLOTS_LOGITS = 2;              // 256 rows x 64 B (two k blocks) = 16 KiB each
@@ -26,6 +30,7 @@ constexpr uint32_t TMEM_COLS = 512;                                  // two 256-
 
 struct SmemView {
   uint8_t* base;
+  int stages, stage_bytes;
   uint64_t* full;
   uint64_t* empty;
   uint64_t* tfull;
@@ -35,24 +40,26 @@ struct SmemView {
   uint8_t* codes;       // QUANT only
   uint64_t* cfull;      // [4]
   uint64_t* cempty;     // [4]
-  __device__ uint8_t* a(int s) const { return base + s * STAGE_BYTES; }
-  __device__ uint8_t* b(int s) const { return base + s * STAGE_BYTES + A_BYTES; }
+  __device__ uint8_t* a(int s) const { return base + s * stage_bytes; }
+  __device__ uint8_t* b(int s) const { return base + s * stage_bytes + A_BYTES; }
 };
 
-__device__ __forceinline__ SmemView carve_smem(uint8_t* raw, bool quant = false) {
+__device__ __forceinline__ SmemView carve_smem(uint8_t* raw, bool quant = false, bool pair = false) {
   const uint32_t addr = smem_u32(raw);
   const uint32_t aligned = (addr + 1023u) & ~1023u;
   SmemView v;
   v.base = raw + (aligned - addr);
+  v.stages = pair ? PAIR_STAGES : STAGES;
+  v.stage_bytes = pair ? PAIR_STAGE_BYTES : STAGE_BYTES;
   v.codes = v.base + STAGES * STAGE_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(v.base + STAGES * STAGE_BYTES + (quant ? CODE_BYTES : 0));
   v.cfull = bars + 2 * STAGES + 6;
   v.cempty = bars + 2 * STAGES + 10;
   v.full = bars;
-  v.empty = bars + STAGES;
-  v.tfull = bars + 2 * STAGES;
-  v.tempty = bars + 2 * STAGES + 2;
-  v.tmem_ptr = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  v.empty = bars + v.stages;
+  v.tfull = bars + 2 * v.stages;
+  v.tempty = bars + 2 * v.stages + 2;
+  v.tmem_ptr = reinterpret_cast<uint32_t*>(bars + 2 * v.stages + 4);
   v.abort_flag = reinterpret_cast<int*>(v.tmem_ptr + 1);
   return v;
 }
@@ -64,9 +71,9 @@ __device__ __forceinline__ void raise_abort(const SmemView& sm, int* status, int
 
 // Common prologue: barriers, TMEM allocation.  Returns the TMEM base address.
 __device__ __forceinline__ uint32_t cta_setup(const SmemView& sm, int warp, uint32_t full_count = 1,
-                                              uint32_t epi_warps = 4) {
+                                              uint32_t epi_warps = 4, bool pair = false) {
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < sm.stages; ++s) {
       mbar_init(&sm.full[s], full_count);   // the TMA producer's arrive.expect_tx (+ one per dequantising warp)
       mbar_init(&sm.empty[s], 1);
     }
@@ -84,29 +91,38 @@ __device__ __forceinline__ uint32_t cta_setup(const SmemView& sm, int warp, uint
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc(sm.tmem_ptr, TMEM_COLS);
-    tmem_relinquish();
+    if (pair) {
+      tmem_alloc_pair(sm.tmem_ptr, TMEM_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(sm.tmem_ptr, TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before_sync();
-  __syncthreads();
+  if (pair) cluster_sync();   // the other CTA's barriers are initialised too
+  else __syncthreads();
   tc_fence_after_sync();
   return *reinterpret_cast<volatile uint32_t*>(sm.tmem_ptr);
 }
 
-__device__ __forceinline__ void cta_teardown(const SmemView& sm, int warp, uint32_t tmem_base) {
+// (A pair leaves together: until then the other CTA's MMAs, commits and arrivals may reach into this one.)
+__device__ __forceinline__ void cta_teardown(const SmemView& sm, int warp, uint32_t tmem_base, bool pair = false) {
   tc_fence_before_sync();
-  __syncthreads();
+  if (pair) cluster_sync();
+  else __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if (pair) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
 // After an abort the producer may still have bulk copies in flight into this CTA's shared
 // memory: wait (bounded) for every stage it armed before the CTA is allowed to retire.
 __device__ __forceinline__ void producer_drain(const SmemView& sm, uint32_t it) {
-  const uint32_t first = it > STAGES ? it - STAGES : 0;
-  for (uint32_t j = first; j < it; ++j) mbar_wait_drain(&sm.full[j % STAGES], (j / STAGES) & 1);
+  const uint32_t n = sm.stages, first = it > n ? it - n : 0;
+  for (uint32_t j = first; j < it; ++j) mbar_wait_drain(&sm.full[j % n], (j / n) & 1);
 }
 
 }  // namespace

@@ -80,11 +80,15 @@ extern "C" int b200tp_linear_ce_fwd_static(const b200tp_ce_args* a, float* row_m
                 "use b200tp_linear_ce_fwd");
   int rc = require_sm100();
   if (rc) return rc;
-  const int splits = ce_tc_fwd_splits(a->n, a->v_local);
-  const size_t need = 3ull * static_cast<size_t>(splits) * static_cast<size_t>(a->n) * sizeof(float);
+  // as many shares as the kernel likes, and no more than single-CTA tiles would take: what fits does not depend on
+  // which of the two runs
+  const int most = ce_tc_choose_splits(static_cast<int>(ceil_div(a->n, kCeTileRows)),
+                                       static_cast<int>(ceil_div(a->v_local, kCeTileCols)));
+  const int splits = std::min(most, ce_tc_fwd_splits(a->n, a->d, a->v_local));
+  const size_t need = 3ull * static_cast<size_t>(most) * static_cast<size_t>(a->n) * sizeof(float);
   if (need > kStaticScratchBytes)
     return fail(B200TP_ERR_WORKSPACE,
-                "shape needs " + std::to_string(need) + " bytes of partial triples (3 x " + std::to_string(splits) +
+                "shape needs " + std::to_string(need) + " bytes of partial triples (3 x " + std::to_string(most) +
                     " splits x " + std::to_string(a->n) + " rows x 4), more than the built-in " +
                     std::to_string(kStaticScratchBytes) + "-byte scratch; use b200tp_linear_ce_fwd with a workspace");
   float* scratch = nullptr;

@@ -27,7 +27,7 @@ struct LaunchGuard {
 
 // Vocab splits the forward uses for (n rows, v_rows vocab rows): one partial triple per
 // (row, split) lands in the workspace.
-int ce_tc_fwd_splits(int64_t n, int64_t v_rows);
+int ce_tc_fwd_splits(int64_t n, int d, int64_t v_rows);
 // The split count behind it, for `num_rb` row groups and `num_vt` vocab tiles.
 int ce_tc_choose_splits(int num_rb, int num_vt);
 
