@@ -381,13 +381,6 @@ __global__ void dequant_int4_kernel(const uint32_t* __restrict__ wq, const TP* _
   }
 }
 
-// One 32-byte store (a whole sector); `p` 32-byte aligned.
-__device__ __forceinline__ void st_global_32b(void* p, const uint32_t (&v)[8]) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
-               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-               : "memory");
-}
-
 // Four packed words (32 codes of one group) per thread: one 16-byte load, one scale / bias pair, and the
 // thread's 64 (bf16) or 128 (fp32) contiguous output bytes as whole 32-byte sectors (`st.global.v8.b32`).
 // Needs d % 32 == 0, group % 32 == 0 and 32-byte aligned output rows.  (A variant whose warps wrote 512

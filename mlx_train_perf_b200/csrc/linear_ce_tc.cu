@@ -86,6 +86,15 @@ __device__ __forceinline__ void release_acc(uint64_t* bar) {
   else mbar_arrive(bar);
 }
 
+// 32 columns of a row of g as whole sectors.  With 16-byte stores every sector was written in two halves, and at
+// D = 1024 the L2 took them no faster than the tensor cores made them (15194 vocab rows x 4096 rows: 115 -> 90 us).
+__device__ __forceinline__ void store_g(__nv_bfloat16* dst, const uint32_t (&v)[16]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    st_global_32b(dst + h * 16, {v[8 * h], v[8 * h + 1], v[8 * h + 2], v[8 * h + 3], v[8 * h + 4], v[8 * h + 5],
+                                 v[8 * h + 6], v[8 * h + 7]});
+}
+
 struct LogitsParams {
   int n_rows;            // N
   int k_dim;             // D
@@ -496,10 +505,7 @@ ce_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_consta
             }
             run_s += (acc4[0] + acc4[1]) + (acc4[2] + acc4[3]);
             if (row_ok) {
-              uint4* dst = reinterpret_cast<uint4*>(p.g + static_cast<size_t>(row) * p.ldg + (vt * BN + c * 32));
-#pragma unroll
-              for (int q4 = 0; q4 < 4; ++q4)
-                dst[q4] = make_uint4(packed[4 * q4], packed[4 * q4 + 1], packed[4 * q4 + 2], packed[4 * q4 + 3]);
+              store_g(p.g + static_cast<size_t>(row) * p.ldg + (vt * BN + c * 32), packed);
             }
           } else {
             uint32_t packed[16];
@@ -514,10 +520,7 @@ ce_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_consta
               packed[j >> 1] = pack_bf16x2(g0, g1);
             }
             if (row_ok) {
-              uint4* dst = reinterpret_cast<uint4*>(p.g + static_cast<size_t>(row) * p.ldg + vt * BN + c * 32);
-#pragma unroll
-              for (int q4 = 0; q4 < 4; ++q4)
-                dst[q4] = make_uint4(packed[4 * q4], packed[4 * q4 + 1], packed[4 * q4 + 2], packed[4 * q4 + 3]);
+              store_g(p.g + static_cast<size_t>(row) * p.ldg + vt * BN + c * 32, packed);
             }
           }
         }
