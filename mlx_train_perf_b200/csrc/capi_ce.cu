@@ -38,19 +38,25 @@ constexpr int kReservedChunked = 0x20000;   // 4-bit head: dequantise chunk by c
 constexpr int kReservedSplit = 0x40000;     // fp32, dense head: the tensor cores whatever the size
 constexpr int64_t kInlineMaxRows = 2048;    // default: the forward expands in the kernel up to this many rows of hidden
 
-// `grow` (the forward that also forms the gradient, dense heads): few rows take wider chunks, up to the scratch that
+// `grow` (the forward that also forms the gradient): few rows take wider chunks, up to the scratch that
 // 8192 rows use anyway.  A chunk ends in a partly filled wave of tiles and an fp32 round trip of d_hidden in each of
 // its two GEMMs: at 1000 x 4096 x 151936 ten chunks make 40 tile times of logits out of 32.1 full waves, two make
 // 34 (training step 2.63 -> 2.30 ms; 60 x 1024 x 32768 in one chunk instead of two: GPU time 94 -> 58 us).
+// A 4-bit head's chunk is dequantised too: at most twice the rows of the default, within what both tiles take at 8192
+// rows and D = 4096 (2048 x 4096 x 151936: training step 4.64 -> 4.46 ms).
 constexpr int64_t kGrowScratchBytes = 256ll << 20;
+constexpr int64_t kGrowQuantBytes = 384ll << 20, kGrowQuantRows = 2 * kTcChunkRowsMax;
 
 int64_t tc_chunk_rows(const b200tp_ce_args* a, int64_t* num_chunks, bool grow = false) {
   int64_t bound = static_cast<int64_t>(a->reserved & 0xFFFF) * kCeTileCols;
   if (bound <= 0) {
     const int64_t fit = kTcScratchBytes / (2 * std::max<int64_t>(a->n, 1)) / kCeTileCols * kCeTileCols;
     bound = std::min(kTcChunkRowsMax, std::max(kTcChunkRowsMin, fit));
-    if (grow && a->quant_bits == 0)
-      bound = std::max(bound, kGrowScratchBytes / (2 * a->n) / kCeTileCols * kCeTileCols);
+    if (grow) {
+      const int64_t fits = a->quant_bits == 0 ? kGrowScratchBytes / (2 * a->n)
+                                              : std::min(kGrowQuantRows, kGrowQuantBytes / (2 * (a->n + a->d)));
+      bound = std::max(bound, fits / kCeTileCols * kCeTileCols);
+    }
   }
   const int64_t nc = ceil_div(a->v_local, bound);
   *num_chunks = nc;
