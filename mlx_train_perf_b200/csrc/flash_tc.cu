@@ -16,6 +16,7 @@
 //                      On a grid smaller than the SM count with long sequences, 2-4 CTAs share
 //                      each query block's key range and write un-normalised fp32 partials;
 //   flash_fwd_combine_kernel  merges those partials into O and L.
+//                      At head_dim 64 one tile per CTA and two CTAs per SM.
 //   flash_fwd_kernel   one tile per CTA, P through shared memory: taken for small grids that are
 //                      not split, and selectable as a cross-check of the two-tile kernel.
 //   flash_dq_kernel    one CTA per (batch, q head, 128-query block): Q and dO staged into tensor
@@ -556,11 +557,20 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 // of its tile.  The two warps of a row exchange their block maxima (and, once, their row sums)
 // through shared memory with a two-arrival mbarrier; that exchange also orders "both have loaded
 // their S values" before either overwrites S columns with P.
-constexpr int FWD2_SM_WARPS = 16;
-constexpr int FWD2_THREADS = 64 + 32 * FWD2_SM_WARPS;
 constexpr int FWD2_RING = 4;
 constexpr int FWD2_XCHG_BYTES = 2 * 2 * TILE * 4;       // [tile][column half][row] fp32 block maxima
-constexpr int FWD2_SMEM_BYTES = (2 + FWD2_RING) * TILE_BYTES + 256 + FWD2_XCHG_BYTES + 1024;
+// One tile per CTA (head_dim 64): half of the threads and of tensor memory and 16 KiB tiles, so an SM holds two CTAs.
+// The same two tiles are in flight, but a CTA's start and end overlap the other's work and the causal triangle is cut
+// into smaller pieces; in exchange a K / V tile is brought in once per tile, which 16 KiB tiles leave room for.
+// Forward, 32 / 8 heads, two tiles against one: 2 x 2500 tokens 111 / 101 us, 1 x 8192 439 / 394; 12 / 4 heads, 1 x 16384
+// 629 / 568.
+template <int D, int TILES>
+__host__ __device__ constexpr int fwd2_tile_bytes() { return TILES == 1 && D == 64 ? SUB_BYTES : TILE_BYTES; }
+template <int D, int TILES>
+constexpr int fwd2_smem_bytes() {
+  return (TILES + FWD2_RING) * fwd2_tile_bytes<D, TILES>() + 256 + FWD2_XCHG_BYTES + 1024;
+}
+constexpr int fwd2_threads(int tiles) { return 64 + 256 * tiles; }
 constexpr float kRescaleSlack = 8.f;
 
 struct Fwd2Tile {
@@ -588,7 +598,7 @@ __device__ __forceinline__ void mma_pv(uint32_t d_tmem, uint32_t p_tmem, uint32_
 }
 
 // 18 warps: five share one scheduler's 16 K registers, so 96 per thread is the most a launch accepts
-template <int D>
+template <int D, int TILES = 2>
 __global__ void __maxnreg__(96)
 flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                   const __grid_constant__ CUtensorMap tmap_v, const AttnParams p, const int head_pair) {
@@ -596,8 +606,9 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = align1024(smem_raw);
   uint8_t* q_sm = sm;                                   // [2]
-  uint8_t* ring_sm = sm + 2 * TILE_BYTES;               // [FWD2_RING]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + (2 + FWD2_RING) * TILE_BYTES);
+  constexpr int kTile = fwd2_tile_bytes<D, TILES>();
+  uint8_t* ring_sm = sm + TILES * kTile;                // [FWD2_RING]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + (TILES + FWD2_RING) * kTile);
   uint64_t* q_full = bars;
   uint64_t* kv_full = bars + 1;                   // [FWD2_RING]
   uint64_t* kv_empty = bars + 1 + FWD2_RING;      // [FWD2_RING]
@@ -606,7 +617,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   uint64_t* o_final = s_full + 4;                 // [2] per tile: the last P V is complete
   uint64_t* xb = s_full + 6;                      // [2][4] per (tile, quadrant): the row pair's exchange
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(s_full + 14);
-  float* xchg = reinterpret_cast<float*>(sm + (2 + FWD2_RING) * TILE_BYTES + 256);
+  float* xchg = reinterpret_cast<float*>(sm + (TILES + FWD2_RING) * kTile + 256);
   int* abort_flag = reinterpret_cast<int*>(tmem_ptr + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // provably warp-uniform
@@ -623,7 +634,11 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   // the heaviest block are still dispatched before any lighter block
   const int yslot = p.nsplit > 1 ? blockIdx.z : blockIdx.y, ny = p.nsplit > 1 ? gridDim.z : gridDim.y;
   Fwd2Tile tl[2];
-  if (head_pair) {
+  if (TILES == 1) {
+    const int qi = ny - 1 - yslot;
+    tl[0] = {qi * TILE, hslot, 0, qi, 1};
+    tl[1] = {0, hslot, 0, -1, 0};
+  } else if (head_pair) {
     const int qi = ny - 1 - yslot;
     for (int t = 0; t < 2; ++t) tl[t] = {qi * TILE, 2 * hslot + t, 0, qi, 1};
   } else {
@@ -682,7 +697,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_ptr, TMEM_COLS);
+    tmem_alloc(tmem_ptr, TILES * 256);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -698,7 +713,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       tma_prefetch_desc(&tmap_v);
       mbar_arrive_expect_tx(q_full, (tl[1].active ? 2 : 1) * tile_tx_bytes<D>());
       load_tile<D>(q_sm, &tmap_q, q_full, tl[0].q0, tl[0].h, b);
-      if (tl[1].active) load_tile<D>(q_sm + TILE_BYTES, &tmap_q, q_full, tl[1].q0, tl[1].h, b);
+      if (tl[1].active) load_tile<D>(q_sm + kTile, &tmap_q, q_full, tl[1].q0, tl[1].h, b);
       int issued = 0;
       bool ok = true;
       const int total = 2 * (jmax - jmin + 1);
@@ -710,7 +725,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           break;
         }
         mbar_arrive_expect_tx(&kv_full[slot], tile_tx_bytes<D>());
-        load_tile<D>(ring_sm + slot * TILE_BYTES, (idx & 1) ? &tmap_v : &tmap_k, &kv_full[slot],
+        load_tile<D>(ring_sm + slot * kTile, (idx & 1) ? &tmap_v : &tmap_k, &kv_full[slot],
                      (jmin + (idx >> 1)) * TILE, kvh, b);
         ++issued;
       }
@@ -743,11 +758,11 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         tc_fence_after_sync();
         if (elect_one()) {
           if (has_prev) {
-            mma_pv<D>(tmem_base + 256 + t * 128, tmem_base + t * 128, ring_a + v_slot * TILE_BYTES, np[t] > 0);
+            mma_pv<D>(tmem_base + TILES * 128 + t * 128, tmem_base + t * 128, ring_a + v_slot * kTile, np[t] > 0);
             if (j - 1 == tl[t].jhi) umma_commit(&o_final[t]);
           }
           if (has_cur) {
-            mma_kk<D>(tmem_base + t * 128, q_a + t * TILE_BYTES, ring_a + k_slot * TILE_BYTES, false);
+            mma_kk<D>(tmem_base + t * 128, q_a + t * kTile, ring_a + k_slot * kTile, false);
             umma_commit(&s_full[t]);
           }
         }
@@ -784,7 +799,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const int igc = min(ig, p.S - 1);
       const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
       const uint32_t tm_s = tmem_base + t * 128 + lane_off;
-      const uint32_t tm_o = tmem_base + 256 + t * 128 + lane_off + ch * 64;
+      const uint32_t tm_o = tmem_base + TILES * 128 + t * 128 + lane_off + ch * 64;
       uint64_t* my_xb = &xb[t * 4 + quad];
       // exchange slots: block maxima xchg[(t * 2 + half) * 128 + row] (single-buffered: a warp
       // writes block n+1's value only after its partner has arrived on p_full for block n, i.e. after
@@ -792,7 +807,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       // tile's Q buffer, which nothing reads once the tile's last MMA has completed.
       auto slot = [&](int half) -> volatile float* { return xchg + (t * 2 + half) * TILE + r; };
       auto sum_slot = [&](int half) -> volatile float* {
-        return reinterpret_cast<float*>(q_sm + t * TILE_BYTES) + half * TILE + r;
+        return reinterpret_cast<float*>(q_sm + t * kTile) + half * TILE + r;
       };
       const int row_lo = packed ? segment_first(segs, p.seg_start + static_cast<long long>(b) * p.S, igc) : 0;
       const int lo_max = __reduce_max_sync(0xffffffffu, row_lo);   // of this warp's rows
@@ -957,7 +972,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc(tmem_base, TILES * 256);
   }
 }
 
@@ -1739,7 +1754,7 @@ int configure() {
   B200TP_CUDA_OK(cudaFuncSetAttribute(flash_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
                                       FWD_SMEM_BYTES));                                                            \
   B200TP_CUDA_OK(cudaFuncSetAttribute(flash_fwd2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
-                                      FWD2_SMEM_BYTES));                                                           \
+                                      fwd2_smem_bytes<D, 2>()));                                                   \
   B200TP_CUDA_OK(cudaFuncSetAttribute(flash_dq_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,             \
                                       DQ_SMEM_BYTES));                                                             \
   B200TP_CUDA_OK(cudaFuncSetAttribute(flash_dkv_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
@@ -1747,6 +1762,8 @@ int configure() {
   B200TP_SET_SMEM(64)
   B200TP_SET_SMEM(96)
   B200TP_SET_SMEM(128)
+  B200TP_CUDA_OK(cudaFuncSetAttribute(flash_fwd2_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      fwd2_smem_bytes<64, 1>()));
 #undef B200TP_SET_SMEM
   if (dev >= 0 && dev < 64) done[dev].store(1, std::memory_order_release);
   return B200TP_OK;
@@ -1831,7 +1848,7 @@ static int fwd_impl(const b200tp_attn_args* a, const void* q, const void* k, con
     p.o_part = static_cast<float*>(workspace);
     p.ml_part = reinterpret_cast<float*>(static_cast<char*>(workspace) + align_up(rows * HD * sizeof(float), 256));
     dim3 grid(a->hq / 2 * a->b, ns, nqb);
-    B200TP_CUDA_OK(launch_pdl(flash_fwd2_kernel<D>, grid, dim3(FWD2_THREADS), FWD2_SMEM_BYTES, stream, tq, tk, tv, p, 1));
+    B200TP_CUDA_OK(launch_pdl(flash_fwd2_kernel<D>, grid, dim3(fwd2_threads(2)), fwd2_smem_bytes<D, 2>(), stream, tq, tk, tv, p, 1));
     dim3 gc((a->s + 3) / 4, a->hq, a->b);
     B200TP_CUDA_OK(launch_pdl(flash_fwd_combine_kernel, gc, dim3(128), 0, stream, a->s, a->hq, D, ns, p.split_min,
                               a->seg_start, static_cast<const float*>(p.o_part), static_cast<const float*>(p.ml_part),
@@ -1843,12 +1860,16 @@ static int fwd_impl(const b200tp_attn_args* a, const void* q, const void* k, con
     // single-tile kernel (reserved & 3 == 1 / 2 force the single- / two-tile kernel, for cross-checks)
     dim3 grid(a->hq * a->b, nqb, 1);
     B200TP_CUDA_OK(launch_pdl(flash_fwd_kernel<D>, grid, dim3(FWD_THREADS), FWD_SMEM_BYTES, stream, tq, tk, tv, p));
+  } else if (D == 64 && fwd_choice != 2) {
+    dim3 grid(a->hq * a->b, nqb, 1);           // one tile per CTA, two CTAs per SM
+    B200TP_CUDA_OK(launch_pdl(flash_fwd2_kernel<64, 1>, grid, dim3(fwd2_threads(1)), fwd2_smem_bytes<64, 1>(), stream,
+                              tq, tk, tv, p, 0));
   } else if (group % 2 == 0) {
     dim3 grid(a->hq / 2 * a->b, nqb, 1);       // two heads of a GQA group per CTA
-    B200TP_CUDA_OK(launch_pdl(flash_fwd2_kernel<D>, grid, dim3(FWD2_THREADS), FWD2_SMEM_BYTES, stream, tq, tk, tv, p, 1));
+    B200TP_CUDA_OK(launch_pdl(flash_fwd2_kernel<D>, grid, dim3(fwd2_threads(2)), fwd2_smem_bytes<D, 2>(), stream, tq, tk, tv, p, 1));
   } else {
     dim3 grid(a->hq * a->b, (nqb + 1) / 2, 1); // two consecutive query blocks of a head per CTA
-    B200TP_CUDA_OK(launch_pdl(flash_fwd2_kernel<D>, grid, dim3(FWD2_THREADS), FWD2_SMEM_BYTES, stream, tq, tk, tv, p, 0));
+    B200TP_CUDA_OK(launch_pdl(flash_fwd2_kernel<D>, grid, dim3(fwd2_threads(2)), fwd2_smem_bytes<D, 2>(), stream, tq, tk, tv, p, 0));
   }
   return B200TP_OK;
 }
