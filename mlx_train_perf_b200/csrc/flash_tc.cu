@@ -16,7 +16,7 @@
 //                      On a grid smaller than the SM count with long sequences, 2-4 CTAs share
 //                      each query block's key range and write un-normalised fp32 partials;
 //   flash_fwd_combine_kernel  merges those partials into O and L.
-//                      At head_dim 64 one tile per CTA and two CTAs per SM.
+//                      At head_dim 64 and 96 one tile per CTA and two CTAs per SM.
 //   flash_fwd_kernel   one tile per CTA, P through shared memory: taken for small grids that are
 //                      not split, and selectable as a cross-check of the two-tile kernel.
 //   flash_dq_kernel    one CTA per (batch, q head, 128-query block): Q and dO staged into tensor
@@ -559,16 +559,20 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 // their S values" before either overwrites S columns with P.
 constexpr int FWD2_RING = 4;
 constexpr int FWD2_XCHG_BYTES = 2 * 2 * TILE * 4;       // [tile][column half][row] fp32 block maxima
-// One tile per CTA (head_dim 64): half of the threads and of tensor memory and 16 KiB tiles, so an SM holds two CTAs.
+// One tile per CTA (head_dim 64 and 96): half of the threads and of tensor memory, and 16 KiB tiles or a ring of one K
+// and one V tile, so an SM holds two CTAs.
 // The same two tiles are in flight, but a CTA's start and end overlap the other's work and the causal triangle is cut
-// into smaller pieces; in exchange a K / V tile is brought in once per tile, which 16 KiB tiles leave room for.
+// into smaller pieces; in exchange a K / V tile is brought in once per tile.
 // Forward, 32 / 8 heads, two tiles against one: 2 x 2500 tokens 111 / 101 us, 1 x 8192 439 / 394; 12 / 4 heads, 1 x 16384
-// 629 / 568.
+// 629 / 568; head_dim 96, 2 x 2500 130 / 123, 1 x 8192 522 / 516, 8 x 512 (16 / 16 heads) 27 / 24; head_dim 128, where it is
+// not taken, 2 x 2500 129 / 125, 1 x 8192 470 / 489.
 template <int D, int TILES>
 __host__ __device__ constexpr int fwd2_tile_bytes() { return TILES == 1 && D == 64 ? SUB_BYTES : TILE_BYTES; }
 template <int D, int TILES>
+__host__ __device__ constexpr int fwd2_ring() { return TILES == 1 && D > 64 ? 2 : FWD2_RING; }
+template <int D, int TILES>
 constexpr int fwd2_smem_bytes() {
-  return (TILES + FWD2_RING) * fwd2_tile_bytes<D, TILES>() + 256 + FWD2_XCHG_BYTES + 1024;
+  return (TILES + fwd2_ring<D, TILES>()) * fwd2_tile_bytes<D, TILES>() + 256 + FWD2_XCHG_BYTES + 1024;
 }
 constexpr int fwd2_threads(int tiles) { return 64 + 256 * tiles; }
 constexpr float kRescaleSlack = 8.f;
@@ -606,18 +610,18 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = align1024(smem_raw);
   uint8_t* q_sm = sm;                                   // [2]
-  constexpr int kTile = fwd2_tile_bytes<D, TILES>();
-  uint8_t* ring_sm = sm + TILES * kTile;                // [FWD2_RING]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + (TILES + FWD2_RING) * kTile);
+  constexpr int kTile = fwd2_tile_bytes<D, TILES>(), kRing = fwd2_ring<D, TILES>();
+  uint8_t* ring_sm = sm + TILES * kTile;                // [kRing]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + (TILES + kRing) * kTile);
   uint64_t* q_full = bars;
-  uint64_t* kv_full = bars + 1;                   // [FWD2_RING]
-  uint64_t* kv_empty = bars + 1 + FWD2_RING;      // [FWD2_RING]
-  uint64_t* s_full = bars + 1 + 2 * FWD2_RING;    // [2] per tile: S(j) is complete (and so is every earlier MMA)
+  uint64_t* kv_full = bars + 1;                   // [kRing]
+  uint64_t* kv_empty = bars + 1 + kRing;      // [kRing]
+  uint64_t* s_full = bars + 1 + 2 * kRing;    // [2] per tile: S(j) is complete (and so is every earlier MMA)
   uint64_t* p_full = s_full + 2;                  // [2] per tile: P(j) is in tensor memory
   uint64_t* o_final = s_full + 4;                 // [2] per tile: the last P V is complete
   uint64_t* xb = s_full + 6;                      // [2][4] per (tile, quadrant): the row pair's exchange
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(s_full + 14);
-  float* xchg = reinterpret_cast<float*>(sm + (TILES + FWD2_RING) * kTile + 256);
+  float* xchg = reinterpret_cast<float*>(sm + (TILES + kRing) * kTile + 256);
   int* abort_flag = reinterpret_cast<int*>(tmem_ptr + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // provably warp-uniform
@@ -683,7 +687,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int s = 0; s < FWD2_RING; ++s) {
+    for (int s = 0; s < kRing; ++s) {
       mbar_init(&kv_full[s], 1);
       mbar_init(&kv_empty[s], 1);
     }
@@ -718,8 +722,8 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       bool ok = true;
       const int total = 2 * (jmax - jmin + 1);
       for (int idx = 0; idx < total; ++idx) {  // even: K of block jmin + idx/2, odd: its V
-        const int slot = idx % FWD2_RING;
-        if (!mbar_wait(&kv_empty[slot], ((idx / FWD2_RING) & 1) ^ 1, abort_flag)) {
+        const int slot = idx % kRing;
+        if (!mbar_wait(&kv_empty[slot], ((idx / kRing) & 1) ^ 1, abort_flag)) {
           raise(abort_flag, p.status, kDevTimeoutProducer);
           ok = false;
           break;
@@ -731,8 +735,8 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       }
       if (!ok) {
         mbar_wait_drain(q_full, 0);
-        for (int idx = max(0, issued - FWD2_RING); idx < issued; ++idx)
-          mbar_wait_drain(&kv_full[idx % FWD2_RING], (idx / FWD2_RING) & 1);
+        for (int idx = max(0, issued - kRing); idx < issued; ++idx)
+          mbar_wait_drain(&kv_full[idx % kRing], (idx / kRing) & 1);
       }
     }
   } else if (warp == 1) {
@@ -744,9 +748,9 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     bool ok = cta_empty || mbar_wait_warp(q_full, 0, abort_flag);
     for (int j = jmin; j <= jmax + 1 && ok && !cta_empty; ++j) {
       const int k_idx = 2 * (j - jmin), v_idx = 2 * (j - 1 - jmin) + 1;   // ring sequence numbers
-      const int k_slot = k_idx % FWD2_RING, v_slot = (v_idx + FWD2_RING) % FWD2_RING;
-      if (j <= jmax) ok = mbar_wait_warp(&kv_full[k_slot], (k_idx / FWD2_RING) & 1, abort_flag);
-      if (ok && j > jmin) ok = mbar_wait_warp(&kv_full[v_slot], (v_idx / FWD2_RING) & 1, abort_flag);
+      const int k_slot = k_idx % kRing, v_slot = (v_idx + kRing) % kRing;
+      if (j <= jmax) ok = mbar_wait_warp(&kv_full[k_slot], (k_idx / kRing) & 1, abort_flag);
+      if (ok && j > jmin) ok = mbar_wait_warp(&kv_full[v_slot], (v_idx / kRing) & 1, abort_flag);
       for (int t = 0; t < 2 && ok; ++t) {
         if (!tl[t].active) continue;
         const bool has_prev = j - 1 >= tl[t].jlo && j - 1 <= tl[t].jhi;
@@ -1764,6 +1768,8 @@ int configure() {
   B200TP_SET_SMEM(128)
   B200TP_CUDA_OK(cudaFuncSetAttribute(flash_fwd2_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       fwd2_smem_bytes<64, 1>()));
+  B200TP_CUDA_OK(cudaFuncSetAttribute(flash_fwd2_kernel<96, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      fwd2_smem_bytes<96, 1>()));
 #undef B200TP_SET_SMEM
   if (dev >= 0 && dev < 64) done[dev].store(1, std::memory_order_release);
   return B200TP_OK;
@@ -1856,13 +1862,14 @@ static int fwd_impl(const b200tp_attn_args* a, const void* q, const void* k, con
     return B200TP_OK;
   }
   const int fwd_choice = a->reserved & 3;
+  constexpr int kOne = D <= 96 ? D : 96;   // (head_dim 128 has no one-tile form)
   if (fwd_choice == 1 || (fwd_choice != 2 && two_tile_ctas <= sm_count())) {
     // single-tile kernel (reserved & 3 == 1 / 2 force the single- / two-tile kernel, for cross-checks)
     dim3 grid(a->hq * a->b, nqb, 1);
     B200TP_CUDA_OK(launch_pdl(flash_fwd_kernel<D>, grid, dim3(FWD_THREADS), FWD_SMEM_BYTES, stream, tq, tk, tv, p));
-  } else if (D == 64 && fwd_choice != 2) {
+  } else if (D <= 96 && fwd_choice != 2) {
     dim3 grid(a->hq * a->b, nqb, 1);           // one tile per CTA, two CTAs per SM
-    B200TP_CUDA_OK(launch_pdl(flash_fwd2_kernel<64, 1>, grid, dim3(fwd2_threads(1)), fwd2_smem_bytes<64, 1>(), stream,
+    B200TP_CUDA_OK(launch_pdl(flash_fwd2_kernel<kOne, 1>, grid, dim3(fwd2_threads(1)), fwd2_smem_bytes<kOne, 1>(), stream,
                               tq, tk, tv, p, 0));
   } else if (group % 2 == 0) {
     dim3 grid(a->hq / 2 * a->b, nqb, 1);       // two heads of a GQA group per CTA
