@@ -207,6 +207,15 @@ size_t b200tp_linear_ce_bwd_grad_workspace_bytes(const b200tp_ce_args* a);
 int b200tp_linear_ce_bwd_grad(const b200tp_ce_args* a, const float* lse, const float* tgt_logit, const float* cotangent,
                               void* state, size_t state_bytes, void* d_hidden, void* workspace, size_t workspace_bytes,
                               void* stream, int* status);
+/* Both for a reduced loss, in one call each: the forward followed by b200tp_linear_ce_reduce into out3, and the backward
+ * with cotangent[i] = upstream[0] (/ max(count[0], 1) when count != NULL) on rows whose target != ignore_index. */
+int b200tp_linear_ce_fwd_grad_reduced(const b200tp_ce_args* a, float* tgt_logit, float* lse, float* nll, float* out3,
+                                      void* state, size_t state_bytes, void* workspace, size_t workspace_bytes,
+                                      void* stream, int* status);
+int b200tp_linear_ce_bwd_grad_reduced(const b200tp_ce_args* a, const float* lse, const float* tgt_logit,
+                                      const float* upstream, const float* count, void* state, size_t state_bytes,
+                                      void* d_hidden, void* workspace, size_t workspace_bytes, void* stream,
+                                      int* status);
 
 /* Dequantise rows [row0, row0 + rows) of a 4-bit affine head into `out` (rows, D) bf16/f32:
  * w = scale * code + bias in fp32, rounded once; `out` 16-byte aligned.  core/kernel/source.py:193-208. */

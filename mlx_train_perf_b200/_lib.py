@@ -89,6 +89,12 @@ SIGNATURES = {
     "b200tp_linear_ce_fwd_grad_workspace_bytes": (C.c_size_t, [C.POINTER(CeArgs)]),
     "b200tp_linear_ce_fwd_grad": (C.c_int, [C.POINTER(CeArgs), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                             C.c_size_t, C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]),
+    "b200tp_linear_ce_fwd_grad_reduced": (C.c_int, [C.POINTER(CeArgs), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                                    C.c_void_p, C.c_size_t, C.c_void_p, C.c_size_t, C.c_void_p,
+                                                    C.c_void_p]),
+    "b200tp_linear_ce_bwd_grad_reduced": (C.c_int, [C.POINTER(CeArgs), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                                    C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p, C.c_size_t,
+                                                    C.c_void_p, C.c_void_p]),
     "b200tp_linear_ce_bwd_grad_workspace_bytes": (C.c_size_t, [C.POINTER(CeArgs)]),
     "b200tp_linear_ce_bwd_grad": (C.c_int, [C.POINTER(CeArgs), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                             C.c_size_t, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p,

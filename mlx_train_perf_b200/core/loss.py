@@ -350,9 +350,10 @@ def _forms_grad(impl: str, hidden_wants_grad: bool, hidden: torch.Tensor, head: 
 
 
 def ce_forward_grad(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, *,
-                    ignore_index: int = IGNORE_INDEX, impl: str = "tc"):
+                    ignore_index: int = IGNORE_INDEX, impl: str = "tc", out3: torch.Tensor | None = None):
     """((3, N) fp32 rows tgt_logit, lse, nll; state): the forward that also forms the gradient.  `state` is what
-    `ce_backward_grad` needs: fp32 sums of d_hidden and a few words per row."""
+    `ce_backward_grad` needs: fp32 sums of d_hidden and a few words per row.  `out3` receives the masked sum, mean and
+    count of the losses."""
     lib = _lib.load()
     dev = hidden.device
     n = hidden.shape[0]
@@ -363,30 +364,41 @@ def ce_forward_grad(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, 
     state, ws = _workspace(sbytes, dev), _workspace(nbytes, dev)
     base = out.data_ptr()
     with _lib.on(dev):
-        rc = lib.b200tp_linear_ce_fwd_grad(C.byref(a), base, base + 4 * n, base + 8 * n, _ptr(state), sbytes,
-                                           _ptr(ws), nbytes, _lib.stream(dev), device_status(dev).data_ptr())
+        if out3 is None:
+            rc = lib.b200tp_linear_ce_fwd_grad(C.byref(a), base, base + 4 * n, base + 8 * n, _ptr(state), sbytes,
+                                               _ptr(ws), nbytes, _lib.stream(dev), device_status(dev).data_ptr())
+        else:
+            rc = lib.b200tp_linear_ce_fwd_grad_reduced(C.byref(a), base, base + 4 * n, base + 8 * n, out3.data_ptr(),
+                                                       _ptr(state), sbytes, _ptr(ws), nbytes, _lib.stream(dev),
+                                                       device_status(dev).data_ptr())
     _lib.check(rc)
     del keep
     return out, state
 
 
 def ce_backward_grad(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, out: torch.Tensor,
-                     state: torch.Tensor, cotangent: torch.Tensor, *, ignore_index: int = IGNORE_INDEX,
-                     impl: str = "tc") -> torch.Tensor:
-    """d_hidden (N, D) from what `ce_forward_grad` returned and the upstream gradient of the per-row losses."""
+                     state: torch.Tensor, cotangent: torch.Tensor | None, *, ignore_index: int = IGNORE_INDEX,
+                     impl: str = "tc", upstream: torch.Tensor | None = None, count: int | None = None) -> torch.Tensor:
+    """d_hidden (N, D) from what `ce_forward_grad` returned and the upstream gradient of the per-row losses, or of a
+    reduced loss: `upstream` (one fp32 element), divided by the count at device address `count` where that is given."""
     lib = _lib.load()
     dev = hidden.device
     n = hidden.shape[0]
     a, keep = _ce_args(hidden, head, targets, v_offset=0, ignore_index=ignore_index, impl=impl)
     d_hidden = torch.empty_like(hidden)
-    ct = cotangent.to(torch.float32).contiguous()
     nbytes = lib.b200tp_linear_ce_bwd_grad_workspace_bytes(C.byref(a))
     ws = _workspace(nbytes, dev)
     base = out.data_ptr()
     with _lib.on(dev):
-        rc = lib.b200tp_linear_ce_bwd_grad(C.byref(a), base + 4 * n, base, ct.data_ptr(), state.data_ptr(),
-                                           state.numel(), d_hidden.data_ptr(), _ptr(ws), nbytes, _lib.stream(dev),
-                                           device_status(dev).data_ptr())
+        if upstream is not None:
+            rc = lib.b200tp_linear_ce_bwd_grad_reduced(C.byref(a), base + 4 * n, base, upstream.data_ptr(), count,
+                                                       state.data_ptr(), state.numel(), d_hidden.data_ptr(), _ptr(ws),
+                                                       nbytes, _lib.stream(dev), device_status(dev).data_ptr())
+        else:
+            ct = cotangent.to(torch.float32).contiguous()
+            rc = lib.b200tp_linear_ce_bwd_grad(C.byref(a), base + 4 * n, base, ct.data_ptr(), state.data_ptr(),
+                                               state.numel(), d_hidden.data_ptr(), _ptr(ws), nbytes, _lib.stream(dev),
+                                               device_status(dev).data_ptr())
     _lib.check(rc)
     del keep
     return d_hidden
@@ -477,20 +489,18 @@ class _FusedLinearCEReduced(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, weight, targets, head, ignore_index, impl, mean):
         use = DenseHead(weight=weight) if weight is not None else head
+        dev = hidden.device
+        out3 = torch.empty(3, dtype=torch.float32, device=dev)
         if weight is None and _forms_grad(impl, ctx.needs_input_grad[0], hidden, use, targets):
-            rows, state = ce_forward_grad(hidden, use, targets, ignore_index=ignore_index, impl=impl)
-            nll, saved = rows[2], [rows, state]
+            saved = list(ce_forward_grad(hidden, use, targets, ignore_index=ignore_index, impl=impl, out3=out3))
         else:
             _, _, _, lse, nll = ce_forward_raw(hidden, use, targets, ignore_index=ignore_index, impl=impl)
             saved = [lse] + ([weight] if weight is not None else [])
+            with _lib.on(dev):
+                rc = _lib.load().b200tp_linear_ce_reduce(nll.data_ptr(), targets.data_ptr(), hidden.shape[0],
+                                                         ignore_index, out3.data_ptr(), _lib.stream(dev))
+            _lib.check(rc)
         ctx.trains_weight, ctx.has_grad = weight is not None, weight is None and len(saved) == 2
-        lib = _lib.load()
-        dev = hidden.device
-        out3 = torch.empty(3, dtype=torch.float32, device=dev)
-        with _lib.on(dev):
-            rc = lib.b200tp_linear_ce_reduce(nll.data_ptr(), targets.data_ptr(), hidden.shape[0], ignore_index,
-                                             out3.data_ptr(), _lib.stream(dev))
-        _lib.check(rc)
         ctx.save_for_backward(hidden, targets, out3, *saved)
         ctx.head, ctx.ignore_index, ctx.impl, ctx.mean = head, ignore_index, impl, mean
         ctx.set_materialize_grads(False)      # no zeros for the count's gradient
@@ -512,15 +522,15 @@ class _FusedLinearCEReduced(torch.autograd.Function):
         dev = hidden.device
         n = hidden.shape[0]
         g = g_loss.to(torch.float32).reshape(1).contiguous()
+        if ctx.has_grad:
+            d_hidden = ce_backward_grad(hidden, head, targets, rows, saved[4], None, ignore_index=ctx.ignore_index,
+                                        impl=ctx.impl, upstream=g, count=out3.data_ptr() + 8 if ctx.mean else None)
+            return d_hidden, None, None, None, None, None, None
         ct = torch.empty(n, dtype=torch.float32, device=dev)
         with _lib.on(dev):
             rc = lib.b200tp_linear_ce_cotangent(targets.data_ptr(), n, ctx.ignore_index, g.data_ptr(),
                                                 out3.data_ptr() + 8 if ctx.mean else None, ct.data_ptr(), _lib.stream(dev))
         _lib.check(rc)
-        if ctx.has_grad:
-            d_hidden = ce_backward_grad(hidden, head, targets, rows, saved[4], ct, ignore_index=ctx.ignore_index,
-                                        impl=ctx.impl)
-            return d_hidden, None, None, None, None, None, None
         d_w = None
         if weight is not None and ctx.needs_input_grad[1]:
             d_w = torch.empty_like(weight, memory_format=torch.contiguous_format)

@@ -318,7 +318,8 @@ struct GradPlan {
   void* deq;
   float* pm; float* ps; float* pt;
   size_t bytes;          // forward
-  size_t bwd_bytes;      // backward: g and deq alone, for calls whose overflow flag is set
+  float* ct;             // (n): the cotangents of a reduced loss
+  size_t bwd_bytes;      // backward: g, deq and ct
   // fp32: planes; `logits` overlays g's
   void* h3; void* w3;
   float* logits;
@@ -342,6 +343,7 @@ GradPlan plan_grad(const b200tp_ce_args* a, void* state, void* ws) {
     p.g = b.take<char>(static_cast<size_t>(a->n) * p.chunk * 6);
     p.logits = static_cast<float*>(p.g);
     p.simt_chunk = std::min<int64_t>(a->v_local, p.chunk * 6 / 4);
+    p.ct = b.take<float>(a->n);
     p.bwd_bytes = align_up(b.off, 256);
     p.h3 = b.take<char>(static_cast<size_t>(a->n) * a->d * 6);
     p.w3 = b.take<char>(static_cast<size_t>(p.chunk) * a->d * 6);
@@ -363,6 +365,7 @@ GradPlan plan_grad(const b200tp_ce_args* a, void* state, void* ws) {
   Bump b(ws);
   p.g = b.take<char>(static_cast<size_t>(a->n) * p.chunk * 2);
   if (a->quant_bits != 0) p.deq = b.take<char>(static_cast<size_t>(p.chunk) * a->d * 2);
+  p.ct = b.take<float>(a->n);
   p.bwd_bytes = align_up(b.off, 256);
   for (int64_t c = 0; c < p.num_chunks; ++c)
     p.total_splits += ce_tc_fwd_splits(a->n, a->d, std::min<int64_t>(p.chunk, a->v_local - c * p.chunk));
@@ -785,12 +788,13 @@ int b200tp_linear_ce_fwd_grad(const b200tp_ce_args* a, float* tgt_logit, float* 
                         nullptr, nullptr, tgt_logit, lse, nll, stream);
 }
 
-int b200tp_linear_ce_bwd_grad(const b200tp_ce_args* a, const float* lse, const float* tgt_logit, const float* cotangent,
-                              void* state, size_t state_bytes, void* d_hidden, void* workspace, size_t workspace_bytes,
-                              void* stream_v, int* status) {
+// The rows' cotangents are `cotangent`, or formed here from `upstream` and `count`.
+static int bwd_grad_impl(const b200tp_ce_args* a, const float* lse, const float* tgt_logit, const float* cotangent,
+                         const float* upstream, const float* count, void* state, size_t state_bytes, void* d_hidden,
+                         void* workspace, size_t workspace_bytes, void* stream_v, int* status) {
   int rc = check_grad_args(a);
   if (rc) return rc;
-  if (lse == nullptr || tgt_logit == nullptr || cotangent == nullptr || d_hidden == nullptr)
+  if (lse == nullptr || tgt_logit == nullptr || (cotangent == nullptr && upstream == nullptr) || d_hidden == nullptr)
     return fail(B200TP_ERR_LOSS_INPUT, "lse / tgt_logit / cotangent / d_hidden is null");
   rc = require_sm100();
   if (rc) return rc;
@@ -802,6 +806,11 @@ int b200tp_linear_ce_bwd_grad(const b200tp_ce_args* a, const float* lse, const f
   rc = check_workspace(workspace, workspace_bytes, p.bwd_bytes);
   if (rc) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  if (cotangent == nullptr) {
+    rc = launch_loss_cotangent(a->targets, a->n, a->ignore_index, upstream, count, p.ct, stream);
+    if (rc) return rc;
+    cotangent = p.ct;
+  }
   if (p.impl == 3) {
     const float* weight = static_cast<const float*>(a->weight);
     float* out = static_cast<float*>(d_hidden);
@@ -847,6 +856,31 @@ int b200tp_linear_ce_bwd_grad(const b200tp_ce_args* a, const float* lse, const f
     if (rc) return rc;
   }
   return B200TP_OK;
+}
+
+int b200tp_linear_ce_bwd_grad(const b200tp_ce_args* a, const float* lse, const float* tgt_logit, const float* cotangent,
+                              void* state, size_t state_bytes, void* d_hidden, void* workspace, size_t workspace_bytes,
+                              void* stream, int* status) {
+  return bwd_grad_impl(a, lse, tgt_logit, cotangent, nullptr, nullptr, state, state_bytes, d_hidden, workspace,
+                       workspace_bytes, stream, status);
+}
+
+int b200tp_linear_ce_bwd_grad_reduced(const b200tp_ce_args* a, const float* lse, const float* tgt_logit,
+                                      const float* upstream, const float* count, void* state, size_t state_bytes,
+                                      void* d_hidden, void* workspace, size_t workspace_bytes, void* stream,
+                                      int* status) {
+  return bwd_grad_impl(a, lse, tgt_logit, nullptr, upstream, count, state, state_bytes, d_hidden, workspace,
+                       workspace_bytes, stream, status);
+}
+
+int b200tp_linear_ce_fwd_grad_reduced(const b200tp_ce_args* a, float* tgt_logit, float* lse, float* nll, float* out3,
+                                      void* state, size_t state_bytes, void* workspace, size_t workspace_bytes,
+                                      void* stream, int* status) {
+  if (out3 == nullptr) return fail(B200TP_ERR_LOSS_INPUT, "the reduced forward needs its output triple");
+  const int rc = b200tp_linear_ce_fwd_grad(a, tgt_logit, lse, nll, state, state_bytes, workspace, workspace_bytes,
+                                           stream, status);
+  if (rc) return rc;
+  return launch_loss_reduce(nll, a->targets, a->n, a->ignore_index, out3, static_cast<cudaStream_t>(stream));
 }
 
 int b200tp_dequant_int4(const uint32_t* w_q, const void* scales, const void* biases, int32_t qparam_dtype, int64_t row0,
