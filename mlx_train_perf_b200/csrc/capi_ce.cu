@@ -384,6 +384,15 @@ int check_grad_args(const b200tp_ce_args* a) {
   return B200TP_OK;
 }
 
+// The bf16 row kernels around the forward that forms the gradient read whole 16-byte words ahead of any tensor map.
+int check_grad_alignment(const b200tp_ce_args* a, const GradPlan& p, const void* d_hidden) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(a->hidden) | reinterpret_cast<uintptr_t>(d_hidden) |
+                        (a->quant_bits == 0 ? reinterpret_cast<uintptr_t>(a->weight) : 0);
+  if (p.impl == 1 && (all & 15) != 0)
+    return fail(B200TP_ERR_LOSS_INPUT, "tensor base address must be 16-byte aligned for TMA");
+  return B200TP_OK;
+}
+
 int check_workspace(void* ws, size_t have, size_t need) {
   if (need == 0) return B200TP_OK;
   if (ws == nullptr) return fail(B200TP_ERR_WORKSPACE, "workspace is null but " + std::to_string(need) + " bytes are needed");
@@ -710,6 +719,8 @@ int b200tp_linear_ce_fwd_grad(const b200tp_ce_args* a, float* tgt_logit, float* 
   const GradPlan p = plan_grad(a, state, workspace);
   if (!p.ok)
     return fail(B200TP_ERR_UNSUPPORTED_HEAD, "the forward with gradient runs on the tensor-core path, 4-bit heads chunk-wise");
+  rc = check_grad_alignment(a, p, nullptr);
+  if (rc) return rc;
   rc = check_workspace(state, state_bytes, p.state_bytes);
   if (rc) return rc;
   rc = check_workspace(workspace, workspace_bytes, p.bytes);
@@ -801,6 +812,8 @@ static int bwd_grad_impl(const b200tp_ce_args* a, const float* lse, const float*
   const GradPlan p = plan_grad(a, state, workspace);
   if (!p.ok)
     return fail(B200TP_ERR_UNSUPPORTED_HEAD, "the forward with gradient runs on the tensor-core path, 4-bit heads chunk-wise");
+  rc = check_grad_alignment(a, p, d_hidden);
+  if (rc) return rc;
   rc = check_workspace(state, state_bytes, p.state_bytes);
   if (rc) return rc;
   rc = check_workspace(workspace, workspace_bytes, p.bwd_bytes);

@@ -117,3 +117,19 @@ def test_no_gradient_wanted_runs_the_plain_forward(cuda_device):
     assert a[0].grad_fn is None and b[0].grad_fn is not None
     for x, y in zip(a, b):
         assert (x - y.detach()).abs().max().item() < 1e-5
+
+
+@pytest.mark.parametrize("operand", ["hidden", "weight"])
+def test_misaligned_operands_are_refused(cuda_device, operand):
+    """Before any kernel reads them: the row kernels load whole 16-byte words."""
+    from mlx_train_perf_b200.errors import LossInputError
+    n, d, v = 40, 64, 300
+    h = torch.zeros(n * d + 1, dtype=torch.bfloat16, device=cuda_device)[1:].reshape(n, d)
+    w = torch.zeros(v * d + 1, dtype=torch.bfloat16, device=cuda_device)[1:].reshape(v, d)
+    h, w = (h, w.clone()) if operand == "hidden" else (h.clone(), w)
+    assert (h.data_ptr() | w.data_ptr()) % 16 != 0
+    t = torch.zeros(n, dtype=torch.int64, device=cuda_device)
+    with pytest.raises(LossInputError, match="16-byte aligned"):
+        fused_linear_ce(h.requires_grad_(True), DenseHead(w, trainable=False), t)
+    with pytest.raises(LossInputError, match="16-byte aligned"):
+        fused_linear_ce(h.detach(), DenseHead(w, trainable=False), t)
