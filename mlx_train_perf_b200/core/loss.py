@@ -469,12 +469,18 @@ class _FusedLinearCETrainable(torch.autograd.Function):
         return d_hidden, d_w, None, None, None
 
 
+def _trained(impl: str) -> str:
+    """The gradient of a trained fp32 head is formed on the CUDA cores, and lse has to come from the same logits: errors
+    that the two share cancel in exp(z - lse)."""
+    return "simt" if impl == "auto" else impl
+
+
 def _apply(hidden2, targets2, head, ignore_index, impl):
     """Route to the trainable form only when autograd will actually ask for d_weight."""
     if (isinstance(head, DenseHead) and head.trainable and head.weight.requires_grad
             and torch.is_grad_enabled()):
         w = head.weight if head.weight.is_contiguous() else head.weight.contiguous()
-        return _FusedLinearCETrainable.apply(hidden2, w, targets2, ignore_index, impl)
+        return _FusedLinearCETrainable.apply(hidden2, w, targets2, ignore_index, _trained(impl))
     return _FusedLinearCE.apply(hidden2, targets2, head, ignore_index, impl)
 
 
@@ -573,6 +579,7 @@ def _apply_reduced(hidden2, targets2, head, ignore_index, impl, mean):
     w = None
     if trainable:
         w = head.weight if head.weight.is_contiguous() else head.weight.contiguous()
+        impl = _trained(impl)
     return _FusedLinearCEReduced.apply(hidden2, w, targets2, head, ignore_index, impl, mean)
 
 

@@ -10,7 +10,7 @@ import pytest
 import torch
 
 from mlx_train_perf_b200.core import loss as L
-from mlx_train_perf_b200.core.loss import DenseHead
+from mlx_train_perf_b200.core.loss import DenseHead, fused_linear_ce, reduced_linear_cross_entropy
 from oracle import linear_ce as oc
 
 pytestmark = pytest.mark.gpu
@@ -139,3 +139,19 @@ def test_forward_that_forms_the_gradient_without_planes(cuda_device):
     nll, lse, tgt, s_dh = _run(dev, h, w, t, ct, impl="simt")
     for a, b in ((rows[0], tgt), (rows[1], lse), (rows[2], nll), (dh, s_dh)):
         assert torch.equal(a.cpu().nan_to_num(7e7), b.nan_to_num(7e7))
+
+
+def test_trained_head_keeps_one_kind_of_logits(cuda_device):
+    """A size that would be split: with the head trained, forward and backward are the CUDA-core ones."""
+    n, d, v = 300, 1024, 1000
+    h, w, t = (x.to(cuda_device) for x in _inputs(n, d, v))
+    out = []
+    for impl in ("auto", "simt"):
+        hh, ww = h.clone().requires_grad_(True), w.clone().requires_grad_(True)
+        nll, lse, _ = fused_linear_ce(hh, DenseHead(ww), t, impl=impl)
+        loss, _ = reduced_linear_cross_entropy(hh, DenseHead(ww), t, impl=impl)
+        out.append((nll.detach(), lse, loss.detach(), *torch.autograd.grad(nll.sum(), (hh, ww)),
+                    *torch.autograd.grad(loss, (hh, ww))))
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+    assert n * d * v >= 2 ** 28 and not torch.equal(fused_linear_ce(h, DenseHead(w, trainable=False), t)[1], out[0][1])
