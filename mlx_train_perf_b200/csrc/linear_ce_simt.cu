@@ -296,12 +296,14 @@ combine_kernel(const float* __restrict__ pm, const float* __restrict__ ps, const
   }
   const bool valid = targets == nullptr || targets[row] != ignore_index;
   if (!valid) t = 0.f;
-  const float lse = m + logf(s);
+  // m is a row's reference, not always its maximum, and |log s| may exceed |lse|: in double, so that lse and nll are
+  // each rounded once
+  const double lse = static_cast<double>(m) + log(static_cast<double>(s));
   if (row_max != nullptr) row_max[row] = m;
   if (row_sumexp != nullptr) row_sumexp[row] = s;
   if (tgt_out != nullptr) tgt_out[row] = t;
-  if (lse_out != nullptr) lse_out[row] = lse;
-  if (nll_out != nullptr) nll_out[row] = valid ? lse - t : 0.f;
+  if (lse_out != nullptr) lse_out[row] = static_cast<float>(lse);
+  if (nll_out != nullptr) nll_out[row] = valid ? static_cast<float>(lse - t) : 0.f;
 }
 
 // Masked reduction of the per-row losses (the masked mean of adapters/mlx_lm.py:192-216 of the
