@@ -144,7 +144,7 @@ QuantHead quant_head(const b200tp_ce_args* a, bool backward) {
 }
 
 // 1 = tcgen05, 2 = SIMT, 3 = tcgen05 over the three bf16 planes of fp32 operands, negative = refusal already
-// recorded.  3 is the default for fp32 with a dense head: 2048 x 1024 x 32768 forward + backward 18.5 -> 2.57 ms, with
+// recorded.  3 is the default for fp32 with a dense head: 2048 x 1024 x 32768 forward + backward 18.5 -> 1.65 ms, with
 // a third of the CUDA-core path's distance to float64 .  A trained fp32 head's backward stays on the CUDA
 // cores, and so do D % 8 != 0 (TMA strides), a 4-bit head under fp32 hidden states, and calls whose contraction is
 // under 2^28 multiplications: there the CUDA cores need no longer than the split's extra launches take (forward /

@@ -444,7 +444,7 @@ int num_groups(int64_t n) { return static_cast<int>(ceil_div(n, kMostTokens)); }
 }  // namespace
 
 int ce_int4_fwd_splits(int64_t n, int64_t v_rows) {
-  return ce_tc_choose_splits(num_groups(n), static_cast<int>(ceil_div(v_rows, VROWS)));
+  return ce_tc_choose_splits(num_groups(n), static_cast<int>(ceil_div(v_rows, VROWS)), sm_count());
 }
 
 int ce_int4_launch_fwd(const void* hidden, const QuantHead& q, int64_t v_rows, int64_t n, int d, int64_t vocab_id0,

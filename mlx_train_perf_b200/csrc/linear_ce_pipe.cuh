@@ -2,6 +2,8 @@
 // its barriers, CTA set-up and teardown, and what a timed-out wait does.
 #pragma once
 
+#include <algorithm>
+
 #include "linear_ce_tc.h"
 #include "ptx.cuh"
 
@@ -123,6 +125,43 @@ __device__ __forceinline__ void cta_teardown(const SmemView& sm, int warp, uint3
 __device__ __forceinline__ void producer_drain(const SmemView& sm, uint32_t it) {
   const uint32_t n = sm.stages, first = it > n ? it - n : 0;
   for (uint32_t j = first; j < it; ++j) mbar_wait_drain(&sm.full[j % n], (j / n) & 1);
+}
+
+template <bool PAIR>
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                     uint32_t idesc, uint32_t accumulate) {
+  if (PAIR) umma_ss_pair_w(tmem_d, a_lo, a_hi, b_lo, b_hi, idesc, accumulate);
+  else umma_ss_w(tmem_d, a_lo, a_hi, b_lo, b_hi, idesc, accumulate);
+}
+template <bool PAIR>
+__device__ __forceinline__ void commit(uint64_t* bar) {
+  if (PAIR) umma_commit_pair(bar);
+  else umma_commit(bar);
+}
+// An epilogue warp has read its accumulator: told to the CTA that issues the MMAs.
+template <bool PAIR>
+__device__ __forceinline__ void release_acc(uint64_t* bar) {
+  if (PAIR) mbar_arrive_cluster(map_to_rank(bar, 0));
+  else mbar_arrive(bar);
+}
+
+// `units` of work on pairs (`kernel` is a PAIR instantiation) or on single CTAs.
+template <typename P>
+int launch_units(void (*kernel)(CUtensorMap, CUtensorMap, P), int threads, bool pair, long long units,
+                 cudaStream_t stream, const CUtensorMap& a, const CUtensorMap& b, const P& p) {
+  cudaLaunchConfig_t cfg{};
+  const long long most = pair ? sm_count() / 2 : sm_count();
+  cfg.gridDim = dim3(static_cast<unsigned>(std::min(most, units) * (pair ? 2 : 1)));
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim = {2, 1, 1};
+  cfg.attrs = attr;
+  cfg.numAttrs = pair ? 1 : 0;
+  B200TP_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, a, b, p));
+  return B200TP_OK;
 }
 
 }  // namespace

@@ -11,7 +11,8 @@
 //
 // Tensor-bound: six bf16 products (6 x 2 N V D flops per contraction) against one product on the CUDA cores, whose
 // fp32 rate is 1/25 of the bf16 tensor rate and whose kernels reach a third of it.  2048 x 1024 x 32768, forward +
-// backward: 18.5 -> 2.57 ms, the six-fold products at 1.2 PFLOP/s.
+// backward: 18.5 ms there, 2.57 with three contractions, 1.65 with the gradient's sum formed in the forward and CTA
+// pairs: twelve bf16 products at 1.36 PFLOP/s inside the two kernels.
 //
 //   split_planes_kernel    fp32 rows -> three bf16 planes; raises a flag on values bf16 cannot hold (inf, NaN,
 //                          within 2^-9 of the largest fp32), for which the CUDA-core kernels take over
@@ -20,7 +21,7 @@
 //   split_dh_kernel        dH (128 x 256) (+)= G W over the chunk's vocab rows
 //   share_sum_kernel       adds the shares of a contraction that was spread over several CTAs
 //
-// Roles as in linear_ce_tc.cu (single CTAs), with eight accumulating warps (two per lane quadrant, 128 columns each).
+// Roles and CTA pairs as in linear_ce_tc.cu, with eight accumulating warps (two per lane quadrant, 128 columns each).
 // Replaces core/chunked.py:35-90 of the reference for fp32 heads, beside linear_ce_simt.cu.
 #include "linear_ce_split.h"
 
@@ -53,12 +54,13 @@ __device__ __forceinline__ void split3(float x, uint32_t& hi, uint32_t& mid, uin
   lo = __bfloat16_as_ushort(__float2bfloat16_rn(r - __uint_as_float(mid << 16)));
 }
 
-// Eight consecutive values -> 16 bytes of each plane.
-__device__ __forceinline__ bool split_store8(const float (&x)[8], __nv_bfloat16* dst, long long plane) {
-  uint32_t o[3][4];
+// N (8 or 16) consecutive values -> 2 N bytes of each plane, sixteen as whole sectors.
+template <int N>
+__device__ __forceinline__ bool split_store(const float (&x)[N], __nv_bfloat16* dst, long long plane) {
+  uint32_t o[3][N / 2];
   bool bad = false;
 #pragma unroll
-  for (int e = 0; e < 8; e += 2) {
+  for (int e = 0; e < N; e += 2) {
     uint32_t h0, m0, l0, h1, m1, l1;
     split3(x[e], h0, m0, l0);
     split3(x[e + 1], h1, m1, l1);
@@ -68,8 +70,12 @@ __device__ __forceinline__ bool split_store8(const float (&x)[8], __nv_bfloat16*
     o[2][e >> 1] = l0 | l1 << 16;
   }
 #pragma unroll
-  for (int p = 0; p < 3; ++p)
-    *reinterpret_cast<uint4*>(dst + p * plane) = make_uint4(o[p][0], o[p][1], o[p][2], o[p][3]);
+  for (int p = 0; p < 3; ++p) {
+    if constexpr (N == 16)
+      st_global_32b(dst + p * plane, o[p]);
+    else
+      *reinterpret_cast<uint4*>(dst + p * plane) = make_uint4(o[p][0], o[p][1], o[p][2], o[p][3]);
+  }
   return bad;
 }
 
@@ -89,7 +95,7 @@ split_planes_kernel(const float* __restrict__ x, long long count, __nv_bfloat16*
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = __ldg(x + i + e);
     }
-    bad = split_store8(v, out + i, count);
+    bad = split_store(v, out + i, count);
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) *flag = 1;
 }
@@ -155,12 +161,12 @@ struct SplitWalk {
 };
 
 // The MMA issuer's part of one tile.  B_MN: B is MN-major in 64 x 64 boxes (the weight rows of dH), else K-major.
-template <bool B_MN>
+template <bool B_MN, bool PAIR>
 __device__ __forceinline__ bool issue_tile(const SmemView& sm, uint32_t tmem_base, int kb0, int kb1, uint32_t& it,
                                            uint32_t& seg, int lane, int* status) {
-  constexpr uint32_t idesc = make_idesc_bf16(BM, BN, 0, B_MN ? 1 : 0);
+  constexpr uint32_t idesc = make_idesc_bf16(PAIR ? 2 * BM : BM, BN, 0, B_MN ? 1 : 0);
   constexpr uint32_t dhi = desc_hi_sw128(1024);
-  constexpr uint32_t b_step = B_MN ? 128 : 2;
+  constexpr uint32_t b_step = B_MN ? 128 : 2, kStages = PAIR ? PAIR_STAGES : STAGES;
   for (SplitWalk w(kb0, kb1); !w.done(); w.next(), ++it) {
     const uint32_t as = seg & 1;
     if (w.first()) {
@@ -169,8 +175,8 @@ __device__ __forceinline__ bool issue_tile(const SmemView& sm, uint32_t tmem_bas
         return false;
       }
     }
-    const int s = it % STAGES;
-    if (!mbar_wait_warp(&sm.full[s], (it / STAGES) & 1, sm.abort_flag)) {
+    const int s = it % kStages;
+    if (!mbar_wait_warp(&sm.full[s], (it / kStages) & 1, sm.abort_flag)) {
       if (lane == 0) raise_abort(sm, status, kDevTimeoutMma);
       return false;
     }
@@ -182,9 +188,9 @@ __device__ __forceinline__ bool issue_tile(const SmemView& sm, uint32_t tmem_bas
     if (elect_one()) {
 #pragma unroll
       for (int k = 0; k < BK / 16; ++k)
-        umma_ss_w(d_tmem, a_lo + k * 2, dhi, b_lo + k * b_step, dhi, idesc, (fresh && k == 0) ? 0u : 1u);
-      umma_commit(&sm.empty[s]);
-      if (last) umma_commit(&sm.tfull[as]);
+        umma<PAIR>(d_tmem, a_lo + k * 2, dhi, b_lo + k * b_step, dhi, idesc, (fresh && k == 0) ? 0u : 1u);
+      commit<PAIR>(&sm.empty[s]);
+      if (last) commit<PAIR>(&sm.tfull[as]);
     }
     __syncwarp();
     if (last) ++seg;
@@ -192,7 +198,14 @@ __device__ __forceinline__ bool issue_tile(const SmemView& sm, uint32_t tmem_bas
   return true;
 }
 
+// A pair's CTA leaves only after the commits of its last stages have arrived.
+__device__ __forceinline__ void pair_tail(const SmemView& sm, uint32_t it) {
+  for (uint32_t j = it > PAIR_STAGES ? it - PAIR_STAGES : 0; j < it; ++j)
+    mbar_wait(&sm.empty[j % PAIR_STAGES], (j / PAIR_STAGES) & 1, sm.abort_flag);
+}
+
 // An accumulating warp's part of one tile: acc = sum of the segments' accumulators over its 128 columns.
+template <bool PAIR>
 __device__ __forceinline__ bool gather_tile(const SmemView& sm, uint32_t taddr, int segs, uint32_t& seg, int lane,
                                             float (&acc)[HALF], int* status) {
 #pragma unroll
@@ -215,20 +228,24 @@ __device__ __forceinline__ bool gather_tile(const SmemView& sm, uint32_t taddr, 
     }
     tc_fence_before_sync();
     __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.tempty[as]);
+    if (lane == 0) release_acc<PAIR>(&sm.tempty[as]);
   }
   return true;
 }
 
-template <int MODE>
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1)
 split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_constant__ CUtensorMap tmap_w,
                     const SplitLogitsParams p) {
   extern __shared__ uint8_t smem_raw[];
-  const SmemView sm = carve_smem(smem_raw);
+  const SmemView sm = carve_smem(smem_raw, false, PAIR);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // provably warp-uniform
   const int lane = threadIdx.x & 31;
-  const uint32_t tmem_base = cta_setup(sm, warp, 1, EPI_WARPS);
+  const uint32_t tmem_base = cta_setup(sm, warp, 1, (PAIR ? 2 : 1) * EPI_WARPS, PAIR);
+  constexpr uint32_t kStages = PAIR ? PAIR_STAGES : STAGES;
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0;
+  const int unit0 = PAIR ? blockIdx.x >> 1 : blockIdx.x, unit_step = PAIR ? gridDim.x >> 1 : gridDim.x;
+  auto block_row = [&](int rb) { return (PAIR ? rb * 2 + static_cast<int>(rank) : rb) * BM; };
   const int total_units = p.num_rb * p.splits;
   auto vt_begin = [&](int split) { return static_cast<int>(static_cast<long long>(split) * p.num_vt / p.splits); };
 
@@ -238,15 +255,23 @@ split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
       tma_prefetch_desc(&tmap_w);
       uint32_t it = 0;
       bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+      for (int u = unit0; u < total_units && ok; u += unit_step) {
         const int split = u / p.num_rb, rb = u - split * p.num_rb;
         for (int vt = vt_begin(split); vt < vt_begin(split + 1) && ok; ++vt) {
           for (SplitWalk w(0, p.kblocks); !w.done(); w.next(), ++it) {
-            const int s = it % STAGES;
-            if (!mbar_wait(&sm.empty[s], ((it / STAGES) & 1) ^ 1, sm.abort_flag)) {
+            const int s = it % kStages;
+            if (!mbar_wait(&sm.empty[s], ((it / kStages) & 1) ^ 1, sm.abort_flag)) {
               raise_abort(sm, p.status, kDevTimeoutProducer);
               ok = false;
               break;
+            }
+            if (PAIR) {   // both CTAs' copies complete on CTA 0's barrier
+              if (rank == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * PAIR_STAGE_BYTES);
+              const uint32_t bar = map_to_rank(&sm.full[s], 0);
+              tma_load_4d_pair(sm.a(s), &tmap_h, bar, w.kb * BK, block_row(rb), 0, plane_a(w.pr));
+              tma_load_4d_pair(sm.b(s), &tmap_w, bar, w.kb * BK, vt * BN + static_cast<int>(rank) * (BN / 2), 0,
+                               plane_b(w.pr));
+              continue;
             }
             mbar_arrive_expect_tx(&sm.full[s], STAGE_BYTES);
             tma_load_4d(sm.a(s), &tmap_h, &sm.full[s], w.kb * BK, rb * BM, 0, plane_a(w.pr));
@@ -254,15 +279,16 @@ split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
           }
         }
       }
+      if (PAIR && ok) pair_tail(sm, it);
       if (!ok) producer_drain(sm, it);
     }
   } else if (warp == 1) {
     uint32_t it = 0, seg = 0;
-    bool ok = true;
-    for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+    bool ok = rank == 0;   // CTA 0 issues for both
+    for (int u = unit0; u < total_units && ok; u += unit_step) {
       const int split = u / p.num_rb;
       for (int vt = vt_begin(split); vt < vt_begin(split + 1) && ok; ++vt)
-        ok = issue_tile<false>(sm, tmem_base, 0, p.kblocks, it, seg, lane, p.status);
+        ok = issue_tile<false, PAIR>(sm, tmem_base, 0, p.kblocks, it, seg, lane, p.status);
     }
   } else {
     const int quad = warp & 3, half = (warp - 2) >> 2;
@@ -270,9 +296,9 @@ split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
     const int segs = (p.kblocks + SEG_KB - 1) / SEG_KB;
     uint32_t seg = 0;
     bool ok = true, bad = false;
-    for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+    for (int u = unit0; u < total_units && ok; u += unit_step) {
       const int split = u / p.num_rb, rb = u - split * p.num_rb;
-      const int row = rb * BM + quad * 32 + lane;
+      const int row = block_row(rb) + quad * 32 + lane;
       const bool row_ok = row < p.n_rows;
       const long long target = row_ok ? p.targets[row] : p.ignore_index;
       const bool tvalid = row_ok && target != p.ignore_index;
@@ -285,7 +311,7 @@ split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
       }
       for (int vt = vt_begin(split); vt < vt_begin(split + 1); ++vt) {
         float acc[HALF];
-        ok = gather_tile(sm, taddr, segs, seg, lane, acc, p.status);
+        ok = gather_tile<PAIR>(sm, taddr, segs, seg, lane, acc, p.status);
         if (!ok) break;
         const int col0 = vt * BN + half * HALF;          // chunk-relative column of acc[0]
         const int ncols = min(HALF, p.width - col0);     // columns that exist (may be <= 0)
@@ -332,10 +358,10 @@ split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
           }
           float s4[4] = {run_s, 0.f, 0.f, 0.f};
 #pragma unroll
-          for (int e = 0; e < HALF; e += 8) {
-            float g[8];
+          for (int e = 0; e < HALF; e += 16) {
+            float g[16];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
+            for (int k = 0; k < 16; ++k) {
               if (MODE == SPLIT_FWD_GRAD) {
                 // the target's own term p - 1 is added to d_hidden at the end
                 const float v = expf(acc[e + k]);
@@ -347,7 +373,7 @@ split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
               if (e + k == tcol) v -= 1.f;
               g[k] = e + k < ncols ? v * ct : 0.f;
             }
-            bad = split_store8(g, dst + e, plane) || bad;
+            bad = split_store(g, dst + e, plane) || bad;
           }
           if (MODE == SPLIT_FWD_GRAD) run_s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
         }
@@ -362,17 +388,22 @@ split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
     if (MODE != SPLIT_FWD && bad) *p.flag = 1;
     if (MODE == SPLIT_FWD_GRAD && blockIdx.x == 0 && warp == 2 && lane == 0 && *p.bad != 0) *p.flag = 1;
   }
-  cta_teardown(sm, warp, tmem_base);
+  cta_teardown(sm, warp, tmem_base, PAIR);
 }
 
+template <bool PAIR>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1)
 split_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__ CUtensorMap tmap_w,
                 const SplitDhParams p) {
   extern __shared__ uint8_t smem_raw[];
-  const SmemView sm = carve_smem(smem_raw);
+  const SmemView sm = carve_smem(smem_raw, false, PAIR);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // provably warp-uniform
   const int lane = threadIdx.x & 31;
-  const uint32_t tmem_base = cta_setup(sm, warp, 1, EPI_WARPS);
+  const uint32_t tmem_base = cta_setup(sm, warp, 1, (PAIR ? 2 : 1) * EPI_WARPS, PAIR);
+  constexpr uint32_t kStages = PAIR ? PAIR_STAGES : STAGES;
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0;
+  const int unit0 = PAIR ? blockIdx.x >> 1 : blockIdx.x, unit_step = PAIR ? gridDim.x >> 1 : gridDim.x;
+  auto block_row = [&](int rb) { return (PAIR ? rb * 2 + static_cast<int>(rank) : rb) * BM; };
   const int tiles = p.num_rb * p.num_nt, total_units = tiles * p.ksplit;
   auto kb_begin = [&](int share) { return static_cast<int>(static_cast<long long>(share) * p.kblocks / p.ksplit); };
 
@@ -382,15 +413,25 @@ split_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constan
       tma_prefetch_desc(&tmap_w);
       uint32_t it = 0;
       bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+      for (int u = unit0; u < total_units && ok; u += unit_step) {
         const int share = u / tiles, t = u - share * tiles;
         const int rb = t / p.num_nt, nt = t - rb * p.num_nt;
         for (SplitWalk w(kb_begin(share), kb_begin(share + 1)); !w.done(); w.next(), ++it) {
-          const int s = it % STAGES;
-          if (!mbar_wait(&sm.empty[s], ((it / STAGES) & 1) ^ 1, sm.abort_flag)) {
+          const int s = it % kStages;
+          if (!mbar_wait(&sm.empty[s], ((it / kStages) & 1) ^ 1, sm.abort_flag)) {
             raise_abort(sm, p.status, kDevTimeoutProducer);
             ok = false;
             break;
+          }
+          if (PAIR) {
+            if (rank == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * PAIR_STAGE_BYTES);
+            const uint32_t bar = map_to_rank(&sm.full[s], 0);
+            tma_load_4d_pair(sm.a(s), &tmap_g, bar, w.kb * BK, block_row(rb), 0, plane_a(w.pr));
+#pragma unroll
+            for (int j = 0; j < BN / 128; ++j)
+              tma_load_4d_pair(sm.b(s) + j * (64 * BK * 2), &tmap_w, bar,
+                               nt * BN + static_cast<int>(rank) * (BN / 2) + j * 64, w.kb * BK, 0, plane_b(w.pr));
+            continue;
           }
           mbar_arrive_expect_tx(&sm.full[s], STAGE_BYTES);
           tma_load_4d(sm.a(s), &tmap_g, &sm.full[s], w.kb * BK, rb * BM, 0, plane_a(w.pr));
@@ -400,26 +441,27 @@ split_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constan
                         plane_b(w.pr));
         }
       }
+      if (PAIR && ok) pair_tail(sm, it);
       if (!ok) producer_drain(sm, it);
     }
   } else if (warp == 1) {
     uint32_t it = 0, seg = 0;
-    bool ok = true;
-    for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+    bool ok = rank == 0;   // CTA 0 issues for both
+    for (int u = unit0; u < total_units && ok; u += unit_step) {
       const int share = u / tiles;
-      ok = issue_tile<true>(sm, tmem_base, kb_begin(share), kb_begin(share + 1), it, seg, lane, p.status);
+      ok = issue_tile<true, PAIR>(sm, tmem_base, kb_begin(share), kb_begin(share + 1), it, seg, lane, p.status);
     }
   } else {
     const int quad = warp & 3, half = (warp - 2) >> 2;
     const uint32_t taddr = tmem_base + half * HALF + (static_cast<uint32_t>(quad * 32) << 16);
     uint32_t seg = 0;
-    for (int u = blockIdx.x; u < total_units; u += gridDim.x) {
+    for (int u = unit0; u < total_units; u += unit_step) {
       const int share = u / tiles, t = u - share * tiles;
       const int rb = t / p.num_nt, nt = t - rb * p.num_nt;
       const int segs = (kb_begin(share + 1) - kb_begin(share) + SEG_KB - 1) / SEG_KB;
       float acc[HALF];
-      if (!gather_tile(sm, taddr, segs, seg, lane, acc, p.status)) break;
-      const int row = rb * BM + quad * 32 + lane, col0 = nt * BN + half * HALF;
+      if (!gather_tile<PAIR>(sm, taddr, segs, seg, lane, acc, p.status)) break;
+      const int row = block_row(rb) + quad * 32 + lane, col0 = nt * BN + half * HALF;
       if (row < p.n_rows) {
         float* dst = p.out + (static_cast<long long>(share) * p.n_rows + row) * p.d_cols + col0;
 #pragma unroll
@@ -436,7 +478,7 @@ split_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constan
       }
     }
   }
-  cta_teardown(sm, warp, tmem_base);
+  cta_teardown(sm, warp, tmem_base, PAIR);
 }
 
 // ref[row] = the target's logit (any vocab row's, where there is no target).  One warp per row; no alignment wanted.
@@ -477,19 +519,31 @@ split_finish_kernel(const float* __restrict__ acc, int shares, const float* __re
   out[off] = c * g;
 }
 
+// CTA pairs over 256 rows, as in linear_ce_tc.cu, where an odd number of row blocks does not leave much of the last
+// pair empty (2048 x 1024 x 32768, single CTAs against pairs and whole-sector stores of g: logits 176 / 124 us a chunk,
+// d_hidden 138 / 119; the tensor pipe was 46 and 57 % active).
+bool split_pair(int64_t n) {
+  const int64_t blocks = ceil_div(n, BM);
+  return blocks % 2 == 0 || blocks >= 9;
+}
+
 std::atomic<int> g_configured[64];
 
 int configure() {
   int dev = 0;
   B200TP_CUDA_OK(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && g_configured[dev].load(std::memory_order_acquire)) return B200TP_OK;
-  B200TP_CUDA_OK(cudaFuncSetAttribute(split_logits_kernel<SPLIT_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      SMEM_BYTES));
-  B200TP_CUDA_OK(cudaFuncSetAttribute(split_logits_kernel<SPLIT_BWD_G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      SMEM_BYTES));
-  B200TP_CUDA_OK(cudaFuncSetAttribute(split_logits_kernel<SPLIT_FWD_GRAD>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  B200TP_CUDA_OK(cudaFuncSetAttribute(split_dh_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  const void* kernels[] = {
+      reinterpret_cast<const void*>(split_logits_kernel<SPLIT_FWD, false>),
+      reinterpret_cast<const void*>(split_logits_kernel<SPLIT_BWD_G, false>),
+      reinterpret_cast<const void*>(split_logits_kernel<SPLIT_FWD_GRAD, false>),
+      reinterpret_cast<const void*>(split_dh_kernel<false>),
+      reinterpret_cast<const void*>(split_logits_kernel<SPLIT_FWD, true>),
+      reinterpret_cast<const void*>(split_logits_kernel<SPLIT_BWD_G, true>),
+      reinterpret_cast<const void*>(split_logits_kernel<SPLIT_FWD_GRAD, true>),
+      reinterpret_cast<const void*>(split_dh_kernel<true>)};
+  for (const void* k : kernels)
+    B200TP_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   if (dev >= 0 && dev < 64) g_configured[dev].store(1, std::memory_order_release);
   return B200TP_OK;
 }
@@ -507,23 +561,24 @@ int launch_logits(const void* h3, const void* w3, int64_t n, int d, int64_t widt
   CUtensorMap tmap_h, tmap_w;
   rc = plane_map(&tmap_h, h3, n, d, d, BM);
   if (rc) return rc;
-  rc = plane_map(&tmap_w, w3, width, d, d, BN);
+  const bool pair = split_pair(n);
+  rc = plane_map(&tmap_w, w3, width, d, d, pair ? BN / 2 : BN);
   if (rc) return rc;
   p.n_rows = static_cast<int>(n);
   p.kblocks = static_cast<int>(ceil_div(d, BK));
   p.width = static_cast<int>(width);
-  p.num_rb = static_cast<int>(ceil_div(n, BM));
+  p.num_rb = static_cast<int>(ceil_div(n, pair ? 2 * BM : BM));
   p.num_vt = static_cast<int>(ceil_div(width, BN));
-  const int grid = static_cast<int>(std::min<int64_t>(sm_count(), static_cast<int64_t>(p.num_rb) * p.splits));
-  split_logits_kernel<MODE><<<grid, SPLIT_THREADS, SMEM_BYTES, stream>>>(tmap_h, tmap_w, p);
-  B200TP_CUDA_OK(cudaGetLastError());
-  return B200TP_OK;
+  return launch_units(pair ? split_logits_kernel<MODE, true> : split_logits_kernel<MODE, false>, SPLIT_THREADS, pair,
+                      static_cast<long long>(p.num_rb) * p.splits, stream, tmap_h, tmap_w, p);
 }
 
 }  // namespace
 
 int ce_split_splits(int64_t n, int64_t width) {
-  return ce_tc_choose_splits(static_cast<int>(ceil_div(n, BM)), static_cast<int>(ceil_div(width, BN)));
+  const bool pair = split_pair(n);
+  return ce_tc_choose_splits(static_cast<int>(ceil_div(n, pair ? 2 * BM : BM)), static_cast<int>(ceil_div(width, BN)),
+                             pair ? sm_count() / 2 : sm_count());
 }
 
 int ce_split_planes(const float* x, int64_t count, void* planes, int* flag, cudaStream_t stream) {
@@ -611,7 +666,9 @@ int ce_split_finish(const float* acc, int shares, const float* ref, const int* s
 // Shares of the d_hidden contraction: the fewest that keep the busiest CTA's work (k blocks, plus about two per unit
 // for its prologue and epilogue) lowest, so that few tiles still fill the chip (2048 x 1024 has 64).
 int ce_split_dh_shares(int64_t n, int d, int64_t width) {
-  const int64_t tiles = ceil_div(n, BM) * ceil_div(d, BN), kblocks = ceil_div(width, BK), ctas = sm_count();
+  const bool pair = split_pair(n);
+  const int64_t tiles = ceil_div(n, pair ? 2 * BM : BM) * ceil_div(d, BN), kblocks = ceil_div(width, BK),
+                ctas = pair ? sm_count() / 2 : sm_count();
   int best = 1;
   int64_t best_cost = INT64_MAX;
   for (int ks = 1; ks <= std::min<int64_t>(64, kblocks) && (ks == 1 || tiles * ks <= 4 * ctas); ++ks) {
@@ -632,7 +689,8 @@ int ce_split_dh(const void* g3, int ldg, const void* w3, int64_t n, int d, int64
   p.n_rows = static_cast<int>(n);
   p.d_cols = d;
   p.kblocks = static_cast<int>(ceil_div(width, BK));
-  p.num_rb = static_cast<int>(ceil_div(n, BM));
+  const bool pair = split_pair(n);
+  p.num_rb = static_cast<int>(ceil_div(n, pair ? 2 * BM : BM));
   p.num_nt = static_cast<int>(ceil_div(d, BN));
   p.ksplit = ksplit;
   p.out = out;
@@ -643,11 +701,8 @@ int ce_split_dh(const void* g3, int ldg, const void* w3, int64_t n, int d, int64
   if (rc) return rc;
   rc = plane_map(&tmap_w, w3, width, d, d, BK);
   if (rc) return rc;
-  const int64_t units = static_cast<int64_t>(p.num_rb) * p.num_nt * ksplit;
-  const int grid = static_cast<int>(std::min<int64_t>(sm_count(), units));
-  split_dh_kernel<<<grid, SPLIT_THREADS, SMEM_BYTES, stream>>>(tmap_g, tmap_w, p);
-  B200TP_CUDA_OK(cudaGetLastError());
-  return B200TP_OK;
+  return launch_units(pair ? split_dh_kernel<true> : split_dh_kernel<false>, SPLIT_THREADS, pair,
+                      static_cast<long long>(p.num_rb) * p.num_nt * ksplit, stream, tmap_g, tmap_w, p);
 }
 
 int ce_split_sum(const float* acc, int shares, int64_t count, float* out, int keep, const int* skip_if_set,

@@ -83,7 +83,7 @@ extern "C" int b200tp_linear_ce_fwd_static(const b200tp_ce_args* a, float* row_m
   // as many shares as the kernel likes, and no more than single-CTA tiles would take: what fits does not depend on
   // which of the two runs
   const int most = ce_tc_choose_splits(static_cast<int>(ceil_div(a->n, kCeTileRows)),
-                                       static_cast<int>(ceil_div(a->v_local, kCeTileCols)));
+                                       static_cast<int>(ceil_div(a->v_local, kCeTileCols)), sm_count());
   const int splits = std::min(most, ce_tc_fwd_splits(a->n, a->d, a->v_local));
   const size_t need = 3ull * static_cast<size_t>(most) * static_cast<size_t>(a->n) * sizeof(float);
   if (need > kStaticScratchBytes)

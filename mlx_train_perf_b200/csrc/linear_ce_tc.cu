@@ -68,24 +68,6 @@ __device__ __forceinline__ bool guard_skips(const LaunchGuard& g) {
   return g.flag != nullptr && (*g.flag != 0) != (g.run_if_set != 0);
 }
 
-template <bool PAIR>
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
-                                     uint32_t idesc, uint32_t accumulate) {
-  if (PAIR) umma_ss_pair_w(tmem_d, a_lo, a_hi, b_lo, b_hi, idesc, accumulate);
-  else umma_ss_w(tmem_d, a_lo, a_hi, b_lo, b_hi, idesc, accumulate);
-}
-template <bool PAIR>
-__device__ __forceinline__ void commit(uint64_t* bar) {
-  if (PAIR) umma_commit_pair(bar);
-  else umma_commit(bar);
-}
-// An epilogue warp has read its accumulator: told to the CTA that issues the MMAs.
-template <bool PAIR>
-__device__ __forceinline__ void release_acc(uint64_t* bar) {
-  if (PAIR) mbar_arrive_cluster(map_to_rank(bar, 0));
-  else mbar_arrive(bar);
-}
-
 // 32 columns of a row of g as whole sectors.  With 16-byte stores every sector was written in two halves, and at
 // D = 1024 the L2 took them no faster than the tensor cores made them (15194 vocab rows x 4096 rows: 115 -> 90 us).
 __device__ __forceinline__ void store_g(__nv_bfloat16* dst, const uint32_t (&v)[16]) {
@@ -1052,26 +1034,7 @@ static bool use_pair(int64_t n, int d) {
   return blocks >= 16 || (blocks % 2 == 0 && d >= 2048);
 }
 
-// `units` of work on pairs (`kernel` is a PAIR instantiation) or on single CTAs.
-template <typename P>
-static int launch_units(void (*kernel)(CUtensorMap, CUtensorMap, P), bool pair, long long units, cudaStream_t stream,
-                        const CUtensorMap& a, const CUtensorMap& b, const P& p) {
-  cudaLaunchConfig_t cfg{};
-  const long long most = pair ? sm_count() / 2 : sm_count();
-  cfg.gridDim = dim3(static_cast<unsigned>(std::min(most, units) * (pair ? 2 : 1)));
-  cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim = {2, 1, 1};
-  cfg.attrs = attr;
-  cfg.numAttrs = pair ? 1 : 0;
-  B200TP_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, a, b, p));
-  return B200TP_OK;
-}
-
-int ce_tc_choose_splits(int num_rb, int num_vt) { return choose_splits(num_rb, num_vt, sm_count()); }
+int ce_tc_choose_splits(int num_rb, int num_vt, int ctas) { return choose_splits(num_rb, num_vt, ctas); }
 
 int ce_tc_fwd_splits(int64_t n, int d, int64_t v_rows) {
   const int num_vt = static_cast<int>(ceil_div(v_rows, BN));
@@ -1134,7 +1097,7 @@ int ce_tc_launch_fwd(const void* hidden, const void* w, int64_t w_rows_total, in
     B200TP_CUDA_OK(cudaGetLastError());
     return B200TP_OK;
   }
-  return launch_units(pair ? ce_logits_kernel<MODE_FWD, false, true> : ce_logits_kernel<MODE_FWD, false>, pair,
+  return launch_units(pair ? ce_logits_kernel<MODE_FWD, false, true> : ce_logits_kernel<MODE_FWD, false>, THREADS, pair,
                       static_cast<long long>(p.num_rb) * splits, stream, tmap_h, tmap_w, p);
 }
 
@@ -1176,7 +1139,7 @@ int ce_tc_launch_bwd_g(const void* hidden, const void* w, int64_t w_rows_total, 
     B200TP_CUDA_OK(cudaGetLastError());
     return B200TP_OK;
   }
-  return launch_units(pair ? ce_logits_kernel<MODE_BWD_G, false, true> : ce_logits_kernel<MODE_BWD_G, false>, pair,
+  return launch_units(pair ? ce_logits_kernel<MODE_BWD_G, false, true> : ce_logits_kernel<MODE_BWD_G, false>, THREADS, pair,
                       static_cast<long long>(p.num_rb) * p.splits, stream, tmap_h, tmap_w, p);
 }
 
@@ -1211,7 +1174,7 @@ int ce_tc_launch_fwd_grad(const void* hidden, const void* w, int64_t w_rows_tota
   p.ref2 = ref2;
   p.overflow = overflow;
   p.status = status;
-  return launch_units(pair ? ce_logits_kernel<MODE_FWD_GRAD, false, true> : ce_logits_kernel<MODE_FWD_GRAD, false>, pair,
+  return launch_units(pair ? ce_logits_kernel<MODE_FWD_GRAD, false, true> : ce_logits_kernel<MODE_FWD_GRAD, false>, THREADS, pair,
                       static_cast<long long>(p.num_rb) * splits, stream, tmap_h, tmap_w, p);
 }
 
@@ -1295,7 +1258,7 @@ int ce_tc_launch_dh(const void* g, int ldg, int k_total, int64_t n, const void* 
     B200TP_CUDA_OK(cudaGetLastError());
     return B200TP_OK;
   }
-  return launch_units(pair ? ce_dh_kernel<false, true> : ce_dh_kernel<false>, pair, p.tile1 - p.tile0, stream, tmap_g,
+  return launch_units(pair ? ce_dh_kernel<false, true> : ce_dh_kernel<false>, THREADS, pair, p.tile1 - p.tile0, stream, tmap_g,
                       tmap_w, p);
 }
 
@@ -1317,7 +1280,7 @@ int ce_tc_launch_dw(const void* g, int ldg, int64_t v_rows, int64_t n, const voi
   p.num_nt = static_cast<int>(ceil_div(d, BN));
   p.out = reinterpret_cast<__nv_bfloat16*>(d_weight_block);
   p.status = status;
-  return launch_units(ce_dw_kernel<true>, true, static_cast<long long>(p.num_mt) * p.num_nt, stream, tmap_g, tmap_h, p);
+  return launch_units(ce_dw_kernel<true>, THREADS, true, static_cast<long long>(p.num_mt) * p.num_nt, stream, tmap_g, tmap_h, p);
 }
 
 }  // namespace b200tp

@@ -28,8 +28,8 @@ struct LaunchGuard {
 // Vocab splits the forward uses for (n rows, v_rows vocab rows): one partial triple per
 // (row, split) lands in the workspace.
 int ce_tc_fwd_splits(int64_t n, int d, int64_t v_rows);
-// The split count behind it, for `num_rb` row groups and `num_vt` vocab tiles.
-int ce_tc_choose_splits(int num_rb, int num_vt);
+// The split count behind it, for `num_rb` row groups and `num_vt` vocab tiles on `ctas` CTAs (or pairs).
+int ce_tc_choose_splits(int num_rb, int num_vt, int ctas);
 
 // Forward partials over weight rows [vrow0, vrow1) of a (w_rows_total, d) bf16 matrix whose
 // row 0 has global vocab id `vocab_id0`.  pm/ps/pt: [splits][n] f32.
