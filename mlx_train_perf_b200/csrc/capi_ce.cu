@@ -116,8 +116,8 @@ int check_args(const b200tp_ce_args* a) {
 //     on dequantised weights, and the only ones of the backward) once per 128;
 //   chunk by chunk into a bf16 scratch (one pass over the codes per GEMM pass, 0.03 ms per 16384 x 4096
 //     chunk) followed by the dense kernels.
-// Default, from timings at D=4096, V=151936 (in-kernel / chunked, us): forward 260 / 691 at N=60, 304 / 884 at 257,
-// 563 / 927 at 512, 1176 / 1481 at 1024, 2050 / 2427 at 2048, 4373 / 4228 at 4096 -- in the kernel up to
+// Default, from timings at D=4096, V=151936 (in-kernel / chunked, us): forward 260 / 692 at N=60, 304 / 884 at 257,
+// 563 / 815 at 512, 1176 / 1344 at 1024, 2050 / 2245 at 2048, 4373 / 4194 at 4096 -- in the kernel up to
 // kInlineMaxRows rows, with no weight scratch at all; backward 3.2 / 1.9 ms at N=128, 3.8 / 2.1 at 512 -- always
 // chunked: with few row blocks the d_hidden GEMM has only D / 256 tiles, so a handful of CTAs would each expand their
 // 256 columns of the whole head, while the dequantisation kernel spreads the same work over every SM.  `reserved`

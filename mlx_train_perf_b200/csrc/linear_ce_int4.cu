@@ -12,7 +12,8 @@
 // vocab share the four lane quadrants' triples of a token are merged into one.
 //
 // Tensor-bound from about 200 tokens on, expansion-bound below (about 170 instructions per 64 weights; eight warps in
-// two groups, each taking every other k block, keep it under the MMAs of 272 tokens).
+// two groups, each taking every other k block, keep it under the MMAs of 272 tokens; three groups make 60 tokens 260 ->
+// 239 us, and 257 304 -> 313, 2048 2050 -> 2249).
 //
 // Roles (19 warps): two TMA producers, MMA issuer, eight epilogue warps, eight expanding warps.  Waits are bounded and end
 // like those of linear_ce_tc.cu.  Replaces core/kernel/source.py:199-340 (K2) of the reference.
