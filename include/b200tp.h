@@ -178,7 +178,9 @@ int b200tp_linear_ce_bwd_stage(const b200tp_ce_args* a, const float* lse, const 
  * rounding -- the `d_w_chunks` of core/chunked.py:84-90; replaces core/kernel/launch.py:249-322
  * (`backward_dw`).  Every vocab row belongs to one chunk, so d_weight is written, never
  * accumulated; vocab-sharded callers own disjoint row blocks.  Same workspace as the plain
- * backward.  Quantized heads are frozen and are refused. */
+ * backward.  Quantized heads are frozen and are refused.
+ * Give every backward the `lse` of a forward of the same impl and `reserved`: errors that lse and the backward's logits
+ * share cancel in exp(z - lse). */
 int b200tp_linear_ce_bwd_train(const b200tp_ce_args* a, const float* lse, const float* cotangent, void* d_hidden,
                                int32_t d_hidden_dtype, int32_t accumulate, void* d_weight, void* workspace,
                                size_t workspace_bytes, void* stream, int* status);

@@ -470,8 +470,8 @@ class _FusedLinearCETrainable(torch.autograd.Function):
 
 
 def _trained(impl: str) -> str:
-    """The gradient of a trained fp32 head is formed on the CUDA cores, and lse has to come from the same logits: errors
-    that the two share cancel in exp(z - lse)."""
+    """A trained fp32 head stays on the CUDA cores in both directions (the contraction for its gradient runs there in any
+    case).  lse and the gradient have to come from one kind of logits: errors that the two share cancel in exp(z - lse)."""
     return "simt" if impl == "auto" else impl
 
 

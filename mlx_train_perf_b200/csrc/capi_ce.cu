@@ -145,9 +145,9 @@ QuantHead quant_head(const b200tp_ce_args* a, bool backward) {
 
 // 1 = tcgen05, 2 = SIMT, 3 = tcgen05 over the three bf16 planes of fp32 operands, negative = refusal already
 // recorded.  3 is the default for fp32 with a dense head: 2048 x 1024 x 32768 forward + backward 18.5 -> 1.65 ms, with
-// a third of the CUDA-core path's distance to float64 .  A trained fp32 head's backward stays on the CUDA
-// cores, and so do D % 8 != 0 (TMA strides), a 4-bit head under fp32 hidden states, and calls whose contraction is
-// under 2^28 multiplications: there the CUDA cores need no longer than the split's extra launches take (forward /
+// a third of the CUDA-core path's distance to float64.  The CUDA cores keep the contraction of a trained head's
+// gradient (its g comes from the planes like the forward's lse), D % 8 != 0 (TMA strides), a 4-bit head under fp32
+// hidden states, and calls whose contraction is under 2^28 multiplications: there the CUDA cores need no longer than the split's extra launches take (forward /
 // forward + backward, CUDA cores against split: 128 x 512 x 2000 65 / 259 against 90 / 282 us, 32 x 1024 x 32000
 // 1001 / 4151 against 173 / 430 us).
 int pick_impl(const b200tp_ce_args* a) {
@@ -625,7 +625,7 @@ static int bwd_impl(const b200tp_ce_args* a, const float* lse, const float* cota
   // The other two paths are not staged (everything runs in stage 0).
   if (rows_done != nullptr) *rows_done = a->n;
   if (stage > 0) return B200TP_OK;
-  if (p.impl == 3 && d_weight == nullptr) {
+  if (p.impl == 3) {
     B200TP_CUDA_OK(cudaMemsetAsync(p.flag, 0, sizeof(int), stream));
     rc = ce_split_planes(static_cast<const float*>(a->hidden), a->n * a->d, p.h3, p.flag, stream);
     if (rc) return rc;
@@ -639,12 +639,17 @@ static int bwd_impl(const b200tp_ce_args* a, const float* lse, const float* cota
       if (rc) return rc;
       rc = ce_split_dh(p.g3, p.ldg, p.w3, a->n, a->d, w, p.shares, p.shares_acc, c > 0, stream, status);
       if (rc) return rc;
+      if (d_weight != nullptr) {
+        // g from the same logits as the forward's lse, whose errors cancel in exp(z - lse); the contraction over the
+        // rows on the CUDA cores
+        rc = ce_simt_dw_planes(p.g3, p.ldg, w, static_cast<const float*>(a->hidden), a->n, a->d,
+                               static_cast<float*>(d_weight) + r0 * a->d, p.flag, stream);
+        if (rc) return rc;
+      }
     }
     // d_hidden is only touched once it is known that the planes held every value
     rc = ce_split_sum(p.shares_acc, p.shares, a->n * a->d, static_cast<float*>(d_hidden), accumulate, p.flag, stream);
     if (rc) return rc;
-  } else {
-    p.flag = nullptr;   // the CUDA-core path, unconditionally
   }
   float* acc = out_f32 ? static_cast<float*>(d_hidden) : p.acc;
   for (int64_t r0 = 0; r0 < a->v_local; r0 += p.simt_chunk) {
@@ -664,7 +669,7 @@ static int bwd_impl(const b200tp_ce_args* a, const float* lse, const float* cota
     if (rc) return rc;
     if (d_weight != nullptr) {
       void* block = static_cast<char*>(d_weight) + static_cast<size_t>(r0) * a->d * elem_size(a->dtype);
-      rc = ce_simt_dw_chunk(p.logits, w, a->hidden, a->dtype, a->n, a->d, block, stream);
+      rc = ce_simt_dw_chunk(p.logits, w, a->hidden, a->dtype, a->n, a->d, block, stream, p.flag);
       if (rc) return rc;
     }
   }

@@ -131,12 +131,20 @@ gemm_nn_acc_kernel(const float* __restrict__ A, long long lda, const TB* __restr
   }
 }
 
-// C[M x Nn] = A^T B with A (K x M) fp32 row-major (the g scratch), B (K x Nn) row-major
+// An element of g: fp32, or the exact sum of its three bf16 planes, `plane` elements apart.
+__device__ __forceinline__ float load_g(const float* g, long long i, long long) { return g[i]; }
+__device__ __forceinline__ float load_g(const __nv_bfloat16* g, long long i, long long plane) {
+  return to_f32(g[i]) + to_f32(g[i + plane]) + to_f32(g[i + 2 * plane]);
+}
+
+// C[M x Nn] = A^T B with A (K x M) row-major (the g scratch: see load_g), B (K x Nn) row-major
 // (hidden); written once in the output type.  d_weight of a trainable head, one vocab chunk.
-template <typename TB, typename TO>
+template <typename TA, typename TB, typename TO>
 __global__ void __launch_bounds__(256)
-gemm_tn_out_kernel(const float* __restrict__ A, long long lda, const TB* __restrict__ B, long long ldb,
-                   TO* __restrict__ C, long long ldc, int M, int Nn, int K) {
+gemm_tn_out_kernel(const TA* __restrict__ A, long long lda, long long plane, const TB* __restrict__ B, long long ldb,
+                   TO* __restrict__ C, long long ldc, int M, int Nn, int K, const int* run_if_set,
+                   const int* skip_if_set) {
+  if ((run_if_set != nullptr && *run_if_set == 0) || (skip_if_set != nullptr && *skip_if_set != 0)) return;
   __shared__ float As[TK][TS + 1];
   __shared__ float Bs[TK][TS + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -151,7 +159,7 @@ gemm_tn_out_kernel(const float* __restrict__ A, long long lda, const TB* __restr
     for (int i = 0; i < 4; ++i) {
       const int idx = threadIdx.x + i * 256;
       const int kr = idx >> 6, c = idx & 63;  // kr = k, c = column of A (m) / of B (n)
-      As[kr][c] = (k0 + kr < K && m0 + c < M) ? A[static_cast<long long>(k0 + kr) * lda + m0 + c] : 0.f;
+      As[kr][c] = (k0 + kr < K && m0 + c < M) ? load_g(A, static_cast<long long>(k0 + kr) * lda + m0 + c, plane) : 0.f;
       Bs[kr][c] = (k0 + kr < K && n0 + c < Nn) ? to_f32(B[static_cast<long long>(k0 + kr) * ldb + n0 + c]) : 0.f;
     }
     __syncthreads();
@@ -558,17 +566,27 @@ int ce_simt_bwd_chunk(const void* hidden, const void* w_chunk, int dtype, int64_
 }
 
 int ce_simt_dw_chunk(const float* g_ws, int64_t width, const void* hidden, int dtype, int64_t n, int d,
-                     void* d_weight_block, cudaStream_t stream) {
+                     void* d_weight_block, cudaStream_t stream, const int* run_if_set) {
   dim3 grid(static_cast<unsigned>(ceil_div(d, TS)), static_cast<unsigned>(ceil_div(width, TS)));
   if (dtype == B200TP_F32) {
-    gemm_tn_out_kernel<float, float><<<grid, 256, 0, stream>>>(g_ws, width, static_cast<const float*>(hidden), d,
-                                                               static_cast<float*>(d_weight_block), d,
-                                                               static_cast<int>(width), d, static_cast<int>(n));
+    gemm_tn_out_kernel<<<grid, 256, 0, stream>>>(g_ws, width, 0ll, static_cast<const float*>(hidden), d,
+                                                 static_cast<float*>(d_weight_block), d, static_cast<int>(width), d,
+                                                 static_cast<int>(n), run_if_set, nullptr);
   } else {
-    gemm_tn_out_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, stream>>>(
-        g_ws, width, static_cast<const __nv_bfloat16*>(hidden), d, static_cast<__nv_bfloat16*>(d_weight_block), d,
-        static_cast<int>(width), d, static_cast<int>(n));
+    gemm_tn_out_kernel<<<grid, 256, 0, stream>>>(
+        g_ws, width, 0ll, static_cast<const __nv_bfloat16*>(hidden), d, static_cast<__nv_bfloat16*>(d_weight_block), d,
+        static_cast<int>(width), d, static_cast<int>(n), run_if_set, nullptr);
   }
+  B200TP_CUDA_OK(cudaGetLastError());
+  return B200TP_OK;
+}
+
+int ce_simt_dw_planes(const void* g3, int ldg, int64_t width, const float* hidden, int64_t n, int d,
+                      float* d_weight_block, const int* skip_if_set, cudaStream_t stream) {
+  dim3 grid(static_cast<unsigned>(ceil_div(d, TS)), static_cast<unsigned>(ceil_div(width, TS)));
+  gemm_tn_out_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(g3), ldg, static_cast<long long>(n) * ldg,
+                                               hidden, d, d_weight_block, d, static_cast<int>(width), d,
+                                               static_cast<int>(n), nullptr, skip_if_set);
   B200TP_CUDA_OK(cudaGetLastError());
   return B200TP_OK;
 }

@@ -38,7 +38,10 @@ int ce_simt_bwd_chunk(const void* hidden, const void* w_chunk, int dtype, int64_
 // d_weight block (width, d) in the hidden dtype = g^T @ hidden, g (n, width) f32 as left in
 // logits_ws by ce_simt_bwd_chunk.
 int ce_simt_dw_chunk(const float* g_ws, int64_t width, const void* hidden, int dtype, int64_t n, int d,
-                     void* d_weight_block, cudaStream_t stream);
+                     void* d_weight_block, cudaStream_t stream, const int* run_if_set = nullptr);
+// The same from g as three bf16 planes (n, ldg) each, its exact sum; nothing while *skip_if_set is set.
+int ce_simt_dw_planes(const void* g3, int ldg, int64_t width, const float* hidden, int64_t n, int d,
+                      float* d_weight_block, const int* skip_if_set, cudaStream_t stream);
 
 int launch_cast_f32_to_bf16(const float* src, void* dst, int64_t count, cudaStream_t stream);
 

@@ -9,6 +9,7 @@ import math
 import pytest
 import torch
 
+from mlx_train_perf_b200 import parallel
 from mlx_train_perf_b200.core import loss as L
 from mlx_train_perf_b200.core.loss import DenseHead, fused_linear_ce, reduced_linear_cross_entropy
 from oracle import linear_ce as oc
@@ -155,3 +156,58 @@ def test_trained_head_keeps_one_kind_of_logits(cuda_device):
     for a, b in zip(*out):
         assert torch.equal(a, b)
     assert n * d * v >= 2 ** 28 and not torch.equal(fused_linear_ce(h, DenseHead(w, trainable=False), t)[1], out[0][1])
+
+
+def test_trained_shards_keep_one_kind_of_logits(cuda_device, monkeypatch):
+    """The vocabulary-sharded operator with d_weight, two shards that would each be split: lse and the gradients come from
+    the same logits, so the distance to fp64 is no larger than the CUDA cores', up to the last rounding of the results."""
+    n, d, v = 128, 1024, 4099
+    (h, w, t), ct = _inputs(n, d, v), torch.linspace(-1, 1.5, n)
+    _, r_lse, _ = oc.naive_linear_ce(h, w, t, dtype=torch.float64)
+    r_dh, r_dw = oc.chunked_backward(h, w, t, r_lse, ct.double(), chunk_size=4096, dtype=torch.float64, want_dw=True)
+    hd, td, ctd = h.to(cuda_device), t.to(cuda_device), ct.to(cuda_device)
+    shards = [parallel.shard_dense_head(w.to(cuda_device), 2, rank) for rank in range(2)]
+    assert min(head.weight.shape[0] for head, _ in shards) * n * d >= 2 ** 28
+    err = {}
+    for impl in ("auto", "simt"):
+        ops = [parallel.VocabShardedLinearCE(head, lo, impl=impl) for head, lo in shards]
+        parts = torch.stack([L.ce_forward_buffer(hd, head, td, v_offset=lo, impl=impl, want_lse=False)[:3]
+                             for head, lo in shards])
+        monkeypatch.setattr(parallel, "gather_partials", lambda local, group=None: parts)
+        dh, dw = torch.zeros(n, d, dtype=torch.float64), []
+        for op in ops:
+            monkeypatch.setattr(op, "_reduce", lambda partial, dtype: partial)
+            _, lse, _ = op.forward(hd, td)
+            dw.append(torch.full_like(op.head.weight, float("nan")))
+            dh += op.backward(hd, td, lse, ctd, d_weight=dw[-1]).double().cpu()
+        L.check_device_status()
+        err[impl] = [(dh - r_dh).norm(), (torch.cat(dw).double().cpu() - r_dw).norm()]
+    for got, cores, ref in zip(err["auto"], err["simt"], (r_dh, r_dw)):
+        assert got <= cores + 2.0 ** -24 * ref.norm(), (float(got / ref.norm()), float(cores / ref.norm()))
+
+
+@pytest.mark.parametrize(("n", "d", "v", "what"), [(1, 8, 1, "planes"), (129, 136, 4099, "planes"),
+                                                   (300, 264, 25000, "planes"), (129, 136, 4095, "inf")])
+def test_gradient_of_the_weight(cuda_device, n, d, v, what):
+    """Against the CUDA cores' d_weight; with a value that has no planes it is theirs, bit for bit (one chunk).  Bound: g moves by
+    the errors of z and lse (as above, for both kinds), the sum over n rows by n 2^-24 of its terms, for both."""
+    h, w, t = _inputs(n, d, v)
+    if what == "inf":
+        w[0] = 0
+        w[0, 3] = -math.inf
+        h[:, 3] = h[:, 3].abs() + 0.1
+    ct, out = torch.linspace(-1, 1.5, n).to(cuda_device), []
+    hd, td, head = h.to(cuda_device), t.to(cuda_device), DenseHead(w.to(cuda_device))
+    for impl in ("split", "simt"):
+        lse = L.ce_forward_raw(hd, head, td, impl=impl)[3]
+        dw = torch.full_like(head.weight, 7.0)
+        dh = L.ce_backward_raw(hd, head, td, lse, ct, impl=impl, d_weight=dw)
+        out.append((dh.cpu(), dw.cpu()))
+    L.check_device_status()
+    if what == "inf":
+        for a, b in zip(*out):
+            assert torch.equal(a.nan_to_num(7e7), b.nan_to_num(7e7))
+        return
+    z = (9 + d) * 2.0 ** -23 * (h.norm(dim=1) * w.norm(dim=1).max()).max() + 2.0 ** -20
+    terms = ct.abs().cpu() @ h.abs()                  # a row of d_weight, were every |g| as large as |ct|
+    assert ((out[0][1] - out[1][1]).abs() <= (4 * z + n * 2.0 ** -23) * terms + 1e-12).all()
