@@ -340,7 +340,8 @@ def _forms_grad(impl: str, hidden_wants_grad: bool, hidden: torch.Tensor, head: 
     """Whether the forward of a frozen head also forms the gradient of the hidden states (two contractions over
     N x V x D in all, where a backward that computes the logits again makes it three): on the tensor-core path,
     when autograd may ask for that gradient.  A forward whose gradient is never wanted is best run under
-    `torch.no_grad()`, where it stays at one contraction."""
+    `torch.no_grad()`, where it stays at one contraction.  (`ctx.needs_input_grad` says whether a tensor requires grad,
+    not whether autograd records, and inside `forward` it never does: the callers below ask before `apply`.)"""
     if not hidden_wants_grad or impl in ("tc", "tc_chunked"):
         return hidden_wants_grad
     if impl not in ("auto", "split") or hidden.dtype != torch.float32:
@@ -408,8 +409,8 @@ class _FusedLinearCE(torch.autograd.Function):
     """(hidden, targets) -> (nll, lse, tgt); the head is a constant (frozen)."""
 
     @staticmethod
-    def forward(ctx, hidden, targets, head, ignore_index, impl):
-        if _forms_grad(impl, ctx.needs_input_grad[0], hidden, head, targets):
+    def forward(ctx, hidden, targets, head, ignore_index, impl, recorded):
+        if _forms_grad(impl, recorded and ctx.needs_input_grad[0], hidden, head, targets):
             out, state = ce_forward_grad(hidden, head, targets, ignore_index=ignore_index, impl=impl)
             tgt, lse, nll = out[0], out[1], out[2]
             ctx.save_for_backward(hidden, targets, out, state)
@@ -426,7 +427,7 @@ class _FusedLinearCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_nll, _g_lse, _g_tgt):
         if g_nll is None:
-            return (None,) * 5
+            return (None,) * 6
         key = "quantized" if isinstance(ctx.head, QuantizedHead) else "dense"
         VJP_CALLS[key] = VJP_CALLS.get(key, 0) + 1
         saved = ctx.saved_tensors
@@ -438,7 +439,7 @@ class _FusedLinearCE(torch.autograd.Function):
             hidden, targets, lse = saved
             d_hidden = ce_backward_raw(hidden, ctx.head, targets, lse, g_nll, ignore_index=ctx.ignore_index,
                                        impl=ctx.impl)
-        return d_hidden, None, None, None, None
+        return d_hidden, None, None, None, None, None
 
 
 class _FusedLinearCETrainable(torch.autograd.Function):
@@ -481,7 +482,7 @@ def _apply(hidden2, targets2, head, ignore_index, impl):
             and torch.is_grad_enabled()):
         w = head.weight if head.weight.is_contiguous() else head.weight.contiguous()
         return _FusedLinearCETrainable.apply(hidden2, w, targets2, ignore_index, _trained(impl))
-    return _FusedLinearCE.apply(hidden2, targets2, head, ignore_index, impl)
+    return _FusedLinearCE.apply(hidden2, targets2, head, ignore_index, impl, torch.is_grad_enabled())
 
 
 class _FusedLinearCEReduced(torch.autograd.Function):
@@ -493,11 +494,11 @@ class _FusedLinearCEReduced(torch.autograd.Function):
     wanted (then `head` is ignored), else None."""
 
     @staticmethod
-    def forward(ctx, hidden, weight, targets, head, ignore_index, impl, mean):
+    def forward(ctx, hidden, weight, targets, head, ignore_index, impl, mean, recorded):
         use = DenseHead(weight=weight) if weight is not None else head
         dev = hidden.device
         out3 = torch.empty(3, dtype=torch.float32, device=dev)
-        if weight is None and _forms_grad(impl, ctx.needs_input_grad[0], hidden, use, targets):
+        if weight is None and _forms_grad(impl, recorded and ctx.needs_input_grad[0], hidden, use, targets):
             saved = list(ce_forward_grad(hidden, use, targets, ignore_index=ignore_index, impl=impl, out3=out3))
         else:
             _, _, _, lse, nll = ce_forward_raw(hidden, use, targets, ignore_index=ignore_index, impl=impl)
@@ -517,7 +518,7 @@ class _FusedLinearCEReduced(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_loss, _g_count):
         if g_loss is None:
-            return (None,) * 7
+            return (None,) * 8
         saved = ctx.saved_tensors
         hidden, targets, out3, rows = saved[:4]      # rows: lse, or the three rows of `ce_forward_grad`
         weight = saved[4] if ctx.trains_weight else None
@@ -531,7 +532,7 @@ class _FusedLinearCEReduced(torch.autograd.Function):
         if ctx.has_grad:
             d_hidden = ce_backward_grad(hidden, head, targets, rows, saved[4], None, ignore_index=ctx.ignore_index,
                                         impl=ctx.impl, upstream=g, count=out3.data_ptr() + 8 if ctx.mean else None)
-            return d_hidden, None, None, None, None, None, None
+            return d_hidden, None, None, None, None, None, None, None
         ct = torch.empty(n, dtype=torch.float32, device=dev)
         with _lib.on(dev):
             rc = lib.b200tp_linear_ce_cotangent(targets.data_ptr(), n, ctx.ignore_index, g.data_ptr(),
@@ -542,7 +543,7 @@ class _FusedLinearCEReduced(torch.autograd.Function):
             d_w = torch.empty_like(weight, memory_format=torch.contiguous_format)
         d_hidden = ce_backward_raw(hidden, head, targets, rows, ct, ignore_index=ctx.ignore_index, impl=ctx.impl,
                                    d_weight=d_w)
-        return d_hidden, d_w, None, None, None, None, None
+        return d_hidden, d_w, None, None, None, None, None, None
 
 
 def masked_loss(nll: torch.Tensor, targets: torch.Tensor, *, mean: bool = True,
@@ -580,7 +581,7 @@ def _apply_reduced(hidden2, targets2, head, ignore_index, impl, mean):
     if trainable:
         w = head.weight if head.weight.is_contiguous() else head.weight.contiguous()
         impl = _trained(impl)
-    return _FusedLinearCEReduced.apply(hidden2, w, targets2, head, ignore_index, impl, mean)
+    return _FusedLinearCEReduced.apply(hidden2, w, targets2, head, ignore_index, impl, mean, torch.is_grad_enabled())
 
 
 def _prepare(hidden, head, targets, *, impl, validate_targets, ignore_index):

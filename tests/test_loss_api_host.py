@@ -163,3 +163,39 @@ def test_masked_loss_refuses_host_tensors():
     from mlx_train_perf_b200.core.loss import masked_loss
     with pytest.raises(LossInputError, match="CUDA"):
         masked_loss(torch.zeros(4), torch.zeros(4, dtype=torch.int64))
+
+
+@pytest.mark.parametrize("reduced", [False, True])
+@pytest.mark.parametrize("mode", ["grad", "no_grad", "inference", "frozen"])
+def test_gradient_is_formed_only_where_autograd_records(monkeypatch, mode, reduced):
+    """Which forward a frozen head's loss asks the library for: hidden states that require grad under `no_grad` or
+    `inference_mode` (an evaluation on a training pass's activations, a reentrant checkpoint's first pass) take the plain
+    one, like those that do not require grad."""
+    import contextlib
+    from types import SimpleNamespace
+
+    from mlx_train_perf_b200.core import loss as L
+    asked = []
+
+    def raw(hidden, head, targets, **kw):
+        asked.append("plain")
+        return tuple(torch.zeros(5, hidden.shape[0]))
+
+    def grad(hidden, head, targets, **kw):
+        asked.append("gradient")
+        return torch.zeros(3, hidden.shape[0]), torch.zeros(256, dtype=torch.uint8)
+
+    monkeypatch.setattr(L, "ce_forward_raw", raw)
+    monkeypatch.setattr(L, "ce_forward_grad", grad)
+    monkeypatch.setattr(L._lib, "load", lambda: SimpleNamespace(b200tp_linear_ce_reduce=lambda *a: 0))
+    monkeypatch.setattr(L._lib, "on", lambda device: contextlib.nullcontext())
+    monkeypatch.setattr(L._lib, "stream", lambda device: 0)
+    hidden, head, targets = _dense(dtype=torch.bfloat16)
+    hidden.requires_grad_(mode != "frozen")
+    with {"no_grad": torch.no_grad, "inference": torch.inference_mode}.get(mode, contextlib.nullcontext)():
+        if reduced:
+            out = L._apply_reduced(hidden, targets, DenseHead(head.weight, trainable=False), -100, "tc", True)
+        else:
+            out = L._apply(hidden, targets, DenseHead(head.weight, trainable=False), -100, "tc")
+    assert asked == ["gradient" if mode == "grad" else "plain"]
+    assert out[0].requires_grad == (mode == "grad")
