@@ -4,9 +4,9 @@
 Peak = (weights + base + LoRA + AdamW + linear activations + attention + loss) x (1 + overhead).
 Attention is either "stock" (a materialised (N, N) backward) or "flash" (saved O + L plus a
 linear transient); the loss is "naive" (full logits), "chunked" (one 8192-column tile) or
-"kernel" (no logits: three N-length fp32 vectors, plus -- with the B200 calibration -- the
-backward's (N, chunk) bf16 tile and (N, D) fp32 accumulator).  Pure arithmetic; the only
-device query is the default budget.
+"kernel" (no logits: three N-length fp32 vectors, plus -- with the B200 calibration -- the (N, chunk)
+tile of g, one chunk of a 4-bit or fp32 head in bf16 and the fp32 sums of d_hidden, as the library sizes
+them).  Pure arithmetic; the only device query is the default budget.
 """
 from __future__ import annotations
 
@@ -22,6 +22,7 @@ CHUNK_TILE = 8192          # the chunked loss impl's fixed vocab tile
 LORA_MODULES = 2           # q_proj, v_proj
 LORA_MATRICES = 2          # A, B
 B200_HBM_BYTES = 183_359 * 1024 ** 2   # what nvidia-smi reports for one B200
+B200_SMS = 148
 BUDGET_FRACTION = 0.92     # default share of device memory the plan may use
 
 
@@ -135,18 +136,65 @@ def _attention_bytes(cfg: TrainConfig, shape: ModelShape, calib: Calibration) ->
     raise PlanInputError(f"unknown attention {cfg.attention!r}; expected 'stock' or 'flash'")
 
 
+def _chunk_bound(n: int, calib: Calibration) -> int:
+    bound = calib.kernel_loss_chunk_rows
+    if calib.kernel_loss_scratch_bytes > 0:
+        bound = min(bound, max(2048, calib.kernel_loss_scratch_bytes // (2 * max(n, 1)) // 256 * 256))
+    return bound
+
+
+def _even_chunks(vocab: int, bound: int) -> int:
+    """Rows of a chunk when the vocabulary is spread over the fewest chunks of at most `bound` rows."""
+    return -(-(-(-vocab // (-(-vocab // bound)))) // 256) * 256
+
+
 def kernel_loss_chunks(n: int, vocab: int, calib: Calibration) -> tuple[int, int]:
-    """(rows per chunk, chunk count) of the fused loss backward, as the library picks them: the bound is
+    """(rows per chunk, chunk count) of the recomputing backward (trained heads), as the library picks them: the bound is
     `kernel_loss_chunk_rows`, lowered (not below 2048) so that the (N, chunk) bf16 tile fits
     `kernel_loss_scratch_bytes`; the vocabulary is spread evenly over the fewest chunks the bound allows,
     in multiples of 256 rows."""
-    bound = calib.kernel_loss_chunk_rows
-    if calib.kernel_loss_scratch_bytes > 0:
-        fit = calib.kernel_loss_scratch_bytes // (2 * max(n, 1)) // 256 * 256
-        bound = min(bound, max(2048, fit))
-    count = -(-vocab // bound)
-    rows = -(-(-(-vocab // count)) // 256) * 256
-    return rows, count
+    bound = _chunk_bound(n, calib)
+    return _even_chunks(vocab, bound), -(-vocab // bound)
+
+
+def _shares(tiles: int, kblocks: int, ctas: int, unit_cost: int, first_past: bool) -> int:
+    """Partial sums a contraction of few tiles is spread over: the fewest whose busiest CTA has the least to do."""
+    best, best_cost = 1, None
+    for ks in range(1, min(64, kblocks) + 1):
+        if not first_past and ks > 1 and tiles * ks > 4 * ctas:
+            break
+        cost = -(-tiles * ks // ctas) * (-(-kblocks // ks) + unit_cost)
+        if best_cost is None or cost < best_cost:
+            best, best_cost = ks, cost
+        if first_past and tiles * ks >= 4 * ctas:
+            break
+    return best
+
+
+def kernel_grad_bytes(n: int, d: int, vocab: int, calib: Calibration, *, quantized: bool = False,
+                      fp32: bool = False) -> int:
+    """What a frozen head's training step holds while its forward runs, beside a few words per row and vocabulary
+    split: the fp32 sums of d_hidden (kept until the backward), the (N, chunk) tile of g and a 4-bit head's chunk in
+    bf16; fp32: g, the chunk and hidden as three bf16 planes, or one fp32 tile of logits where the CUDA cores run."""
+    blocks = -(-n // 128)
+    if fp32:
+        if quantized or d % 8 != 0 or n * vocab < 2 ** 28 // d:
+            tile = min(4096, vocab)
+            return n * tile * 4 + (tile * d * 4 if quantized else 0)
+        rows = _even_chunks(vocab, min(16384, max(2048, 2 ** 27 // (6 * (n + d)) // 256 * 256)))
+        pair = blocks % 2 == 0 or blocks >= 9
+        groups, ctas = (-(-blocks // 2), B200_SMS // 2) if pair else (blocks, B200_SMS)
+        shares = _shares(groups * -(-d // 256), -(-rows // 64), ctas, 2, first_past=False)
+        # many chunks, and two triples a row for each split of one: as many splits as the library would consider
+        splits = -(-vocab // rows) * min(-(-rows // 256), 8 * ctas // groups + 1)
+        return shares * n * d * 4 + 6 * (n * rows + n * d + rows * d) + 24 * n * splits
+    bound = _chunk_bound(n, calib)
+    grown = min(2 * calib.kernel_loss_chunk_rows, 384 * 2 ** 20 // (2 * (n + d))) if quantized else 256 * 2 ** 20 // (2 * n)
+    rows = _even_chunks(vocab, max(bound, grown // 256 * 256))
+    pair = blocks >= 16 or (blocks % 2 == 0 and d >= 2048)
+    groups, ctas = (-(-blocks // 2), B200_SMS // 2) if pair else (blocks, B200_SMS)
+    shares = _shares(groups * -(-d // 256), rows // 64, ctas, 8, first_past=True)
+    return shares * n * d * 4 + n * rows * 2 + (rows * d * 2 if quantized else 0)
 
 
 def _loss_bytes(cfg: TrainConfig, shape: ModelShape, calib: Calibration) -> int:
@@ -158,11 +206,14 @@ def _loss_bytes(cfg: TrainConfig, shape: ModelShape, calib: Calibration) -> int:
     elif cfg.impl == "kernel":
         base = 3 * n * 4
         if calib.kernel_loss_chunk_rows > 0:
-            quantized = bool(shape.quant_bits)
-            rows, count = kernel_loss_chunks(n, shape.vocab, calib)
-            base += n * rows * 2 + (n * shape.hidden * 4 if count > 1 else 0)   # g tile; fp32 accumulator over chunks
-            if quantized and n > 512:
-                base += rows * shape.hidden * 2                                   # one dequantised chunk of the head
+            if cfg.lora_rank > 0:                                               # a frozen head
+                base += kernel_grad_bytes(n, shape.hidden, shape.vocab, calib, quantized=bool(shape.quant_bits),
+                                          fp32=cfg.dtype == "float32")
+            elif cfg.dtype == "float32":                                        # trained, on the CUDA cores
+                base += n * min(4096, shape.vocab) * 4
+            else:
+                rows, count = kernel_loss_chunks(n, shape.vocab, calib)
+                base += n * rows * 2 + (n * shape.hidden * 4 if count > 1 else 0)   # g tile; fp32 sums over chunks
     else:
         raise PlanInputError(f"unknown impl {cfg.impl!r}; expected 'naive', 'chunked', or 'kernel'")
     if cfg.lora_rank == 0:          # full fine-tuning: the head's fp32 gradient, doubled by the concat

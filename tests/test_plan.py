@@ -114,3 +114,37 @@ def test_kernel_loss_chunks_follow_the_library():
             want = n * rows * 2 + (n * d * 4 if count > 1 else 0) + rows * d * 2
             got = lib.b200tp_linear_ce_bwd_workspace_bytes(C.byref(a), _lib.BF16)
             assert want <= got <= want + 1024, ("quant", n, d, v, rows, count, got)
+
+
+def test_frozen_head_step_follows_the_library():
+    """The planner's model of a frozen head's training step (sums of d_hidden kept until the backward, and the forward's
+    scratch) against the library's own sizes.  It leaves out the partial triples of 3 words per row and vocabulary split
+    (few rows have up to 704 splits, many rows little of them beside the rest); fp32 counts as many of them as there may be."""
+    import ctypes as C
+    import random
+    from mlx_train_perf_b200 import _lib
+    lib = _lib.load()
+    calib = load_calibration()
+    rng = random.Random(7)
+    shapes = [(1000, 4096, 151936), (2048, 4096, 151936), (4096, 2560, 151936), (512, 2048, 32000), (8192, 4096, 151936),
+              (60, 1024, 32768), (1, 8, 1), (16384, 4096, 151936), (2048, 1024, 32768), (100000, 1024, 50000)]
+    shapes += [(int(2 ** rng.uniform(0, 14.5)), 8 * rng.randint(1, 640), int(2 ** rng.uniform(8, 17.3)))
+               for _ in range(300)]
+    for n, d, v in shapes:
+        for quantized, fp32 in ((False, False), (True, False), (False, True)):
+            if quantized and d % 64 != 0:
+                continue
+            a = _lib.CeArgs()
+            a.hidden = a.targets = 1 << 20        # placeholders; nothing is dereferenced
+            a.n, a.d, a.v_local, a.dtype, a.impl = n, d, v, _lib.F32 if fp32 else _lib.BF16, 0
+            if quantized:
+                a.w_q, a.scales, a.biases = 1 << 20, 1 << 20, 1 << 20
+                a.quant_bits, a.group_size, a.qparam_dtype = 4, 64, _lib.BF16
+            else:
+                a.weight = 1 << 20
+            state = lib.b200tp_linear_ce_grad_state_bytes(C.byref(a))
+            got = state + (lib.b200tp_linear_ce_fwd_grad_workspace_bytes(C.byref(a)) if state
+                           else lib.b200tp_linear_ce_fwd_workspace_bytes(C.byref(a)))
+            want = E.kernel_grad_bytes(n, d, v, calib, quantized=quantized, fp32=fp32)
+            least, most = (0.75 * want, 1.001 * want) if fp32 else (want, want + min(12 * n * 800, max(0.06 * want, 2 ** 20)))
+            assert least <= got <= most + 4096, (n, d, v, quantized, fp32, got, want)
