@@ -349,7 +349,7 @@ split_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
               xm = fmaxf(xm, acc[e]);
             }
             if (xm > kHeadroom) {   // rare: this thread's own sum moves to a larger reference; g is void then
-              bad = true;
+              bad = bad || tvalid;  // (an ignored row's g is zero, and its reference an arbitrary logit)
               run_s *= expf(-xm);
               run_m += xm;
 #pragma unroll

@@ -27,7 +27,7 @@ int ce_split_bwd_g(const void* h3, const void* w3, int64_t n, int d, int64_t wid
 
 // The forward that also forms the gradient's sum (see linear_ce_grad.h): ref, then per chunk the partials and
 // g3 = exp(z - ref), zero at the target and on ignored rows; *flag is set when g3 is void (a logit more than 69 above
-// its reference, or *bad), the partials are right unless *bad.
+// the reference of a row that is not ignored, or *bad), the partials are right unless *bad.
 int ce_split_reference(const float* hidden, const float* w, int64_t n, int d, int64_t v, const int64_t* targets,
                        int64_t ignore_index, float* ref, cudaStream_t stream);
 int ce_split_fwd_grad(const void* h3, const void* w3, int64_t n, int d, int64_t width, int64_t vocab_id0,

@@ -96,7 +96,7 @@ struct LogitsParams {
   int ldg;
   // FWD_GRAD
   const float* ref2;        // per row: reference of the exponentials, log2 units
-  int* overflow;            // set to 1 when some logit exceeds its row's reference by kRefHeadroom
+  int* overflow;            // set to 1 when some logit exceeds its (not ignored) row's reference by kRefHeadroom
   LaunchGuard guard;
   int* status;
   // QUANT: the packed head (rows indexed like the tensor map of a dense weight would be)
@@ -467,7 +467,7 @@ ce_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_consta
               xm = fmaxf(xm, x[j]);
             }
             if (xm > kRefHeadroom) {   // rare: move this thread's own sum to a larger reference; g is void then
-              over = true;
+              over = over || tvalid;   // (an ignored row's g is zero, and its reference an arbitrary logit)
               run_s *= fast_exp2(-xm);
               run_m += xm;
 #pragma unroll

@@ -51,7 +51,7 @@ int ce_tc_launch_bwd_g(const void* hidden, const void* w, int64_t w_rows_total, 
                        const LaunchGuard& guard, cudaStream_t stream, int* status);
 
 // Forward partials as ce_tc_launch_fwd and, from the same exponentials, g[n][ldg] (bf16) = exp(z - ref) with
-// `ref2` = ref log2(e) per row, zero at the target's column and on ignored rows.  A row whose logits reach
+// `ref2` = ref log2(e) per row, zero at the target's column and on ignored rows.  Any other row whose logits reach
 // 69 above its reference sets *overflow (g is void then; the partials are right in any case).  Dense weights.
 int ce_tc_launch_fwd_grad(const void* hidden, const void* w, int64_t w_rows_total, int64_t n, int d, int64_t vrow0,
                           int64_t vrow1, int64_t vocab_id0, const int64_t* targets, int64_t ignore_index,

@@ -85,7 +85,7 @@ def test_int4(cuda_device, n, d, v, params):
 @pytest.mark.parametrize("scale", [20.0, 200.0])
 def test_logits_far_above_the_target(cuda_device, quant, scale):
     """Logits 70 and more above the target's leave the range of the fixed reference: the backward then computes
-    them again.  At 20 some rows do, at 200 all; ignored rows (reference: vocab row 0) do as well."""
+    them again.  At 20 some rows do, at 200 all; ignored rows' logits (reference: vocab row 0) do as well, to no effect."""
     n, d, v = 200, 128, 20000
     if quant:
         inp = configs.ce_quant(n, d, v, ignore_frac=0.1, seed=3)
@@ -133,3 +133,36 @@ def test_misaligned_operands_are_refused(cuda_device, operand):
         fused_linear_ce(h.requires_grad_(True), DenseHead(w, trainable=False), t)
     with pytest.raises(LossInputError, match="16-byte aligned"):
         fused_linear_ce(h.detach(), DenseHead(w, trainable=False), t)
+
+
+@pytest.mark.parametrize("kind", ["dense", "quant", "fp32"])
+def test_ignored_rows_do_not_void_the_sums(cuda_device, kind):
+    """Their gradient is zero whatever their logits are; the reference of such a row is the logit of vocab row 0."""
+    n, d, v = 200, 128, 20000
+    if kind == "quant":
+        inp = configs.ce_quant(n, d, v, seed=3)
+        w = oc.dequantize_int4(inp.w_q, inp.scales, inp.biases, out_dtype=torch.bfloat16)
+        head = QuantizedHead(*(x.to(cuda_device) for x in (inp.w_q, inp.scales, inp.biases)))
+    else:
+        inp = configs.ce_dense(n, d, v, dtype=torch.float32 if kind == "fp32" else torch.bfloat16, seed=3)
+        w, head = inp.weight, DenseHead(inp.weight.to(cuda_device), trainable=False)
+    t = inp.targets.clone()
+    t[::3] = configs.IGNORE_INDEX
+    ign = t == configs.IGNORE_INDEX
+    hidden = torch.where(ign[:, None], inp.hidden.float() * 200, inp.hidden.float()).to(inp.hidden.dtype)
+    ct = torch.full((n,), 1.0 / n)
+    impl = "split" if kind == "fp32" else "tc"
+    hd, td = hidden.to(cuda_device), t.to(cuda_device)
+    rows, state = L.ce_forward_grad(hd, head, td, impl=impl)
+    dh = L.ce_backward_grad(hd, head, td, rows, state, ct.to(cuda_device), impl=impl)
+    L.check_device_status()
+    r_nll, r_lse, _ = oc.naive_linear_ce(hidden, w, t, dtype=torch.float64)
+    zmax = (hidden.double() @ w.double().T).max(dim=1).values - hidden.double() @ w.double()[0]
+    assert zmax[ign].max() > 80 and r_nll.max() < 60
+    assert state[:4].view(torch.int32).item() == 0
+    # D / 16 accumulation steps at 2^-23 of the running sum, |h| |w| at most, and the roundings of lse
+    z = (d / 16 + 4) * 2.0 ** -23 * hidden.double().norm(dim=1) * w.double().norm(dim=1).max()
+    assert ((rows[1].double().cpu() - r_lse).abs() <= z + 2.0 ** -22 * r_lse.abs()).all()
+    r_dh, _ = oc.chunked_backward(hidden, w, t, r_lse, ct.double(), chunk_size=4096, dtype=torch.float64)
+    assert (dh[ign.to(cuda_device)] == 0).all()
+    assert ((dh.double().cpu() - r_dh).norm() / r_dh.norm()).item() < 1e-2
