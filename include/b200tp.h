@@ -197,7 +197,7 @@ int b200tp_linear_ce_bwd_train(const b200tp_ce_args* a, const float* lse, const 
  *   state : b200tp_linear_ce_grad_state_bytes, 256-byte aligned, kept by the caller until the backward
  *           (fp32 sums of d_hidden, the references and the flag)
  * bf16 hidden, or fp32 where the tensor cores serve it (see `reserved`: its exponentials keep fp32 precision, and
- * inputs without bf16 planes set the flag too); D % 8 == 0, the whole vocabulary (v_offset = 0); the *_bytes functions
+ * inputs without bf16 planes set the flag too; these, and calls under 2^28 multiplications, fall back to the CUDA cores); D % 8 == 0, the whole vocabulary (v_offset = 0); the *_bytes functions
  * return 0 where the call would be refused.  b200tp_linear_ce_bwd_grad may be called more than once on one state. */
 size_t b200tp_linear_ce_grad_state_bytes(const b200tp_ce_args* a);
 size_t b200tp_linear_ce_fwd_grad_workspace_bytes(const b200tp_ce_args* a);

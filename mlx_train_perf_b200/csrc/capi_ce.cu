@@ -143,6 +143,9 @@ QuantHead quant_head(const b200tp_ce_args* a, bool backward) {
   return quant_inline(a, backward) ? packed_head(a) : QuantHead{};
 }
 
+// Whether a contraction is large enough for the planes to be the faster form (see pick_impl).
+bool split_pays(const b200tp_ce_args* a) { return a->n * a->v_local >= kSplitWorkMin / a->d; }
+
 // 1 = tcgen05, 2 = SIMT, 3 = tcgen05 over the three bf16 planes of fp32 operands, negative = refusal already
 // recorded.  3 is the default for fp32 with a dense head: 2048 x 1024 x 32768 forward + backward 18.5 -> 1.65 ms, with
 // a third of the CUDA-core path's distance to float64.  The CUDA cores keep the contraction of a trained head's
@@ -166,7 +169,7 @@ int pick_impl(const b200tp_ce_args* a) {
     return 1;
   }
   if (tc_ok) return 1;
-  const bool large = (a->reserved & kReservedSplit) != 0 || a->n * a->v_local >= kSplitWorkMin / a->d;
+  const bool large = (a->reserved & kReservedSplit) != 0 || split_pays(a);
   return a->dtype == B200TP_F32 && a->quant_bits == 0 && a->d % 8 == 0 && large ? 3 : 2;
 }
 
@@ -309,7 +312,7 @@ struct GradPlan {
   int shares;            // partial sums of d_hidden (see ce_tc_dh_ksplit)
   int64_t total_splits;
   // state
-  int* overflow;         // [0]: the sums are void; [1]: (fp32) an operand had no planes
+  int* overflow;         // [0]: the sums are void; fp32: [1]: an operand had no planes; [2]: that, or g's own had none
   float* ref2;           // (n), log2 units; fp32: natural units
   float* acc;            // (shares, n, d)
   size_t state_bytes;
@@ -324,6 +327,10 @@ struct GradPlan {
   void* h3; void* w3;
   float* logits;
   int64_t simt_chunk;
+  // fp32: void sums are computed again from planes, by the CUDA cores only where a value has none -- or where these are
+  // the faster form anyway.  One row of 2048 x 1024 x 32768 at 100 nats: 3.0 ms a step (2.1 without such a row), on the
+  // CUDA cores 19.9.
+  bool planes_again;
 };
 
 GradPlan plan_grad(const b200tp_ce_args* a, void* state, void* ws) {
@@ -334,8 +341,9 @@ GradPlan plan_grad(const b200tp_ce_args* a, void* state, void* ws) {
   if (p.impl == 3) {
     p.chunk = split_chunk_rows(a, 6ll * (a->n + a->d), &p.num_chunks);
     p.shares = ce_split_dh_shares(a->n, a->d, p.chunk);
+    p.planes_again = split_pays(a);
     Bump st(state);
-    p.overflow = st.take<int>(2);
+    p.overflow = st.take<int>(3);
     p.ref2 = st.take<float>(a->n);
     p.acc = st.take<float>(static_cast<size_t>(p.shares) * a->n * a->d);
     p.state_bytes = align_up(st.off, 256);
@@ -344,9 +352,10 @@ GradPlan plan_grad(const b200tp_ce_args* a, void* state, void* ws) {
     p.logits = static_cast<float*>(p.g);
     p.simt_chunk = std::min<int64_t>(a->v_local, p.chunk * 6 / 4);
     p.ct = b.take<float>(a->n);
-    p.bwd_bytes = align_up(b.off, 256);
+    if (!p.planes_again) p.bwd_bytes = align_up(b.off, 256);
     p.h3 = b.take<char>(static_cast<size_t>(a->n) * a->d * 6);
     p.w3 = b.take<char>(static_cast<size_t>(p.chunk) * a->d * 6);
+    if (p.planes_again) p.bwd_bytes = align_up(b.off, 256);
     for (int64_t c = 0; c < p.num_chunks; ++c)
       p.total_splits += 2 * ce_split_splits(a->n, std::min<int64_t>(p.chunk, a->v_local - c * p.chunk));
     p.pm = b.take<float>(static_cast<size_t>(p.total_splits) * a->n);
@@ -648,7 +657,8 @@ static int bwd_impl(const b200tp_ce_args* a, const float* lse, const float* cota
       }
     }
     // d_hidden is only touched once it is known that the planes held every value
-    rc = ce_split_sum(p.shares_acc, p.shares, a->n * a->d, static_cast<float*>(d_hidden), accumulate, p.flag, stream);
+    rc = ce_split_sum(p.shares_acc, p.shares, a->n * a->d, static_cast<float*>(d_hidden), accumulate,
+                      SplitGuard{nullptr, p.flag}, stream);
     if (rc) return rc;
   }
   float* acc = out_f32 ? static_cast<float*>(d_hidden) : p.acc;
@@ -752,22 +762,25 @@ int b200tp_linear_ce_fwd_grad(const b200tp_ce_args* a, float* tgt_logit, float* 
                              static_cast<int>(p.chunk), bad, void_sums, stream, status);
       if (rc) return rc;
       slot += 2 * splits;
-      rc = ce_split_dh(p.g, static_cast<int>(p.chunk), p.w3, a->n, a->d, w, p.shares, p.acc, c > 0, stream, status);
+      // once the flag is set the sums are void: no need to go on with them
+      rc = ce_split_dh(p.g, static_cast<int>(p.chunk), p.w3, a->n, a->d, w, p.shares, p.acc, c > 0, stream, status,
+                       SplitGuard{nullptr, void_sums});
       if (rc) return rc;
     }
     rc = launch_combine(p.pm, p.ps, p.pt, a->n, static_cast<int>(p.total_splits), a->n, a->targets, a->ignore_index,
                         nullptr, nullptr, tgt_logit, lse, nll, stream);
     if (rc) return rc;
-    // void sums: the CUDA cores, here and in the backward (which wants lse from the same logits as its own); the
-    // partials' space holds their running triples
+    // the CUDA cores, here and in the backward (which wants lse from the same logits as its own); the partials' space
+    // holds their running triples
+    const int* on_cores = p.planes_again ? bad : void_sums;
     for (int64_t r0 = 0; r0 < a->v_local; r0 += p.simt_chunk) {
       const int64_t w = std::min<int64_t>(p.simt_chunk, a->v_local - r0);
       rc = ce_simt_fwd_chunk(hidden, weight + r0 * a->d, a->dtype, a->n, a->d, w, r0, a->targets, a->ignore_index,
-                             p.logits, p.pm, p.ps, tgt_logit, r0 == 0 ? 1 : 0, stream, void_sums);
+                             p.logits, p.pm, p.ps, tgt_logit, r0 == 0 ? 1 : 0, stream, on_cores);
       if (rc) return rc;
     }
     return launch_combine(p.pm, p.ps, tgt_logit, a->n, 1, a->n, a->targets, a->ignore_index, nullptr, nullptr,
-                          tgt_logit, lse, nll, stream, void_sums);
+                          tgt_logit, lse, nll, stream, on_cores);
   }
   const QuantHead q = packed_head(a);
   rc = launch_ce_reference(a->hidden, a->weight, a->quant_bits != 0 ? &q : nullptr, a->n, a->d, a->v_local, a->targets,
@@ -835,10 +848,31 @@ static int bwd_grad_impl(const b200tp_ce_args* a, const float* lse, const float*
     rc = ce_split_finish(p.acc, p.shares, p.ref2, p.overflow, weight, a->n, a->d, a->v_local, a->targets,
                          a->ignore_index, lse, tgt_logit, cotangent, out, stream);
     if (rc) return rc;
+    if (p.planes_again) {   // as bwd_impl; the void sums' space serves the shares
+      const SplitGuard again{p.overflow, p.overflow + 1};
+      const int ldg = static_cast<int>(p.chunk);
+      int* flag = p.overflow + 2;
+      rc = ce_split_planes(static_cast<const float*>(a->hidden), a->n * a->d, p.h3, flag, stream, again);
+      if (rc) return rc;
+      for (int64_t c = 0; c < p.num_chunks; ++c) {
+        const int64_t r0 = c * p.chunk;
+        const int64_t w = std::min<int64_t>(p.chunk, a->v_local - r0);
+        rc = ce_split_planes(weight + r0 * a->d, w * a->d, p.w3, flag, stream, again);
+        if (rc) return rc;
+        rc = ce_split_bwd_g(p.h3, p.w3, a->n, a->d, w, r0, a->targets, a->ignore_index, lse, cotangent,
+                            ce_split_splits(a->n, w), p.g, ldg, flag, stream, status, again);
+        if (rc) return rc;
+        rc = ce_split_dh(p.g, ldg, p.w3, a->n, a->d, w, p.shares, p.acc, c > 0, stream, status, again);
+        if (rc) return rc;
+      }
+      rc = ce_split_sum(p.acc, p.shares, a->n * a->d, out, 0, SplitGuard{p.overflow, flag}, stream);
+      if (rc) return rc;
+    }
+    const int* on_cores = p.planes_again ? p.overflow + 2 : p.overflow;
     for (int64_t r0 = 0; r0 < a->v_local; r0 += p.simt_chunk) {
       const int64_t w = std::min<int64_t>(p.simt_chunk, a->v_local - r0);
       rc = ce_simt_bwd_chunk(a->hidden, weight + r0 * a->d, a->dtype, a->n, a->d, w, r0, a->targets, a->ignore_index,
-                             lse, cotangent, p.logits, out, r0 > 0, stream, p.overflow);
+                             lse, cotangent, p.logits, out, r0 > 0, stream, on_cores);
       if (rc) return rc;
     }
     return B200TP_OK;
@@ -848,7 +882,8 @@ static int bwd_grad_impl(const b200tp_ce_args* a, const float* lse, const float*
                              a->d, a->v_local, a->targets, a->ignore_index, lse, tgt_logit, cotangent, d_hidden, stream);
   if (rc) return rc;
   // Overflowed references: recompute the logits chunk by chunk.  The sums in `state` are void then, so their
-  // first share serves as the fp32 accumulator.
+  // first share serves as the fp32 accumulator.  (1000 x 4096 x 151936, steps without such a row / with one / all of
+  // them: 1.86 / 2.68 / 2.75 ms; 8192 rows 16.1 / 25.3 / 24.4; a forward and a recomputing backward took 3.16 and 25.5.)
   const LaunchGuard guard{p.overflow, 1};
   for (int64_t c = 0; c < p.num_chunks; ++c) {
     const int64_t r0 = c * p.chunk;

@@ -145,21 +145,26 @@ __device__ __forceinline__ void release_acc(uint64_t* bar) {
   else mbar_arrive(bar);
 }
 
-// `units` of work on pairs (`kernel` is a PAIR instantiation) or on single CTAs.
+// `units` of work on pairs (`kernel` is a PAIR instantiation) or on single CTAs.  `pdl`: the kernel calls griddep_wait().
 template <typename P>
 int launch_units(void (*kernel)(CUtensorMap, CUtensorMap, P), int threads, bool pair, long long units,
-                 cudaStream_t stream, const CUtensorMap& a, const CUtensorMap& b, const P& p) {
+                 cudaStream_t stream, const CUtensorMap& a, const CUtensorMap& b, const P& p, bool pdl = false) {
   cudaLaunchConfig_t cfg{};
   const long long most = pair ? sm_count() / 2 : sm_count();
   cfg.gridDim = dim3(static_cast<unsigned>(std::min(most, units) * (pair ? 2 : 1)));
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = SMEM_BYTES;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim = {2, 1, 1};
+  cudaLaunchAttribute attr[2];
+  if (pair) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs++].val.clusterDim = {2, 1, 1};
+  }
+  if (pdl && pdl_enabled()) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = pair ? 1 : 0;
   B200TP_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, a, b, p));
   return B200TP_OK;
 }

@@ -23,6 +23,14 @@ __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
+// A guarded launch (`run_if_set`) may be scheduled under its predecessor's tail: one that has nothing to do, as almost
+// always, then costs little more than this read.
+__device__ __forceinline__ bool guard_skips(const int* run_if_set) {
+  if (run_if_set == nullptr) return false;
+  griddep_wait();
+  return *run_if_set == 0;
+}
+
 constexpr int TS = 64;  // tile side
 constexpr int TK = 16;
 
@@ -31,7 +39,7 @@ template <typename TA, typename TB>
 __global__ void __launch_bounds__(256)
 gemm_nt_kernel(const TA* __restrict__ A, long long lda, const TB* __restrict__ B, long long ldb, float* __restrict__ C,
                long long ldc, int M, int Nn, int K, const int* run_if_set) {
-  if (run_if_set != nullptr && *run_if_set == 0) return;
+  if (guard_skips(run_if_set)) return;
   __shared__ float As[TK][TS + 1];
   __shared__ float Bs[TK][TS + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -82,7 +90,7 @@ __global__ void __launch_bounds__(256)
 gemm_nn_acc_kernel(const float* __restrict__ A, long long lda, const TB* __restrict__ B, long long ldb,
                    float* __restrict__ C, long long ldc, int M, int Nn, int K, int accumulate,
                    const int* run_if_set) {
-  if (run_if_set != nullptr && *run_if_set == 0) return;
+  if (guard_skips(run_if_set)) return;
   __shared__ float As[TK][TS + 1];
   __shared__ float Bs[TK][TS + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -205,7 +213,7 @@ __global__ void __launch_bounds__(256)
 rows_fwd_kernel(const float* __restrict__ logits, long long ld, int n_rows, int width, long long vocab_id0,
                 const long long* __restrict__ targets, long long ignore_index, float* run_m, float* run_s,
                 float* run_t, int first, const int* run_if_set) {
-  if (run_if_set != nullptr && *run_if_set == 0) return;
+  if (guard_skips(run_if_set)) return;
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= n_rows) return;
@@ -239,7 +247,7 @@ __global__ void __launch_bounds__(256)
 rows_bwd_kernel(float* __restrict__ logits, long long ld, int n_rows, int width, long long vocab_id0,
                 const long long* __restrict__ targets, long long ignore_index, const float* __restrict__ lse,
                 const float* __restrict__ ct, const int* run_if_set) {
-  if (run_if_set != nullptr && *run_if_set == 0) return;
+  if (guard_skips(run_if_set)) return;
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= n_rows) return;
@@ -274,7 +282,7 @@ combine_kernel(const float* __restrict__ pm, const float* __restrict__ ps, const
                long long stride, int parts, long long n, const long long* __restrict__ targets,
                long long ignore_index, float* row_max, float* row_sumexp, float* tgt_out, float* lse_out,
                float* nll_out, const int* run_if_set) {
-  if (run_if_set != nullptr && *run_if_set == 0) return;
+  if (guard_skips(run_if_set)) return;
   __shared__ float s_m[kCombineGroups][32], s_s[kCombineGroups][32], s_t[kCombineGroups][32];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const long long row = static_cast<long long>(blockIdx.x) * 32 + lane;
@@ -463,11 +471,10 @@ int launch_combine(const float* pm, const float* ps, const float* pt, int64_t st
                    const int64_t* targets, int64_t ignore_index, float* row_max, float* row_sumexp, float* tgt_out,
                    float* lse_out, float* nll_out, cudaStream_t stream, const int* run_if_set) {
   if (n <= 0) return B200TP_OK;
-  const unsigned blocks = static_cast<unsigned>(ceil_div(n, 32));
-  combine_kernel<<<blocks, 32 * kCombineGroups, 0, stream>>>(pm, ps, pt, stride, parts, n,
-                                                 reinterpret_cast<const long long*>(targets), ignore_index, row_max,
-                                                 row_sumexp, tgt_out, lse_out, nll_out, run_if_set);
-  B200TP_CUDA_OK(cudaGetLastError());
+  B200TP_CUDA_OK(launch_kernel(run_if_set != nullptr, combine_kernel, dim3(static_cast<unsigned>(ceil_div(n, 32))),
+                               dim3(32 * kCombineGroups), 0, stream, pm, ps, pt, stride, parts, n,
+                               reinterpret_cast<const long long*>(targets), ignore_index, row_max, row_sumexp, tgt_out,
+                               lse_out, nll_out, run_if_set));
   return B200TP_OK;
 }
 
@@ -507,23 +514,44 @@ int launch_dequant_int4(const uint32_t* w_q, const void* scales, const void* bia
   return B200TP_OK;
 }
 
+template <typename T>
+static int launch_logits_chunk(const void* hidden, const void* w_chunk, int64_t n, int d, int64_t width, float* logits_ws,
+                               cudaStream_t stream, const int* run_if_set) {
+  const dim3 grid(static_cast<unsigned>(ceil_div(width, TS)), static_cast<unsigned>(ceil_div(n, TS)));
+  B200TP_CUDA_OK(launch_kernel(run_if_set != nullptr, gemm_nt_kernel<T, T>, grid, dim3(256), 0, stream,
+                               static_cast<const T*>(hidden), d, static_cast<const T*>(w_chunk), d, logits_ws, width, n,
+                               width, d, run_if_set));
+  return B200TP_OK;
+}
+
 int ce_simt_fwd_chunk(const void* hidden, const void* w_chunk, int dtype, int64_t n, int d, int64_t width,
                       int64_t vocab_id0, const int64_t* targets, int64_t ignore_index, float* logits_ws, float* run_m,
                       float* run_s, float* run_t, int first, cudaStream_t stream, const int* run_if_set) {
-  dim3 grid(static_cast<unsigned>(ceil_div(width, TS)), static_cast<unsigned>(ceil_div(n, TS)));
-  if (dtype == B200TP_F32)
-    gemm_nt_kernel<float, float><<<grid, 256, 0, stream>>>(static_cast<const float*>(hidden), d,
-                                                           static_cast<const float*>(w_chunk), d, logits_ws, width,
-                                                           static_cast<int>(n), static_cast<int>(width), d, run_if_set);
-  else
-    gemm_nt_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(hidden), d, static_cast<const __nv_bfloat16*>(w_chunk), d, logits_ws, width,
-        static_cast<int>(n), static_cast<int>(width), d, run_if_set);
-  B200TP_CUDA_OK(cudaGetLastError());
-  rows_fwd_kernel<<<static_cast<unsigned>(ceil_div(n, 8)), 256, 0, stream>>>(
-      logits_ws, width, static_cast<int>(n), static_cast<int>(width), vocab_id0,
-      reinterpret_cast<const long long*>(targets), ignore_index, run_m, run_s, run_t, first, run_if_set);
-  B200TP_CUDA_OK(cudaGetLastError());
+  const int rc = dtype == B200TP_F32
+                     ? launch_logits_chunk<float>(hidden, w_chunk, n, d, width, logits_ws, stream, run_if_set)
+                     : launch_logits_chunk<__nv_bfloat16>(hidden, w_chunk, n, d, width, logits_ws, stream, run_if_set);
+  if (rc) return rc;
+  B200TP_CUDA_OK(launch_kernel(run_if_set != nullptr, rows_fwd_kernel, dim3(static_cast<unsigned>(ceil_div(n, 8))),
+                               dim3(256), 0, stream, logits_ws, width, n, width, vocab_id0,
+                               reinterpret_cast<const long long*>(targets), ignore_index, run_m, run_s, run_t, first,
+                               run_if_set));
+  return B200TP_OK;
+}
+
+template <typename T>
+static int bwd_chunk(const void* hidden, const void* w_chunk, int64_t n, int d, int64_t width, int64_t vocab_id0,
+                     const int64_t* targets, int64_t ignore_index, const float* lse, const float* ct, float* logits_ws,
+                     float* dh_acc, int accumulate, cudaStream_t stream, const int* run_if_set) {
+  const int rc = launch_logits_chunk<T>(hidden, w_chunk, n, d, width, logits_ws, stream, run_if_set);
+  if (rc) return rc;
+  B200TP_CUDA_OK(launch_kernel(run_if_set != nullptr, rows_bwd_kernel<sizeof(T) == 2>,
+                               dim3(static_cast<unsigned>(ceil_div(n, 8))), dim3(256), 0, stream, logits_ws, width, n,
+                               width, vocab_id0, reinterpret_cast<const long long*>(targets), ignore_index, lse, ct,
+                               run_if_set));
+  const dim3 grid(static_cast<unsigned>(ceil_div(d, TS)), static_cast<unsigned>(ceil_div(n, TS)));
+  B200TP_CUDA_OK(launch_kernel(run_if_set != nullptr, gemm_nn_acc_kernel<T>, grid, dim3(256), 0, stream, logits_ws,
+                               width, static_cast<const T*>(w_chunk), d, dh_acc, d, n, d, width, accumulate,
+                               run_if_set));
   return B200TP_OK;
 }
 
@@ -531,38 +559,9 @@ int ce_simt_bwd_chunk(const void* hidden, const void* w_chunk, int dtype, int64_
                       int64_t vocab_id0, const int64_t* targets, int64_t ignore_index, const float* lse,
                       const float* ct, float* logits_ws, float* dh_acc, int accumulate, cudaStream_t stream,
                       const int* run_if_set) {
-  dim3 grid(static_cast<unsigned>(ceil_div(width, TS)), static_cast<unsigned>(ceil_div(n, TS)));
-  dim3 grid2(static_cast<unsigned>(ceil_div(d, TS)), static_cast<unsigned>(ceil_div(n, TS)));
-  const unsigned row_blocks = static_cast<unsigned>(ceil_div(n, 8));
-  if (dtype == B200TP_F32) {
-    gemm_nt_kernel<float, float><<<grid, 256, 0, stream>>>(static_cast<const float*>(hidden), d,
-                                                           static_cast<const float*>(w_chunk), d, logits_ws, width,
-                                                           static_cast<int>(n), static_cast<int>(width), d, run_if_set);
-    B200TP_CUDA_OK(cudaGetLastError());
-    rows_bwd_kernel<false><<<row_blocks, 256, 0, stream>>>(logits_ws, width, static_cast<int>(n),
-                                                           static_cast<int>(width), vocab_id0,
-                                                           reinterpret_cast<const long long*>(targets), ignore_index,
-                                                           lse, ct, run_if_set);
-    B200TP_CUDA_OK(cudaGetLastError());
-    gemm_nn_acc_kernel<float><<<grid2, 256, 0, stream>>>(logits_ws, width, static_cast<const float*>(w_chunk), d,
-                                                         dh_acc, d, static_cast<int>(n), d, static_cast<int>(width),
-                                                         accumulate, run_if_set);
-  } else {
-    gemm_nt_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(hidden), d, static_cast<const __nv_bfloat16*>(w_chunk), d, logits_ws, width,
-        static_cast<int>(n), static_cast<int>(width), d, run_if_set);
-    B200TP_CUDA_OK(cudaGetLastError());
-    rows_bwd_kernel<true><<<row_blocks, 256, 0, stream>>>(logits_ws, width, static_cast<int>(n),
-                                                          static_cast<int>(width), vocab_id0,
-                                                          reinterpret_cast<const long long*>(targets), ignore_index,
-                                                          lse, ct, run_if_set);
-    B200TP_CUDA_OK(cudaGetLastError());
-    gemm_nn_acc_kernel<__nv_bfloat16><<<grid2, 256, 0, stream>>>(
-        logits_ws, width, static_cast<const __nv_bfloat16*>(w_chunk), d, dh_acc, d, static_cast<int>(n), d,
-        static_cast<int>(width), accumulate, run_if_set);
-  }
-  B200TP_CUDA_OK(cudaGetLastError());
-  return B200TP_OK;
+  return (dtype == B200TP_F32 ? bwd_chunk<float> : bwd_chunk<__nv_bfloat16>)(
+      hidden, w_chunk, n, d, width, vocab_id0, targets, ignore_index, lse, ct, logits_ws, dh_acc, accumulate, stream,
+      run_if_set);
 }
 
 int ce_simt_dw_chunk(const float* g_ws, int64_t width, const void* hidden, int dtype, int64_t n, int d,

@@ -211,3 +211,41 @@ def test_gradient_of_the_weight(cuda_device, n, d, v, what):
     z = (9 + d) * 2.0 ** -23 * (h.norm(dim=1) * w.norm(dim=1).max()).max() + 2.0 ** -20
     terms = ct.abs().cpu() @ h.abs()                  # a row of d_weight, were every |g| as large as |ct|
     assert ((out[0][1] - out[1][1]).abs() <= (4 * z + n * 2.0 ** -23) * terms + 1e-12).all()
+
+
+@pytest.mark.parametrize("what", ["one row", "all rows", "no planes"])
+def test_void_sums_of_a_large_call(cuda_device, what):
+    """Logits 69 and more above a target's, at a size where the planes are the faster form: the backward computes them
+    again from planes, bit for bit as the recomputing backward does from the same lse, and the CUDA cores give the result
+    only where a value has none."""
+    n, d, v = 200, 1024, 2600
+    dev, (h, w, t) = cuda_device, _inputs(n, d, v)
+    assert n * d * v >= 2 ** 28
+    if what == "no planes":
+        w[5] = 0
+        w[5, 3] = -math.inf
+        h[:, 3] = h[:, 3].abs() + 0.1
+    else:
+        rows = slice(17, 18) if what == "one row" else slice(None)
+        h[rows] += -110.0 * w[t[rows].clamp(min=0)]
+    ct = torch.linspace(-1, 1.5, n)
+    hd, td, head = h.to(dev), t.to(dev), DenseHead(w.to(dev), trainable=False)
+    rows, state = L.ce_forward_grad(hd, head, td, impl="auto")
+    got = [L.ce_backward_grad(hd, head, td, rows, state, ct.to(dev), impl="auto") for _ in range(2)]
+    L.check_device_status()
+    assert torch.equal(got[0].nan_to_num(7e7), got[1].nan_to_num(7e7))
+    flags = state[:12].view(torch.int32).tolist()
+    s_nll, s_lse, _, s_dh = _run(dev, h, w, t, ct, impl="simt")
+    if what == "no planes":
+        assert flags == [1, 1, 1]
+        for a, b in ((rows[1], s_lse), (rows[2], s_nll), (got[0], s_dh)):
+            assert torch.equal(a.cpu().nan_to_num(7e7), b.nan_to_num(7e7))
+        return
+    assert flags == [1, 0, 0]
+    assert torch.equal(got[0], L.ce_backward_raw(hd, head, td, rows[1], ct.to(dev), impl="auto"))
+    r_nll, r_lse, _ = oc.naive_linear_ce(h, w, t, dtype=torch.float64)
+    r_dh, _ = oc.chunked_backward(h, w, t, r_lse, ct.double(), chunk_size=4096, dtype=torch.float64)
+    assert r_nll.max() > 75
+    lse, dh = rows[1].double().cpu(), got[0].double().cpu()
+    assert (lse - r_lse).norm() <= (s_lse.double() - r_lse).norm() + 2.0 ** -24 * r_lse.norm()
+    assert (dh - r_dh).norm() <= (s_dh.double() - r_dh).norm() + 2.0 ** -24 * r_dh.norm()
