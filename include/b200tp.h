@@ -191,7 +191,7 @@ int b200tp_linear_ce_bwd_train(const b200tp_ce_args* a, const float* lse, const 
  *   exp(ref - lse) * sum_{v != t} exp(z_v - ref) W_v  +  (p_t - 1) W_t
  * for any reference `ref`; with ref = the target's logit the sum is formed chunk by chunk beside the row sums,
  * its exponentials rounded to bf16 before the second contraction like g in b200tp_linear_ce_bwd, the target's
- * term in fp32.  Rows (not ignored ones) whose logits exceed the target's by 69 would overflow: the call then sets a flag in
+ * term in fp32.  Rows (not ignored ones) whose logits exceed the target's by 69 may overflow, and sums over weights of 2^11 and more: the call then sets a flag in
  * `state` and b200tp_linear_ce_bwd_grad recomputes as b200tp_linear_ce_bwd does (lse / nll / tgt_logit are
  * right in any case, and every decision is taken on the device).
  *   state : b200tp_linear_ce_grad_state_bytes, 256-byte aligned, kept by the caller until the backward

@@ -6,8 +6,9 @@
 // is the same vector, and the sum can be formed chunk by chunk beside the forward's row sums: two contractions
 // over N x V x D where forward + recomputing backward take three.  The reference is the target's own logit: it
 // never exceeds the row maximum, so nothing that matters underflows, and logits may lie 69 above it before
-// anything overflows (a loss of 69 nats; such calls set a flag and the backward recomputes, as it always did
-// before: core/chunked.py:52-90 of the reference).
+// an exponential overflows (a loss of 69 nats; such calls set a flag and the backward recomputes, as it always did
+// before: core/chunked.py:52-90 of the reference).  A sum over weights of 2^11 and more may overflow before that:
+// the finish kernel then sets the flag.
 #include "linear_ce_grad.h"
 
 #include "dequant.cuh"
@@ -70,7 +71,7 @@ constexpr int kFinishThreads = 128;
 template <bool QUANT>
 __global__ void __launch_bounds__(kFinishThreads)
 ce_grad_finish_kernel(const float* __restrict__ acc, int shares, const float* __restrict__ ref2,
-                      const int* __restrict__ overflow, const __nv_bfloat16* __restrict__ w, const QuantHead q, int n,
+                      int* overflow, const __nv_bfloat16* __restrict__ w, const QuantHead q, int n,
                       int d, long long v, const long long* __restrict__ targets, long long ignore_index,
                       const float* __restrict__ lse, const float* __restrict__ tgt, const float* __restrict__ ct,
                       __nv_bfloat16* __restrict__ out) {
@@ -93,22 +94,30 @@ ce_grad_finish_kernel(const float* __restrict__ acc, int shares, const float* __
     s[0] += a.x; s[1] += a.y; s[2] += a.z; s[3] += a.w;
     s[4] += b.x; s[5] += b.y; s[6] += b.z; s[7] += b.w;
   }
+  bool finite = true;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) finite = finite && isfinite(s[k]);
+  if (!finite) {
+    *overflow = 1;
+    return;
+  }
+  // c last: exp(ref - lse) may be as small as 2^-117, and c too is often small
   const float c = ct[row], l = lse[row];
-  const float f = c * exp2f(ref2[row] - l * kLog2e);
+  const float f = exp2f(ref2[row] - l * kLog2e);
   const long long t = target_row(target, ignore_index, v);
   uint32_t o[4];
   if (t >= 0) {
-    const float g = c * expm1f(tgt[row] - l);   // ct * (p_target - 1)
+    const float g = expm1f(tgt[row] - l);   // p_target - 1
     const uint4 w8 = weight8<QUANT>(w, q, t, d, i);
     const uint32_t wv[4] = {w8.x, w8.y, w8.z, w8.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wv[k]));
-      o[k] = pack_bf16x2(fmaf(f, s[2 * k], g * x.x), fmaf(f, s[2 * k + 1], g * x.y));
+      o[k] = pack_bf16x2(c * fmaf(f, s[2 * k], g * x.x), c * fmaf(f, s[2 * k + 1], g * x.y));
     }
   } else {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) o[k] = pack_bf16x2(f * s[2 * k], f * s[2 * k + 1]);
+    for (int k = 0; k < 4; ++k) o[k] = pack_bf16x2(c * (f * s[2 * k]), c * (f * s[2 * k + 1]));
   }
   *reinterpret_cast<uint4*>(out + off) = make_uint4(o[0], o[1], o[2], o[3]);
 }
@@ -132,7 +141,7 @@ int launch_ce_reference(const void* hidden, const void* w, const QuantHead* q, i
   return B200TP_OK;
 }
 
-int launch_ce_grad_finish(const float* acc, int shares, const float* ref2, const int* overflow, const void* w,
+int launch_ce_grad_finish(const float* acc, int shares, const float* ref2, int* overflow, const void* w,
                           const QuantHead* q, int64_t n, int d, int64_t v, const int64_t* targets,
                           int64_t ignore_index, const float* lse, const float* tgt, const float* ct, void* d_hidden,
                           cudaStream_t stream) {

@@ -12,8 +12,8 @@ int launch_ce_reference(const void* hidden, const void* w, const QuantHead* q, i
                         cudaStream_t stream);
 
 // d_hidden[n][d] (bf16) = ct * (exp(ref - lse) * sum_s acc[s] + (p_target - 1) * W[target]), 0 on ignored rows;
-// does nothing when *overflow is set.
-int launch_ce_grad_finish(const float* acc, int shares, const float* ref2, const int* overflow, const void* w,
+// does nothing when *overflow is set, and sets it when a sum overflowed (d_hidden is void then).
+int launch_ce_grad_finish(const float* acc, int shares, const float* ref2, int* overflow, const void* w,
                           const QuantHead* q, int64_t n, int d, int64_t v, const int64_t* targets,
                           int64_t ignore_index, const float* lse, const float* tgt, const float* ct, void* d_hidden,
                           cudaStream_t stream);

@@ -529,6 +529,10 @@ split_finish_kernel(const float* __restrict__ acc, int shares, const float* __re
   float s = 0.f;
 #pragma unroll 4
   for (int k = 0; k < shares; ++k) s += __ldcs(acc + static_cast<long long>(k) * n * d + off);
+  if (!isfinite(s)) {   // large weights: the sum is void
+    flags[0] = 1;
+    return;
+  }
   const float c = ct[row], l = lse[row];
   float g = expf(ref[row] - l) * s;
   if (t >= 0 && t < v) g = fmaf(expm1f(tgt[row] - l), __ldg(w + t * d + i), g);

@@ -42,7 +42,7 @@ int ce_split_reference(const float* hidden, const float* w, int64_t n, int d, in
 int ce_split_fwd_grad(const void* h3, const void* w3, int64_t n, int d, int64_t width, int64_t vocab_id0,
                       const int64_t* targets, int64_t ignore_index, const float* ref, int splits, float* pm, float* ps,
                       float* pt, void* g3, int ldg, const int* bad, int* flag, cudaStream_t stream, int* status);
-// d_hidden from the shares' sums, nothing while flags[0] (they are void) is set; flags[2] = flags[1] (an operand has no
+// d_hidden from the shares' sums, nothing while flags[0] (they are void; set here when one overflowed) is set; flags[2] = flags[1] (an operand has no
 // planes) in any case.
 int ce_split_finish(const float* acc, int shares, const float* ref, int* flags, const float* w, int64_t n, int d,
                     int64_t v, const int64_t* targets, int64_t ignore_index, const float* lse, const float* tgt,

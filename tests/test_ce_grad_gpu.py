@@ -166,3 +166,30 @@ def test_ignored_rows_do_not_void_the_sums(cuda_device, kind):
     r_dh, _ = oc.chunked_backward(hidden, w, t, r_lse, ct.double(), chunk_size=4096, dtype=torch.float64)
     assert (dh[ign.to(cuda_device)] == 0).all()
     assert ((dh.double().cpu() - r_dh).norm() / r_dh.norm()).item() < 1e-2
+
+
+@pytest.mark.parametrize(("kind", "n", "d"), [("bf16", 4, 64), ("fp32", 4, 64), ("fp32", 128, 1024)])
+@pytest.mark.parametrize(("weight", "ct"), [(3e9, 1.0), (1.0, 1e-20)])
+def test_products_at_the_ends_of_fp32(cuda_device, kind, n, d, weight, ct):
+    """Logits 66 above the target's are inside the reference's range; 3000 exponentials of e^66 times weights of 3e9 are
+    not inside fp32's, and exp(ref - lse) times a cotangent of 1e-20 is not either.  p = 1 / 2999 everywhere but at the
+    target, so d_hidden = ct (mean of the other rows - W_t), to the rounding of p and of the result (2^-9 each; fp32:
+    (9 + 3000 / 128) 2^-23 for the sum) and what 2^-22 of lse = 74 moves p by."""
+    v = 3000
+    dtype = torch.bfloat16 if kind == "bf16" else torch.float32
+    w, h = torch.zeros(v, d), torch.zeros(n, d)
+    w[:, 0], w[:, 1] = 1.0, weight
+    w[7] = 0.0
+    h[:, 0] = 66.0
+    t = torch.full((n,), 7)
+    impl = "tc" if kind == "bf16" else "split"
+    hd, td, head = (h.to(dtype).to(cuda_device), t.to(cuda_device),
+                    DenseHead(w.to(dtype).to(cuda_device), trainable=False))
+    rows, state = L.ce_forward_grad(hd, head, td, impl=impl)
+    for _ in range(2):
+        dh = L.ce_backward_grad(hd, head, td, rows, state, torch.full((n,), ct, device=cuda_device), impl=impl)
+        L.check_device_status()
+        want = torch.zeros(n, d, dtype=torch.float64)
+        want[:, 0], want[:, 1] = ct, ct * float(torch.tensor(weight).to(dtype))
+        tol = 1e-2 if kind == "bf16" else 1e-4
+        assert ((dh.double().cpu() - want).abs() <= tol * want.abs()).all(), dh[:, :2]
