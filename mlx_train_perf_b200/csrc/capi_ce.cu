@@ -904,7 +904,7 @@ static int bwd_grad_impl(const b200tp_ce_args* a, const float* lse, const float*
     if (rc) return rc;
     const bool last = c == p.num_chunks - 1;
     rc = ce_tc_launch_dh(p.g, static_cast<int>(p.chunk), static_cast<int>(align_up(w, kCeTileCols)), a->n, wmat, wrows,
-                         a->d, row0, c == 0 ? nullptr : p.acc, last ? nullptr : p.acc, last ? d_hidden : nullptr, -1, -1,
+                         a->d, row0, c == 0 ? nullptr : p.acc, p.acc, last ? d_hidden : nullptr, -1, -1,
                          1, nullptr, guard, stream, status);
     if (rc) return rc;
   }

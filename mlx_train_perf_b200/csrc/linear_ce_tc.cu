@@ -64,6 +64,8 @@ enum { MODE_FWD = 0, MODE_BWD_G = 1, MODE_FWD_GRAD = 2 };
 // Sums of 2^27 terms of 2^100 stay below the largest fp32, and 2^100 = e^69.
 constexpr float kRefHeadroom = 100.f;
 
+constexpr int kMostAccumulated = 16384;   // vocab rows per accumulation of d_hidden (see ce_dh_kernel)
+
 __device__ __forceinline__ bool guard_skips(const LaunchGuard& g) {
   return g.flag != nullptr && (*g.flag != 0) != (g.run_if_set != 0);
 }
@@ -121,6 +123,8 @@ struct DhParams {
   int tile0, tile1;         // units [tile0, tile1) are computed by this launch; unit = split * tiles + tile
   int ksplit;               // shares of the contraction: share s adds into acc + s * split_stride (ksplit 1: no shares)
   long long split_stride;
+  int seg_kb;               // most k blocks of one accumulation; a unit's parts are added in acc_out
+  int wide;                 // acc_in and acc_out are 32-byte aligned
   // QUANT: the packed head
   const uint32_t* wq;
   const void* scales;
@@ -530,6 +534,12 @@ ce_logits_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_consta
 // in order as the persistent CTAs advance, and a launch can be given a sub-range [tile0, tile1) of
 // them: vocab-sharded callers run the last chunk in a few such launches and start reducing the
 // finished rows across ranks while the later ones are still being computed.
+//
+// The tensor core rounds its accumulator towards zero at every step of 16 terms, an error that is biased and grows with
+// the steps.  A chunk wider than kMostAccumulated vocab rows is therefore accumulated in parts, which the epilogue adds in
+// acc_out with round-to-nearest while the next part runs.  (One large row and 76000 small ones: the sum 1.6e-4 of itself
+// too small in one part, 3.2e-5 in five; 1000 x 4096 x 151936, d_hidden of a chunk 444 -> 453 us with whole sectors read
+// and written, 465 with halves: what the epilogue moves through L1 is taken from the operands.)
 template <bool QUANT, bool PAIR = false>
 __global__ void __launch_bounds__(QUANT ? THREADS_Q : THREADS, 1)
 ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__ CUtensorMap tmap_w,
@@ -554,6 +564,7 @@ ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
     kb0 = static_cast<int>(static_cast<long long>(split) * kblocks / p.ksplit);
     kb1 = static_cast<int>(static_cast<long long>(split + 1) * kblocks / p.ksplit);
   };
+  auto num_segs = [&](int kb0, int kb1) { return (kb1 - kb0 + p.seg_kb - 1) / p.seg_kb; };
 
   if (QUANT && warp >= THREADS / 32) {
     // ------------------------------ dequantising warps ------------------------------
@@ -706,90 +717,108 @@ ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
     for (int u = first_tile; u < total_tiles && ok; u += unit_step) {
       int kb0, kb1;
       k_range(u / tiles, kb0, kb1);
-      if (kb0 >= kb1) continue;
-      const uint32_t as = tile & 1;
-      if (!mbar_wait_warp(&sm.tempty[as], ((tile >> 1) & 1) ^ 1, sm.abort_flag)) {
-        if (lane == 0) raise_abort(sm, p.status, kDevTimeoutMma);
-        break;
-      }
-      tc_fence_after_sync();
-      const uint32_t d_tmem = tmem_base + as * BN;
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        const int s = it % kStages;
-        if (!mbar_wait_warp(&sm.full[s], (it / kStages) & 1, sm.abort_flag)) {
+      const int segs = num_segs(kb0, kb1);
+      for (int seg = 0; seg < segs && ok; ++seg, ++tile) {
+        const int ks0 = kb0 + (kb1 - kb0) * seg / segs, ks1 = kb0 + (kb1 - kb0) * (seg + 1) / segs;
+        const uint32_t as = tile & 1;
+        if (!mbar_wait_warp(&sm.tempty[as], ((tile >> 1) & 1) ^ 1, sm.abort_flag)) {
           if (lane == 0) raise_abort(sm, p.status, kDevTimeoutMma);
           ok = false;
           break;
         }
         tc_fence_after_sync();
-        const uint32_t a_lo = desc_lo(smem_u32(sm.a(s)), 16);
-        // 16 k rows of 128 B each per step; 64-column chunks are 8 KiB apart.
-        const uint32_t b_lo = desc_lo(smem_u32(sm.b(s)), 64 * BK * 2);
-        if (elect_one()) {
+        const uint32_t d_tmem = tmem_base + as * BN;
+        for (int kb = ks0; kb < ks1; ++kb, ++it) {
+          const int s = it % kStages;
+          if (!mbar_wait_warp(&sm.full[s], (it / kStages) & 1, sm.abort_flag)) {
+            if (lane == 0) raise_abort(sm, p.status, kDevTimeoutMma);
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+          const uint32_t a_lo = desc_lo(smem_u32(sm.a(s)), 16);
+          // 16 k rows of 128 B each per step; 64-column chunks are 8 KiB apart.
+          const uint32_t b_lo = desc_lo(smem_u32(sm.b(s)), 64 * BK * 2);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma<PAIR>(d_tmem, a_lo + k * 2, dhi, b_lo + k * 128, dhi, idesc, kb != kb0 || k != 0 ? 1u : 0u);
-          commit<PAIR>(&sm.empty[s]);
+            for (int k = 0; k < BK / 16; ++k)
+              umma<PAIR>(d_tmem, a_lo + k * 2, dhi, b_lo + k * 128, dhi, idesc, kb != ks0 || k != 0 ? 1u : 0u);
+            commit<PAIR>(&sm.empty[s]);
+          }
+          __syncwarp();
         }
+        if (ok && elect_one()) commit<PAIR>(&sm.tfull[as]);
         __syncwarp();
       }
-      if (ok && elect_one()) commit<PAIR>(&sm.tfull[as]);
-      __syncwarp();
-      ++tile;
     }
     }
   } else {
     const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;
     uint32_t tile = 0;
-    for (int u = first_tile; u < total_tiles; u += unit_step) {
+    bool ok = true;
+    for (int u = first_tile; u < total_tiles && ok; u += unit_step) {
       const int split = u / tiles, t = u - split * tiles;
       const int rb = t / p.num_nt;
       const int nt = t - rb * p.num_nt;
       int kb0, kb1;
       k_range(split, kb0, kb1);
-      if (kb0 >= kb1) continue;   // nothing to add: the share keeps what earlier chunks left (see the host side)
-      const uint32_t as = tile & 1;
-      if (!mbar_wait_warp(&sm.tfull[as], (tile >> 1) & 1, sm.abort_flag)) {
-        raise_abort(sm, p.status, kDevTimeoutEpilogue);
-        break;
-      }
-      tc_fence_after_sync();
-      const int row = block_row(rb) + row_in_tile;
-      const bool row_ok = row < p.n_rows;
-      const uint32_t taddr0 = tmem_base + as * BN + (static_cast<uint32_t>(quad * 32) << 16);
+      const int segs = num_segs(kb0, kb1);   // 0: the share keeps what earlier chunks left (see the host side)
+      for (int seg = 0; seg < segs; ++seg, ++tile) {
+        const float* acc_in = seg == 0 ? p.acc_in : p.acc_out;
+        const bool last = seg == segs - 1;
+        const uint32_t as = tile & 1;
+        if (!mbar_wait_warp(&sm.tfull[as], (tile >> 1) & 1, sm.abort_flag)) {
+          raise_abort(sm, p.status, kDevTimeoutEpilogue);
+          ok = false;
+          break;
+        }
+        tc_fence_after_sync();
+        const int row = block_row(rb) + row_in_tile;
+        const bool row_ok = row < p.n_rows;
+        const uint32_t taddr0 = tmem_base + as * BN + (static_cast<uint32_t>(quad * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        const int col0 = nt * BN + c * 32;
-        if (col0 >= p.d_cols) break;
-        uint32_t r[32];
-        tmem_ld_x32(taddr0 + c * 32, r);
-        tmem_wait_ld();
-        tmem_regs_ready(r);
-        if (row_ok) {
-          const size_t off = static_cast<size_t>(split) * p.split_stride + static_cast<size_t>(row) * p.d_cols + col0;
+        for (int c = 0; c < BN / 32; ++c) {
+          const int col0 = nt * BN + c * 32;
+          if (col0 >= p.d_cols) break;
+          uint32_t r[32];
+          tmem_ld_x32(taddr0 + c * 32, r);
+          tmem_wait_ld();
+          tmem_regs_ready(r);
+          if (row_ok) {
+            const size_t off = static_cast<size_t>(split) * p.split_stride + static_cast<size_t>(row) * p.d_cols + col0;
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            if (col0 + j < p.d_cols) {  // d_cols is a multiple of 8
-              float4 v = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                                     __uint_as_float(r[j + 3]));
-              if (p.acc_in != nullptr) {
-                const float4 o = *reinterpret_cast<const float4*>(p.acc_in + off + j);
-                v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-              }
-              if (p.acc_out != nullptr) *reinterpret_cast<float4*>(p.acc_out + off + j) = v;
-              if (p.out_bf16 != nullptr) {
-                uint2 w2 = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
-                *reinterpret_cast<uint2*>(p.out_bf16 + off + j) = w2;
+            for (int j = 0; j < 32; j += 8) {
+              if (col0 + j < p.d_cols) {  // d_cols is a multiple of 8
+                uint32_t v[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = r[j + e];
+                if (acc_in != nullptr) {
+                  uint32_t o[8];
+                  if (p.wide) ld_global_32b(acc_in + off + j, o);
+                  else ld_global_2x16b(acc_in + off + j, o);
+#pragma unroll
+                  for (int e = 0; e < 8; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(o[e]));
+                }
+                if (last && p.out_bf16 != nullptr) {
+#pragma unroll
+                  for (int e = 0; e < 8; e += 4)
+                    *reinterpret_cast<uint2*>(p.out_bf16 + off + j + e) =
+                        make_uint2(pack_bf16x2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])),
+                                   pack_bf16x2(__uint_as_float(v[e + 2]), __uint_as_float(v[e + 3])));
+                } else if (p.wide) {
+                  st_global_32b(p.acc_out + off + j, v);
+                } else {
+                  st_global_2x16b(p.acc_out + off + j, v);
+                }
               }
             }
           }
         }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) release_acc<PAIR>(&sm.tempty[as]);
       }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) release_acc<PAIR>(&sm.tempty[as]);
-      ++tile;
     }
   }
   cta_teardown(sm, warp, tmem_base, PAIR);
@@ -1241,6 +1270,8 @@ int ce_tc_launch_dh(const void* g, int ldg, int k_total, int64_t n, const void* 
   p.guard = guard;
   p.ksplit = ksplit;
   p.split_stride = static_cast<long long>(n) * d;
+  p.wide = ((reinterpret_cast<uintptr_t>(acc_in) | reinterpret_cast<uintptr_t>(acc_out)) & 31) == 0;
+  p.seg_kb = acc_out != nullptr ? kMostAccumulated / BK : std::max(1, k_total / BK);
   const int total = p.num_rb * p.num_nt * ksplit;
   p.tile0 = tile0 < 0 ? 0 : tile0;
   p.tile1 = tile1 < 0 ? total : std::min(tile1, total);

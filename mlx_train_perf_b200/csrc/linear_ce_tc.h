@@ -58,8 +58,8 @@ int ce_tc_launch_fwd_grad(const void* hidden, const void* w, int64_t w_rows_tota
                           const float* ref2, int* overflow, int splits, float* pm, float* ps, float* pt, void* g,
                           int ldg, cudaStream_t stream, int* status);
 
-// dH = [acc_in +] G[:, :k_total] @ W[wrow0 : wrow0 + k_total, :]; written to acc_out (f32)
-// and/or out_bf16.  k_total is a multiple of 64; rows of W past w_rows_total read as zero.
+// dH = [acc_in +] G[:, :k_total] @ W[wrow0 : wrow0 + k_total, :]; written to out_bf16, else to acc_out (f32), which
+// also holds the sums of the parts that a k_total above 16384 is accumulated in (without it, in one).  k_total is a multiple of 64; rows of W past w_rows_total read as zero.
 // The 128 x 256 output tiles are numbered row-block-major; this launch computes tiles
 // [tile0, tile1) (negative: from the first / through the last).  `ce_tc_dh_rows_done(n, d, t)` is
 // the number of leading rows of d_hidden that are complete once tiles [0, t) have run.

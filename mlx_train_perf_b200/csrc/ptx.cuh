@@ -444,6 +444,22 @@ __device__ __forceinline__ void st_global_32b(void* p, const uint32_t (&v)[8]) {
                "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
+__device__ __forceinline__ void ld_global_32b(const void* p, uint32_t (&v)[8]) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "l"(p)
+               : "memory");
+}
+// The same 32 bytes in two halves; `p` 16-byte aligned.
+__device__ __forceinline__ void ld_global_2x16b(const void* p, uint32_t (&v)[8]) {
+  const uint4 a = *reinterpret_cast<const uint4*>(p), b = *(reinterpret_cast<const uint4*>(p) + 1);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void st_global_2x16b(void* p, const uint32_t (&v)[8]) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(v[0], v[1], v[2], v[3]);
+  *(reinterpret_cast<uint4*>(p) + 1) = make_uint4(v[4], v[5], v[6], v[7]);
+}
 
 // ---------------------------------------------------------------------------------------
 // small numeric helpers

@@ -193,3 +193,23 @@ def test_products_at_the_ends_of_fp32(cuda_device, kind, n, d, weight, ct):
         want[:, 0], want[:, 1] = ct, ct * float(torch.tensor(weight).to(dtype))
         tol = 1e-2 if kind == "bf16" else 1e-4
         assert ((dh.double().cpu() - want).abs() <= tol * want.abs()).all(), dh[:, :2]
+
+
+def test_accumulations_are_short(cuda_device):
+    """Hidden states of zero make every exponential 1, so a row's sum in `state` is that of the weights but the target's.
+    One large row and many small ones: where the large one is in the accumulator, a step of 16 rows loses up to an ulp
+    (2^-23) of it towards zero, 1024 x 2^-23 in an accumulation of 16384 rows (over all 131072, which are one chunk and
+    one share here, eight times as much); the parts' sums and the small rows add 2 % at most."""
+    n, d, v, dev = 1000, 4096, 131072, cuda_device
+    w = torch.randn(v, d, generator=torch.Generator(device=dev).manual_seed(v), device=dev) * 2.0 ** -8
+    w[17] = 300 * torch.randn(d, generator=torch.Generator(device=dev).manual_seed(17), device=dev)
+    w = w.to(torch.bfloat16)
+    h, t = torch.zeros(n, d, dtype=torch.bfloat16, device=dev), torch.full((n,), 5, device=dev)
+    _, state = L.ce_forward_grad(h, DenseHead(w, trainable=False), t)
+    L.check_device_status()
+    at = 256 + (4 * n + 255) // 256 * 256
+    sums = state[at:at + (state.numel() - at) // (4 * n * d) * (4 * n * d)].view(torch.float32).reshape(-1, n, d)
+    assert sums.shape[0] == 1
+    want = w.sum(dim=0, dtype=torch.float64) - w[5].double()
+    rel = (sums[0].double() - want).norm(dim=1) / want.norm()
+    assert rel.max().item() <= 1.02 * 1024 * 2.0 ** -23, rel.max().item() * 2.0 ** 23
