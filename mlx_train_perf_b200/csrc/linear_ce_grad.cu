@@ -62,7 +62,7 @@ ce_reference_kernel(const __nv_bfloat16* __restrict__ hidden, const __nv_bfloat1
   for (int i = lane; i < d / 8; i += 32) acc = dot8(__ldg(h + i), weight8<QUANT>(w, q, t, d, i), acc);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) ref2[row] = acc * kLog2e;
+  if (lane == 0) ref2[row] = isfinite(acc) ? acc * kLog2e : 0.f;   // (any finite one serves)
 }
 
 // Eight columns of one row per thread.  HBM-bound: the fp32 sums, the target's weight row and the bf16 result

@@ -5,7 +5,8 @@
 
 namespace b200tp {
 
-// ref2[n] = log2(e) * (logit of the row's target, or of vocab row 0 when it has none); *overflow = 0.
+// ref2[n] = log2(e) * (logit of the row's target, or of vocab row 0 when it has none), 0 where that
+// is not finite; *overflow = 0.
 // `q` non-null: 4-bit head, else `w` (v, d) bf16.
 int launch_ce_reference(const void* hidden, const void* w, const QuantHead* q, int64_t n, int d, int64_t v,
                         const int64_t* targets, int64_t ignore_index, float* ref2, int* overflow,

@@ -509,7 +509,7 @@ split_reference_kernel(const float* __restrict__ hidden, const float* __restrict
   for (int i = lane; i < d; i += 32) acc = fmaf(__ldg(h + i), __ldg(wt + i), acc);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) ref[row] = acc;
+  if (lane == 0) ref[row] = isfinite(acc) ? acc : 0.f;   // (any finite one serves)
 }
 
 // d_hidden = ct (exp(ref - lse) sum of shares + (p_t - 1) W_t); HBM-bound, one column per thread.

@@ -213,3 +213,36 @@ def test_accumulations_are_short(cuda_device):
     want = w.sum(dim=0, dtype=torch.float64) - w[5].double()
     rel = (sums[0].double() - want).norm(dim=1) / want.norm()
     assert rel.max().item() <= 1.02 * 1024 * 2.0 ** -23, rel.max().item() * 2.0 ** 23
+
+
+@pytest.mark.parametrize("what", ["targets out of range", "inf weight", "nan hidden"])
+def test_values_outside_the_ordinary(cuda_device, what):
+    """What the recomputing pair gives: a target outside the vocabulary has no logit (loss = lse, d_hidden = ct sum of
+    p W); a value that is not finite reaches the same rows, as one that is not finite."""
+    n, d, v = 130, 64, 700
+    inp = configs.ce_dense(n, d, v, dtype=torch.bfloat16, ignore_frac=0.05, seed=5)
+    h, w, t = inp.hidden.clone(), inp.weight.clone(), inp.targets.clone()
+    if what == "targets out of range":
+        t[3], t[9] = v, -7
+    elif what == "inf weight":
+        t[3] = 5                                  # (also the logit of a target)
+        w[5], w[5, 3] = 0, float("-inf")
+        h[:, 3] = h[:, 3].abs() + 0.1
+    else:
+        h[7, 2] = float("nan")
+    hd, td, head = h.to(cuda_device), t.to(cuda_device), DenseHead(w.to(cuda_device), trainable=False)
+    ct = torch.full((n,), 0.5, device=cuda_device)
+    rows, state = L.ce_forward_grad(hd, head, td)
+    dh = L.ce_backward_grad(hd, head, td, rows, state, ct)
+    _, _, tgt, lse, nll = L.ce_forward_raw(hd, head, td, impl="tc")
+    want = L.ce_backward_raw(hd, head, td, lse, ct, impl="tc")
+    L.check_device_status()
+    # sums of the same logits in another order; g rounded to bf16 in one and its exponentials in the other (see above)
+    for a, b in ((rows[0], tgt), (rows[1], lse), (rows[2], nll)):
+        assert torch.equal(a.isfinite(), b.isfinite())
+        ok = b.isfinite()
+        assert (a[ok] - b[ok]).abs().max() <= 1e-5 * (1 + b[ok].abs().max())
+    ok = want.isfinite()      # (not where a g of zero meets an infinite weight: ignored rows too)
+    assert torch.equal(dh.isfinite(), ok)
+    a, b = dh.double()[ok], want.double()[ok]
+    assert (a - b).norm() <= 1e-2 * b.norm()

@@ -249,3 +249,25 @@ def test_void_sums_of_a_large_call(cuda_device, what):
     lse, dh = rows[1].double().cpu(), got[0].double().cpu()
     assert (lse - r_lse).norm() <= (s_lse.double() - r_lse).norm() + 2.0 ** -24 * r_lse.norm()
     assert (dh - r_dh).norm() <= (s_dh.double() - r_dh).norm() + 2.0 ** -24 * r_dh.norm()
+
+
+@pytest.mark.parametrize("n", [16, 130])
+def test_target_logit_that_overflows(cuda_device, n):
+    """Finite operands whose product is below fp32's range: the target's logit is -inf, its row's loss +inf, everything
+    else finite, as on the CUDA cores (the larger call would compute void sums again from planes)."""
+    d, v, dev = 1024, 2100, cuda_device
+    h, w, t = _inputs(n, d, v)
+    w[5], h[:, 3], t[4] = 0, 3.0, 5
+    w[5, 3] = -3e38
+    ct = torch.linspace(-1, 1.5, n)
+    hd, td, head = h.to(dev), t.to(dev), DenseHead(w.to(dev), trainable=False)
+    rows, state = L.ce_forward_grad(hd, head, td, impl="split")
+    dh = L.ce_backward_grad(hd, head, td, rows, state, ct.to(dev), impl="split").cpu()
+    nll, lse, tgt, s_dh = _run(dev, h, w, t, ct, impl="simt")
+    assert nll[4].item() == math.inf and lse.isfinite().all()
+    for a, b in ((rows[0], tgt), (rows[1], lse), (rows[2], nll), (dh, s_dh)):
+        a, ok = a.cpu(), b.isfinite()
+        assert torch.equal(a.isfinite(), ok) and torch.equal(a[~ok], b[~ok])
+        a, b, ok = (x[torch.arange(n) != 4] for x in (a, b, ok))        # (that row of d_hidden holds 1e38)
+        # logits of up to 40 at (9 + D) 2^-23 of themselves for both kinds: 1e-2 of a probability at most
+        assert (a[ok] - b[ok]).norm() <= 1e-2 * b[ok].norm()
