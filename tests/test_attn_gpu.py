@@ -417,3 +417,32 @@ def test_backward_parts_match_the_whole_backward(cuda_device, s, hq, hkv, d, len
     for name, x, y in (("dK", dk2, dk), ("dV", dv2, dv)):
         rel = (x.float() - y.float()).abs().max().item() / y.float().abs().max().item()
         assert rel < 4e-3, (name, rel)      # half a bf16 ulp of the largest element, at most
+
+
+# one query block and one key; ragged last blocks; more key blocks than the ring of K and V tiles has slots; groups of
+# 1, 2, 3 and 4 q heads; packed rows with boundaries on, beside and inside 128-key blocks
+@pytest.mark.parametrize("d", [64, 96])
+@pytest.mark.parametrize(("b", "hq", "hkv", "s", "lengths"), [
+    (19, 16, 8, 1, None), (19, 16, 8, 100, None), (10, 16, 16, 129, None), (7, 12, 4, 300, None), (4, 16, 4, 640, None),
+    (2, 16, 8, 1153, None), (1, 32, 8, 1300, None), (4, 16, 4, 600, [127, 1, 128, 129, 200, 15]),
+    (7, 12, 4, 300, [1, 299]), (2, 16, 8, 1153, [640, 512, 1])])
+def test_one_tile_forward(cuda_device, b, hq, hkv, s, d, lengths):
+    """Grids that fill the chip at head_dim 64 / 96 take the forward with one query tile per CTA: bit for bit the two-tile
+    kernel ("tc2"), which the cases above hold to the oracle, and within their class of the CUDA-core kernels."""
+    nqb, group = -(-s // 128), hq // hkv
+    ctas = b * (hq // 2 * nqb if group % 2 == 0 else hq * ((nqb + 1) // 2))
+    assert ctas > torch.cuda.get_device_properties(cuda_device).multi_processor_count      # (else another kernel runs)
+    inp = configs.attention(s, b=b, hq=hq, hkv=hkv, d=d, dtype=torch.bfloat16, seed=s + d)
+    q, k, v = (x.to(cuda_device) for x in (inp.q, inp.k, inp.v))
+    seg = None
+    if lengths is not None:
+        ids, starts = oa.segments_from_lengths(lengths, s)
+        seg = PackedMask(*(x.expand(b, -1).contiguous().to(cuda_device) for x in (ids, starts)))
+    o, l = flash_attention_with_lse(q, k, v, scale=inp.scale, segments=seg)
+    o2, l2 = flash_attention_with_lse(q, k, v, scale=inp.scale, segments=seg, impl="tc2")
+    o_s, l_s = flash_attention_with_lse(q, k, v, scale=inp.scale, segments=seg, impl="simt")
+    check_device_status()
+    assert torch.equal(o, o2) and torch.equal(l, l2)
+    # O: P is rounded to bf16 in one of the two and the result in both (the bf16 class); L: fp32 sums, relative to 1 + |L|
+    assert (o.float() - o_s.float()).abs().max().item() < 1.2e-2 + 2.0 ** -8 * o_s.float().abs().max().item()
+    assert ((l - l_s).abs() / (1 + l_s.abs())).max().item() < 2e-5
