@@ -48,8 +48,8 @@ def _check(got, hidden, w, targets, ct):
     assert (err <= 1e-2 * norm + floor).all(), (err / (1e-2 * norm + floor)).max().item()
 
 
-# rows around a tile, hidden sizes around a k block and a column tile, vocabularies around a tile and over
-# several chunks; few rows share each tile's contraction over many CTAs, many rows do not
+# rows around a tile, hidden sizes around a k block and a column tile, vocabularies around a tile, dense ones in one
+# chunk, the 4-bit ones below over several; few rows share each tile's contraction over many CTAs, many rows do not
 SHAPES = [(1, 8, 1), (1, 64, 257), (127, 72, 255), (128, 256, 512), (129, 264, 4099), (60, 1024, 33000),
           (300, 320, 16385), (1500, 136, 2049)]
 
@@ -246,3 +246,15 @@ def test_values_outside_the_ordinary(cuda_device, what):
     assert torch.equal(dh.isfinite(), ok)
     a, b = dh.double()[ok], want.double()[ok]
     assert (a - b).norm() <= 1e-2 * b.norm()
+
+
+# single CTAs and pairs, with shares (some of which the narrower last chunk leaves empty) and without
+@pytest.mark.parametrize(("n", "d", "v", "units"), [(60, 1024, 5000, 4), (129, 264, 4099, 1), (300, 320, 2561, 2),
+                                                    (256, 2056, 3000, 3), (2177, 264, 2600, 4), (1500, 2112, 1100, 2)])
+def test_dense_over_several_chunks(cuda_device, monkeypatch, n, d, v, units):
+    """A chunk bound of `units` x 256 vocabulary rows: sums added up over the chunks, shares among them."""
+    monkeypatch.setitem(L._RESERVED, "tc", units)
+    inp = configs.ce_dense(n, d, v, dtype=torch.bfloat16, ignore_frac=0.05, seed=n + v)
+    ct = torch.linspace(0.5, 1.5, n) * torch.where(torch.arange(n) % 2 == 0, 1.0, -1.0)
+    _check(_run(cuda_device, inp.hidden, DenseHead(inp.weight.to(cuda_device), trainable=False), inp.targets, ct),
+           inp.hidden, inp.weight, inp.targets, ct)
