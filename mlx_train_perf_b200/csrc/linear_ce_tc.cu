@@ -827,24 +827,23 @@ ce_dh_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
 // -----------------------------------------------------------------------------------------
 // dW_chunk = G^T hidden   (trainable dense head; core/chunked.py:84-85, K5 of the reference)
 // -----------------------------------------------------------------------------------------
-// Tile = 128 vocab rows x 256 hidden columns, contraction over the N tokens in 64-row blocks.
+// Tile = 128 vocab rows x 256 hidden columns per CTA of a pair, contraction over the N tokens in 64-row blocks.
 // Both operands are read MN-major straight from their row-major homes: A = G (N, chunk) as two
 // [64 tokens][64 vocab columns] boxes per stage, B = hidden (N, D) as four [64 tokens][64 hidden
 // columns] boxes.  Token rows past N are zero-filled by TMA.  Each vocab row belongs to exactly one
 // chunk, so the fp32 accumulator is complete after one pass and is rounded once to bf16.
-template <bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 ce_dw_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__ CUtensorMap tmap_h,
              const DwParams p) {
   extern __shared__ uint8_t smem_raw[];
-  const SmemView sm = carve_smem(smem_raw, false, PAIR);
+  const SmemView sm = carve_smem(smem_raw, false, true);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // provably warp-uniform
   const int lane = threadIdx.x & 31;
-  const uint32_t tmem_base = cta_setup(sm, warp, 1, PAIR ? 8 : 4, PAIR);
-  constexpr uint32_t kStages = PAIR ? PAIR_STAGES : STAGES;
-  const uint32_t rank = PAIR ? cluster_ctarank() : 0;
-  const int unit0 = PAIR ? blockIdx.x >> 1 : blockIdx.x, unit_step = PAIR ? gridDim.x >> 1 : gridDim.x;
-  auto block_row = [&](int mt) { return (PAIR ? mt * 2 + static_cast<int>(rank) : mt) * BM; };
+  const uint32_t tmem_base = cta_setup(sm, warp, 1, 8, true);
+  constexpr uint32_t kStages = PAIR_STAGES;
+  const uint32_t rank = cluster_ctarank();
+  const int unit0 = blockIdx.x >> 1, unit_step = gridDim.x >> 1;
+  auto block_row = [&](int mt) { return (mt * 2 + static_cast<int>(rank)) * BM; };
 
   const int total_tiles = p.num_mt * p.num_nt;
   const int kblocks = (p.n_rows + BK - 1) / BK;
@@ -865,29 +864,19 @@ ce_dw_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
             ok = false;
             break;
           }
-          if (PAIR) {
-            if (rank == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * PAIR_STAGE_BYTES);
-            const uint32_t bar = map_to_rank(&sm.full[s], 0);
-#pragma unroll
-            for (int j = 0; j < BM / 64; ++j)
-              tma_load_2d_pair(sm.a(s) + j * (64 * BK * 2), &tmap_g, bar, block_row(mt) + j * 64, kb * BK);
-#pragma unroll
-            for (int j = 0; j < BN / 128; ++j)
-              tma_load_2d_pair(sm.b(s) + j * (64 * BK * 2), &tmap_h, bar,
-                               nt * BN + static_cast<int>(rank) * (BN / 2) + j * 64, kb * BK);
-            continue;
-          }
-          mbar_arrive_expect_tx(&sm.full[s], STAGE_BYTES);
+          if (rank == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * PAIR_STAGE_BYTES);
+          const uint32_t bar = map_to_rank(&sm.full[s], 0);
 #pragma unroll
           for (int j = 0; j < BM / 64; ++j)
-            tma_load_2d(sm.a(s) + j * (64 * BK * 2), &tmap_g, &sm.full[s], mt * BM + j * 64, kb * BK);
+            tma_load_2d_pair(sm.a(s) + j * (64 * BK * 2), &tmap_g, bar, block_row(mt) + j * 64, kb * BK);
 #pragma unroll
-          for (int j = 0; j < BN / 64; ++j)
-            tma_load_2d(sm.b(s) + j * (64 * BK * 2), &tmap_h, &sm.full[s], nt * BN + j * 64, kb * BK);
+          for (int j = 0; j < BN / 128; ++j)
+            tma_load_2d_pair(sm.b(s) + j * (64 * BK * 2), &tmap_h, bar,
+                             nt * BN + static_cast<int>(rank) * (BN / 2) + j * 64, kb * BK);
         }
       }
       // the other CTA's commits land here: none may be on its way when this one leaves
-      if (PAIR && ok)
+      if (ok)
         for (uint32_t j = it > kStages ? it - kStages : 0; j < it; ++j)
           mbar_wait(&sm.empty[j % kStages], (j / kStages) & 1, sm.abort_flag);
       if (!ok) producer_drain(sm, it);
@@ -895,7 +884,7 @@ ce_dw_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
   } else if (warp == 1) {
     if (rank == 0) {
     // whole-warp issue loop, one elected lane issues (see ce_logits_kernel)
-    constexpr uint32_t idesc = make_idesc_bf16(PAIR ? 2 * BM : BM, BN, 1, 1);  // A and B are MN-major
+    constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, 1, 1);  // A and B are MN-major
     constexpr uint32_t dhi = desc_hi_sw128(1024);
     uint32_t it = 0, tile = 0;
     bool ok = true;
@@ -921,12 +910,12 @@ ce_dw_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
         if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
-            umma<PAIR>(d_tmem, a_lo + k * 128, dhi, b_lo + k * 128, dhi, idesc, (kb | k) != 0 ? 1u : 0u);
-          commit<PAIR>(&sm.empty[s]);
+            umma<true>(d_tmem, a_lo + k * 128, dhi, b_lo + k * 128, dhi, idesc, (kb | k) != 0 ? 1u : 0u);
+          commit<true>(&sm.empty[s]);
         }
         __syncwarp();
       }
-      if (ok && elect_one()) commit<PAIR>(&sm.tfull[as]);
+      if (ok && elect_one()) commit<true>(&sm.tfull[as]);
       __syncwarp();
     }
     }
@@ -970,10 +959,10 @@ ce_dw_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__
       }
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) release_acc<PAIR>(&sm.tempty[as]);
+      if (lane == 0) release_acc<true>(&sm.tempty[as]);
     }
   }
-  cta_teardown(sm, warp, tmem_base, PAIR);
+  cta_teardown(sm, warp, tmem_base, true);
 }
 
 // -----------------------------------------------------------------------------------------
@@ -1037,7 +1026,7 @@ static int configure_kernels() {
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES_Q));
   B200TP_CUDA_OK(cudaFuncSetAttribute(ce_dh_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   B200TP_CUDA_OK(cudaFuncSetAttribute(ce_dh_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES_Q));
-  B200TP_CUDA_OK(cudaFuncSetAttribute(ce_dw_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  B200TP_CUDA_OK(cudaFuncSetAttribute(ce_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   B200TP_CUDA_OK(cudaFuncSetAttribute(ce_logits_kernel<MODE_FWD, false, true>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   B200TP_CUDA_OK(cudaFuncSetAttribute(ce_logits_kernel<MODE_BWD_G, false, true>,
@@ -1311,7 +1300,7 @@ int ce_tc_launch_dw(const void* g, int ldg, int64_t v_rows, int64_t n, const voi
   p.num_nt = static_cast<int>(ceil_div(d, BN));
   p.out = reinterpret_cast<__nv_bfloat16*>(d_weight_block);
   p.status = status;
-  return launch_units(ce_dw_kernel<true>, THREADS, true, static_cast<long long>(p.num_mt) * p.num_nt, stream, tmap_g, tmap_h, p);
+  return launch_units(ce_dw_kernel, THREADS, true, static_cast<long long>(p.num_mt) * p.num_nt, stream, tmap_g, tmap_h, p);
 }
 
 }  // namespace b200tp
