@@ -80,10 +80,12 @@ typedef struct b200tp_ce_args {
   int32_t qparam_dtype;
   int64_t ignore_index;
   int32_t impl;       /* B200TP_IMPL_* */
-  int32_t reserved;   /* low 16 bits: 0, or an upper bound on the vocab rows per tensor-core backward chunk in units
-                       * of 256 (default: 16384 rows, fewer when N is so large that an (N, chunk) bf16 matrix would exceed
-                       * 512 MiB): the backward's scratch is that matrix, so
-                       * a smaller bound trades launches for memory.  4-bit heads on the tensor-core path:
+  int32_t reserved;   /* low 16 bits: 0, or an upper bound on the vocab rows per tensor-core chunk in units of 256.  The
+                       * scratch is the (N, chunk) matrix of g, so a smaller bound trades launches for memory.
+                       * Default, bf16: 16384 rows, fewer where that matrix would exceed 512 MiB; the forward that
+                       * also forms the gradient takes more where it stays within 256 MiB (a 4-bit head: up to 32768
+                       * where g and the dequantised chunk stay within 384 MiB together).  fp32: 2048 to 16384 rows,
+                       * what 128 MiB of planes hold.  4-bit heads on the tensor-core path:
                        * 0x10000 expands the head inside the kernels whatever N is, 0x20000 always dequantises chunk
                        * by chunk into the workspace (default: the forward expands inside the kernel for N <= 2048,
                        * where that is the cheaper form and needs no weight scratch, and is chunked beyond; the
@@ -92,11 +94,12 @@ typedef struct b200tp_ce_args {
                        * from 2^28 multiplications a contraction; impl = auto, D % 8 == 0) */
 } b200tp_ce_args;
 
-/* Forward: per-row log-sum-exp pieces and target logit over this call's vocab rows.  A 4-bit head is
- * expanded either inside the tensor-core kernels, tile by tile in shared memory (it then never exists as a
- * bf16 matrix in global memory and needs no scratch beyond the partial triples; w_q 16-byte aligned), or
- * chunk by chunk into the workspace ahead of the dense kernels; both give the same bits
- * (w = fma(scale, code, bias) in fp32, rounded once to bf16).  See `reserved` for the choice.
+/* Forward: per-row log-sum-exp pieces and target logit over this call's vocab rows.  A 4-bit head
+ * (w = fma(scale, code, bias) in fp32, rounded once to bf16) is expanded either inside the tensor-core kernels (it then
+ * never exists as a bf16 matrix in global memory and needs no scratch beyond the partial triples; w_q 16-byte
+ * aligned), or chunk by chunk into the workspace ahead of the dense kernels.  The default in-kernel form expands into
+ * tensor memory and sums a row in another order than the dense kernels; the forms that 0x10000 and 0x20000 of
+ * `reserved` select give the same bits as each other.
  *   row_max, row_sumexp : (N,) f32, max logit and sum exp(logit - max)   [always written]
  *   tgt_logit           : (N,) f32, logit of the target if it lies in this shard, else 0
  *   lse, nll            : (N,) f32, may be NULL (vocab-sharded callers combine first);

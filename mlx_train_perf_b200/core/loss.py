@@ -119,7 +119,8 @@ def resolve_impl(*, head: HeadRef, dtype: torch.dtype, n: int, d: int | None = N
         return Resolution(impl, f"explicit impl={impl!r}")
     if tc_ok:
         return Resolution("tc", "bf16 operands: tcgen05 kernels")
-    return Resolution("simt", f"{dtype} operands: fp32 sums, no bf16 rounding of an operand")
+    return Resolution("simt", f"{dtype} operands at fp32 precision: CUDA cores, or three bf16 planes each on the tensor "
+                              "cores for fp32, a frozen dense head and 2^28 multiplications or more")
 
 
 def _validate_inputs(hidden: torch.Tensor, head: HeadRef, targets: torch.Tensor, *,

@@ -1413,7 +1413,7 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q64, const __grid_cons
   const int nqb = (p.S + 63) / 64;   // 64-row query blocks
   const int ilo = k0 / 64;           // first query block that can see a key of this block
 
-  if (packed) griddep_wait();   // thread 0 reads the segment table below
+  if (packed) griddep_wait();   // warp 2 reads the segment table below
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int s = 0; s < DKV_RING; ++s) {

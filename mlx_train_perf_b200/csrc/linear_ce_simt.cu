@@ -1,8 +1,8 @@
 // CUDA-core (SIMT) linear cross-entropy path and the small kernels both paths share.
 //
-// The SIMT path serves fp32 heads (exact fp32 FMA accumulation, which the tensor cores do
-// not offer) and shapes the tcgen05 path refuses (D not a multiple of 8).  It streams the
-// vocabulary in chunks through an (N, chunk) fp32 scratch tile -- the structure of the
+// The SIMT path serves what the tensor cores do not: small fp32 losses, fp32 values that have no
+// bf16 planes (linear_ce_split.cu), 4-bit heads under fp32 hidden states, a hidden size that is not a
+// multiple of 8, and any call that asks for it (impl = simt).  It streams the vocabulary in chunks through an (N, chunk) fp32 scratch tile -- the structure of the
 // reference's pure-array implementation, core/chunked.py:35-90 -- and so never holds (N, V).
 //
 // Shared kernels: `combine_kernel` merges per-split (max, sum-exp, target) triples into

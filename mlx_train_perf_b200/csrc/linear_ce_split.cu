@@ -541,7 +541,13 @@ split_finish_kernel(const float* __restrict__ acc, int shares, const float* __re
 
 // CTA pairs over 256 rows, as in linear_ce_tc.cu, where an odd number of row blocks does not leave much of the last
 // pair empty (2048 x 1024 x 32768, single CTAs against pairs and whole-sector stores of g: logits 176 / 124 us a chunk,
-// d_hidden 138 / 119; the tensor pipe was 46 and 57 % active).
+// d_hidden 138 / 119; the tensor pipe was 46 and 57 % active).  Forward / whole step in us, single CTAs, pairs, V = 32768:
+//   D = 512:   200 rows 117 / 281, 115 / 274;  1024 rows 244 / 596, 211 / 563;  1100 rows (9 blocks) 246 / 621, 248 / 606
+//   D = 1024:  200 rows 186 / 397, 176 / 375;  640 rows (5) 330 / 705, 291 / 666;  1100 rows 435 / 1020, 426 / 1147;
+//              1300 rows (11) 531 / 1340, 509 / 1180;  2048 rows 756 / 1842, 631 / 1612
+//   D = 2048:  200 rows 471 / 859, 408 / 774;  1024 rows 852 / 2003, 721 / 1798;  1100 rows 882 / 2112, 990 / 2092
+//   D = 4096:  300 rows (3) 1311 / 2144, 1090 / 1989;  500 rows 1327 / 2339, 1101 / 2025
+// Even counts gain throughout; of the odd ones 9 is about even and those below, left to single CTAs, would gain too.
 bool split_pair(int64_t n) {
   const int64_t blocks = ceil_div(n, BM);
   return blocks % 2 == 0 || blocks >= 9;

@@ -24,8 +24,8 @@
 // PAIR instantiations (dense heads): a cluster of two CTAs works on 256 rows.  Each holds its 128 rows of A, half of
 // the weight tile and its rows' accumulators; CTA 0 issues one `cta_group::2` MMA for both, whose commits arrive in
 // both.  Both CTAs' copies complete on CTA 0's full barriers; accumulators are handed back to it across the cluster.
-// Training step of 8192 x 4096 x 151936: 18.2 -> 17.0 ms, 1000 rows 2.30 -> 2.10 ms, a trained head of 4096 x 1024 x
-// 151936 4.94 -> 4.72 ms.
+// Training step of 8192 x 4096 x 151936: 18.2 -> 16.6 ms, 1000 rows 2.30 -> 2.05 ms, a trained head of 4096 x 1024 x
+// 151936 4.94 -> 4.62 ms.
 //
 // 4-bit affine group-64 heads (QUANT instantiations of ce_logits_kernel and ce_dh_kernel): the
 // weight operand is never materialised in global memory.  The TMA producer copies the packed codes
@@ -1047,6 +1047,11 @@ static int configure_kernels() {
 //   1978 / 4386, 1769 / 4134;  8192 rows 7624 / 17976, 7234 / 16916
 //   D = 1024, V = 50000:   200 rows 53 / 110, 59 / 125;  400 rows 60 / 129, 66 / 139;  2100 rows (17) 156 / 377, 153 / 368;
 //   8192 rows 535 / 1530, 509 / 1378
+// That head (102 MB) was in the L2.  Forward / whole step from a cold L2, V = 50000, where the line at D = 2048 leaves
+// something to pairs below it:
+//   D = 1024:  200 rows 46 / 101, 42 / 97;  1000 rows 87 / 210, 77 / 187;  1400 rows (11) 111 / 273, 108 / 265
+//   D = 1536:  200 rows 64 / 144, 60 / 134;  1000 rows 140 / 337, 126 / 300;  1400 rows 161 / 394, 156 / 366
+//   D = 2048:  200 rows 79 / 163, 71 / 150;  1000 rows 161 / 370, 140 / 331;  1400 rows 222 / 486, 208 / 478
 static bool use_pair(int64_t n, int d) {
   const int64_t blocks = ceil_div(n, BM);
   return blocks >= 16 || (blocks % 2 == 0 && d >= 2048);
