@@ -6,7 +6,8 @@
 Headline (`metric` / `value`): fused linear-cross-entropy forward+backward tokens/s at
 N=8192, D=4096, V=151936, bf16 (3 % of rows ignore_index), d_hidden with fp32 accumulation.
 A "step" is one forward + one backward over that batch with the inputs already resident in
-HBM.  The inputs are the seeded tensors of `configs.ce_dense(..., seed=0)`, drawn on the CPU:
+HBM: the plain forward and the backward that computes the logits again, three contractions, which is what
+a vocabulary shard runs at every N (the public operator of a frozen head on one GPU makes two: `e2e`).  The inputs are the seeded tensors of `configs.ce_dense(..., seed=0)`, drawn on the CPU:
 the same tensors the full-size parity test feeds the kernels.  At N GPUs the lm_head is
 vocab-sharded V/N per rank (strong scaling: the problem is fixed): forward partial triples are
 all-gathered and the fp32 partial d_hidden is all-reduced across ranks, both inside the timed
