@@ -150,9 +150,9 @@ bool split_pays(const b200tp_ce_args* a) { return a->n * a->v_local >= kSplitWor
 // recorded.  3 is the default for fp32 with a dense head: 2048 x 1024 x 32768 forward + backward 18.5 -> 1.65 ms, with
 // a third of the CUDA-core path's distance to float64.  The CUDA cores keep the contraction of a trained head's
 // gradient (its g comes from the planes like the forward's lse), D % 8 != 0 (TMA strides), a 4-bit head under fp32
-// hidden states, and calls whose contraction is under 2^28 multiplications: there the CUDA cores need no longer than the split's extra launches take (forward /
-// forward + backward, CUDA cores against split: 128 x 512 x 2000 65 / 259 against 90 / 282 us, 32 x 1024 x 32000
-// 1001 / 4151 against 173 / 430 us).
+// hidden states, and calls whose contraction is under 2^28 multiplications: there the CUDA cores need no longer than
+// the split's extra launches take (forward / forward + backward, CUDA cores against split: 128 x 512 x 2000 65 / 259
+// against 90 / 282 us, 32 x 1024 x 32000 1001 / 4151 against 173 / 430 us).
 int pick_impl(const b200tp_ce_args* a) {
   const bool tc_ok = a->dtype == B200TP_BF16 && a->d % 8 == 0;
   if (a->impl == B200TP_IMPL_SIMT) return 2;
